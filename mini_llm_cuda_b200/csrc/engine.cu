@@ -2,29 +2,17 @@
 // state, step scratch), the launch chain of one decode step, CUDA-graph replay, and the C ABI
 // declared in include/mlb.h.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
-#include <cstdlib>
-#include <chrono>
-#include <cstring>
-#include <string>
-#include <type_traits>
-#include <mutex>
-#include <vector>
 
-#include "../../include/mlb.h"
-#include "errors.h"
-#include "kernels.cuh"
-#include "gemm_tc.cuh"
-#include "tc_host.h"
-#include "ring.cuh"
-#include "grid_params.h"
+#include "session.h"
+#include "cols_host.h"
+#include "gemm_cols.cuh"
 #include "grid_host.h"
-#include "lean_params.h"
 #include "lean_host.h"
 #include "model_file.h"
-#include "sgemv.cuh"
 
 namespace mlb {
 
@@ -43,30 +31,9 @@ int fail(int code, const char* fmt, ...) {
     return code;
 }
 
-#define CU(expr)                                                                              \
-    do {                                                                                      \
-        cudaError_t e__ = (expr);                                                             \
-        if (e__ != cudaSuccess)                                                               \
-            return fail(MLB_E_CUDA, "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e__), __FILE__, __LINE__); \
-    } while (0)
-
-static size_t elt_size(int dt) { return dt == MLB_DT_F32 ? 4 : (dt == MLB_DT_BF16 ? 2 : 1); }
-static int ple_dtype(int wdt) { return wdt == MLB_DT_FP8_E4M3 ? MLB_DT_BF16 : wdt; }
-
 // --------------------------------------------------------------------------------------
 // KV page allocator (host only)
 // --------------------------------------------------------------------------------------
-}  // namespace mlb
-
-struct mlb_kv_alloc {
-    std::vector<int> free_list;                 // stack; back() is handed out next
-    std::vector<std::vector<int>> seq_pages;
-    int max_pages_per_seq = 0;
-    int num_pages = 0;
-};
-
-namespace mlb {
-
 static int kv_ensure(mlb_kv_alloc* a, int seq, int n_positions, int block) {
     if (!a || seq < 0 || seq >= (int)a->seq_pages.size() || block <= 0 || n_positions < 0)
         return fail(MLB_E_INVALID, "kv allocator: bad argument");
@@ -86,32 +53,6 @@ static int kv_ensure(mlb_kv_alloc* a, int seq, int n_positions, int block) {
 // --------------------------------------------------------------------------------------
 // model
 // --------------------------------------------------------------------------------------
-struct DevLayer {
-    int type = MLB_LAYER_ATTENTION;
-    float *g1 = nullptr, *g2 = nullptr, *gq = nullptr, *gk = nullptr;
-    void* Wqkv = nullptr; float* Sqkv = nullptr; int n_qkv = 0;
-    int nq = 0, nk = 0, nv = 0, ng = 0;
-    void* Wo = nullptr; float* So = nullptr; int o_in = 0;
-    void *W1a = nullptr, *W1b = nullptr, *W2 = nullptr;
-    float *S1a = nullptr, *S1b = nullptr, *S2 = nullptr;
-    void *pleT = nullptr, *pleP = nullptr;
-};
-
-}  // namespace mlb
-
-struct mlb_model {
-    mlb_config cfg;
-    int device = 0;
-    void* E = nullptr; float* Es = nullptr; float* g_final = nullptr; float* rope = nullptr;
-    std::vector<mlb::DevLayer> layers;      // execution order
-    uint64_t weight_bytes = 0;
-    std::vector<void*> allocs;
-    // FP8 models: the same weights as bf16 (code * row scale, rounded), made on first use for the
-    // tensor-core steps that consume a prompt as columns; shares gains, RoPE table and PLE tensors
-};
-
-namespace mlb {
-
 struct Uploader {
     mlb_model* m;
     const std::vector<unsigned char>* file;
@@ -348,113 +289,6 @@ extern "C" void mlb_model_free(mlb_model* m) { free_model(m); }
 // session
 // --------------------------------------------------------------------------------------
 namespace mlb {
-enum ChainKind { CHAIN_PREFILL = 0, CHAIN_GREEDY = 1, CHAIN_TOPK = 2 };
-
-struct LaunchRec {
-    const char* name;
-    uint64_t bytes, flops;
-    cudaEvent_t e0, e1;
-};
-struct Recorder {
-    cudaStream_t st;
-    std::vector<LaunchRec> recs;
-    int begin(const char* name, uint64_t bytes, uint64_t flops) {
-        LaunchRec r{name, bytes, flops, nullptr, nullptr};
-        CU(cudaEventCreate(&r.e0));
-        CU(cudaEventCreate(&r.e1));
-        CU(cudaEventRecord(r.e0, st));
-        recs.push_back(r);
-        return MLB_OK;
-    }
-    int end() {
-        CU(cudaEventRecord(recs.back().e1, st));
-        return MLB_OK;
-    }
-};
-}  // namespace mlb
-
-struct TcShape { int nb, split, stages, group; size_t smem; uint32_t tmem_cols; };
-
-struct mlb_session {
-    mlb_model* m = nullptr;
-    int B = 0, max_ctx = 0, max_pages = 0, kv_pages = 0;
-    cudaStream_t stream = nullptr;
-    int *pos = nullptr, *tok = nullptr, *limit_prefill = nullptr, *limit_decode = nullptr;
-    int *prompt = nullptr, *out_ring = nullptr, *out_idx = nullptr, *page_table = nullptr;
-    unsigned long long* seeds = nullptr;
-    float *x = nullptr, *qbuf = nullptr, *gbuf = nullptr, *abuf = nullptr, *hbuf = nullptr, *raw = nullptr;
-    float *logits = nullptr, *part = nullptr, *part_val = nullptr, *probe = nullptr;
-    int *part_idx = nullptr, *attn_ticket = nullptr, *lm_ticket = nullptr;
-    std::vector<void*> kpool, vpool;
-    std::vector<float*> state;
-    std::vector<void*> allocs;
-    // host mirrors
-    std::vector<int> h_pos;
-    std::vector<char> h_stopped;            // the sequence drew the stop token: it takes no further step
-    int stop_token = -1;
-    std::vector<int> h_table;
-    bool table_dirty = true;
-    bool have_logits = false;
-    mlb_kv_alloc alloc;
-    int attn_min_pps = 11;                    // KV pages a flash-decode split must hold before a sequence uses it
-    int splits = 1, lm_rows = 32, lm_parts = 1, raw_stride = 0, max_q = 0;
-    // graphs
-    cudaGraphExec_t graphs[3] = {nullptr, nullptr, nullptr};
-    int g_topk = -1; float g_temp = 0.f;
-    int cur_topk = 50; float cur_temp = 1.f;
-    int launches_per_step[3] = {0, 0, 0};
-    // one-token call as ONE graph: upload of the pending ids, the step, read-back of ids and error word
-    cudaGraphExec_t tgraphs[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};     // [kind][with input ids]
-    int tg_topk[2] = {-1, -1}; float tg_temp[2] = {0.f, 0.f};
-    int* pinned_out = nullptr;
-    int ctl_host_io = 0;                    // while the one-token graph is captured: 1 = ids and error word to the host, 2 = + ids from the host
-    int tok_arg = -1;                       // single-kernel step: the pending id travels with the launch (>= 0), else it is read from `tok`
-    float4* flush_buf = nullptr; size_t flush_n = 0;
-    int* pinned_tok = nullptr;
-    bool use_pdl = true;
-    bool use_sgemv = false;                 // TMA-streamed GEMV for very small batches and large matrices
-    bool force_sgemv = false;               // MLB_GEMV=stream: also for small matrices (tests)
-    int sg_stage_kb = 48, sg_max_stages = 8; // ring geometry of the streamed GEMV (MLB_SG_STAGE_KB, MLB_SG_STAGES)
-    int sm_count = 148;
-    mlb::StepLayer* step_layers = nullptr;   // device table of per-layer pointers (single-kernel step)
-    int* dev_err = nullptr;                 // set by a kernel whose bounded wait ran out
-    // whole-GPU single-kernel step (batch 1)
-    bool use_grid = false;
-    int grid_ctas = 0;
-    size_t grid_smem = 0;
-    mlb::GridParams grid;
-    // the same step with compile-time shapes, for the models it is built for
-    bool use_lean = false;
-    int lean_idx = -1;
-    size_t lean_smem = 0;
-    mlb::LeanParams lean;
-    // tensor-core projections (bf16 weights, batch >= 16)
-    bool use_tc = false;
-    int tc_nb = 0, tc_stages = 0, tc_stages_swiglu = 0;
-    int tc_max_split = 8;                     // largest cluster that may split a GEMM's k-blocks
-    bool tc_split_forced = false;             // MLB_TC_SPLIT given: take it as the limit without the k-blocks-per-CTA rule
-    int tc_cluster_cap[4] = {0, 0, 0, 0};     // clusters of 1, 2, 4, 8 GEMM CTAs that can be resident at once
-    unsigned long long* tc_trace = nullptr;   // MLB_TC_TRACE=1: [64][8] timer stamps of the step's GEMM launches
-    int tc_trace_n = 0;
-    TcShape tc_shape_down{};                  // launch shape of the down projection (its per-layer embedding map has this batch tile)
-    mlb::bf16_t *xn16 = nullptr, *a16 = nullptr, *h16 = nullptr;
-    float* rawq = nullptr;
-    struct alignas(64) TcLayerMaps { CUtensorMap qkv, o, w1a, w1b, w2, pleP, pleT; };   // pleP / pleT: [d][ple] projection, gathered [B][ple] rows
-    float* tc_ssq = nullptr;                 // [B][ceil(d / 128)] partial sums of squares of the residual stream
-    mlb::bf16_t* tple16 = nullptr;           // [layers][B][ple] per-layer embedding rows of the step's tokens
-    std::vector<TcLayerMaps> tc_maps;
-    // activation operand maps per batch tile 16, 32, 64, 128, 256 (index log2(Nb/16))
-    struct alignas(64) TcGlobalMaps { CUtensorMap E, xn[5], a_attn[5], a_dn[5], h[5]; } tc_g;
-    int* pinned_err = nullptr;
-    // prompt columns: a second set of step buffers, `B` columns wide, that shares this session's KV
-    // pool, delta-net state and stream; a column is one prompt token of one sequence
-    mlb_session* cols = nullptr;            // owned by the session it serves
-    mlb_session* parent = nullptr;          // set in the column set
-    bool cols_tried = false;
-    int* seq_of = nullptr;                  // [B] in the column set: column -> sequence of the parent
-};
-
-namespace mlb {
 
 static int sess_alloc(mlb_session* s, void** p, size_t bytes, bool zero) {
     cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
@@ -485,7 +319,9 @@ static void free_session(mlb_session* s) {
     if (!s) return;
     cudaSetDevice(s->m->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->cols) free_session(s->cols);
+    for (auto* cs : s->cols) free_session(cs);
+    for (auto& e : s->plan_free) if (e) cudaEventDestroy(e);
+    if (s->plan_host) cudaFreeHost(s->plan_host);
     for (auto& g : s->graphs) if (g) cudaGraphExecDestroy(g);
     for (auto& g : s->tgraphs) if (g) cudaGraphExecDestroy(g);
     for (void* p : s->allocs) cudaFree(p);
@@ -496,8 +332,6 @@ static void free_session(mlb_session* s) {
     delete s;
 }
 
-// Host mirror of seq_active for the decode chains.
-static bool seq_live(const mlb_session* s, int b) { return s->h_pos[b] < s->max_ctx && !s->h_stopped[b]; }
 // After a decode call returned `n` ids of sequence b (ring order): advance the mirror, stop at the stop token,
 // blank what lies behind it.
 static void note_outputs(mlb_session* s, int b, int32_t* out, int n) {
@@ -513,589 +347,102 @@ static void note_outputs(mlb_session* s, int b, int32_t* out, int n) {
     s->h_pos[b] += room;
 }
 
-static StepCtl make_ctl(mlb_session* s, int kind) {
-    StepCtl c;
-    c.B = s->B;
-    c.vocab = s->m->cfg.vocab;
-    c.pos = s->pos;
-    c.tok = s->tok;
-    c.limit = kind == CHAIN_PREFILL ? s->limit_prefill : s->limit_decode;
-    c.stop_token = kind == CHAIN_PREFILL ? -1 : s->stop_token;
-    c.prompt = kind == CHAIN_PREFILL ? s->prompt : nullptr;
-    c.prompt_stride = s->max_ctx;
-    c.out_ring = s->out_ring;
-    c.out_idx = s->out_idx;
-    c.out_cap = s->parent ? 0 : s->max_ctx;     // a column set has no output ring
-    c.tok_src = s->ctl_host_io == 2 ? s->pinned_tok : nullptr;
-    c.host_out = s->ctl_host_io ? s->pinned_out : nullptr;
-    c.host_err = s->ctl_host_io ? s->pinned_err : nullptr;
-    c.dev_err = s->dev_err;
-    return c;
-}
-
-static int pick_bt(int B, size_t per_seq_floats) {
-    int bt = B >= 8 ? 8 : (B >= 4 ? 4 : (B >= 2 ? 2 : 1));
-    while (bt > 1 && (size_t)bt * per_seq_floats * 4 > 200 * 1024) bt >>= 1;
-    return bt;
-}
-
-// Launch with the programmatic-dependent-launch attribute: the kernel may start while its
-// predecessor in the stream still runs and orders itself with griddepcontrol.wait.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_chain(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                Args... args) {
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof cfg);
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
-
-// launch_chain for a grid whose z extent is one thread-block cluster (cluster_z CTAs share an output tile).
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_cluster(bool pdl, int cluster_z, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                  Args... args) {
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof cfg);
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (pdl) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
-    if (cluster_z > 1) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = 1;
-        attr[n].val.clusterDim.y = 1;
-        attr[n].val.clusterDim.z = (unsigned)cluster_z;
-        ++n;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
-
-// Shape of one tensor-core GEMM launch: batch tile (UMMA N), how many CTAs of a cluster split the k-blocks of
-// an output tile, and the ring. Measured on B200: a tcgen05.mma of M = 128 costs about 0.1 us whatever its N
-// (16..128), so a CTA's k-loop takes 0.4 us per 64-wide k-block (0.8 with two weight tiles) whatever the ring
-// depth, and is the time of the kernel unless the k-blocks are spread over CTAs. Exchanging partial
-// accumulators through distributed shared memory costs 2-3 us per launch with clusters of 4 and 8, more than
-// it saves at cfg1's sizes (8-23 k-blocks per tile); pairs pay off at small batches (cfg1 step at 32 sequences:
-// 452 -> 424 us) and are neutral at 256. Larger clusters are taken only where a CTA keeps 8 k-blocks or more
-// (cfg4: 32-90 k-blocks per tile and few tiles). MLB_TC_SPLIT sets the limit by hand. One wave of CTAs per
-// launch where possible.
-static TcShape tc_pick_shape(const mlb_session* s, int N, int nkb_all, int na, bool w8, int nacc) {
-    const int tiles_m = (N + kTcM - 1) / kTcM;
-    const int cap = std::min(256, (s->B + 15) / 16 * 16);
-    TcShape best{};
-    double best_cost = -1.0;
-    for (int nb = 16; nb <= cap && nacc * nb <= 512; nb <<= 1) {
-        for (int li = 0; li < 4; ++li) {
-            const int S = 1 << li;
-            if (S > s->tc_max_split || S > nkb_all) break;
-            // clusters of 4 and 8 only where a CTA keeps 8 k-blocks or more: their exchange costs 2-3 us
-            if (S > 2 && !s->tc_split_forced && (nkb_all + S - 1) / S < 8) break;
-            if (S > 1 && (nb % S != 0 || s->tc_cluster_cap[li] <= 0)) continue;
-            const size_t stage_bytes = (size_t)na * kTcM * 128 + (size_t)nb * 128;      // FP8 codes land inside the operand tile
-            const int kpc = (nkb_all + S - 1) / S;
-            int st = (int)std::max<size_t>(1, std::min<size_t>(std::min(kpc, 12), kTcRingBytes / stage_bytes));
-            const int g = st >= kpc ? 1 : (st >= 8 ? 4 : (st >= 4 ? 2 : 1));
-            st -= st % g;
-            const size_t body = std::max((size_t)st * stage_bytes, S > 1 ? (size_t)nacc * nb * kTcM * 4 : (size_t)0);
-            const size_t smem = 1024 + kTcHeadBytes + kTcStageBytes + body;
-            if (smem > 227 * 1024) continue;
-            const long ctas = (long)tiles_m * ((s->B + nb - 1) / nb) * S;
-            const long resident = S == 1 ? s->sm_count : (long)s->tc_cluster_cap[li] * S;
-            const long waves = (ctas + resident - 1) / resident;
-            const double t_loop = 0.4 * na * kpc;
-            const double t_red = S > 2 ? 2.5 + (double)nacc * nb * 512.0 / 65536.0 : (S > 1 ? 0.5 + (double)nacc * nb * 512.0 / 65536.0 : 0.0);
-            const double t_epi = 0.25 * ((nb / S + 15) / 16);
-            const double cost = (double)waves * (t_loop + t_red + t_epi + 0.5);
-            if (best_cost < 0 || cost < best_cost) {
-                best_cost = cost;
-                uint32_t cols = 32;
-                while (cols < (uint32_t)(nacc * nb)) cols <<= 1;
-                best = TcShape{nb, S, st, g, smem, cols};
-            }
-        }
-    }
-    return best;
-}
-static int nb_index(int nb) { return nb == 16 ? 0 : nb == 32 ? 1 : nb == 64 ? 2 : nb == 128 ? 3 : 4; }
-
-template <typename T, typename T2, typename KVT>
-struct Chain {
-    // TMA-streamed variant: one contiguous slab of rows per CTA (one head per CTA for QKV).
-    template <int MODE>
-    static int sgemv(mlb_session* s, const StepCtl& c, GemvParams p, Recorder* rec, const char* name, bool* done) {
-        *done = false;
-        // Worth it only when the matrix is large: below a few MB the per-thread-load kernel's
-        // shorter latency chain wins (measured on the 1-GPU latency configuration).
-        const size_t mat_bytes = (size_t)p.N * p.K * sizeof(T) * (MODE == GEMV_SWIGLU ? 2 : 1);
-        if (!s->force_sgemv && mat_bytes < (4u << 20)) return MLB_OK;
-        SgemvGeom g;
-        g.stage_bytes = s->sg_stage_kb * 1024;
-        if ((size_t)p.K * sizeof(T) > (size_t)g.stage_bytes || (size_t)p.Kp * sizeof(T2) > (size_t)g.stage_bytes) return MLB_OK;
-        int grid_x;
-        if (MODE == GEMV_QKV) {
-            // whole heads when the per-head norm needs them, else 32-row groups (RoPE pairs stay together)
-            g.rows_per_cta = p.qk_norm ? p.hd : 32;
-            grid_x = p.N / g.rows_per_cta;
-        } else {
-            const int n_ctas = std::max(1, std::min(s->sm_count, (p.N + 3) / 4));
-            g.rows_per_cta = (p.N + n_ctas - 1) / n_ctas;
-            grid_x = (p.N + g.rows_per_cta - 1) / g.rows_per_cta;
-        }
-        auto up4 = [](int v) { return (v + 3) / 4 * 4; };
-        int off = 0;
-        g.off_xs = off; off += up4(p.K);
-        g.off_xs2 = off; off += up4(std::max(p.Kp, 4));
-        g.off_outs = off; off += up4(std::max(p.hd, 64));
-        g.off_pacc = off; off += up4(g.rows_per_cta + 4);
-        g.off_red = off; off += 64;
-        off = (off + 31) / 32 * 32;
-        g.off_bar = off; off += 8 * 4;
-        off = (off + 31) / 32 * 32;
-        g.off_ring = off;
-        const size_t fixed = (size_t)off * 4;
-        if (fixed + 3 * (size_t)g.stage_bytes > 210 * 1024) return MLB_OK;
-        g.n_stages = (int)std::min<size_t>(s->sg_max_stages, (210 * 1024 - fixed) / g.stage_bytes);
-        g.err = s->dev_err;
-        const size_t smem = fixed + (size_t)g.n_stages * g.stage_bytes;
-        if (rec) {
-            const uint64_t wbytes = (uint64_t)p.N * p.K * sizeof(T) * (MODE == GEMV_SWIGLU ? 2 : 1) +
-                                    (uint64_t)p.N * p.Kp * sizeof(T2) + (p.wscale ? (uint64_t)p.N * 4 : 0);
-            const uint64_t abytes = (uint64_t)s->B * ((uint64_t)p.K + p.N) * 4;
-            int rc = rec->begin(name, wbytes + abytes, 2ull * p.N * (p.K + p.Kp) * s->B * (MODE == GEMV_SWIGLU ? 2 : 1));
-            if (rc) return rc;
-        }
-        cudaError_t e = launch_chain(s->use_pdl, sgemv_kernel<T, T2, KVT, MODE>, dim3(grid_x, s->B), dim3(kSgThreads), smem,
-                                     s->stream, c, p, g);
-        if (e != cudaSuccess) return fail(MLB_E_CUDA, "launch of %s (streamed) failed: %s", name, cudaGetErrorString(e));
-        *done = true;
-        if (rec) return rec->end();
-        return MLB_OK;
-    }
-
-    template <int MODE>
-    static int gemv(mlb_session* s, const StepCtl& c, GemvParams p, int R, Recorder* rec, const char* name) {
-        if (s->use_sgemv) {
-            bool done = false;
-            int rc = sgemv<MODE>(s, c, p, rec, name, &done);
-            if (rc || done) return rc;
-        }
-        p.R = R;
-        const size_t per_seq = (size_t)p.K + p.Kp + R + 1 + 8;
-        const int BT = pick_bt(s->B, per_seq);
-        if (per_seq * 4 > 200 * 1024) return fail(MLB_E_UNSUPPORTED, "projection input of %d floats does not fit shared memory", p.K);
-        const int rwf = BT == 1 ? 2 : 4;                                  // GemvShape<BT>::RW
-        const int rw = MODE == GEMV_SWIGLU ? rwf / 2 : rwf;
-        const int warps = std::max(1, std::min(8, (R + rw - 1) / rw));
-        dim3 grid((p.N + R - 1) / R, (s->B + BT - 1) / BT);
-        const size_t smem = (size_t)BT * per_seq * 4;
-        if (rec) {
-            const uint64_t wbytes = (uint64_t)p.N * p.K * sizeof(T) * (MODE == GEMV_SWIGLU ? 2 : 1) +
-                                    (uint64_t)p.N * p.Kp * sizeof(T2) + (p.wscale ? (uint64_t)p.N * 4 : 0);
-            const uint64_t abytes = (uint64_t)s->B * ((uint64_t)p.K + p.N) * 4;
-            int rc = rec->begin(name, wbytes + abytes, 2ull * p.N * (p.K + p.Kp) * s->B * (MODE == GEMV_SWIGLU ? 2 : 1));
-            if (rc) return rc;
-        }
-        cudaError_t e;
-        switch (BT) {
-            case 1: e = launch_chain(s->use_pdl, gemv_kernel<T, T2, KVT, 1, MODE>, grid, dim3(warps * 32), smem, s->stream, c, p); break;
-            case 2: e = launch_chain(s->use_pdl, gemv_kernel<T, T2, KVT, 2, MODE>, grid, dim3(warps * 32), smem, s->stream, c, p); break;
-            case 4: e = launch_chain(s->use_pdl, gemv_kernel<T, T2, KVT, 4, MODE>, grid, dim3(warps * 32), smem, s->stream, c, p); break;
-            default: e = launch_chain(s->use_pdl, gemv_kernel<T, T2, KVT, 8, MODE>, grid, dim3(warps * 32), smem, s->stream, c, p); break;
-        }
-        if (e != cudaSuccess) return fail(MLB_E_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
-        if (rec) return rec->end();
-        return MLB_OK;
-    }
-
-    template <int MODE>
-    static int configure_mode() {
-        const int big = 200 * 1024;
-        CU(cudaFuncSetAttribute(sgemv_kernel<T, T2, KVT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
-        CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 4, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 8, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        return MLB_OK;
-    }
-    static int configure() {
-        int rc;
-        if ((rc = configure_mode<GEMV_RAW>())) return rc;
-        if ((rc = configure_mode<GEMV_RESID>())) return rc;
-        if ((rc = configure_mode<GEMV_SWIGLU>())) return rc;
-        if ((rc = configure_mode<GEMV_QKV>())) return rc;
-        if ((rc = configure_mode<GEMV_LMHEAD>())) return rc;
-        return MLB_OK;
-    }
-
-    template <int HD>
-    static int attn_g(mlb_session* s, const StepCtl& c, const AttnParams& p0, int G) {
-        AttnParams p = p0;
-        p.hg = 1;
-        // few CTAs (small batch): two query heads per CTA, G/2 CTAs per kv head (cfg4 at batch 1: 1.28 -> 1.14 ms
-        // per step); with the GPU already full the extra CTAs only re-read K/V (62 -> 69 us at 64 sequences)
-        if (G >= 4 && G % 2 == 0 && s->splits * p.kv_heads * s->B < 2 * s->sm_count) { p.hg = G / 2; G = 2; }
-        dim3 grid(s->splits, p.kv_heads * p.hg, s->B);
-        cudaError_t e;
-        switch (G) {
-            case 1: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 1>, grid, dim3(128), 0, s->stream, c, p); break;
-            case 2: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 2>, grid, dim3(128), 0, s->stream, c, p); break;
-            case 4: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 4>, grid, dim3(128), 0, s->stream, c, p); break;
-            default: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 8>, grid, dim3(128), 0, s->stream, c, p); break;
-        }
-        if (e != cudaSuccess) return fail(MLB_E_CUDA, "attention launch failed: %s", cudaGetErrorString(e));
-        return MLB_OK;
-    }
-
-    // Launch shape of the embedding kernel: with per-layer embeddings and a small batch, the rows
-    // of a sequence are spread over several CTAs of 64 threads (one projection row per thread).
-    static int embed_split(int B, int d, int ple) {
-        if (ple <= 0) return 1;
-        return std::max(1, std::min((d + 63) / 64, 1024 / std::max(1, B)));
-    }
-    static dim3 embed_grid(int B, int d, int ple) { return dim3(B, embed_split(B, d, ple)); }
-    static dim3 embed_block(int B, int d, int ple) { return dim3(embed_split(B, d, ple) > 1 ? 64 : 256); }
-
-    // One decode (or prefill) step of a batch-1 session as a single cooperative kernel over all
-    // SMs (plus the sampler for top-k).
-    static int run_grid(mlb_session* s, int kind, const StepCtl& c, Recorder* rec, int* n_launches) {
-        int rc, launches = 0;
-        if (rec) {
-            uint64_t w, kv, st, rows;
-            mlb_session_step_bytes(s, &w, &kv, &st, &rows);
-            if ((rc = rec->begin(s->use_lean ? "lean_decode_step" : "grid_decode_step", w + kv + st + rows, 0))) return rc;
-        }
-        if (s->use_lean) {
-            LeanParams lp = s->lean;
-            lp.tok_arg = s->tok_arg;
-            lp.with_lm_head = kind == CHAIN_PREFILL ? 0 : 1;
-            lp.do_pick = kind == CHAIN_GREEDY ? 1 : 0;
-            CU(lean_kernel_launch(s->lean_idx, s->m->cfg.kv_dtype, s->lean_smem, s->stream, c, lp));
-        } else {
-            GridParams gp = s->grid;
-            gp.tok_arg = s->tok_arg;
-            gp.with_lm_head = kind == CHAIN_PREFILL ? 0 : 1;
-            gp.do_pick = kind == CHAIN_GREEDY ? 1 : 0;
-            CU(grid_kernel_launch(s->m->cfg.weight_dtype, s->m->cfg.kv_dtype, s->grid_ctas, s->grid_smem, s->stream, c, gp));
-        }
-        if (rec && (rc = rec->end())) return rc;
+// A chunk of prompt columns: embedding, then per layer projection, attention or recurrence, o-projection, gate/up and
+// down projection, as persistent column GEMMs with the element-wise work in their epilogues; the LM head if the columns
+// are scored.
+static int run_cols(mlb_session* s, int kind, int* n_launches) {
+    const mlb_model* m = s->m;
+    const mlb_config& cfg = m->cfg;
+    const int d = cfg.dim, F = cfg.ffn_dim, ple = cfg.ple_dim;
+    const bool w8 = cfg.weight_dtype == MLB_DT_FP8_E4M3;
+    const StepCtl c = make_ctl(s, kind);
+    int launches = 0, rc;
+    EmbedColsParams e;
+    e.E = m->E; e.escale = m->Es; e.d = d; e.layers = s->step_layers; e.n_layers = cfg.layers; e.ple = ple; e.gain = m->layers[0].g1;
+    const int parts = (d + 127) / 128 * 4;
+    e.x = s->x; e.xg16 = s->xn16; e.ssq = s->tc_ssq; e.parts = parts; e.tple16 = s->tple16; e.T = s->B;
+    CU(embed_cols_launch(w8, false, s->stream, c, e));
+    ++launches;
+    const QkvPostParams q0{};
+    auto gemm = [&](int mode, const ColsGemm& g, const CUtensorMap& X, const CUtensorMap& W, const CUtensorMap& W2, int N, int K, float* y, bf16_t* h16,
+                    bool normed, const float* next_gain, const mlb_session::TcLayerMaps* ext, const QkvPostParams* q, const float* s1, const float* s2) -> int {
+        GemmColsParams p;
+        p.N = N; p.K = K; p.BN = g.bn; p.stages = g.stages; p.nkb_x = ext ? (ple + kTcKB - 1) / kTcKB : 0;
+        p.split = g.split; p.mains = g.mains; p.exts = g.exts; p.nbuf = g.nbuf; p.tmem_cols = g.tmem_cols; p.early_w = 1;
+        p.y = y; p.h16 = h16; p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = parts; p.eps = cfg.rms_eps;
+        p.xg16 = s->xn16; p.gain_next = next_gain; p.ssq_out = s->tc_ssq;
+        p.s1 = s1; p.s2 = s2; p.err = s->dev_err;
+        CU(gemm_cols_launch(mode, cfg.kv_dtype, s->use_pdl, g.ctas, s->stream, X, W, W2, ext ? ext->pleT : X, ext ? ext->pleP : W, p, c, q ? *q : q0));
         ++launches;
-        if (kind == CHAIN_TOPK) {
-            SampleParams sp;
-            sp.logits = s->logits; sp.V = s->m->cfg.vocab; sp.top_k = s->cur_topk; sp.temperature = s->cur_temp; sp.seeds = s->seeds;
-            if (rec && (rc = rec->begin("sample_topk_philox", (uint64_t)s->B * s->m->cfg.vocab * 4 * 5, 0))) return rc;
-            CU(launch_chain(false, sample_topk_kernel, dim3(s->B), dim3(256), 0, s->stream, c, sp));
-            if (rec && (rc = rec->end())) return rc;
-            ++launches;
-        }
-        if (n_launches) *n_launches = launches;
         return MLB_OK;
-    }
-
-    // One tensor-core projection. `normed`: the activation operand is bf16(x * gain) and the accumulator
-    // columns are scaled by 1 / rms(x) from the partial sums its producer left. `next_gain` (RESID): also
-    // write the operand and the partial sums for the next norm. `ext`: the per-layer embedding pair whose
-    // k-blocks follow the main operands' (RESID of the down projection).
-    template <int MODE>
-    static int gemm_tc(mlb_session* s, const StepCtl& c, const CUtensorMap& A, const CUtensorMap& A2, const CUtensorMap* Bmaps, int N, int K,
-                       float* y, bf16_t* h16, bool normed, const float* next_gain, const mlb_session::TcLayerMaps* ext,
-                       const QkvPostParams* q, const float* sA, const float* sA2, Recorder* rec, const char* name) {
-        GemmTcParams p;
-        const int ple = s->m->cfg.ple_dim;
-        const int na = MODE == TC_SWIGLU ? 2 : 1;
-        p.nkb_x = ext ? (ple + kTcKB - 1) / kTcKB : 0;
-        constexpr bool w8 = sizeof(T) == 1;
-        const int nacc = (MODE == TC_SWIGLU || (w8 && MODE == TC_RESID)) ? 2 : 1;
-        const TcShape sh = ext ? s->tc_shape_down : tc_pick_shape(s, N, (K + kTcKB - 1) / kTcKB, na, w8, nacc);
-        if (sh.nb == 0) return fail(MLB_E_UNSUPPORTED, "%s: no launch shape fits", name);
-        const int nb = sh.nb;
-        p.N = N; p.K = K; p.B = s->B; p.Nb = nb;
-        p.stages = sh.stages; p.group = sh.group; p.tmem_cols = sh.tmem_cols;
-        p.y = y; p.resid = MODE == TC_RESID ? y : nullptr; p.h16 = h16; p.err = s->dev_err;
-        p.sA = sA; p.sA2 = sA2;
-        p.trace = s->tc_trace ? s->tc_trace + 8 * (size_t)(s->tc_trace_n++ % 64) : nullptr;
-        p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = (s->m->cfg.dim + kTcM - 1) / kTcM; p.eps = s->m->cfg.rms_eps;
-        p.xg16 = next_gain ? s->xn16 : nullptr; p.gain_next = next_gain; p.ssq_out = next_gain ? s->tc_ssq : nullptr;
-        const size_t smem = sh.smem;
-        dim3 grid((N + kTcM - 1) / kTcM, (s->B + nb - 1) / nb, sh.split);
-        int rc;
-        if (rec && (rc = rec->begin(name, ((uint64_t)N * K * sizeof(T) + (uint64_t)N * (ext ? ple : 0) * 2) * na + (uint64_t)s->B * K * 2 + (uint64_t)s->B * N * 4,
-                                    2ull * N * (K + (ext ? ple : 0)) * s->B * na)))
+    };
+    for (int i = 0; i < cfg.layers; ++i) {
+        const DevLayer& L = m->layers[i];
+        const mlb_session::TcLayerMaps& M = s->tc_maps[i];
+        const bool attn = L.type == MLB_LAYER_ATTENTION;
+        if (attn) {
+            QkvPostParams q;
+            q.nq = L.nq; q.nk = L.nk; q.nv = L.nv; q.ng = L.ng; q.hd = cfg.head_dim;
+            q.kv_heads = cfg.kv_heads; q.qk_norm = cfg.qk_norm; q.eps = cfg.rms_eps; q.gq = L.gq; q.gk = L.gk; q.rope = m->rope;
+            q.kpool = s->kpool[i]; q.vpool = s->vpool[i]; q.page_table = s->page_table; q.pt_stride = s->max_pages;
+            q.qbuf = s->qbuf; q.gbuf = s->gbuf;
+            if ((rc = gemm(TC_QKV, s->cg_qkv, s->tc_g.xn[0], M.qkv, M.qkv, L.n_qkv, d, nullptr, nullptr, true, nullptr, nullptr, &q, L.Sqkv, nullptr))) return rc;
+            if (cfg.kv_dtype == MLB_DT_BF16) {
+                AttnColsParams ac;
+                ac.kpool = static_cast<const bf16_t*>(s->kpool[i]); ac.vpool = static_cast<const bf16_t*>(s->vpool[i]);
+                ac.page_table = s->page_table; ac.pt_stride = s->max_pages;
+                ac.qbuf = s->qbuf; ac.gbuf = L.ng ? s->gbuf : nullptr; ac.out16 = s->a16;
+                ac.heads = cfg.heads; ac.kv_heads = cfg.kv_heads;
+                ac.hdr = s->plan.hdr; ac.tiles = reinterpret_cast<const int4*>(s->plan.tiles);
+                CU(attn_cols_launch(cfg.head_dim, cfg.heads / cfg.kv_heads, s->use_pdl, s->plan.max_tiles, s->stream, ac));
+            } else {
+                // fp32 K/V: the decode kernel, one column at a time
+                AttnParams a;
+                a.kpool = s->kpool[i]; a.vpool = s->vpool[i]; a.page_table = s->page_table; a.pt_stride = s->max_pages;
+                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16; a.part = s->part; a.ticket = s->attn_ticket;
+                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
+                rc = chain_attn_f32kv(s, c, a);
+                if (rc) return rc;
+            }
+        } else {
+            if ((rc = gemm(TC_RAW, s->cg_dn, s->tc_g.xn[0], M.qkv, M.qkv, L.n_qkv, d, s->raw, nullptr, true, nullptr, nullptr, nullptr, L.Sqkv, nullptr))) return rc;
+            DeltaColsParams dc;
+            dc.raw = s->raw; dc.raw_stride = s->raw_stride; dc.state = s->state[i]; dc.H = cfg.heads; dc.dv = cfg.dn_value_dim;
+            dc.out = nullptr; dc.out16 = s->a16; dc.l2_eps = 1e-6f;
+            dc.hdr = s->plan.hdr; dc.runs = reinterpret_cast<const int4*>(s->plan.runs);
+            CU(delta_cols_launch(cfg.dn_key_dim, s->use_pdl, s->plan.max_runs, s->stream, dc));
+        }
+        ++launches;
+        if ((rc = gemm(TC_RESID, attn ? s->cg_o_attn : s->cg_o_dn, attn ? s->tc_g.a_attn[0] : s->tc_g.a_dn[0], M.o, M.o, d, L.o_in, s->x, nullptr, false, L.g2, nullptr, nullptr, L.So, nullptr)))
             return rc;
-        QkvPostParams q0{};
-        const CUtensorMap& Ax = ext ? ext->pleP : A;
-        const CUtensorMap& Bx = ext ? ext->pleT : A;
-        cudaError_t e = launch_cluster(s->use_pdl, sh.split, gemm_tc_kernel<MODE, KVT, T>, grid, dim3(kTcThreads), smem, s->stream, A, A2, Bmaps[nb_index(nb)], Ax, Bx, p,
-                                       c, q ? *q : q0);
-        if (e != cudaSuccess) return fail(MLB_E_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
-        if (rec) return rec->end();
-        return MLB_OK;
+        if ((rc = gemm(TC_SWIGLU, s->cg_up, s->tc_g.xn[0], M.w1a, M.w1b, F, d, nullptr, s->h16, true, nullptr, nullptr, nullptr, L.S1a, L.S1b))) return rc;
+        const bool last = i + 1 == cfg.layers;
+        const bool ext = !last && ple > 0;
+        if ((rc = gemm(TC_RESID, ext ? s->cg_down : s->cg_last, s->tc_g.h[0], M.w2, M.w2, d, F, s->x, nullptr, false, last ? m->g_final : m->layers[i + 1].g1,
+                       ext ? &s->tc_maps[i + 1] : nullptr, nullptr, L.S2, nullptr)))
+            return rc;
     }
-
-    // Large-batch step: projections as tcgen05 GEMMs on bf16 operands with the element-wise work in their
-    // epilogues; per layer: projection, attention / delta-net, o-projection, gate-up, down.
-    static int run_tc(mlb_session* s, int kind, const StepCtl& c, Recorder* rec, int* n_launches) {
-        if (std::is_same<T, float>::value) return fail(MLB_E_UNSUPPORTED, "tensor-core projections need bf16 or FP8 weights");
-        const mlb_model* m = s->m;
-        const mlb_config& cfg = m->cfg;
-        const int d = cfg.dim, F = cfg.ffn_dim, B = s->B, ple = cfg.ple_dim;
-        int launches = 0, rc;
-        if (rec && (rc = rec->begin("embed_ple_gather_norm", (uint64_t)B * d * 8 + (uint64_t)B * ple * 2 * cfg.layers, 0))) return rc;
-        CU(launch_chain(s->use_pdl, embed_tc_kernel<T>, dim3(B, (d + kTcM - 1) / kTcM), dim3(128), (size_t)ple * 4, s->stream, c,
-                        static_cast<const T*>(m->E), static_cast<const float*>(m->Es), d, static_cast<const StepLayer*>(s->step_layers), cfg.layers, ple,
-                        static_cast<const float*>(m->layers[0].g1), s->x, s->xn16, s->tc_ssq, s->tple16));
-        if (rec && (rc = rec->end())) return rc;
-        ++launches;
-        for (int i = 0; i < cfg.layers; ++i) {
-            const DevLayer& L = m->layers[i];
-            const mlb_session::TcLayerMaps& M = s->tc_maps[i];
-            if (L.type == MLB_LAYER_ATTENTION) {
-                QkvPostParams q;
-                q.nq = L.nq; q.nk = L.nk; q.nv = L.nv; q.ng = L.ng; q.hd = cfg.head_dim;
-                q.kv_heads = cfg.kv_heads; q.qk_norm = cfg.qk_norm; q.eps = cfg.rms_eps; q.gq = L.gq; q.gk = L.gk; q.rope = m->rope;
-                q.kpool = s->kpool[i]; q.vpool = s->vpool[i]; q.page_table = s->page_table; q.pt_stride = s->max_pages;
-                q.qbuf = s->qbuf; q.gbuf = s->gbuf;
-                if ((rc = gemm_tc<TC_QKV>(s, c, M.qkv, M.qkv, s->tc_g.xn, L.n_qkv, d, nullptr, nullptr, true, nullptr, nullptr, &q, L.Sqkv, nullptr, rec,
-                                          "qkv_gemm_tcgen05_norm_rope_kvappend")))
-                    return rc;
-                ++launches;
-                AttnParams a;
-                a.kpool = s->kpool[i]; a.vpool = s->vpool[i];
-                a.page_table = s->page_table; a.pt_stride = s->max_pages;
-                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16;
-                a.part = s->part; a.ticket = s->attn_ticket;
-                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
-                if (rec) {
-                    uint64_t kvb = 0, fl = 0;
-                    for (int b = 0; b < B; ++b) {
-                        if (!seq_live(s, b)) continue;
-                        kvb += 2ull * cfg.kv_heads * cfg.head_dim * sizeof(KVT) * (s->h_pos[b] + 1);
-                        fl += 4ull * cfg.heads * cfg.head_dim * (s->h_pos[b] + 1);
-                    }
-                    if ((rc = rec->begin("attn_flash_decode_paged", kvb, fl))) return rc;
-                }
-                const int G = cfg.heads / cfg.kv_heads;
-                if (cfg.head_dim == 64) rc = attn_g<64>(s, c, a, G); else rc = attn_g<128>(s, c, a, G);
-                if (rc) return rc;
-                if (rec && (rc = rec->end())) return rc;
-                ++launches;
-            } else {
-                if ((rc = gemm_tc<TC_RAW>(s, c, M.qkv, M.qkv, s->tc_g.xn, L.n_qkv, d, s->raw, nullptr, true, nullptr, nullptr, nullptr, L.Sqkv, nullptr, rec,
-                                          "deltanet_proj_gemm_tcgen05")))
-                    return rc;
-                ++launches;
-                const int dk = cfg.dn_key_dim, dv = cfg.dn_value_dim, H = cfg.heads;
-                if (rec && (rc = rec->begin("deltanet_state_update", (uint64_t)B * 2ull * H * dk * dv * 4, (uint64_t)B * 6ull * H * dk * dv))) return rc;
-                if (s->parent) {
-                    // prompt columns: the recurrence runs over the columns of a sequence in order
-                    dim3 ngrid(H, B), grid((dv + 31) / 32, H, B);
-                    if (dk == 64) {
-                        CU(launch_chain(s->use_pdl, delta_cols_norm_kernel<64>, ngrid, dim3(64), 0, s->stream, c, s->raw, s->raw_stride, H, dv, 1e-6f));
-                        CU(launch_chain(s->use_pdl, delta_net_cols_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const int*>(s->seq_of), B, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16));
-                    } else {
-                        CU(launch_chain(s->use_pdl, delta_cols_norm_kernel<128>, ngrid, dim3(64), 0, s->stream, c, s->raw, s->raw_stride, H, dv, 1e-6f));
-                        CU(launch_chain(s->use_pdl, delta_net_cols_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const int*>(s->seq_of), B, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16));
-                    }
-                    ++launches;
-                } else {
-                    dim3 grid((dv + 31) / 32, H, B);
-                    if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, 1e-6f));
-                    else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, 1e-6f));
-                }
-                if (rec && (rc = rec->end())) return rc;
-                ++launches;
-            }
-            const CUtensorMap* amap = L.type == MLB_LAYER_ATTENTION ? s->tc_g.a_attn : s->tc_g.a_dn;
-            if ((rc = gemm_tc<TC_RESID>(s, c, M.o, M.o, amap, d, L.o_in, s->x, nullptr, false, L.g2, nullptr, nullptr, L.So, nullptr, rec,
-                                        "oproj_gemm_tcgen05_residual_norm")))
-                return rc;
-            ++launches;
-            if ((rc = gemm_tc<TC_SWIGLU>(s, c, M.w1a, M.w1b, s->tc_g.xn, F, d, nullptr, s->h16, true, nullptr, nullptr, nullptr, L.S1a, L.S1b, rec,
-                                         "ffn_gateup_gemm_tcgen05_swiglu")))
-                return rc;
-            ++launches;
-            const bool last = i + 1 == cfg.layers;
-            const float* g_next = last ? m->g_final : m->layers[i + 1].g1;
-            if ((rc = gemm_tc<TC_RESID>(s, c, M.w2, M.w2, s->tc_g.h, d, F, s->x, nullptr, false, g_next,
-                                        (!last && ple > 0) ? &s->tc_maps[i + 1] : nullptr, nullptr, L.S2, nullptr, rec, "ffn_down_gemm_tcgen05_residual_ple_norm")))
-                return rc;
-            ++launches;
-        }
-        if (kind == CHAIN_PREFILL && s->parent) {
-            // prompt columns: positions and tokens of the next chunk come from the host
-        } else if (kind == CHAIN_PREFILL) {
-            if (rec && (rc = rec->begin("advance_prompt", (uint64_t)B * 12, 0))) return rc;
-            CU(launch_chain(s->use_pdl, advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s->stream, c));
-            if (rec && (rc = rec->end())) return rc;
-            ++launches;
-        } else {
-            if ((rc = gemm_tc<TC_RAW>(s, c, s->tc_g.E, s->tc_g.E, s->tc_g.xn, cfg.vocab, d, s->logits, nullptr, true, nullptr, nullptr, nullptr, static_cast<const float*>(m->Es), nullptr, rec,
-                                      "lmhead_gemm_tcgen05")))
-                return rc;
-            ++launches;
-            if (kind == CHAIN_GREEDY) {
-                if (rec && (rc = rec->begin("argmax_pick", (uint64_t)B * cfg.vocab * 4, 0))) return rc;
-                CU(launch_chain(s->use_pdl, argmax_advance_kernel, dim3(B), dim3(256), 0, s->stream, c, static_cast<const float*>(s->logits), cfg.vocab));
-                if (rec && (rc = rec->end())) return rc;
-            } else {
-                SampleParams sp;
-                sp.logits = s->logits; sp.V = cfg.vocab; sp.top_k = s->cur_topk; sp.temperature = s->cur_temp; sp.seeds = s->seeds;
-                if (rec && (rc = rec->begin("sample_topk_philox", (uint64_t)B * cfg.vocab * 4 * 5, 0))) return rc;
-                CU(launch_chain(s->use_pdl, sample_topk_kernel, dim3(B), dim3(256), 0, s->stream, c, sp));
-                if (rec && (rc = rec->end())) return rc;
-            }
-            ++launches;
-        }
-        if (n_launches) *n_launches = launches;
-        return MLB_OK;
-    }
-
-    // One decode (or prefill) step as a chain of launches on the session's stream.
-    static int run(mlb_session* s, int kind, Recorder* rec, int* n_launches) {
-        const mlb_model* m = s->m;
-        const mlb_config& cfg = m->cfg;
-        const StepCtl c = make_ctl(s, kind);
-        const int d = cfg.dim, F = cfg.ffn_dim, B = s->B, p = cfg.ple_dim;
-        int launches = 0, rc;
-        if (s->use_lean || s->use_grid) return run_grid(s, kind, c, rec, n_launches);
-        if (s->use_tc) return run_tc(s, kind, c, rec, n_launches);
-
-        if (rec && (rc = rec->begin("embed_ple_gather", (uint64_t)B * (d * sizeof(T) + (uint64_t)p * sizeof(T2) + (uint64_t)d * 4) + (uint64_t)d * p * sizeof(T2), 0))) return rc;
-        CU(launch_chain(s->use_pdl, embed_kernel<T, T2>, embed_grid(B, d, p), embed_block(B, d, p), (size_t)p * 4, s->stream, c,
-                        static_cast<const T*>(m->E), static_cast<const float*>(m->Es), d, static_cast<const T2*>(m->layers[0].pleT),
-                        static_cast<const T2*>(m->layers[0].pleP), p, s->x));
-        if (rec && (rc = rec->end())) return rc;
-        ++launches;
-
-        for (int i = 0; i < cfg.layers; ++i) {
-            const DevLayer& L = m->layers[i];
-            GemvParams g;
-            std::memset(&g, 0, sizeof g);
-            g.W = L.Wqkv; g.wscale = L.Sqkv; g.N = L.n_qkv; g.K = d;
-            g.xin = s->x; g.gain = L.g1; g.eps = cfg.rms_eps; g.do_norm = 1;
-            if (L.type == MLB_LAYER_ATTENTION) {
-                g.nq = L.nq; g.nk = L.nk; g.nv = L.nv; g.ng = L.ng;
-                g.hd = cfg.head_dim; g.kv_heads = cfg.kv_heads; g.qk_norm = cfg.qk_norm;
-                g.gq = L.gq; g.gk = L.gk; g.rope = m->rope;
-                g.kpool = s->kpool[i]; g.vpool = s->vpool[i];
-                g.page_table = s->page_table; g.pt_stride = s->max_pages;
-                g.qbuf = s->qbuf; g.gbuf = s->gbuf;
-                const int R = cfg.qk_norm ? cfg.head_dim : 16;
-                if ((rc = gemv<GEMV_QKV>(s, c, g, R, rec, "qkv_gemv_norm_rope_kvappend"))) return rc;
-                ++launches;
-                AttnParams a;
-                a.kpool = s->kpool[i]; a.vpool = s->vpool[i];
-                a.page_table = s->page_table; a.pt_stride = s->max_pages;
-                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = nullptr;
-                a.part = s->part; a.ticket = s->attn_ticket;
-                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
-                if (rec) {
-                    uint64_t kvb = 0, fl = 0;
-                    for (int b = 0; b < B; ++b) {
-                        if (!seq_live(s, b)) continue;
-                        kvb += 2ull * cfg.kv_heads * cfg.head_dim * sizeof(KVT) * (s->h_pos[b] + 1);
-                        fl += 4ull * cfg.heads * cfg.head_dim * (s->h_pos[b] + 1);
-                    }
-                    if ((rc = rec->begin("attn_flash_decode_paged", kvb, fl))) return rc;
-                }
-                const int G = cfg.heads / cfg.kv_heads;
-                if (cfg.head_dim == 64) rc = attn_g<64>(s, c, a, G); else rc = attn_g<128>(s, c, a, G);
-                if (rc) return rc;
-                if (rec && (rc = rec->end())) return rc;
-                ++launches;
-            } else {
-                g.y = s->raw;
-                if ((rc = gemv<GEMV_RAW>(s, c, g, 16, rec, "deltanet_proj_gemv_norm"))) return rc;
-                ++launches;
-                const int dk = cfg.dn_key_dim, dv = cfg.dn_value_dim, H = cfg.heads;
-                if (rec && (rc = rec->begin("deltanet_state_update", (uint64_t)B * 2ull * H * dk * dv * 4, (uint64_t)B * 6ull * H * dk * dv))) return rc;
-                dim3 grid((dv + 31) / 32, H, B);
-                if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
-                else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
-                if (rec && (rc = rec->end())) return rc;
-                ++launches;
-            }
-            // output projection + residual (in place on the residual stream)
-            std::memset(&g, 0, sizeof g);
-            g.W = L.Wo; g.wscale = L.So; g.N = d; g.K = L.o_in;
-            g.xin = s->abuf; g.y = s->x; g.resid = s->x;
-            if ((rc = gemv<GEMV_RESID>(s, c, g, d <= 1024 ? 8 : 16, rec, "oproj_gemv_residual"))) return rc;
-            ++launches;
-            // FFN gate/up with RMS norm prologue and SwiGLU epilogue
-            std::memset(&g, 0, sizeof g);
-            g.W = L.W1a; g.Wb = L.W1b; g.wscale = L.S1a; g.wscale_b = L.S1b; g.N = F; g.K = d;
-            g.xin = s->x; g.gain = L.g2; g.eps = cfg.rms_eps; g.do_norm = 1; g.y = s->hbuf;
-            if ((rc = gemv<GEMV_SWIGLU>(s, c, g, 8, rec, "ffn_gateup_gemv_norm_swiglu"))) return rc;
-            ++launches;
-            // FFN down + residual (+ the next layer's per-layer embedding)
-            std::memset(&g, 0, sizeof g);
-            g.W = L.W2; g.wscale = L.S2; g.N = d; g.K = F;
-            g.xin = s->hbuf; g.y = s->x; g.resid = s->x;
-            if (p > 0 && i + 1 < cfg.layers) { g.P = m->layers[i + 1].pleP; g.Ptab = m->layers[i + 1].pleT; g.Kp = p; }
-            if ((rc = gemv<GEMV_RESID>(s, c, g, d <= 1024 ? 8 : 16, rec, "ffn_down_gemv_residual_ple"))) return rc;
-            ++launches;
-        }
-        if (kind == CHAIN_PREFILL) {
-            if (rec && (rc = rec->begin("advance_prompt", (uint64_t)B * 12, 0))) return rc;
-            CU(launch_chain(s->use_pdl, advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s->stream, c));
-            if (rec && (rc = rec->end())) return rc;
-            ++launches;
-        } else {
-            GemvParams g;
-            std::memset(&g, 0, sizeof g);
-            g.W = m->E; g.wscale = m->Es; g.N = cfg.vocab; g.K = d;
-            g.xin = s->x; g.gain = m->g_final; g.eps = cfg.rms_eps; g.do_norm = 1; g.y = s->logits;
-            g.part_val = s->part_val; g.part_idx = s->part_idx; g.ticket = s->lm_ticket;
-            g.do_pick = kind == CHAIN_GREEDY ? 1 : 0;
-            if ((rc = gemv<GEMV_LMHEAD>(s, c, g, s->lm_rows, rec, "lmhead_gemv_norm_argmax"))) return rc;
-            ++launches;
-            if (kind == CHAIN_TOPK) {
-                SampleParams sp;
-                sp.logits = s->logits; sp.V = cfg.vocab; sp.top_k = s->cur_topk; sp.temperature = s->cur_temp; sp.seeds = s->seeds;
-                if (rec && (rc = rec->begin("sample_topk_philox", (uint64_t)B * cfg.vocab * 4 * 5, 0))) return rc;
-                CU(launch_chain(s->use_pdl, sample_topk_kernel, dim3(B), dim3(256), 0, s->stream, c, sp));
-                if (rec && (rc = rec->end())) return rc;
-                ++launches;
-            }
-        }
-        if (n_launches) *n_launches = launches;
-        return MLB_OK;
-    }
-};
+    if (kind != CHAIN_PREFILL && (rc = gemm(TC_RAW, s->cg_head, s->tc_g.xn[0], s->tc_g.E, s->tc_g.E, cfg.vocab, d, s->logits, nullptr, true, nullptr, nullptr, nullptr,
+                                            static_cast<const float*>(m->Es), nullptr)))
+        return rc;
+    if (n_launches) *n_launches = launches;
+    return MLB_OK;
+}
 
 static int chain_run(mlb_session* s, int kind, Recorder* rec, int* n_launches) {
-    const int w = s->m->cfg.weight_dtype, k = s->m->cfg.kv_dtype;
-    if (w == MLB_DT_F32 && k == MLB_DT_F32) return Chain<float, float, float>::run(s, kind, rec, n_launches);
-    if (w == MLB_DT_F32 && k == MLB_DT_BF16) return Chain<float, float, bf16_t>::run(s, kind, rec, n_launches);
-    if (w == MLB_DT_BF16 && k == MLB_DT_F32) return Chain<bf16_t, bf16_t, float>::run(s, kind, rec, n_launches);
-    if (w == MLB_DT_BF16 && k == MLB_DT_BF16) return Chain<bf16_t, bf16_t, bf16_t>::run(s, kind, rec, n_launches);
-    if (w == MLB_DT_FP8_E4M3 && k == MLB_DT_F32) return Chain<fp8_t, bf16_t, float>::run(s, kind, rec, n_launches);
-    return Chain<fp8_t, bf16_t, bf16_t>::run(s, kind, rec, n_launches);
+    if (s->use_cols) return run_cols(s, kind, n_launches);
+    switch (s->m->cfg.weight_dtype) {
+        case MLB_DT_F32: return chain_run_f32(s, kind, rec, n_launches);
+        case MLB_DT_BF16: return chain_run_bf16(s, kind, rec, n_launches);
+        default: return chain_run_fp8(s, kind, rec, n_launches);
+    }
 }
 static int chain_configure(mlb_session* s) {
-    const int w = s->m->cfg.weight_dtype, k = s->m->cfg.kv_dtype;
-    if (w == MLB_DT_F32 && k == MLB_DT_F32) return Chain<float, float, float>::configure();
-    if (w == MLB_DT_F32 && k == MLB_DT_BF16) return Chain<float, float, bf16_t>::configure();
-    if (w == MLB_DT_BF16 && k == MLB_DT_F32) return Chain<bf16_t, bf16_t, float>::configure();
-    if (w == MLB_DT_BF16 && k == MLB_DT_BF16) return Chain<bf16_t, bf16_t, bf16_t>::configure();
-    if (w == MLB_DT_FP8_E4M3 && k == MLB_DT_F32) return Chain<fp8_t, bf16_t, float>::configure();
-    return Chain<fp8_t, bf16_t, bf16_t>::configure();
+    switch (s->m->cfg.weight_dtype) {
+        case MLB_DT_F32: return chain_configure_f32(s);
+        case MLB_DT_BF16: return chain_configure_bf16(s);
+        default: return chain_configure_fp8(s);
+    }
 }
 
 // Device copy of the per-layer pointer table of the single-kernel steps.
@@ -1361,18 +708,23 @@ static int setup_grid_path(mlb_session* s) {
     return MLB_OK;
 }
 
-template <typename KVT, typename WT>
-static int tc_allow_big_smem_t() {
-    const int big = 227 * 1024;
-    CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_RAW, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_RESID, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_SWIGLU, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_QKV, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+// How far a cluster may split the k-blocks of a GEMM tile here.
+static int tc_probe_clusters(mlb_session* s) {
+    s->tc_max_split = 8;
+    if (const char* v = std::getenv("MLB_TC_SPLIT")) {
+        s->tc_max_split = std::max(1, std::min(8, std::atoi(v)));
+        s->tc_split_forced = true;
+    }
+    {
+        // how many clusters of GEMM CTAs fit on the GPU at once (a 100 KB CTA, typical of a split launch)
+        s->tc_cluster_cap[0] = s->sm_count;
+        for (int li = 1; li < 4; ++li) {
+            int n = 0, rc;
+            if ((rc = tc_max_clusters(1 << li, 100 * 1024, &n))) return rc;
+            s->tc_cluster_cap[li] = n;
+        }
+    }
     return MLB_OK;
-}
-static int tc_allow_big_smem(int wdt, int kvdt) {
-    if (wdt == MLB_DT_FP8_E4M3) return kvdt == MLB_DT_BF16 ? tc_allow_big_smem_t<bf16_t, fp8_t>() : tc_allow_big_smem_t<float, fp8_t>();
-    return kvdt == MLB_DT_BF16 ? tc_allow_big_smem_t<bf16_t, bf16_t>() : tc_allow_big_smem_t<float, bf16_t>();
 }
 
 // Tensor-core projections for batches of 4 sequences or more with bf16 weights (MLB_GEMM=simt turns it off).
@@ -1407,35 +759,8 @@ static int setup_tc_path(mlb_session* s) {
     if ((rc = build_step_layers(s))) return rc;
     if (const char* v = std::getenv("MLB_TC_TRACE"))
         if (v[0] == '1' && (rc = sess_alloc(s, (void**)&s->tc_trace, 64 * 8 * 8, true))) return rc;
-    s->tc_max_split = 8;
-    if (const char* v = std::getenv("MLB_TC_SPLIT")) {
-        s->tc_max_split = std::max(1, std::min(8, std::atoi(v)));
-        s->tc_split_forced = true;
-    }
-    {
-        // how many clusters of GEMM CTAs fit on the GPU at once (a 100 KB CTA, typical of a split launch)
-        const int big = 227 * 1024;
-        void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmTcParams, StepCtl, QkvPostParams) =
-            gemm_tc_kernel<TC_RESID, float, bf16_t>;
-        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        s->tc_cluster_cap[0] = s->sm_count;
-        for (int li = 1; li < 4; ++li) {
-            cudaLaunchConfig_t cfg;
-            std::memset(&cfg, 0, sizeof cfg);
-            cfg.gridDim = dim3(1, 1, 1u << li);
-            cfg.blockDim = dim3(kTcThreads);
-            cfg.dynamicSmemBytes = 100 * 1024;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1u << li;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-            s->tc_cluster_cap[li] = n;
-        }
-    }
-    s->tc_shape_down = tc_pick_shape(s, c.dim, (c.ffn_dim + kTcKB - 1) / kTcKB + (c.ple_dim + kTcKB - 1) / kTcKB, 1, w8, w8 ? 2 : 1);
+    if ((rc = tc_probe_clusters(s))) return rc;
+    s->tc_shape_down = tc_pick_shape(s, B, c.dim, (c.ffn_dim + kTcKB - 1) / kTcKB + (c.ple_dim + kTcKB - 1) / kTcKB, 1, w8, w8 ? 2 : 1);
     const int parts = (c.dim + kTcM - 1) / kTcM;
     if ((rc = sess_alloc(s, (void**)&s->xn16, (size_t)B * c.dim * 2, true))) return rc;
     if ((rc = sess_alloc(s, (void**)&s->a16, (size_t)B * std::max(nq, a_dn) * 2, true))) return rc;
@@ -1466,8 +791,162 @@ static int setup_tc_path(mlb_session* s) {
         if ((rc = make_bf16_map(enc, &s->tc_g.a_dn[i], s->a16, B, a_dn, nb))) return rc;
         if ((rc = make_bf16_map(enc, &s->tc_g.h[i], s->h16, B, c.ffn_dim, nb))) return rc;
     }
-    if ((rc = tc_allow_big_smem(c.weight_dtype, c.kv_dtype))) return rc;
+    if ((rc = w8 ? tc_allow_big_smem_fp8(c.kv_dtype) : tc_allow_big_smem_bf16(c.kv_dtype))) return rc;
     s->use_tc = true;
+    return MLB_OK;
+}
+
+// The FP8 codes of a model as bf16. Leaves `wide` empty where there is no memory for them.
+static int model_widen(mlb_model* m, cudaStream_t st) {
+    std::lock_guard<std::mutex> hold(m->wide_mutex);
+    if (!m->wide.empty() || m->wide_failed) return MLB_OK;
+    const mlb_config& c = m->cfg;
+    std::vector<void*> made;
+    int rc = MLB_OK;
+    auto widen = [&](const void* codes, size_t n) -> void* {
+        void* p = nullptr;
+        if (rc) return p;
+        if (cudaMalloc(&p, n * 2) != cudaSuccess) {
+            cudaGetLastError();
+            rc = MLB_E_NOMEM;
+            return nullptr;
+        }
+        made.push_back(p);
+        if (widen_e4m3_launch(codes, static_cast<bf16_t*>(p), n, st) != cudaSuccess) rc = MLB_E_CUDA;
+        return p;
+    };
+    std::vector<mlb_model::Wide> w(c.layers);
+    for (int i = 0; i < c.layers; ++i) {
+        const DevLayer& L = m->layers[i];
+        w[i].Wqkv = widen(L.Wqkv, (size_t)L.n_qkv * c.dim);
+        w[i].Wo = widen(L.Wo, (size_t)c.dim * L.o_in);
+        w[i].W1a = widen(L.W1a, (size_t)c.ffn_dim * c.dim);
+        w[i].W1b = widen(L.W1b, (size_t)c.ffn_dim * c.dim);
+        w[i].W2 = widen(L.W2, (size_t)c.dim * c.ffn_dim);
+    }
+    void* we = widen(m->E, (size_t)c.vocab * c.dim);
+    const cudaError_t e = cudaStreamSynchronize(st);      // sessions on other streams read them from here on
+    if (rc || e != cudaSuccess) {
+        for (void* p : made) cudaFree(p);
+        m->wide_failed = true;
+        if (rc == MLB_E_NOMEM && e == cudaSuccess) return MLB_OK;
+        return fail(MLB_E_CUDA, "widening of the FP8 weights failed: %s", cudaGetErrorString(e));
+    }
+    m->allocs.insert(m->allocs.end(), made.begin(), made.end());
+    m->wide_E = we;
+    m->wide.swap(w);
+    return MLB_OK;
+}
+
+// Launch shape of a column GEMM: `T` columns, `N` output features, `nkb` k-blocks of 64, the last `nkb_x` of a second
+// operand pair (`exts_apart`: with accumulators of its own), in `split` ranges. Tensor memory (512 columns) bounds BN x
+// accumulators x buffers. A 128 x BN x 64 k-block takes about 0.30 / 0.19 / 0.14 us at BN = 256 / 128 / 64 (the MMA's own
+// rate at 256, operand reads below), an epilogue 3 us at 256, hidden under the next tile's k-loop where there are two
+// buffers; the cheapest in the sum over a CTA's tiles wins.
+static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode, bool exts_apart, int split, int min_bn) {
+    ColsGemm best{};
+    double best_cost = -1.0;
+    static const int bns[3] = {256, 128, 64};
+    static const double t_kb[3] = {0.30, 0.19, 0.14};
+    int mains = 0, exts = 0;
+    for (int r = 0; r < split; ++r) {
+        const int lo = (int)((long)nkb * r / split), hi = (int)((long)nkb * (r + 1) / split);
+        if (exts_apart ? lo < nkb - nkb_x : hi > lo) ++mains;
+        if (exts_apart && hi > nkb - nkb_x) ++exts;
+    }
+    for (int i = 0; i < 3; ++i) {
+        const int bn = bns[i];
+        for (int nbuf = 2; nbuf >= 1; --nbuf) {
+            if (bn < min_bn || bn * (mains + exts) * nbuf > 512) continue;
+            const int bn_out = mode == TC_SWIGLU ? bn / 2 : bn;
+            const long tiles = (long)((T + kGcM - 1) / kGcM) * ((N + bn_out - 1) / bn_out);
+            const long waves = (tiles + sm_count - 1) / sm_count;
+            const double loop = nkb * t_kb[i], epi = 3.0 * bn / 256 + 0.5;
+            const double cost = 1.5 + loop + epi + (waves - 1) * (nbuf == 2 ? std::max(loop, epi) : loop + epi);
+            if (best_cost < 0 || cost < best_cost) {
+                best_cost = cost;
+                const int fit = (int)((kGcSmem - 1024) / ((size_t)(kGcM + bn) * 128));
+                best.bn = bn;
+                best.stages = (int)std::min<long>(std::min(fit, kGcMaxStages), std::max<long>(2, nkb * waves));
+                best.ctas = (int)std::min<long>(tiles, sm_count);
+                best.split = split; best.mains = mains; best.exts = exts; best.nbuf = nbuf;
+                best.tmem_cols = 32;
+                while (best.tmem_cols < (uint32_t)(bn * (mains + exts) * nbuf)) best.tmem_cols <<= 1;
+            }
+            break;
+        }
+    }
+    return best;
+}
+
+// Buffers, tensor maps and launch shapes of a column set.
+static int setup_cols_path(mlb_session* s) {
+    const mlb_model* m = s->m;
+    const mlb_config& c = m->cfg;
+    s->use_cols = false;
+    EncodeTiledFn enc = get_encode_tiled();
+    if (!enc) return MLB_OK;
+    const bool w8 = c.weight_dtype == MLB_DT_FP8_E4M3;
+    int rc;
+    if (w8) {
+        if ((rc = model_widen(s->m, s->stream))) return rc;
+        if (m->wide.empty()) return MLB_OK;
+    }
+    if ((rc = build_step_layers(s))) return rc;
+    const int T = s->B, nq = c.heads * c.head_dim, a_dn = c.heads * c.dn_value_dim;
+    auto kb = [](int k) { return (k + kTcKB - 1) / kTcKB; };
+    const bool ext2 = w8 && c.ple_dim > 0;
+    int n_qkv = 0, n_dn = 0;
+    for (const DevLayer& L : m->layers) (L.type == MLB_LAYER_ATTENTION ? n_qkv : n_dn) = L.n_qkv;
+    // The ranges of k-blocks are those of gemm_tc_kernel's launches with kTcRefCols columns, whatever the width of this set, so
+    // that a prompt's cache does not depend on how it is cut into chunks.
+    if ((rc = tc_probe_clusters(s))) return rc;
+    bool fits = true;
+    auto pick = [&](int N, int nkb, int nkb_x, int mode, bool apart) {
+        const bool resid8 = w8 && mode == TC_RESID;
+        const TcShape ref = tc_pick_shape(s, kTcRefCols, N, nkb, mode == TC_SWIGLU ? 2 : 1, w8, mode == TC_SWIGLU || resid8 ? 2 : 1);
+        const ColsGemm g = gc_pick(s->sm_count, T, N, nkb, nkb_x, mode, apart, std::max(1, ref.split),
+                                    mode == TC_QKV && c.qk_norm ? c.head_dim : 64);       // a tile holds whole heads for their norm
+        fits = fits && g.bn > 0;
+        return g;
+    };
+    if (n_qkv) s->cg_qkv = pick(n_qkv, kb(c.dim), 0, TC_QKV, false);
+    if (n_dn) s->cg_dn = pick(n_dn, kb(c.dim), 0, TC_RAW, false);
+    if (n_qkv) s->cg_o_attn = pick(c.dim, kb(nq), 0, TC_RESID, false);
+    if (n_dn) s->cg_o_dn = pick(c.dim, kb(a_dn), 0, TC_RESID, false);
+    s->cg_up = pick(c.ffn_dim, kb(c.dim), 0, TC_SWIGLU, false);
+    s->cg_down = pick(c.dim, kb(c.ffn_dim) + kb(c.ple_dim), kb(c.ple_dim), TC_RESID, ext2);
+    s->cg_last = pick(c.dim, kb(c.ffn_dim), 0, TC_RESID, false);
+    s->cg_head = pick(c.vocab, kb(c.dim), 0, TC_RAW, false);
+    if (!fits) return MLB_OK;      // a forced split that tensor memory does not hold
+    if ((rc = sess_alloc(s, (void**)&s->xn16, (size_t)T * c.dim * 2, true))) return rc;
+    if ((rc = sess_alloc(s, (void**)&s->a16, (size_t)T * std::max(nq, a_dn) * 2, true))) return rc;
+    if ((rc = sess_alloc(s, (void**)&s->h16, (size_t)T * c.ffn_dim * 2, true))) return rc;
+    if ((rc = sess_alloc(s, (void**)&s->tc_ssq, (size_t)T * ((c.dim + 127) / 128) * 4 * 4, true))) return rc;
+    if (c.ple_dim > 0 && (rc = sess_alloc(s, (void**)&s->tple16, (size_t)c.layers * T * c.ple_dim * 2, true))) return rc;
+    s->tc_maps.resize(c.layers);
+    for (int i = 0; i < c.layers; ++i) {
+        const DevLayer& L = m->layers[i];
+        auto& M = s->tc_maps[i];
+        const void *wqkv = L.Wqkv, *wo = L.Wo, *w1a = L.W1a, *w1b = L.W1b, *w2 = L.W2;
+        if (w8) { const auto& w = m->wide[i]; wqkv = w.Wqkv; wo = w.Wo; w1a = w.W1a; w1b = w.W1b; w2 = w.W2; }
+        const int bn_qkv = L.type == MLB_LAYER_ATTENTION ? s->cg_qkv.bn : s->cg_dn.bn;
+        if ((rc = make_bf16_map(enc, &M.qkv, wqkv, L.n_qkv, c.dim, bn_qkv))) return rc;
+        if ((rc = make_bf16_map(enc, &M.o, wo, c.dim, L.o_in, L.type == MLB_LAYER_ATTENTION ? s->cg_o_attn.bn : s->cg_o_dn.bn))) return rc;
+        if ((rc = make_bf16_map(enc, &M.w1a, w1a, c.ffn_dim, c.dim, s->cg_up.bn / 2))) return rc;
+        if ((rc = make_bf16_map(enc, &M.w1b, w1b, c.ffn_dim, c.dim, s->cg_up.bn / 2))) return rc;
+        if ((rc = make_bf16_map(enc, &M.w2, w2, c.dim, c.ffn_dim, (i + 1 < c.layers && c.ple_dim > 0) ? s->cg_down.bn : s->cg_last.bn))) return rc;
+        if (c.ple_dim > 0) {
+            if ((rc = make_bf16_map(enc, &M.pleP, L.pleP, c.dim, c.ple_dim, s->cg_down.bn))) return rc;
+            if ((rc = make_bf16_map(enc, &M.pleT, s->tple16 + (size_t)i * T * c.ple_dim, T, c.ple_dim, kGcM))) return rc;
+        }
+    }
+    if ((rc = make_bf16_map(enc, &s->tc_g.E, w8 ? m->wide_E : m->E, c.vocab, c.dim, s->cg_head.bn))) return rc;
+    if ((rc = make_bf16_map(enc, &s->tc_g.xn[0], s->xn16, T, c.dim, kGcM))) return rc;
+    if ((rc = make_bf16_map(enc, &s->tc_g.a_attn[0], s->a16, T, nq, kGcM))) return rc;
+    if ((rc = make_bf16_map(enc, &s->tc_g.a_dn[0], s->a16, T, a_dn, kGcM))) return rc;
+    if ((rc = make_bf16_map(enc, &s->tc_g.h[0], s->h16, T, c.ffn_dim, kGcM))) return rc;
+    s->use_cols = true;
     return MLB_OK;
 }
 
@@ -1562,6 +1041,21 @@ static int grow_pages(mlb_session* s, int extra_steps) {
     return sync_page_table(s);
 }
 
+// Where the parts of a column plan lie, for `T` columns of a session of `B` sequences.
+struct ColsLayout {
+    size_t tok, pos, lim, seq, runs, tiles, ints;
+    int max_runs, max_tiles;
+};
+static ColsLayout cols_layout(const mlb_config& c, int B, int T) {
+    ColsLayout l;
+    l.max_runs = std::min(B, T);
+    l.max_tiles = T / attn_cols_queries(c.heads / c.kv_heads) + l.max_runs;      // every run may end in a partial tile
+    l.tok = 4; l.pos = l.tok + T; l.lim = l.pos + T; l.seq = l.lim + T;
+    l.runs = l.seq + T; l.tiles = l.runs + 4 * (size_t)l.max_runs;
+    l.ints = l.tiles + 4 * (size_t)l.max_tiles;
+    return l;
+}
+
 static int apply_sampling(mlb_session* s, const mlb_sampling* sp, int* kind) {
     *kind = CHAIN_GREEDY;
     if (!sp || sp->mode == 0) return MLB_OK;
@@ -1604,29 +1098,44 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     if (parent) s->stream = parent->stream;
     else SCU(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     const size_t B = batch;
-    const size_t ctx_rows = parent ? 1 : (size_t)max_context;      // a column set has no prompt / output ring of its own
-    SA(sess_alloc(s, (void**)&s->pos, B * 4, true));
-    SA(sess_alloc(s, (void**)&s->tok, B * 4, true));
-    SA(sess_alloc(s, (void**)&s->limit_prefill, B * 4, true));
-    SA(sess_alloc(s, (void**)&s->limit_decode, B * 4, true));
-    SA(sess_alloc(s, (void**)&s->prompt, B * ctx_rows * 4, true));
-    SA(sess_alloc(s, (void**)&s->out_ring, B * ctx_rows * 4, true));
-    if (parent) SA(sess_alloc(s, (void**)&s->seq_of, B * 4, true));
-    SA(sess_alloc(s, (void**)&s->out_idx, B * 4, true));
-    SA(sess_alloc(s, (void**)&s->page_table, B * s->max_pages * 4, true));
-    SA(sess_alloc(s, (void**)&s->seeds, B * 8, true));
+    if (parent) {
+        // positions, tokens, limits and sequences of the columns are one array, so that a chunk is one copy; no prompt
+        // or output ring, no page table of its own
+        const ColsLayout lay = cols_layout(c, parent->B, batch);
+        SA(sess_alloc(s, (void**)&s->plan_dev, lay.ints * 4, true));
+        s->tok = s->plan_dev + lay.tok; s->pos = s->plan_dev + lay.pos; s->seq_of = s->plan_dev + lay.seq;
+        s->limit_prefill = s->limit_decode = s->plan_dev + lay.lim;
+        s->plan.hdr = s->plan_dev;
+        s->plan.runs = s->plan_dev + lay.runs; s->plan.max_runs = lay.max_runs;
+        s->plan.tiles = s->plan_dev + lay.tiles; s->plan.max_tiles = lay.max_tiles;
+        s->page_table = parent->page_table;
+    } else {
+        SA(sess_alloc(s, (void**)&s->pos, B * 4, true));
+        SA(sess_alloc(s, (void**)&s->tok, B * 4, true));
+        SA(sess_alloc(s, (void**)&s->limit_prefill, B * 4, true));
+        SA(sess_alloc(s, (void**)&s->limit_decode, B * 4, true));
+        SA(sess_alloc(s, (void**)&s->prompt, B * max_context * 4, true));
+        SA(sess_alloc(s, (void**)&s->out_ring, B * max_context * 4, true));
+        SA(sess_alloc(s, (void**)&s->out_idx, B * 4, true));
+        SA(sess_alloc(s, (void**)&s->page_table, B * s->max_pages * 4, true));
+        SA(sess_alloc(s, (void**)&s->seeds, B * 8, true));
+    }
     const int nq = c.heads * c.head_dim;
     const int a_dim = std::max(nq, c.heads * c.dn_value_dim);
+    bool has_dn = false;
+    for (int i = 0; i < c.layers; ++i) has_dn = has_dn || c.layer_types[i] == MLB_LAYER_DELTA_NET;
     s->max_q = nq;
     s->raw_stride = 2 * c.heads * c.dn_key_dim + c.heads * c.dn_value_dim + 2 * c.heads;
     SA(sess_alloc(s, (void**)&s->x, B * c.dim * 4, true));
     SA(sess_alloc(s, (void**)&s->qbuf, B * nq * 4, true));
-    SA(sess_alloc(s, (void**)&s->gbuf, B * nq * 4, true));
+    if (c.query_gating || !parent) SA(sess_alloc(s, (void**)&s->gbuf, B * nq * 4, true));
     SA(sess_alloc(s, (void**)&s->abuf, B * a_dim * 4, true));
-    SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
-    SA(sess_alloc(s, (void**)&s->raw, B * s->raw_stride * 4, true));
-    SA(sess_alloc(s, (void**)&s->logits, B * c.vocab * 4, true));
-    SA(sess_alloc(s, (void**)&s->probe, (size_t)c.vocab * 4, true));
+    if (has_dn || !parent) SA(sess_alloc(s, (void**)&s->raw, B * s->raw_stride * 4, true));
+    if (!parent) {
+        SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
+        SA(sess_alloc(s, (void**)&s->logits, B * c.vocab * 4, true));        // a column set's are made when a text is scored
+        SA(sess_alloc(s, (void**)&s->probe, (size_t)c.vocab * 4, true));
+    }
     // split count of the flash-decode: enough CTAs to cover the GPU at small batch, at least
     // four pages of work per split at full context
     int sm_count = 148;
@@ -1670,19 +1179,25 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
         s->flush_n = (192ull << 20) / 16;
         SA(sess_alloc(s, (void**)&s->flush_buf, s->flush_n * 16, false));
     }
-    SCU(cudaMallocHost((void**)&s->pinned_tok, B * 4));
-    SCU(cudaMallocHost((void**)&s->pinned_out, B * 4));
     SCU(cudaMallocHost((void**)&s->pinned_err, 4));
+    if (!parent) {
+        SCU(cudaMallocHost((void**)&s->pinned_tok, B * 4));
+        SCU(cudaMallocHost((void**)&s->pinned_out, B * 4));
+    }
     *s->pinned_err = 0;
-    s->alloc.num_pages = s->kv_pages;
-    s->alloc.max_pages_per_seq = s->max_pages;
-    s->alloc.seq_pages.assign(batch, {});
-    for (int p = s->kv_pages - 1; p >= 0; --p) s->alloc.free_list.push_back(p);
+    if (!parent) {
+        s->alloc.num_pages = s->kv_pages;
+        s->alloc.max_pages_per_seq = s->max_pages;
+        s->alloc.seq_pages.assign(batch, {});
+        for (int p = s->kv_pages - 1; p >= 0; --p) s->alloc.free_list.push_back(p);
+    }
     s->h_pos.assign(batch, 0);
     s->h_stopped.assign(batch, 0);
-    s->h_table.assign(B * s->max_pages, 0);
-    std::vector<int> lim(batch, max_context);
-    SCU(cudaMemcpy(s->limit_decode, lim.data(), B * 4, cudaMemcpyHostToDevice));
+    if (!parent) {
+        s->h_table.assign(B * s->max_pages, 0);
+        std::vector<int> lim(batch, max_context);
+        SCU(cudaMemcpy(s->limit_decode, lim.data(), B * 4, cudaMemcpyHostToDevice));
+    }
     {
         const char* e = std::getenv("MLB_NO_PDL");     // measurement switch: plain stream-ordered launches
         s->use_pdl = !(e && e[0] == '1');
@@ -1695,13 +1210,14 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
         cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, m->device);
     }
     SA(sess_alloc(s, (void**)&s->dev_err, 4, true));
-    SA(chain_configure(s));
     if (!parent) {
+        SA(chain_configure(s));
         SA(setup_lean_path(s));
         if (!s->use_lean) SA(setup_grid_path(s));
     }
-    SA(setup_tc_path(s));
-    if (parent && !s->use_tc) {
+    if (parent) SA(setup_cols_path(s));
+    if (!s->use_cols) SA(setup_tc_path(s));
+    if (parent && !s->use_cols && !s->use_tc) {
         free_session(s);
         return fail(MLB_E_UNSUPPORTED, "prompt columns need the tensor-core step (bf16 weights)");
     }
@@ -1716,25 +1232,14 @@ extern "C" int mlb_session_new(mlb_model* m, int batch, int max_context, int kv_
     return session_create(m, batch, max_context, kv_block, kv_pages, nullptr, out);
 }
 
-extern "C" int mlb_session_reset(mlb_session* s) {
-    if (!s) return fail(MLB_E_INVALID, "null session");
-    CU(cudaSetDevice(s->m->device));
-    CU(cudaStreamSynchronize(s->stream));
+// Queues the reset of the device state and resets the host's.
+static int reset_queued(mlb_session* s) {
     const size_t B = s->B;
-    CU(cudaMemsetAsync(s->pos, 0, B * 4, s->stream));
-    CU(cudaMemsetAsync(s->tok, 0, B * 4, s->stream));
-    CU(cudaMemsetAsync(s->limit_prefill, 0, B * 4, s->stream));
-    CU(cudaMemsetAsync(s->out_idx, 0, B * 4, s->stream));
-    {
-        // a sequence that stopped had its decode limit lowered on the device
-        const std::vector<int> lim(B, s->max_ctx);
-        CU(cudaMemcpyAsync(s->limit_decode, lim.data(), B * 4, cudaMemcpyHostToDevice, s->stream));
-        CU(cudaStreamSynchronize(s->stream));
-    }
+    session_reset_kernel<<<(s->B + 127) / 128, 128, 0, s->stream>>>(s->B, s->max_ctx, s->pos, s->tok, s->limit_prefill, s->limit_decode, s->out_idx);
+    CU(cudaGetLastError());
     const mlb_config& c = s->m->cfg;
     for (int i = 0; i < c.layers; ++i)
         if (s->state[i]) CU(cudaMemsetAsync(s->state[i], 0, B * c.heads * c.dn_value_dim * c.dn_key_dim * 4, s->stream));
-    CU(cudaStreamSynchronize(s->stream));
     for (int b = 0; b < s->B; ++b) {
         for (int pg : s->alloc.seq_pages[b]) s->alloc.free_list.push_back(pg);
         s->alloc.seq_pages[b].clear();
@@ -1746,18 +1251,41 @@ extern "C" int mlb_session_reset(mlb_session* s) {
     return MLB_OK;
 }
 
+extern "C" int mlb_session_reset(mlb_session* s) {
+    if (!s) return fail(MLB_E_INVALID, "null session");
+    CU(cudaSetDevice(s->m->device));
+    int rc = reset_queued(s);
+    if (rc) return rc;
+    CU(cudaStreamSynchronize(s->stream));
+    return MLB_OK;
+}
+
 extern "C" void mlb_session_free(mlb_session* s) { free_session(s); }
 
 // Prompt by columns. The token loop consumes a prompt one token per step and sequence: a
 // 512-token prompt costs 511 steps. Here the prompt tokens of all sequences become the columns of
-// tensor-core steps (bf16 weights): the projections of up to kPromptCols (256) tokens are one GEMM each,
-// every column appends its K/V row and attends to the rows before it (same kernels as a decode
-// step, the column's page-table row is its sequence's), and the delta-net recurrence walks the
-// columns of a sequence in order (delta_net_cols_kernel). All tokens but the last of each prompt
+// tensor-core steps (bf16 or FP8 weights): the projections of up to kColMax tokens are one GEMM each,
+// every column appends its K/V row and attends to the rows before it, and the delta-net recurrence walks the
+// columns of a sequence in order (cols.cu). All tokens but the last of each prompt
 // are consumed; the last one stays pending, as after the token loop. MLB_PREFILL = auto | step |
 // chunk: auto takes this path from 64 prompt tokens on (its activations are bf16, so the cache
 // differs from the token loop's within the low-precision tolerance); `*done` tells whether it ran.
-static const int kPromptCols = 256;
+//
+// Width of a step: a column set of 256 leaves most SMs without a tile (d = 512: 4 row tiles of 128) and pays the
+// step's ~45 launches once per 256 tokens; at 4096 columns the same launches carry 16 times the work.
+
+// The narrowest column set that holds `n` columns (n <= kColMax).
+static int cols_get(mlb_session* s, int n, mlb_session** out) {
+    int i = 0;
+    while ((kColMin << i) < n) ++i;
+    if (!s->cols[i]) {
+        int rc = session_create(s->m, kColMin << i, s->max_ctx, 0, 0, s, &s->cols[i]);
+        if (rc) { s->cols[i] = nullptr; return rc; }
+    }
+    *out = s->cols[i];
+    return MLB_OK;
+}
+
 // score_out != null: the scoring forward instead (mlb_score_tokens): every token of sequence 0 is a
 // column, the LM head runs on the columns too, and the logits of each chunk go to score_out.
 static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t* lens, int stride, bool* done, float* score_out = nullptr) {
@@ -1771,74 +1299,96 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     long total = 0;
     for (int b = 0; b < B; ++b) total += lens[b] - keep;
     if (total < 1 || (mode == "auto" && total < 64)) return MLB_OK;
-    if (s->m->cfg.weight_dtype != MLB_DT_BF16 && s->m->cfg.weight_dtype != MLB_DT_FP8_E4M3) {
+    const mlb_config& cfg = s->m->cfg;
+    if (cfg.weight_dtype != MLB_DT_BF16 && cfg.weight_dtype != MLB_DT_FP8_E4M3) {
         if (mode == "chunk") return fail(MLB_E_UNSUPPORTED, "MLB_PREFILL=chunk needs bf16 or FP8 weights");
         return MLB_OK;
     }
-    if (!s->cols && !s->cols_tried) {
-        s->cols_tried = true;
-        int rc = session_create(s->m, kPromptCols, s->max_ctx, 0, 0, s, &s->cols);
-        if (rc) {
-            s->cols = nullptr;
-            if (mode == "chunk") return rc;
-        }
-    }
-    mlb_session* cs = s->cols;
-    if (!cs) return MLB_OK;
-    const int T = cs->B, MP = s->max_pages;
     int rc;
-    if ((rc = ensure_graph(cs, kind))) return rc;
-    const size_t V = (size_t)s->m->cfg.vocab;
+    mlb_session* cs = nullptr;
+    if (s->cols_failed && mode != "chunk") return MLB_OK;
+    if ((rc = cols_get(s, (int)std::min<long>(total, kColMax), &cs))) {
+        s->cols_failed = true;
+        return mode == "chunk" ? rc : (int)MLB_OK;
+    }
+    if (!s->plan_host) {
+        s->plan_host_ints = cols_layout(cfg, s->B, kColMax).ints;
+        CU(cudaMallocHost((void**)&s->plan_host, kPlanSlots * s->plan_host_ints * 4));
+        for (auto& e : s->plan_free) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    const size_t V = (size_t)cfg.vocab;
+    const int qt = attn_cols_queries(cfg.heads / cfg.kv_heads);
     size_t scored = 0;
-    std::vector<int> h_tok(T), h_pos(T), h_lim(T), h_seq(T), h_tab((size_t)T * MP);
     // A chunk takes the next tokens of as many sequences as it can, an equal share each: the
-    // delta-net recurrence is serial along a sequence and parallel across sequences, so 64 sequences
-    // with 2 columns each beat 1 sequence with 128. Columns stay grouped by sequence, positions ascending.
+    // delta-net recurrence is serial along a sequence and parallel across sequences. Columns stay grouped by
+    // sequence, positions ascending.
     std::vector<int> cursor(B, 0);
     long left = total;
-    while (left > 0) {
-        int n_active = 0;
-        for (int b = 0; b < B; ++b) n_active += cursor[b] < lens[b] - keep ? 1 : 0;
-        const int share = std::max(1, T / n_active);
-        int n = 0;
-        for (int b = 0; b < B && n < T; ++b) {
-            const int take = std::min(std::min(share, lens[b] - keep - cursor[b]), T - n);
+    for (int slot = 0, used = 0; left > 0; slot = (slot + 1) % kPlanSlots, ++used) {
+        const int want = (int)std::min<long>(left, kColMax);
+        if ((rc = cols_get(s, want, &cs))) return rc;
+        if (kind == CHAIN_GREEDY && !cs->logits && (rc = sess_alloc(cs, (void**)&cs->logits, (size_t)cs->B * V * 4, false))) return rc;
+        if ((rc = ensure_graph(cs, kind))) return rc;
+        // the largest equal share that fits; what is left over goes to the first sequences
+        int lo = 0, hi = want;
+        auto filled = [&](int share) {
+            long n = 0;
+            for (int b = 0; b < B; ++b) n += std::min(share, lens[b] - keep - cursor[b]);
+            return n;
+        };
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (filled(mid) <= want) lo = mid; else hi = mid - 1;
+        }
+        int extra = want - (int)filled(lo);
+        const ColsLayout lay = cols_layout(cfg, s->B, cs->B);
+        int* pl = s->plan_host + slot * s->plan_host_ints;
+        if (used >= kPlanSlots) CU(cudaEventSynchronize(s->plan_free[slot]));
+        int n = 0, runs = 0, tiles = 0;
+        for (int b = 0; b < B; ++b) {
+            const int rest = lens[b] - keep - cursor[b];
+            int take = std::min(rest, lo);
+            if (extra > 0 && take < rest) { ++take; --extra; }
+            if (take <= 0) continue;
+            int* r = pl + lay.runs + 4 * (size_t)runs++;
+            r[0] = n; r[1] = take; r[2] = b; r[3] = cursor[b];
+            for (int q = 0; q < take; q += qt) {
+                int* t = pl + lay.tiles + 4 * (size_t)tiles++;
+                t[0] = n + q; t[1] = std::min(qt, take - q); t[2] = b; t[3] = cursor[b] + q;
+            }
             for (int i = 0; i < take; ++i, ++n) {
                 const int t = cursor[b] + i;
-                h_tok[n] = tokens[(size_t)b * stride + t];
-                h_pos[n] = t;
-                h_lim[n] = t + 1;        // active: pos < limit
-                h_seq[n] = b;
-                std::memcpy(&h_tab[(size_t)n * MP], &s->h_table[(size_t)b * MP], (size_t)MP * 4);
+                pl[lay.tok + n] = tokens[(size_t)b * stride + t];
+                pl[lay.pos + n] = t;
+                pl[lay.lim + n] = t + 1;        // active: pos < limit
+                pl[lay.seq + n] = b;
             }
-            if (take > 0) cursor[b] += take;
+            cursor[b] += take;
         }
+        for (int i = n; i < cs->B; ++i) pl[lay.tok + i] = pl[lay.pos + i] = pl[lay.lim + i] = pl[lay.seq + i] = 0;      // idle columns
+        pl[0] = n; pl[1] = runs; pl[2] = tiles; pl[3] = 0;
         left -= n;
-        for (int i = n; i < T; ++i) { h_tok[i] = 0; h_pos[i] = 0; h_lim[i] = 0; h_seq[i] = 0; }      // idle columns
-        CU(cudaMemcpyAsync(cs->tok, h_tok.data(), (size_t)T * 4, cudaMemcpyHostToDevice, s->stream));
-        CU(cudaMemcpyAsync(cs->pos, h_pos.data(), (size_t)T * 4, cudaMemcpyHostToDevice, s->stream));
-        CU(cudaMemcpyAsync(kind == CHAIN_PREFILL ? cs->limit_prefill : cs->limit_decode, h_lim.data(), (size_t)T * 4, cudaMemcpyHostToDevice, s->stream));
-        CU(cudaMemcpyAsync(cs->seq_of, h_seq.data(), (size_t)T * 4, cudaMemcpyHostToDevice, s->stream));
-        CU(cudaMemcpyAsync(cs->page_table, h_tab.data(), h_tab.size() * 4, cudaMemcpyHostToDevice, s->stream));
+        CU(cudaMemcpyAsync(cs->plan_dev, pl, lay.ints * 4, cudaMemcpyHostToDevice, s->stream));
+        CU(cudaEventRecord(s->plan_free[slot], s->stream));
         CU(cudaGraphLaunch(cs->graphs[kind], s->stream));
         if (score_out) {
             // one sequence: the columns of a chunk are its next n positions, in order
             CU(cudaMemcpyAsync(score_out + scored * V, cs->logits, (size_t)n * V * 4, cudaMemcpyDeviceToHost, s->stream));
             scored += (size_t)n;
         }
-        CU(cudaStreamSynchronize(s->stream));          // the host arrays are rewritten for the next chunk
+        if ((rc = queue_err_readback(cs))) return rc;
     }
     if (!score_out) {
         // what the token loop would have left: position len-1 with the last prompt token pending
-        std::vector<int> pos(B), last(B);
-        for (int i = 0; i < B; ++i) { pos[i] = lens[i] - 1; last[i] = tokens[(size_t)i * stride + lens[i] - 1]; }
-        CU(cudaMemcpyAsync(s->pos, pos.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
-        CU(cudaMemcpyAsync(s->tok, last.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
+        for (int i = 0; i < B; ++i) { s->pinned_out[i] = lens[i] - 1; s->pinned_tok[i] = tokens[(size_t)i * stride + lens[i] - 1]; }
+        CU(cudaMemcpyAsync(s->pos, s->pinned_out, (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
+        CU(cudaMemcpyAsync(s->tok, s->pinned_tok, (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
     }
-    if ((rc = queue_err_readback(cs))) return rc;
     CU(cudaStreamSynchronize(s->stream));
     *done = true;
-    return check_err_readback(cs);
+    for (auto* c2 : s->cols)
+        if (c2 && (rc = check_err_readback(c2))) return rc;
+    return MLB_OK;
 }
 
 extern "C" int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t* lens, int stride) {
@@ -1856,16 +1406,9 @@ extern "C" int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t*
         }
         max_len = std::max(max_len, lens[b]);
     }
-    int rc = mlb_session_reset(s);
+    int rc = reset_queued(s);
     if (rc) return rc;
-    std::vector<int> hp((size_t)B * s->max_ctx, 0), first(B), lim(B);
-    for (int b = 0; b < B; ++b) {
-        std::memcpy(&hp[(size_t)b * s->max_ctx], &tokens[(size_t)b * stride], (size_t)lens[b] * 4);
-        first[b] = tokens[(size_t)b * stride];
-        lim[b] = lens[b] - 1;
-    }
     // pages for the whole prompt before any launch
-    for (int b = 0; b < B; ++b) s->h_pos[b] = 0;
     bool has_attn = false;
     for (auto* p : s->kpool) if (p) has_attn = true;
     if (has_attn) {
@@ -1875,21 +1418,28 @@ extern "C" int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t*
         s->table_dirty = true;
         if ((rc = sync_page_table(s))) return rc;
     }
-    CU(cudaMemcpyAsync(s->prompt, hp.data(), hp.size() * 4, cudaMemcpyHostToDevice, s->stream));
-    CU(cudaMemcpyAsync(s->tok, first.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
-    CU(cudaMemcpyAsync(s->limit_prefill, lim.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
-    CU(cudaStreamSynchronize(s->stream));
     bool by_columns = false;
     if ((rc = prefill_columns(s, tokens, lens, stride, &by_columns))) return rc;
-    if (!by_columns && max_len > 1) {
-        if ((rc = ensure_graph(s, CHAIN_PREFILL))) return rc;
-        for (int t = 0; t < max_len - 1; ++t)
-            if ((rc = launch_step(s, CHAIN_PREFILL))) return rc;
+    if (!by_columns) {
+        std::vector<int> hp((size_t)B * s->max_ctx, 0), first(B), lim(B);
+        for (int b = 0; b < B; ++b) {
+            std::memcpy(&hp[(size_t)b * s->max_ctx], &tokens[(size_t)b * stride], (size_t)lens[b] * 4);
+            first[b] = tokens[(size_t)b * stride];
+            lim[b] = lens[b] - 1;
+        }
+        CU(cudaMemcpyAsync(s->prompt, hp.data(), hp.size() * 4, cudaMemcpyHostToDevice, s->stream));
+        CU(cudaMemcpyAsync(s->tok, first.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
+        CU(cudaMemcpyAsync(s->limit_prefill, lim.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s->stream));
+        if (max_len > 1) {
+            if ((rc = ensure_graph(s, CHAIN_PREFILL))) { cudaStreamSynchronize(s->stream); return rc; }
+            for (int t = 0; t < max_len - 1; ++t)
+                if ((rc = launch_step(s, CHAIN_PREFILL))) { cudaStreamSynchronize(s->stream); return rc; }
+        }
+        if ((rc = queue_err_readback(s))) { cudaStreamSynchronize(s->stream); return rc; }
+        CU(cudaStreamSynchronize(s->stream));
     }
-    if ((rc = queue_err_readback(s))) return rc;
-    CU(cudaStreamSynchronize(s->stream));
     for (int b = 0; b < B; ++b) s->h_pos[b] = lens[b] - 1;
-    return check_err_readback(s);
+    return by_columns ? (int)MLB_OK : check_err_readback(s);
 }
 
 extern "C" int mlb_score_tokens(mlb_session* s, const int32_t* tokens, int len, float* logits_out) {

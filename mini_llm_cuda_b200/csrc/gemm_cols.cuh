@@ -1,0 +1,464 @@
+// Projections of many prompt columns on the 5th-generation tensor cores: Y[c][n] = sum_k X[c][k] W[n][k], bf16 operands,
+// fp32 accumulation in tensor memory, persistent CTAs.
+//
+// A decode batch is at most a few tiles wide and gemm_tc.cuh gives its MMA rows to the weights. A prompt chunk has up to
+// 4096 columns, so here the columns are the MMA's M = 128 and BN weight rows its N: a thread of the epilogue then owns
+// one column (token), and what the step does per token - the 1/rms scale, QK norm over a head, RoPE pairs, the K/V row,
+// the sum of squares for the next norm - stays in its registers; every thread reads and writes whole 32- or 64-byte
+// pieces of its token's row.
+//   warp 0     TMA loader: [128 x 64] activation tile and [BN x 64] weight tile (gate and up halves for SwiGLU) per stage
+//   warp 1     MMA issuer: tcgen05.mma M128 x BN x K16, four per stage, into one of two accumulators
+//   warps 2-9  epilogue of the other accumulator: two warps per TMEM lane quarter, half of the columns each
+// One CTA per SM walks tiles of the output; the epilogue of a tile runs under the k-loop of the next one where tensor
+// memory holds the accumulators twice.
+// FP8 weights come as an exact bf16 copy of their codes; their row scales are applied to the accumulator, and the bf16
+// per-layer-embedding operand that rides behind the down projection has an accumulator of its own.
+//
+// The results are gemm_tc_kernel's to the last bit: behind every layer the activations are rounded to bf16, so sums taken
+// in another order end, some layers later, in other roundings and now and then in another token. That kernel splits the
+// k-blocks of a tile over the CTAs of a cluster and adds their partial accumulators in order; here the same ranges of
+// k-blocks go to accumulators of their own (`split`), and the sums of squares are taken over 32 features at a time in the
+// order of its warp shuffles.
+// Every mbarrier wait is bounded; one that runs out records a code and the CTA drains without waiting further.
+#pragma once
+#include "gemm_tc.cuh"
+
+namespace mlb {
+
+constexpr int kGcM = 128;
+constexpr int kGcEpiWarps = 8;
+constexpr int kGcThreads = 64 + 32 * kGcEpiWarps;
+constexpr int kGcMaxStages = 8;
+constexpr size_t kGcSmem = 224 * 1024;
+
+struct GemmColsParams {
+    int N, K, BN;                  // output features (SWIGLU: of h), width of the main operands, MMA N
+    int stages, nkb_x;             // ring depth; k-blocks taken from the second operand pair
+    int split, mains, exts;        // ranges of k-blocks; of them, how many hold k-blocks of the main pair / of a second pair that
+                                   // accumulates separately (scaled weights; 0: it shares the main accumulators)
+    int nbuf;                      // sets of accumulators in tensor memory: 2 = epilogue under the next k-loop
+    uint32_t tmem_cols;
+    int early_w;                   // weight tiles may be fetched before the predecessor kernel has finished
+    float* y;                      // RAW: fp32 [c][N]; RESID: residual stream, updated in place
+    bf16_t* h16;                   // SWIGLU: bf16 [c][N]
+    const float* ssq_in; int ssq_parts; float eps;      // deferred RMS norm, as in GemmTcParams
+    bf16_t* xg16; const float* gain_next; float* ssq_out;      // sums of squares of 32 features each: [c][ssq_parts], a multiple of 4
+    const float *s1, *s2;          // row scales of FP8 weights (SWIGLU: gate, up), or null
+    int* err;
+};
+
+// 32 bytes per thread: one whole sector, so that rows of different tokens do not cost partial sectors
+__device__ __forceinline__ void st_f32x8(float* p, const float* v) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
+                 "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void ld_f32x8(const float* p, float* v) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t gc_pack(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ void st_bf16x16(bf16_t* p, const float* v) {
+    uint4 a, b;
+    a.x = gc_pack(v[0], v[1]); a.y = gc_pack(v[2], v[3]); a.z = gc_pack(v[4], v[5]); a.w = gc_pack(v[6], v[7]);
+    b.x = gc_pack(v[8], v[9]); b.y = gc_pack(v[10], v[11]); b.z = gc_pack(v[12], v[13]); b.w = gc_pack(v[14], v[15]);
+    reinterpret_cast<uint4*>(p)[0] = a;
+    reinterpret_cast<uint4*>(p)[1] = b;
+}
+__device__ __forceinline__ void put16(float* p, const float* v) { st_f32x8(p, v); st_f32x8(p + 8, v + 8); }
+__device__ __forceinline__ void put16(bf16_t* p, const float* v) { st_bf16x16(p, v); }
+// 16 per-feature values, the same for every lane
+__device__ __forceinline__ void ld_feat16(const float* p, float* v) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p) + i);
+        v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+    }
+}
+
+template <int MODE, typename KVT>
+__global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
+                                                                  const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmXx,
+                                                                  const __grid_constant__ CUtensorMap tmWx, const __grid_constant__ GemmColsParams p,
+                                                                  const __grid_constant__ StepCtl c, const __grid_constant__ QkvPostParams q) {
+    extern __shared__ unsigned char smem_raw[];
+    const int n_cols = *c.n_cols;                                  // in place before the step's first kernel starts
+    const int bn_out = MODE == TC_SWIGLU ? p.BN / 2 : p.BN;
+    const int n_m = (n_cols + kGcM - 1) / kGcM, n_n = (p.N + bn_out - 1) / bn_out;
+    const int n_tiles = n_m * n_n;
+    if ((int)blockIdx.x >= n_tiles) return;
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t bars[2 * kGcMaxStages + 4];
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8u * kGcMaxStages;
+    const uint32_t tfull0 = empty0 + 8u * kGcMaxStages, tempty0 = tfull0 + 16u;
+    const int a_bytes = kGcM * 128, stage_bytes = a_bytes + p.BN * 128;
+    const int nkb1 = (p.K + kTcKB - 1) / kTcKB, nkb = nkb1 + p.nkb_x;
+    const uint32_t acc_cols = (uint32_t)((p.mains + p.exts) * p.BN);
+    if (tid == 0) {
+        for (int i = 0; i < p.stages; ++i) {
+            mbar_init(full0 + 8u * i, 1);
+            mbar_init(empty0 + 8u * i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(tfull0 + 8u * i, 1);
+            mbar_init(tempty0 + 8u * i, kGcEpiWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(p.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            auto load_w = [&](int kb, int n0, uint32_t base, uint32_t bar) {
+                if (kb < nkb1) {
+                    tma_load_2d(base + a_bytes, &tmW, kb * kTcKB, n0, bar);
+                    if (MODE == TC_SWIGLU) tma_load_2d(base + a_bytes + bn_out * 128, &tmW2, kb * kTcKB, n0, bar);
+                } else {
+                    tma_load_2d(base + a_bytes, &tmWx, (kb - nkb1) * kTcKB, n0, bar);
+                }
+            };
+            auto load_x = [&](int kb, int m0, uint32_t base, uint32_t bar) {
+                if (kb < nkb1) tma_load_2d(base, &tmX, kb * kTcKB, m0, bar);
+                else tma_load_2d(base, &tmXx, (kb - nkb1) * kTcKB, m0, bar);
+            };
+            const uint32_t ring = smem_u32(smem);
+            // the first tile's first weight tiles depend on nothing: on their way before the predecessor is waited for
+            const int first = blockIdx.x;
+            const int pre = p.early_w ? min(p.stages, nkb) : 0;
+            for (int kb = 0; kb < pre; ++kb) {
+                mbar_expect_tx(full0 + 8u * kb, (uint32_t)stage_bytes);
+                load_w(kb, first / n_m * bn_out, ring + (uint32_t)(kb * stage_bytes), full0 + 8u * kb);
+            }
+            pdl_wait();
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int t = first; t < n_tiles && ok; t += gridDim.x) {
+                const int m0 = t % n_m * kGcM, n0 = t / n_m * bn_out;
+                for (int kb = 0; kb < nkb; ++kb) {
+                    const uint32_t bar = full0 + 8u * s, base = ring + (uint32_t)(s * stage_bytes);
+                    if (t != first || kb >= pre) {
+                        if (!tc_wait(empty0 + 8u * s, ph, p.err, 21)) { ok = false; break; }
+                        mbar_expect_tx(bar, (uint32_t)stage_bytes);
+                        load_w(kb, n0, base, bar);
+                    }
+                    load_x(kb, m0, base, bar);
+                    if (++s == p.stages) { s = 0; ph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = umma_idesc_bf16(kGcM, p.BN);
+            const uint32_t ring = smem_u32(smem);
+            int s = 0, i = 0, buf = 0, use = 0;        // use: how often this buffer has been filled before
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++i) {
+                if (i >= p.nbuf && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t acc = tmem + buf * acc_cols;
+                int r = 0, hi = nkb / p.split;           // range of k-blocks: [nkb r / split, nkb (r + 1) / split)
+                bool fresh = true, xfresh = true;        // the next MMA starts its accumulator
+                for (int kb = 0; kb < nkb; ++kb) {
+                    while (kb >= hi) {
+                        ++r;
+                        hi = (int)((long)nkb * (r + 1) / p.split);
+                        fresh = xfresh = true;
+                    }
+                    if (!tc_wait(full0 + 8u * s, ph, p.err, 23)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t base = ring + (uint32_t)(s * stage_bytes);
+                    const uint64_t ad = umma_desc_sw128(base), bd = umma_desc_sw128(base + a_bytes);
+                    const bool ext = p.exts > 0 && kb >= nkb1;
+                    // the separate accumulators of the second pair lie behind the main ones, its ranges are the last ones
+                    const uint32_t dst = acc + (uint32_t)((ext ? p.mains + r - (p.split - p.exts) : r) * p.BN);
+                    const bool first = ext ? xfresh : fresh;
+#pragma unroll
+                    for (int j = 0; j < kTcKB / 16; ++j) umma_bf16(dst, ad + 2u * j, bd + 2u * j, idesc, (first && j == 0) ? 0u : 1u);
+                    if (ext) xfresh = false; else fresh = false;
+                    umma_commit(empty0 + 8u * s);
+                    if (++s == p.stages) { s = 0; ph ^= 1u; }
+                }
+                umma_commit(tfull0 + 8u * buf);      // also after a wait that ran out: the epilogue must not hang on it
+                if (++buf == p.nbuf) { buf = 0; ++use; }
+            }
+        }
+    } else {
+        // ---- epilogue: one token per thread, half of the tile's columns per warp ---------------------------------
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const int span = bn_out / 2;                  // features of this thread per tile, in chunks of 16
+        pdl_wait();
+        int buf = 0, use = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            const int m0 = t % n_m * kGcM, n0 = t / n_m * bn_out;
+            const int tok = m0 + quarter * 32 + lane;
+            const bool live = tok < n_cols;
+            const int f_begin = n0 + half * span;
+            float rinv = 1.0f;
+            if (p.ssq_in != nullptr && live) {
+                float tot = 0.f;
+                const float4* sp = reinterpret_cast<const float4*>(p.ssq_in + (size_t)tok * p.ssq_parts);
+                for (int j = 0; j < p.ssq_parts / 4; ++j) {
+                    const float4 x = __ldcg(sp + j);
+                    tot += (x.x + x.y) + (x.z + x.w);
+                }
+                rinv = 1.0f / sqrtf(tot / (float)p.K + p.eps);
+            }
+            int pos = 0;
+            size_t kv_row = 0;                        // row of the token in this layer's pools, for kv head 0
+            if (MODE == TC_QKV && live) {
+                pos = c.pos[tok];
+                const int page = q.page_table[kv_seq(c, tok) * q.pt_stride + pos / kKvBlock];
+                kv_row = (size_t)page * q.kv_heads * kKvBlock + (pos % kKvBlock);
+            }
+            float rnext[16];
+            auto load_resid = [&](int f0) {
+                if (live && f0 < p.N) {               // N is a multiple of 8, chunks end inside it only at 8
+                    const float* r = p.y + (size_t)tok * p.N + f0;
+                    ld_f32x8(r, rnext);
+                    if (f0 + 8 < p.N) ld_f32x8(r + 8, rnext + 8);
+                }
+            };
+            if (MODE == TC_RESID) load_resid(f_begin);
+            if (!tc_wait(tfull0 + 8u * buf, (uint32_t)use & 1u, p.err, 24)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t acc = tmem + buf * acc_cols + lane_base;
+            float head_sc = 1.0f, sqp[16];
+            // 16 columns of the sum of `n` accumulators, in their order
+            auto load_acc = [&](uint32_t col, int n, float* o) {
+                uint32_t ta[16];
+                tmem_ld16_issue(col, ta);
+                if (n == 1) {
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) o[j] = __uint_as_float(ta[j]);
+                    return;
+                }
+                uint32_t tb[16];
+                tmem_ld16_issue(col + (uint32_t)p.BN, tb);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) o[j] = __uint_as_float(ta[j]) + __uint_as_float(tb[j]);
+                for (int r = 2; r < n; ++r) {
+                    tmem_ld16_issue(col + (uint32_t)(r * p.BN), ta);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) o[j] += __uint_as_float(ta[j]);
+                }
+            };
+            // sum of 16 + 16 values in the order of warp_colsum16
+            auto sum32 = [](const float* x, const float* y) {
+                float t[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) t[j] = x[j] + y[j];
+#pragma unroll
+                for (int w = 8; w >= 1; w >>= 1)
+#pragma unroll
+                    for (int j = 0; j < w; ++j) t[j] += t[j + w];
+                return t[0];
+            };
+            for (int cc = 0; cc < span; cc += 16) {
+                const int f0 = f_begin + cc, col = half * span + cc;
+                if (f0 >= p.N) {                       // uniform for the warp; the sums of squares behind the last feature are zero
+                    if (MODE == TC_RESID) {
+                        if ((f0 & 16) && live) {
+                            float z[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) z[j] = 0.f;
+                            p.ssq_out[(size_t)tok * p.ssq_parts + f0 / 32] = sum32(sqp, z);
+                        }
+                        if (live)
+                            for (int g = (f0 + 16) / 32; g < (f_begin + span) / 32 && g < p.ssq_parts; ++g) p.ssq_out[(size_t)tok * p.ssq_parts + g] = 0.f;
+                    }
+                    break;
+                }
+                const bool whole = f0 + 16 <= p.N;
+                __syncwarp();                          // tcgen05.ld is a warp-wide instruction
+                float v[16], w2[16];
+                load_acc(acc + (uint32_t)col, p.mains, v);
+                if (MODE == TC_SWIGLU) load_acc(acc + (uint32_t)(bn_out + col), p.mains, w2);
+                if (MODE == TC_RESID && p.exts > 0) load_acc(acc + (uint32_t)(p.mains * p.BN + col), p.exts, w2);
+                if (MODE == TC_SWIGLU) {
+                    float sa[16], sb[16];
+                    if (p.s1 != nullptr && whole) {
+                        ld_feat16(p.s1 + f0, sa);
+                        ld_feat16(p.s2 + f0, sb);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int f = min(f0 + j, p.N - 1);
+                            sa[j] = p.s1 != nullptr ? __ldg(p.s1 + f) : 1.0f;
+                            sb[j] = p.s2 != nullptr ? __ldg(p.s2 + f) : 1.0f;
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float g = v[j] * sa[j] * rinv, u = w2[j] * sb[j] * rinv;
+                        v[j] = __fdividef(g, 1.0f + __expf(-g)) * u;            // inference.cu:262-281
+                    }
+                    if (live) {
+                        bf16_t* o = p.h16 + (size_t)tok * p.N + f0;
+                        if (whole) {
+                            st_bf16x16(o, v);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (f0 + j < p.N) o[j] = __float2bfloat16_rn(v[j]);
+                        }
+                    }
+                    continue;
+                }
+                float sa[16];
+                if (p.s1 != nullptr) {
+                    if (whole) {
+                        ld_feat16(p.s1 + f0, sa);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sa[j] = __ldg(p.s1 + min(f0 + j, p.N - 1));
+                    }
+                    if (MODE != TC_RESID) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] *= sa[j];
+                    }
+                }
+                if (MODE == TC_RAW) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] *= rinv;
+                    if (live) {
+                        float* o = p.y + (size_t)tok * p.N + f0;
+                        if (whole && (p.N & 7) == 0) {
+                            put16(o, v);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (f0 + j < p.N) o[j] = v[j];
+                        }
+                    }
+                } else if (MODE == TC_RESID) {
+                    float r[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[j] = rnext[j];
+                    if (cc + 16 < span) load_resid(f0 + 16);
+                    // (roundings as in gemm_tc_kernel: scale and second pair in one fma, then the residual)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (p.s1 != nullptr) v[j] = fmaf(v[j], sa[j], p.exts > 0 ? w2[j] : 0.f);
+                        v[j] = __fadd_rn(v[j], r[j]);                           // inference.cu:252-260, :283-291
+                    }
+                    if (live) {
+                        float g[16];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            // N is a multiple of 8: a chunk ends inside the matrix after 8 or 16 features
+                            const float4 t4 = (whole || j < 2) ? __ldg(reinterpret_cast<const float4*>(p.gain_next + f0) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            g[4 * j] = t4.x; g[4 * j + 1] = t4.y; g[4 * j + 2] = t4.z; g[4 * j + 3] = t4.w;
+                        }
+                        float* o = p.y + (size_t)tok * p.N + f0;
+                        bf16_t* ox = p.xg16 + (size_t)tok * p.N + f0;
+                        st_f32x8(o, v);
+                        uint4 a;
+                        a.x = gc_pack(v[0] * g[0], v[1] * g[1]); a.y = gc_pack(v[2] * g[2], v[3] * g[3]);
+                        a.z = gc_pack(v[4] * g[4], v[5] * g[5]); a.w = gc_pack(v[6] * g[6], v[7] * g[7]);
+                        reinterpret_cast<uint4*>(ox)[0] = a;
+                        if (whole) {
+                            st_f32x8(o + 8, v + 8);
+                            a.x = gc_pack(v[8] * g[8], v[9] * g[9]); a.y = gc_pack(v[10] * g[10], v[11] * g[11]);
+                            a.z = gc_pack(v[12] * g[12], v[13] * g[13]); a.w = gc_pack(v[14] * g[14], v[15] * g[15]);
+                            reinterpret_cast<uint4*>(ox)[1] = a;
+                        }
+                    }
+                    float sq[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sq[j] = (whole || j < 8) ? __fmul_rn(v[j], v[j]) : 0.f;
+                    if (f0 & 16) {
+                        if (live) p.ssq_out[(size_t)tok * p.ssq_parts + f0 / 32] = sum32(sqp, sq);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sqp[j] = sq[j];
+                    }
+                } else {
+                    // q | k | v | gate: whole heads of 64 or 128 features each
+                    const int seg_k = q.nq, seg_v = q.nq + q.nk, seg_g = seg_v + q.nv;
+                    const int seg = f0 < seg_k ? 0 : (f0 < seg_v ? 1 : (f0 < seg_g ? 2 : 3));
+                    const int fs = f0 - (seg == 0 ? 0 : (seg == 1 ? seg_k : (seg == 2 ? seg_v : seg_g)));     // feature inside its segment
+                    const int e0 = fs % q.hd, head = fs / q.hd;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] *= rinv;
+                    if (seg < 2 && q.qk_norm) {
+                        // per-head RMS norm (inference.cu:52-81, :97-111): the head's other features come from tensor memory
+                        if (e0 == 0 || cc == 0) {
+                            float ss = 0.f;
+                            for (int e = 0; e < q.hd; e += 32) {
+                                float x[2][16];
+#pragma unroll
+                                for (int b = 0; b < 2; ++b) {
+                                    load_acc(acc + (uint32_t)(col - e0 + e + 16 * b), p.mains, x[b]);
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j) {
+                                        if (p.s1 != nullptr) x[b][j] *= __ldg(p.s1 + f0 - e0 + e + 16 * b + j);
+                                        x[b][j] *= rinv;
+                                        x[b][j] = __fmul_rn(x[b][j], x[b][j]);
+                                    }
+                                }
+                                ss += sum32(x[0], x[1]);
+                            }
+                            head_sc = rsqrtf(ss * (1.0f / (float)q.hd) + q.eps);
+                        }
+                        float g[16];
+                        ld_feat16((seg == 0 ? q.gq : q.gk) + fs, g);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] *= head_sc * g[j];
+                    }
+                    if (live) {
+                        if (seg < 2) {
+                            // RoPE on adjacent pairs (inference.cu:113-134)
+                            float r[16];
+                            const float* rp = q.rope + (size_t)pos * q.hd + e0;
+                            ld_feat16(rp, r);
+#pragma unroll
+                            for (int j = 0; j < 16; j += 2) {
+                                const float a = v[j], b = v[j + 1];
+                                v[j] = fmaf(r[j], a, -(r[j + 1] * b));
+                                v[j + 1] = fmaf(r[j + 1], a, r[j] * b);
+                            }
+                        }
+                        if (seg == 0) put16(q.qbuf + (size_t)tok * q.nq + fs, v);
+                        else if (seg == 1) put16(reinterpret_cast<KVT*>(q.kpool) + (kv_row + (size_t)head * kKvBlock) * q.hd + e0, v);
+                        else if (seg == 2) put16(reinterpret_cast<KVT*>(q.vpool) + (kv_row + (size_t)head * kKvBlock) * q.hd + e0, v);
+                        else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = __fdividef(1.0f, 1.0f + __expf(-v[j]));      // inference.cu:248
+                            put16(q.gbuf + (size_t)tok * q.ng + fs, v);
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty0 + 8u * buf);
+            if (++buf == p.nbuf) { buf = 0; ++use; }
+        }
+    }
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
+}
+
+}  // namespace mlb

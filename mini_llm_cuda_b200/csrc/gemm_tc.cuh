@@ -248,6 +248,9 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
                                                        const __grid_constant__ CUtensorMap tmAx,
                                                        const __grid_constant__ CUtensorMap tmBx, GemmTcParams p,
                                                        StepCtl c, QkvPostParams q) {
+    // prompt columns: a tile behind the last column that carries a token has nothing to do (all CTAs of a cluster
+    // agree; the tiles that do work order this launch behind its predecessor)
+    if (c.n_cols != nullptr && (int)blockIdx.y * p.Nb >= *c.n_cols) return;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const bool tracing = p.trace != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
@@ -457,7 +460,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
                 int pos = -1, page = 0;
                 if (seq_active(c, b)) {
                     pos = c.pos[b];
-                    page = q.page_table[(size_t)b * q.pt_stride + pos / kKvBlock];
+                    page = q.page_table[kv_seq(c, b) * q.pt_stride + pos / kKvBlock];
                 }
                 pos_s[j] = pos;
                 page_s[j] = page;

@@ -130,7 +130,14 @@ struct StepCtl {
     int* host_out;       // [B] picked ids, written where the sequence advances
     int* host_err;       // copy of *dev_err at the end of the step
     const int* dev_err;
+    // prompt columns: the sequence whose page-table row and state a column uses, and (first word) how many columns
+    // of the launch carry a token (the rest lie behind them); null in a decode session, where column = sequence
+    const int* seq_of;
+    const int* n_cols;
 };
+
+// row of the page table that column b's K/V rows live in
+__device__ __forceinline__ size_t kv_seq(const StepCtl& c, int b) { return (size_t)(c.seq_of != nullptr ? c.seq_of[b] : b); }
 
 __device__ __forceinline__ bool seq_active(const StepCtl& c, int b) {
     return b < c.B && c.pos[b] < c.limit[b];
@@ -157,6 +164,17 @@ __device__ __forceinline__ void advance_seq(const StepCtl& c, int b, int sampled
         if (sampled == c.stop_token) c.limit[b] = p + 1;          // end of this sequence: later steps skip it
     }
     c.pos[b] = p + 1;
+}
+
+// State of a session without tokens.
+static __global__ void session_reset_kernel(int B, int max_ctx, int* pos, int* tok, int* limit_prefill, int* limit_decode, int* out_idx) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= B) return;
+    pos[b] = 0;
+    tok[b] = 0;
+    limit_prefill[b] = 0;
+    limit_decode[b] = max_ctx;       // a sequence that stopped had it lowered
+    out_idx[b] = 0;
 }
 
 // Prefill chain has no LM head: a one-thread-per-sequence advance.
@@ -550,7 +568,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(StepCtl c, GemvParams p) {
                     p.qbuf[(size_t)bg * p.nq + srow + 1] = rc;
                 } else {
                     int kvh = srow / hd;
-                    int page = p.page_table[(size_t)bg * p.pt_stride + pos / kKvBlock];
+                    int page = p.page_table[kv_seq(c, bg) * p.pt_stride + pos / kKvBlock];
                     size_t off = (((size_t)page * p.kv_heads + kvh) * kKvBlock + (pos % kKvBlock)) * hd + e;
                     Elem<KVT>::put(kpool, off, ra);
                     Elem<KVT>::put(kpool, off + 1, rc);
@@ -558,7 +576,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(StepCtl c, GemvParams p) {
             } else if (seg == 2) {
                 int srow = row - seg_k;
                 int kvh = srow / hd, e = srow % hd;
-                int page = p.page_table[(size_t)bg * p.pt_stride + pos / kKvBlock];
+                int page = p.page_table[kv_seq(c, bg) * p.pt_stride + pos / kKvBlock];
                 size_t off = (((size_t)page * p.kv_heads + kvh) * kKvBlock + (pos % kKvBlock)) * hd + e;
                 Elem<KVT>::put(vpool, off, a);
                 Elem<KVT>::put(vpool, off + 1, cc);
@@ -724,7 +742,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(StepCtl c, AttnParams 
     // (refreshed every 32 pages), so that the page loop does not start with a dependent load.
     constexpr int ITERS = kKvBlock / PPI;
     constexpr int CH = ITERS < 4 ? ITERS : 4;      // positions per lane group handled together
-    const int* pt = p.page_table + (size_t)b * p.pt_stride;
+    const int* pt = p.page_table + kv_seq(c, b) * p.pt_stride;
     const int span = pg_end - pg_begin - warp;
     const int npw = span > 0 ? (span + NW - 1) / NW : 0;
     int pidx = 0;
@@ -1004,142 +1022,6 @@ __global__ void __launch_bounds__(256) delta_net_kernel(StepCtl c, const float* 
             }
         }
     }
-}
-
-// The same update for prompt columns: the columns of a chunk are consecutive tokens of one or
-// several sequences (seq_of[col], grouped by sequence, positions ascending inside a sequence), and
-// the recurrence S_t = f(S_{t-1}) runs over a sequence's columns in order.
-//
-// delta_cols_norm_kernel first turns the raw projections of every (column, head) into what the
-// recurrence consumes - L2-normalised q and k, sigmoid gates - in place, in parallel over columns.
-// grid = (H, columns), block = 64.
-template <int DK>
-__global__ void __launch_bounds__(64) delta_cols_norm_kernel(StepCtl c, float* __restrict__ raw, int raw_stride, int H, int dv,
-                                                             float l2_eps) {
-    constexpr int EPL = DK / 32;
-    const int h = blockIdx.x, col = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    pdl_launch_dependents();
-    pdl_wait();
-    if (!seq_active(c, col)) return;
-    float* r = raw + (size_t)col * raw_stride;
-    float* vec = r + (size_t)(warp == 0 ? 0 : H) * DK + (size_t)h * DK;       // q heads, then k heads
-    float v[EPL], ss = 0.f;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) { v[e] = vec[lane * EPL + e]; ss = fmaf(v[e], v[e], ss); }
-    ss = warp_sum(ss);
-    const float n = sqrtf(ss + l2_eps);
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) vec[lane * EPL + e] = v[e] / n;
-    if (warp == 0 && lane < 2) {
-        float* g = r + (size_t)2 * H * DK + (size_t)H * dv + (size_t)lane * H + h;       // beta[H] then alpha[H]
-        *g = 1.0f / (1.0f + expf(-*g));
-    }
-}
-
-// The recurrence itself. A warp owns 4 rows of one head's state and keeps them in registers
-// across the columns of a sequence; the state is read and written once per sequence and chunk, and
-// the next column's q, k, v and gates are requested while the current one is applied (no block
-// barrier in the loop). The sequences of a chunk are independent: CTA z serves the run of columns
-// that starts at column z, if a sequence starts there, and leaves otherwise.
-// grid = (ceil(dv / 32), H, columns), block = 256.
-template <int DK>
-__global__ void __launch_bounds__(256) delta_net_cols_kernel(StepCtl c, const int* __restrict__ seq_of, int n_cols,
-                                                             const float* __restrict__ raw, int raw_stride, float* __restrict__ state,
-                                                             int H, int dv, float* __restrict__ abuf, bf16_t* __restrict__ abuf16) {
-    constexpr int EPL = DK / 32;
-    constexpr int ROWS_PER_WARP = 4;
-    const int h = blockIdx.y;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    pdl_launch_dependents();
-    pdl_wait();
-    const int row0 = blockIdx.x * (8 * ROWS_PER_WARP) + warp * ROWS_PER_WARP;
-    const int first = blockIdx.z;
-    if (first >= n_cols || !seq_active(c, first)) return;
-    const int cur = seq_of[first];
-    if (first > 0 && seq_active(c, first - 1) && seq_of[first - 1] == cur) return;     // not the start of a run
-    if (row0 >= dv) return;
-    float* Sh = state + ((size_t)cur * H + h) * (size_t)dv * DK;
-    float s[ROWS_PER_WARP][EPL];
-#pragma unroll
-    for (int i = 0; i < ROWS_PER_WARP; ++i) {
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) s[i][e] = 0.f;
-        if (row0 + i < dv) {                     // one vector load per lane and row, as in delta_net_kernel
-            if (EPL == 4) {
-                const float4 t = __ldcg(reinterpret_cast<const float4*>(&Sh[(size_t)(row0 + i) * DK + lane * 4]));
-                s[i][0] = t.x; s[i][1] = t.y; s[i][2 % EPL] = t.z; s[i][3 % EPL] = t.w;
-            } else {
-                const float2 t = __ldcg(reinterpret_cast<const float2*>(&Sh[(size_t)(row0 + i) * DK + lane * 2]));
-                s[i][0] = t.x; s[i][1] = t.y;
-            }
-        }
-    }
-    // one column's inputs: normalised q and k of the head (EPL values per lane), the warp's 4 values
-    // of v, the two gates
-    float qn[EPL], kn[EPL], vr[ROWS_PER_WARP], beta, alpha;
-    auto fetch = [&](int col, float* q_, float* k_, float* v_, float& b_, float& a_) {
-        const float* r = raw + (size_t)col * raw_stride;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) {
-            q_[e] = __ldcg(r + (size_t)h * DK + lane * EPL + e);
-            k_[e] = __ldcg(r + (size_t)H * DK + (size_t)h * DK + lane * EPL + e);
-        }
-#pragma unroll
-        for (int i = 0; i < ROWS_PER_WARP; ++i) v_[i] = row0 + i < dv ? __ldcg(r + (size_t)2 * H * DK + (size_t)h * dv + row0 + i) : 0.f;
-        b_ = __ldcg(r + (size_t)2 * H * DK + (size_t)H * dv + h);
-        a_ = __ldcg(r + (size_t)2 * H * DK + (size_t)H * dv + H + h);
-    };
-    fetch(first, qn, kn, vr, beta, alpha);
-    for (int col = first; col < n_cols; ++col) {
-        const bool more = col + 1 < n_cols && seq_active(c, col + 1) && seq_of[col + 1] == cur;
-        float qx[EPL], kx[EPL], vx[ROWS_PER_WARP], bx = 0.f, ax = 0.f;
-        if (more) fetch(col + 1, qx, kx, vx, bx, ax);
-        float d1[ROWS_PER_WARP], d2[ROWS_PER_WARP];
-#pragma unroll
-        for (int i = 0; i < ROWS_PER_WARP; ++i) {
-            d1[i] = 0.f;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) { s[i][e] *= alpha; d1[i] = fmaf(s[i][e], kn[e], d1[i]); }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int i = 0; i < ROWS_PER_WARP; ++i) d1[i] += __shfl_xor_sync(0xffffffffu, d1[i], o);
-#pragma unroll
-        for (int i = 0; i < ROWS_PER_WARP; ++i) {
-            const float cf = beta * (vr[i] - d1[i]);
-            d2[i] = 0.f;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) { s[i][e] = fmaf(cf, kn[e], s[i][e]); d2[i] = fmaf(s[i][e], qn[e], d2[i]); }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int i = 0; i < ROWS_PER_WARP; ++i) d2[i] += __shfl_xor_sync(0xffffffffu, d2[i], o);
-        if (lane == 0) {
-#pragma unroll
-            for (int i = 0; i < ROWS_PER_WARP; ++i) {
-                if (row0 + i < dv) {
-                    abuf[((size_t)col * H + h) * dv + row0 + i] = d2[i];
-                    if (abuf16) abuf16[((size_t)col * H + h) * dv + row0 + i] = __float2bfloat16_rn(d2[i]);
-                }
-            }
-        }
-        if (!more) break;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) { qn[e] = qx[e]; kn[e] = kx[e]; }
-#pragma unroll
-        for (int i = 0; i < ROWS_PER_WARP; ++i) vr[i] = vx[i];
-        beta = bx;
-        alpha = ax;
-    }
-#pragma unroll
-    for (int i = 0; i < ROWS_PER_WARP; ++i)
-        if (row0 + i < dv) {
-            if (EPL == 4) *reinterpret_cast<float4*>(&Sh[(size_t)(row0 + i) * DK + lane * 4]) = make_float4(s[i][0], s[i][1], s[i][2 % EPL], s[i][3 % EPL]);
-            else *reinterpret_cast<float2*>(&Sh[(size_t)(row0 + i) * DK + lane * 2]) = make_float2(s[i][0], s[i][1]);
-        }
 }
 
 // ------------------------------------------------------------------------------------

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) sgemv_kernel(StepCtl c, GemvPar
                         p.qbuf[(size_t)b * p.nq + srow + 1] = rc;
                     } else {
                         const int kvh = srow / hd;
-                        const int page = p.page_table[(size_t)b * p.pt_stride + pos / kKvBlock];
+                        const int page = p.page_table[kv_seq(c, b) * p.pt_stride + pos / kKvBlock];
                         const size_t off = (((size_t)page * p.kv_heads + kvh) * kKvBlock + (pos % kKvBlock)) * hd + e;
                         Elem<KVT>::put(kpool, off, ra);
                         Elem<KVT>::put(kpool, off + 1, rc);
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kSgThreads, 1) sgemv_kernel(StepCtl c, GemvPar
                 } else if (seg == 2) {
                     const int srow = row - seg_k;
                     const int kvh = srow / hd, e = srow % hd;
-                    const int page = p.page_table[(size_t)b * p.pt_stride + pos / kKvBlock];
+                    const int page = p.page_table[kv_seq(c, b) * p.pt_stride + pos / kKvBlock];
                     const size_t off = (((size_t)page * p.kv_heads + kvh) * kKvBlock + (pos % kKvBlock)) * hd + e;
                     Elem<KVT>::put(vpool, off, a);
                     Elem<KVT>::put(vpool, off + 1, cc);

@@ -1,0 +1,70 @@
+"""Prompt columns at the edges of their tiles: column sets of 64 to 4096, attention tiles of 64 (query, head) rows over
+64-position K/V tiles, delta-net chunks of 4 columns in groups of 16, GEMM tiles of 128 columns; against the oracle."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from helpers import TOL_LOWP, load_oracle, logits_error, oracle_rollout, random_prompts, write_model
+from mini_llm_cuda_b200.model_file import ModelSpec, periodic_layer_types
+
+pytestmark = pytest.mark.gpu
+
+BF16 = dict(weight_dtype="bfloat16", kv_dtype="bfloat16", rms_eps=1e-5, vocab=512)
+SPECS = {
+    "mha64": ModelSpec(dim=128, layers=3, heads=2, head_dim=64, ffn_dim=256, ple_dim=32, layer_types=periodic_layer_types(3, 2), **BF16),
+    "gqa4_128": ModelSpec(dim=256, layers=2, heads=4, kv_heads=1, head_dim=128, ffn_dim=264, qk_norm=True, query_gating=True, **BF16),
+    "gqa8_64": ModelSpec(dim=256, layers=2, heads=8, kv_heads=1, head_dim=64, ffn_dim=256, **BF16),
+    "gqa2_128": ModelSpec(dim=256, layers=2, heads=4, kv_heads=2, head_dim=128, ffn_dim=256, **BF16),
+    # three heads: the rows of the raw delta-net projection start on 8 bytes; 72 value rows end inside a CTA's 64 and 16
+    "dn_odd": ModelSpec(dim=192, layers=2, heads=3, head_dim=64, ffn_dim=256, dn_key_dim=128, dn_value_dim=72,
+                        layer_types=periodic_layer_types(2, 1), **BF16),
+    "fp8": ModelSpec(dim=256, layers=3, heads=4, kv_heads=1, head_dim=64, ffn_dim=272, ple_dim=24, vocab=512, rms_eps=1e-5,
+                     layer_types=periodic_layer_types(3, 3), weight_dtype="float8_e4m3", kv_dtype="bfloat16"),
+}
+
+
+@pytest.fixture(scope="module")
+def api(built_lib):
+    from mini_llm_cuda_b200 import api as _api
+    return _api
+
+
+@pytest.mark.parametrize("name", list(SPECS))
+def test_scored_columns_at_tile_edges(api, tmp_path, name):
+    """Every position's logits of texts of 1 to 1025 tokens (one session: the column sets are made as they are needed)."""
+    spec = dataclasses.replace(SPECS[name], max_context=1040)
+    path = write_model(tmp_path, spec, seed=41)
+    oracle = load_oracle(path)
+    tokens = random_prompts(spec.vocab, [1025], seed=43)[0]
+    st = oracle.new_state()
+    want = np.stack([np.asarray(oracle.step(st, int(t))) for t in tokens])
+    model = api.Model(path)
+    sess = api.Session(model, 1)
+    for length in (1, 2, 15, 17, 63, 64, 65, 127, 128, 129, 1025):
+        got = sess.score(tokens[:length])
+        worst = max(logits_error(got[i], want[i]) for i in range(length))
+        assert worst < TOL_LOWP, (length, worst)
+    sess.close()
+    model.close()
+
+
+@pytest.mark.parametrize("name,lens", [("mha64", [2100, 1, 2050]), ("dn_odd", [2048, 2049, 3]), ("gqa4_128", [4099]), ("fp8", [65] * 70)])
+def test_prompts_longer_than_one_chunk(api, tmp_path, monkeypatch, name, lens):
+    """More than 4096 prompt tokens: the sequences continue across chunks, in equal shares; many short ones share a chunk."""
+    monkeypatch.setenv("MLB_PREFILL", "chunk")
+    spec = dataclasses.replace(SPECS[name], max_context=max(lens) + 8)
+    path = write_model(tmp_path, spec, seed=45)
+    oracle = load_oracle(path)
+    prompts = random_prompts(spec.vocab, lens, seed=47)
+    model = api.Model(path)
+    sess = api.Session(model, len(lens))
+    sess.prefill(prompts)
+    assert sess.positions().tolist() == [n - 1 for n in lens]
+    sess.decode_step()
+    got = sess.logits()
+    for b in sorted({0, 1 % len(lens), len(lens) - 1}):
+        _, want = oracle_rollout(oracle, prompts[b], 1)
+        assert logits_error(got[b], want[0]) < TOL_LOWP, b
+    sess.close()
+    model.close()
