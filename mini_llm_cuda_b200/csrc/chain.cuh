@@ -343,11 +343,7 @@ struct Chain {
                 if (rec && (rc = rec->begin("deltanet_state_update", (uint64_t)B * 2ull * H * dk * dv * 4, (uint64_t)B * 6ull * H * dk * dv))) return rc;
                 if (s->parent) {
                     // prompt columns: the recurrence runs over the columns of a sequence in order
-                    DeltaColsParams dc;
-                    dc.raw = s->raw; dc.raw_stride = s->raw_stride; dc.state = s->state[i]; dc.H = H; dc.dv = dv;
-                    dc.out = nullptr; dc.out16 = s->a16; dc.l2_eps = 1e-6f;
-                    dc.hdr = s->plan.hdr; dc.runs = reinterpret_cast<const int4*>(s->plan.runs);
-                    CU(delta_cols_launch(dk, s->use_pdl, s->plan.max_runs, s->stream, dc));
+                    CU(delta_cols(s, i, nullptr, s->a16));
                 } else {
                     dim3 grid((dv + 31) / 32, H, B);
                     if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, 1e-6f));
@@ -463,7 +459,8 @@ struct Chain {
                 const int dk = cfg.dn_key_dim, dv = cfg.dn_value_dim, H = cfg.heads;
                 if (rec && (rc = rec->begin("deltanet_state_update", (uint64_t)B * 2ull * H * dk * dv * 4, (uint64_t)B * 6ull * H * dk * dv))) return rc;
                 dim3 grid((dv + 31) / 32, H, B);
-                if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
+                if (s->parent) CU(delta_cols(s, i, s->abuf, nullptr));
+                else if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
                 else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
                 if (rec && (rc = rec->end())) return rc;
                 ++launches;
@@ -488,7 +485,9 @@ struct Chain {
             if ((rc = gemv<GEMV_RESID>(s, c, g, d <= 1024 ? 8 : 16, rec, "ffn_down_gemv_residual_ple"))) return rc;
             ++launches;
         }
-        if (kind == CHAIN_PREFILL) {
+        if (kind == CHAIN_PREFILL && s->parent) {
+            // prompt columns: positions and tokens of the next chunk come from the host
+        } else if (kind == CHAIN_PREFILL) {
             if (rec && (rc = rec->begin("advance_prompt", (uint64_t)B * 12, 0))) return rc;
             CU(launch_chain(s->use_pdl, advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s->stream, c));
             if (rec && (rc = rec->end())) return rc;

@@ -406,11 +406,7 @@ static int run_cols(mlb_session* s, int kind, int* n_launches) {
             }
         } else {
             if ((rc = gemm(TC_RAW, s->cg_dn, s->tc_g.xn[0], M.qkv, M.qkv, L.n_qkv, d, s->raw, nullptr, true, nullptr, nullptr, nullptr, L.Sqkv, nullptr))) return rc;
-            DeltaColsParams dc;
-            dc.raw = s->raw; dc.raw_stride = s->raw_stride; dc.state = s->state[i]; dc.H = cfg.heads; dc.dv = cfg.dn_value_dim;
-            dc.out = nullptr; dc.out16 = s->a16; dc.l2_eps = 1e-6f;
-            dc.hdr = s->plan.hdr; dc.runs = reinterpret_cast<const int4*>(s->plan.runs);
-            CU(delta_cols_launch(cfg.dn_key_dim, s->use_pdl, s->plan.max_runs, s->stream, dc));
+            CU(delta_cols(s, i, nullptr, s->a16));
         }
         ++launches;
         if ((rc = gemm(TC_RESID, attn ? s->cg_o_attn : s->cg_o_dn, attn ? s->tc_g.a_attn[0] : s->tc_g.a_dn[0], M.o, M.o, d, L.o_in, s->x, nullptr, false, L.g2, nullptr, nullptr, L.So, nullptr)))
@@ -1131,8 +1127,8 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     if (c.query_gating || !parent) SA(sess_alloc(s, (void**)&s->gbuf, B * nq * 4, true));
     SA(sess_alloc(s, (void**)&s->abuf, B * a_dim * 4, true));
     if (has_dn || !parent) SA(sess_alloc(s, (void**)&s->raw, B * s->raw_stride * 4, true));
+    if (!parent || c.weight_dtype == MLB_DT_F32) SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
     if (!parent) {
-        SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
         SA(sess_alloc(s, (void**)&s->logits, B * c.vocab * 4, true));        // a column set's are made when a text is scored
         SA(sess_alloc(s, (void**)&s->probe, (size_t)c.vocab * 4, true));
     }
@@ -1203,7 +1199,7 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
         s->use_pdl = !(e && e[0] == '1');
         const char* gv = std::getenv("MLB_GEMV");      // stream | thread | auto (stream for batch <= 4)
         const std::string gmode = gv ? gv : "auto";
-        s->use_sgemv = gmode == "stream" || (gmode == "auto" && batch <= 4);
+        s->use_sgemv = !parent && (gmode == "stream" || (gmode == "auto" && batch <= 4));
         s->force_sgemv = gmode == "stream";
         if (const char* v = std::getenv("MLB_SG_STAGE_KB")) s->sg_stage_kb = std::max(8, std::min(96, std::atoi(v)));
         if (const char* v = std::getenv("MLB_SG_STAGES")) s->sg_max_stages = std::max(2, std::min(8, std::atoi(v)));
@@ -1215,11 +1211,15 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
         SA(setup_lean_path(s));
         if (!s->use_lean) SA(setup_grid_path(s));
     }
-    if (parent) SA(setup_cols_path(s));
-    if (!s->use_cols) SA(setup_tc_path(s));
-    if (parent && !s->use_cols && !s->use_tc) {
-        free_session(s);
-        return fail(MLB_E_UNSUPPORTED, "prompt columns need the tensor-core step (bf16 weights)");
+    if (parent && c.weight_dtype != MLB_DT_F32) {        // columns in fp32 run the GEMV chain
+        SA(setup_cols_path(s));
+        if (!s->use_cols) SA(setup_tc_path(s));
+        if (!s->use_cols && !s->use_tc) {
+            free_session(s);
+            return fail(MLB_E_UNSUPPORTED, "prompt columns need tensor maps from the driver");
+        }
+    } else if (!parent) {
+        SA(setup_tc_path(s));
     }
 #undef SA
 #undef SCU
@@ -1270,9 +1270,15 @@ extern "C" void mlb_session_free(mlb_session* s) { free_session(s); }
 // are consumed; the last one stays pending, as after the token loop. MLB_PREFILL = auto | step |
 // chunk: auto takes this path from 64 prompt tokens on (its activations are bf16, so the cache
 // differs from the token loop's within the low-precision tolerance); `*done` tells whether it ran.
+// Models with fp32 weights run their columns through the GEMV chain instead, eight to a CTA, in fp32 like the token loop,
+// wherever that loop would take kF32ColSteps steps or more.
 //
 // Width of a step: a column set of 256 leaves most SMs without a tile (d = 512: 4 row tiles of 128) and pays the
 // step's ~45 launches once per 256 tokens; at 4096 columns the same launches carry 16 times the work.
+
+// A step of columns costs 3.3 token steps of one sequence (0.27 and 0.59 ms on the two fp32 configurations, 8 or 12 columns), fewer
+// of several sequences.
+constexpr int kF32ColSteps = 4;
 
 // The narrowest column set that holds `n` columns (n <= kColMax).
 static int cols_get(mlb_session* s, int n, mlb_session** out) {
@@ -1298,12 +1304,12 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     const int kind = score_out ? CHAIN_GREEDY : CHAIN_PREFILL;
     long total = 0;
     for (int b = 0; b < B; ++b) total += lens[b] - keep;
-    if (total < 1 || (mode == "auto" && total < 64)) return MLB_OK;
     const mlb_config& cfg = s->m->cfg;
-    if (cfg.weight_dtype != MLB_DT_BF16 && cfg.weight_dtype != MLB_DT_FP8_E4M3) {
-        if (mode == "chunk") return fail(MLB_E_UNSUPPORTED, "MLB_PREFILL=chunk needs bf16 or FP8 weights");
-        return MLB_OK;
-    }
+    const bool f32 = cfg.weight_dtype == MLB_DT_F32;
+    if (f32 && mode == "chunk") return fail(MLB_E_UNSUPPORTED, "MLB_PREFILL=chunk needs bf16 or FP8 weights");
+    int longest = 0;
+    for (int b = 0; b < B; ++b) longest = std::max(longest, lens[b] - keep);
+    if (total < 1 || (mode == "auto" && (f32 ? longest < kF32ColSteps : total < 64))) return MLB_OK;
     int rc;
     mlb_session* cs = nullptr;
     if (s->cols_failed && mode != "chunk") return MLB_OK;

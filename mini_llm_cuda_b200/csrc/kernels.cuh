@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(StepCtl c, GemvParams p) {
     float* red = rs + BT;                              // [8][BT]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     const int b0 = blockIdx.y * BT;
+    if (c.n_cols != nullptr && b0 >= *c.n_cols) return;     // prompt columns: behind the last one that carries a token
     const int row0 = blockIdx.x * R;
     const int nvec = K / EPV;
     const T* W = reinterpret_cast<const T*>(p.W);

@@ -260,6 +260,16 @@ static TcShape tc_pick_shape(const mlb_session* s, int B, int N, int nkb_all, in
 }
 static int nb_index(int nb) { return nb == 16 ? 0 : nb == 32 ? 1 : nb == 64 ? 2 : nb == 128 ? 3 : 4; }
 
+// delta-net recurrence of layer i over the columns of a column set
+static inline cudaError_t delta_cols(const mlb_session* s, int i, float* out, bf16_t* out16) {
+    const mlb_config& cfg = s->m->cfg;
+    DeltaColsParams dc;
+    dc.raw = s->raw; dc.raw_stride = s->raw_stride; dc.state = s->state[i]; dc.H = cfg.heads; dc.dv = cfg.dn_value_dim;
+    dc.out = out; dc.out16 = out16; dc.l2_eps = 1e-6f;
+    dc.hdr = s->plan.hdr; dc.runs = reinterpret_cast<const int4*>(s->plan.runs);
+    return delta_cols_launch(cfg.dn_key_dim, s->use_pdl, s->plan.max_runs, s->stream, dc);
+}
+
 // ---- the launch chains (chain_f32.cu, chain_bf16.cu, chain_fp8.cu) ------------------------------------
 int chain_run_f32(mlb_session* s, int kind, Recorder* rec, int* n_launches);
 int chain_run_bf16(mlb_session* s, int kind, Recorder* rec, int* n_launches);

@@ -5,7 +5,7 @@ import dataclasses
 import numpy as np
 import pytest
 
-from helpers import TOL_LOWP, load_oracle, logits_error, oracle_rollout, random_prompts, write_model
+from helpers import TOL_FP32, TOL_LOWP, load_oracle, logits_error, oracle_rollout, random_prompts, write_model
 from mini_llm_cuda_b200.model_file import ModelSpec, periodic_layer_types
 
 pytestmark = pytest.mark.gpu
@@ -66,5 +66,28 @@ def test_prompts_longer_than_one_chunk(api, tmp_path, monkeypatch, name, lens):
     for b in sorted({0, 1 % len(lens), len(lens) - 1}):
         _, want = oracle_rollout(oracle, prompts[b], 1)
         assert logits_error(got[b], want[0]) < TOL_LOWP, b
+    sess.close()
+    model.close()
+
+
+@pytest.mark.parametrize("name,lens", [("mha64", [4, 5]), ("gqa4_128", [70]), ("dn_odd", [9, 1, 18, 33, 2]), ("gqa8_64", [65, 64, 63, 8, 1, 16, 17, 130, 3])])
+def test_fp32_prompt_columns_match_oracle(api, tmp_path, name, lens):
+    """fp32 weights and cache: a prompt of four tokens or more goes through the GEMV chain eight columns to a CTA; the logits behind
+    it within the fp32 bound, the ids of the steps that follow identical."""
+    spec = dataclasses.replace(SPECS[name], weight_dtype="float32", kv_dtype="float32", max_context=160)
+    path = write_model(tmp_path, spec, seed=51)
+    oracle = load_oracle(path)
+    prompts = random_prompts(spec.vocab, lens, seed=53)
+    model = api.Model(path)
+    sess = api.Session(model, len(lens))
+    for _ in range(2):
+        sess.prefill(prompts)
+        assert sess.positions().tolist() == [n - 1 for n in lens]
+        got = sess.decode(4)
+    logits = sess.logits()
+    for b in range(len(lens)):
+        toks, want = oracle_rollout(oracle, prompts[b], 4)
+        assert got[b].tolist() == toks.tolist(), b
+        assert logits_error(logits[b], want[-1]) < TOL_FP32, b
     sess.close()
     model.close()
