@@ -237,6 +237,39 @@ struct Chain {
         return MLB_OK;
     }
 
+    // The same on mma.sync tiles (gemm_dec.cuh), for decode batches.
+    template <int MODE>
+    static int gemm_dec(mlb_session* s, const StepCtl& c, const CUtensorMap& A, const CUtensorMap& A2, const CUtensorMap* Bmaps, int N, int K,
+                        float* y, bf16_t* h16, bool normed, const float* next_gain, const mlb_session::TcLayerMaps* ext,
+                        const QkvPostParams* q, const float* sA, const float* sA2, Recorder* rec, const char* name) {
+        const int ple = s->m->cfg.ple_dim, na = MODE == TC_SWIGLU ? 2 : 1;
+        constexpr bool w8 = sizeof(T) == 1;
+        using KVQ = typename std::conditional<MODE == TC_QKV, KVT, float>::type;      // only the projection of q, k, v writes the cache
+        GemmDecParams p;
+        p.nkb_x = ext ? (ple + kTcKB - 1) / kTcKB : 0;
+        const GdShape g = gd_pick(s, N, (K + kTcKB - 1) / kTcKB + p.nkb_x, MODE, w8, ext != nullptr);
+        p.N = N; p.K = K; p.B = s->B; p.split = g.split; p.G = g.g; p.stages = g.stages; p.w_bytes = g.w_bytes;
+        p.y = y; p.h16 = h16; p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = (s->m->cfg.dim + kTcM - 1) / kTcM * 4; p.eps = s->m->cfg.rms_eps;
+        p.xg16 = s->xn16; p.gain_next = next_gain; p.ssq_out = s->tc_ssq; p.s1 = sA; p.s2 = sA2; p.err = s->dev_err;
+        p.trace = s->tc_trace ? s->tc_trace + 8 * (size_t)(s->tc_trace_n++ % 64) : nullptr;
+        int rc;
+        if (rec && (rc = rec->begin(name, ((uint64_t)N * K * sizeof(T) + (uint64_t)N * (ext ? ple : 0) * 2) * na + (uint64_t)s->B * K * 2 + (uint64_t)s->B * N * 4,
+                                    2ull * N * (K + (ext ? ple : 0)) * s->B * na)))
+            return rc;
+        const dim3 grid((N + kGdF - 1) / kGdF, (s->B + 16 * g.np - 1) / (16 * g.np)), block(32 * (2 * na * g.split + 1));
+        const CUtensorMap &X = Bmaps[gd_index(g.np, g.g)], &Ax = ext ? ext->pleP : A, &Bx = ext ? ext->pleT : A;
+        const QkvPostParams q0{};
+        cudaError_t e;
+        switch (g.np) {
+            case 1: e = launch_chain(s->use_pdl, gemm_dec_kernel<MODE, KVQ, T, 1>, grid, block, g.smem, s->stream, A, A2, X, Ax, Bx, p, c, q ? *q : q0); break;
+            case 2: e = launch_chain(s->use_pdl, gemm_dec_kernel<MODE, KVQ, T, 2>, grid, block, g.smem, s->stream, A, A2, X, Ax, Bx, p, c, q ? *q : q0); break;
+            default: e = launch_chain(s->use_pdl, gemm_dec_kernel<MODE, KVQ, T, 4>, grid, block, g.smem, s->stream, A, A2, X, Ax, Bx, p, c, q ? *q : q0); break;
+        }
+        if (e != cudaSuccess) return fail(MLB_E_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
+        if (rec) return rec->end();
+        return MLB_OK;
+    }
+
     // One tensor-core projection. `normed`: the activation operand is bf16(x * gain) and the accumulator
     // columns are scaled by 1 / rms(x) from the partial sums its producer left. `next_gain` (RESID): also
     // write the operand and the partial sums for the next norm. `ext`: the per-layer embedding pair whose
@@ -245,6 +278,7 @@ struct Chain {
     static int gemm_tc(mlb_session* s, const StepCtl& c, const CUtensorMap& A, const CUtensorMap& A2, const CUtensorMap* Bmaps, int N, int K,
                        float* y, bf16_t* h16, bool normed, const float* next_gain, const mlb_session::TcLayerMaps* ext,
                        const QkvPostParams* q, const float* sA, const float* sA2, Recorder* rec, const char* name) {
+        if (s->use_dec) return gemm_dec<MODE>(s, c, A, A2, Bmaps, N, K, y, h16, normed, next_gain, ext, q, sA, sA2, rec, name);
         GemmTcParams p;
         const int ple = s->m->cfg.ple_dim;
         const int na = MODE == TC_SWIGLU ? 2 : 1;
@@ -259,7 +293,7 @@ struct Chain {
         p.y = y; p.resid = MODE == TC_RESID ? y : nullptr; p.h16 = h16; p.err = s->dev_err;
         p.sA = sA; p.sA2 = sA2;
         p.trace = s->tc_trace ? s->tc_trace + 8 * (size_t)(s->tc_trace_n++ % 64) : nullptr;
-        p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = (s->m->cfg.dim + kTcM - 1) / kTcM; p.eps = s->m->cfg.rms_eps;
+        p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = (s->m->cfg.dim + kTcM - 1) / kTcM * 4; p.eps = s->m->cfg.rms_eps;
         p.xg16 = next_gain ? s->xn16 : nullptr; p.gain_next = next_gain; p.ssq_out = next_gain ? s->tc_ssq : nullptr;
         const size_t smem = sh.smem;
         dim3 grid((N + kTcM - 1) / kTcM, (s->B + nb - 1) / nb, sh.split);
@@ -284,11 +318,12 @@ struct Chain {
         const mlb_model* m = s->m;
         const mlb_config& cfg = m->cfg;
         const int d = cfg.dim, F = cfg.ffn_dim, B = s->B, ple = cfg.ple_dim;
+        const int perm = s->use_dec && sizeof(T) == 1 ? 1 : 0;       // operand order of the FP8 decode GEMMs
         int launches = 0, rc;
         if (rec && (rc = rec->begin("embed_ple_gather_norm", (uint64_t)B * d * 8 + (uint64_t)B * ple * 2 * cfg.layers, 0))) return rc;
         CU(launch_chain(s->use_pdl, embed_tc_kernel<T>, dim3(B, (d + kTcM - 1) / kTcM), dim3(128), (size_t)ple * 4, s->stream, c,
                         static_cast<const T*>(m->E), static_cast<const float*>(m->Es), d, static_cast<const StepLayer*>(s->step_layers), cfg.layers, ple,
-                        static_cast<const float*>(m->layers[0].g1), s->x, s->xn16, s->tc_ssq, s->tple16));
+                        static_cast<const float*>(m->layers[0].g1), s->x, s->xn16, s->tc_ssq, s->tple16, perm));
         if (rec && (rc = rec->end())) return rc;
         ++launches;
         for (int i = 0; i < cfg.layers; ++i) {
@@ -307,7 +342,7 @@ struct Chain {
                 AttnParams a;
                 a.kpool = s->kpool[i]; a.vpool = s->vpool[i];
                 a.page_table = s->page_table; a.pt_stride = s->max_pages;
-                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16;
+                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16; a.perm = perm;
                 a.part = s->part; a.ticket = s->attn_ticket;
                 a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
                 if (rec) {
@@ -346,8 +381,8 @@ struct Chain {
                     CU(delta_cols(s, i, nullptr, s->a16));
                 } else {
                     dim3 grid((dv + 31) / 32, H, B);
-                    if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, 1e-6f));
-                    else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, 1e-6f));
+                    if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, perm, 1e-6f));
+                    else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, s->a16, perm, 1e-6f));
                 }
                 if (rec && (rc = rec->end())) return rc;
                 ++launches;
@@ -435,7 +470,7 @@ struct Chain {
                 AttnParams a;
                 a.kpool = s->kpool[i]; a.vpool = s->vpool[i];
                 a.page_table = s->page_table; a.pt_stride = s->max_pages;
-                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = nullptr;
+                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = nullptr; a.perm = 0;
                 a.part = s->part; a.ticket = s->attn_ticket;
                 a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
                 if (rec) {
@@ -460,8 +495,8 @@ struct Chain {
                 if (rec && (rc = rec->begin("deltanet_state_update", (uint64_t)B * 2ull * H * dk * dv * 4, (uint64_t)B * 6ull * H * dk * dv))) return rc;
                 dim3 grid((dv + 31) / 32, H, B);
                 if (s->parent) CU(delta_cols(s, i, s->abuf, nullptr));
-                else if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
-                else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 1e-6f));
+                else if (dk == 64) CU(launch_chain(s->use_pdl, delta_net_kernel<64>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 0, 1e-6f));
+                else CU(launch_chain(s->use_pdl, delta_net_kernel<128>, grid, dim3(256), 0, s->stream, c, static_cast<const float*>(s->raw), s->raw_stride, s->state[i], H, dv, s->abuf, static_cast<bf16_t*>(nullptr), 0, 1e-6f));
                 if (rec && (rc = rec->end())) return rc;
                 ++launches;
             }
@@ -515,6 +550,15 @@ struct Chain {
     }
 };
 
+template <int MODE, typename KVT, typename WT>
+static int dec_allow_big_smem() {
+    const int big = 200 * 1024;
+    using KVQ = typename std::conditional<MODE == TC_QKV, KVT, float>::type;
+    CU(cudaFuncSetAttribute(gemm_dec_kernel<MODE, KVQ, WT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    CU(cudaFuncSetAttribute(gemm_dec_kernel<MODE, KVQ, WT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    CU(cudaFuncSetAttribute(gemm_dec_kernel<MODE, KVQ, WT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    return MLB_OK;
+}
 template <typename KVT, typename WT>
 static int tc_allow_big_smem_t() {
     const int big = 227 * 1024;
@@ -522,6 +566,10 @@ static int tc_allow_big_smem_t() {
     CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_RESID, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_SWIGLU, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     CU(cudaFuncSetAttribute(gemm_tc_kernel<TC_QKV, KVT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    int rc;
+    if ((rc = dec_allow_big_smem<TC_RAW, KVT, WT>()) || (rc = dec_allow_big_smem<TC_RESID, KVT, WT>()) || (rc = dec_allow_big_smem<TC_SWIGLU, KVT, WT>()) ||
+        (rc = dec_allow_big_smem<TC_QKV, KVT, WT>()))
+        return rc;
     return MLB_OK;
 }
 

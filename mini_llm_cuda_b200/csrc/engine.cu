@@ -399,7 +399,7 @@ static int run_cols(mlb_session* s, int kind, int* n_launches) {
                 // fp32 K/V: the decode kernel, one column at a time
                 AttnParams a;
                 a.kpool = s->kpool[i]; a.vpool = s->vpool[i]; a.page_table = s->page_table; a.pt_stride = s->max_pages;
-                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16; a.part = s->part; a.ticket = s->attn_ticket;
+                a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16; a.perm = 0; a.part = s->part; a.ticket = s->attn_ticket;
                 a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
                 rc = chain_attn_f32kv(s, c, a);
                 if (rc) return rc;
@@ -756,36 +756,61 @@ static int setup_tc_path(mlb_session* s) {
     if (const char* v = std::getenv("MLB_TC_TRACE"))
         if (v[0] == '1' && (rc = sess_alloc(s, (void**)&s->tc_trace, 64 * 8 * 8, true))) return rc;
     if ((rc = tc_probe_clusters(s))) return rc;
+    const auto kb = [](int k) { return (k + kTcKB - 1) / kTcKB; };
+    // mma.sync tiles for the projections, or tcgen05 ones: gd_small_enough. The QK norm needs whole heads in a tile, the k-block maps
+    // whole k-blocks, the ranges of a tile a warp each: other models stay on gemm_tc.cuh.
+    s->use_dec = !s->parent && !c.qk_norm && gd_small_enough(s) && c.dim % kTcKB == 0 && c.ffn_dim % kTcKB == 0 && c.ple_dim % kTcKB == 0 &&
+                 nq % kTcKB == 0 && a_dn % kTcKB == 0;
+    const auto ranges_fit = [&](int n, int nkb, int mode, bool ext) { return gd_pick(s, n, nkb, mode, w8, ext).split <= kGdMaxSplit; };
+    for (int i = 0; i < c.layers && s->use_dec; ++i)
+        s->use_dec = ranges_fit(s->m->layers[i].n_qkv, kb(c.dim), TC_QKV, false) && ranges_fit(c.dim, kb(s->m->layers[i].o_in), TC_RESID, false);
+    s->use_dec = s->use_dec && ranges_fit(c.ffn_dim, kb(c.dim), TC_SWIGLU, false) && ranges_fit(c.vocab, kb(c.dim), TC_RAW, false) &&
+                 ranges_fit(c.dim, kb(c.ffn_dim) + kb(c.ple_dim), TC_RESID, c.ple_dim > 0) && ranges_fit(c.dim, kb(c.ffn_dim), TC_RESID, false);
     s->tc_shape_down = tc_pick_shape(s, B, c.dim, (c.ffn_dim + kTcKB - 1) / kTcKB + (c.ple_dim + kTcKB - 1) / kTcKB, 1, w8, w8 ? 2 : 1);
-    const int parts = (c.dim + kTcM - 1) / kTcM;
+    const int parts = (c.dim + kTcM - 1) / kTcM * 4;
     if ((rc = sess_alloc(s, (void**)&s->xn16, (size_t)B * c.dim * 2, true))) return rc;
     if ((rc = sess_alloc(s, (void**)&s->a16, (size_t)B * std::max(nq, a_dn) * 2, true))) return rc;
     if ((rc = sess_alloc(s, (void**)&s->h16, (size_t)B * c.ffn_dim * 2, true))) return rc;
     if ((rc = sess_alloc(s, (void**)&s->tc_ssq, (size_t)B * parts * 4, true))) return rc;
     if (c.ple_dim > 0 && (rc = sess_alloc(s, (void**)&s->tple16, (size_t)c.layers * B * c.ple_dim * 2, true))) return rc;
     s->tc_maps.resize(c.layers);
+    // weight maps of a projection, by the launch shape it has
+    auto wmap = [&](CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, int mode, int kb_ext) {
+        if (s->use_dec) return make_kblock_map(enc, out, base, rows, cols, kGdF, gd_pick(s, (int)rows, kb((int)cols) + kb_ext, mode, w8, kb_ext > 0).g, w8);
+        return w8 ? make_u8_map(enc, out, base, rows, cols, kTcM) : make_bf16_map(enc, out, base, rows, cols, kTcM);      // codes are widened in the kernel
+    };
     for (int i = 0; i < c.layers; ++i) {
         const DevLayer& L = s->m->layers[i];
         auto& M = s->tc_maps[i];
-        auto wmap = w8 ? make_u8_map : make_bf16_map;       // FP8: e4m3 codes, widened in the kernel
-        if ((rc = wmap(enc, &M.qkv, L.Wqkv, L.n_qkv, c.dim, kTcM))) return rc;
-        if ((rc = wmap(enc, &M.o, L.Wo, c.dim, L.o_in, kTcM))) return rc;
-        if ((rc = wmap(enc, &M.w1a, L.W1a, c.ffn_dim, c.dim, kTcM))) return rc;
-        if ((rc = wmap(enc, &M.w1b, L.W1b, c.ffn_dim, c.dim, kTcM))) return rc;
-        if ((rc = wmap(enc, &M.w2, L.W2, c.dim, c.ffn_dim, kTcM))) return rc;
+        const int kb_ext = i + 1 < c.layers ? kb(c.ple_dim) : 0;      // k-blocks of the next layer's embedding behind the down projection
+        if ((rc = wmap(&M.qkv, L.Wqkv, L.n_qkv, c.dim, L.type == MLB_LAYER_ATTENTION ? TC_QKV : TC_RAW, 0))) return rc;
+        if ((rc = wmap(&M.o, L.Wo, c.dim, L.o_in, TC_RESID, 0))) return rc;
+        if ((rc = wmap(&M.w1a, L.W1a, c.ffn_dim, c.dim, TC_SWIGLU, 0))) return rc;
+        if ((rc = wmap(&M.w1b, L.W1b, c.ffn_dim, c.dim, TC_SWIGLU, 0))) return rc;
+        if ((rc = wmap(&M.w2, L.W2, c.dim, c.ffn_dim, TC_RESID, kb_ext))) return rc;
         if (c.ple_dim > 0) {
             // operands of the per-layer embedding folded into the previous layer's down projection
-            if ((rc = make_bf16_map(enc, &M.pleP, L.pleP, c.dim, c.ple_dim, kTcM))) return rc;
-            if ((rc = make_bf16_map(enc, &M.pleT, s->tple16 + (size_t)i * B * c.ple_dim, B, c.ple_dim, s->tc_shape_down.nb))) return rc;
+            const bf16_t* rows = s->tple16 + (size_t)i * B * c.ple_dim;
+            if (s->use_dec) {
+                const GdShape g = gd_pick(s, c.dim, kb(c.ffn_dim) + kb(c.ple_dim), TC_RESID, w8, true);
+                if ((rc = make_kblock_map(enc, &M.pleP, L.pleP, c.dim, c.ple_dim, kGdF, g.g, false))) return rc;
+                if ((rc = make_kblock_map(enc, &M.pleT, rows, B, c.ple_dim, 16 * g.np, g.g, false))) return rc;
+            } else {
+                if ((rc = make_bf16_map(enc, &M.pleP, L.pleP, c.dim, c.ple_dim, kTcM))) return rc;
+                if ((rc = make_bf16_map(enc, &M.pleT, rows, B, c.ple_dim, s->tc_shape_down.nb))) return rc;
+            }
         }
     }
-    if ((rc = (w8 ? make_u8_map : make_bf16_map)(enc, &s->tc_g.E, s->m->E, c.vocab, c.dim, kTcM))) return rc;
-    for (int i = 0; i < 5; ++i) {
-        const uint32_t nb = 16u << i;
-        if ((rc = make_bf16_map(enc, &s->tc_g.xn[i], s->xn16, B, c.dim, nb))) return rc;
-        if ((rc = make_bf16_map(enc, &s->tc_g.a_attn[i], s->a16, B, nq, nb))) return rc;
-        if ((rc = make_bf16_map(enc, &s->tc_g.a_dn[i], s->a16, B, a_dn, nb))) return rc;
-        if ((rc = make_bf16_map(enc, &s->tc_g.h[i], s->h16, B, c.ffn_dim, nb))) return rc;
+    if ((rc = wmap(&s->tc_g.E, s->m->E, c.vocab, c.dim, TC_RAW, 0))) return rc;
+    for (int i = 0; i < (s->use_dec ? 9 : 5); ++i) {
+        auto xmap = [&](CUtensorMap* out, const void* base, uint64_t cols) {
+            if (s->use_dec) return make_kblock_map(enc, out, base, B, cols, 16u << (i / 3), 1u << (i % 3), false);
+            return make_bf16_map(enc, out, base, B, cols, 16u << i);
+        };
+        if ((rc = xmap(&s->tc_g.xn[i], s->xn16, c.dim))) return rc;
+        if ((rc = xmap(&s->tc_g.a_attn[i], s->a16, nq))) return rc;
+        if ((rc = xmap(&s->tc_g.a_dn[i], s->a16, a_dn))) return rc;
+        if ((rc = xmap(&s->tc_g.h[i], s->h16, c.ffn_dim))) return rc;
     }
     if ((rc = w8 ? tc_allow_big_smem_fp8(c.kv_dtype) : tc_allow_big_smem_bf16(c.kv_dtype))) return rc;
     s->use_tc = true;

@@ -57,7 +57,8 @@ struct GemmTcParams {
     float* y;                      // RAW / RESID: fp32 [B][N]
     const float* resid;            // RESID: fp32 [B][N] (may alias y)
     bf16_t* h16;                   // SWIGLU: bf16 [B][N]
-    // deferred RMS norm of the activation operand: partial sums of squares [B][ssq_parts]; null = operand is used as is
+    // deferred RMS norm of the activation operand: sums of squares of 32 features each, [B][ssq_parts] (a multiple of 4); null =
+    // operand is used as is
     const float* ssq_in; int ssq_parts; float eps;
     // RESID: operand and partial sums for the next norm (null = not wanted)
     bf16_t* xg16; const float* gain_next; float* ssq_out;
@@ -451,7 +452,11 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
             const int b = b0 + j;
             if (p.ssq_in != nullptr && b < p.B) {
                 float tot = 0.f;
-                for (int t = 0; t < p.ssq_parts; ++t) tot += __ldcg(p.ssq_in + (size_t)b * p.ssq_parts + t);
+                const float4* sp = reinterpret_cast<const float4*>(p.ssq_in + (size_t)b * p.ssq_parts);
+                for (int t = 0; t < p.ssq_parts / 4; ++t) {
+                    const float4 x = __ldcg(sp + t);
+                    tot += (x.x + x.y) + (x.z + x.w);
+                }
                 r = 1.0f / sqrtf(tot / (float)p.K + p.eps);
             }
             rinv_s[j] = r;
@@ -682,8 +687,8 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
         for (int j = cb + tid; j < ce; j += kTcThreads) {
             const int b = b0 + j;
             if (b < p.B)
-                p.ssq_out[(size_t)b * gridDim.x + blockIdx.x] =
-                    (colsum_s[j] + colsum_s[256 + j]) + (colsum_s[512 + j] + colsum_s[768 + j]);
+                reinterpret_cast<float4*>(p.ssq_out + (size_t)b * p.ssq_parts)[blockIdx.x] =
+                    make_float4(colsum_s[j], colsum_s[256 + j], colsum_s[512 + j], colsum_s[768 + j]);
         }
     }
     if (warp == 0) {
@@ -703,7 +708,7 @@ __global__ void __launch_bounds__(128) embed_tc_kernel(StepCtl c, const WT* __re
                                                               const StepLayer* __restrict__ layers, int n_layers, int ple,
                                                               const float* __restrict__ gain, float* __restrict__ x,
                                                               bf16_t* __restrict__ xg16, float* __restrict__ ssq,
-                                                              bf16_t* __restrict__ tple16) {
+                                                              bf16_t* __restrict__ tple16, int perm) {
     pdl_launch_dependents();
     pdl_wait();                      // pos / tok come from the last kernel of the previous step
     const int b = blockIdx.x;
@@ -714,7 +719,6 @@ __global__ void __launch_bounds__(128) embed_tc_kernel(StepCtl c, const WT* __re
         if (blockIdx.y == 0 && threadIdx.x == 0) c.tok[b] = t;
     }
     extern __shared__ __align__(16) float trow[];
-    __shared__ float red[4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (ple > 0) {
         const bf16_t* T0 = static_cast<const bf16_t*>(layers[0].pleT);
@@ -742,12 +746,10 @@ __global__ void __launch_bounds__(128) embed_tc_kernel(StepCtl c, const WT* __re
             v += a;
         }
         x[(size_t)b * d + i] = v;
-        xg16[(size_t)b * d + i] = __float2bfloat16_rn(v * gain[i]);
+        xg16[(size_t)b * d + (perm ? perm16(i) : i)] = __float2bfloat16_rn(v * gain[i] * (perm ? kOperandScale : 1.0f));
     }
     const float ss = warp_sum(v * v);
-    if (lane == 0) red[warp] = ss;
-    __syncthreads();
-    if (tid == 0) ssq[(size_t)b * gridDim.y + blockIdx.y] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (lane == 0) ssq[((size_t)b * gridDim.y + blockIdx.y) * 4 + warp] = ss;
 }
 
 // Greedy pick over the fp32 logits of a batched LM-head GEMM: argmax, lowest index on ties

@@ -80,6 +80,14 @@ template <> struct Elem<fp8_t> {
     }
 };
 
+// Position of a feature in the bf16 activation operand of an FP8 model's decode GEMMs (gemm_dec.cuh): permuted inside every sixteen.
+__device__ __forceinline__ int perm16(int f) {
+    const int k = f & 15;
+    return (f & ~15) | ((k & 2) << 2) | ((k >> 2) << 1) | (k & 1);
+}
+// and its factor, a power of two (kernels that serve both kinds of operand take `perm` for the pair)
+constexpr float kOperandScale = 18446744073709551616.0f;        // 2^64
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -667,6 +675,7 @@ struct AttnParams {
     const float* gbuf;      // [B][heads*hd] sigmoid gates or null
     float* abuf;            // [B][heads*hd]
     bf16_t* abuf16;         // same values as the bf16 operand of a tensor-core O projection, or null
+    int perm;               // features of abuf16 in perm16 order
     float* part;            // [B][heads][splits][hd+2]
     int* ticket;            // [B * gridDim.y]
     int heads, kv_heads;
@@ -885,7 +894,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(StepCtl c, AttnParams 
             float o = at / lt;
             if (p.gbuf) o *= p.gbuf[((size_t)b * p.heads + h) * HD + e];
             p.abuf[((size_t)b * p.heads + h) * HD + e] = o;
-            if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + e] = __float2bfloat16_rn(o);
+            if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
         } else {
             float* pp = p.part + (((size_t)b * p.heads + h) * SG + split) * (HD + 2);
             pp[e] = at;
@@ -928,7 +937,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(StepCtl c, AttnParams 
         for (int s = 0; s < S; ++s) o = fmaf(wsm[g][s], __ldcg(pp + (size_t)s * (HD + 2)), o);
         if (p.gbuf) o *= p.gbuf[((size_t)b * p.heads + h) * HD + e];
         p.abuf[((size_t)b * p.heads + h) * HD + e] = o;
-        if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + e] = __float2bfloat16_rn(o);
+        if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
     }
     if (tid == 0) p.ticket[tslot] = 0;
 }
@@ -946,7 +955,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(StepCtl c, AttnParams 
 template <int DK>
 __global__ void __launch_bounds__(256) delta_net_kernel(StepCtl c, const float* __restrict__ raw, int raw_stride,
                                                         float* __restrict__ state, int H, int dv,
-                                                        float* __restrict__ abuf, bf16_t* __restrict__ abuf16, float l2_eps) {
+                                                        float* __restrict__ abuf, bf16_t* __restrict__ abuf16, int perm, float l2_eps) {
     constexpr int EPL = DK / 32;
     constexpr int ROWS_PER_WARP = 4;
     const int b = blockIdx.z, h = blockIdx.y;
@@ -1019,7 +1028,10 @@ __global__ void __launch_bounds__(256) delta_net_kernel(StepCtl c, const float* 
             else *reinterpret_cast<float2*>(&Sh[(size_t)row * DK + lane * 2]) = make_float2(s[i][0], s[i][1]);
             if (lane == 0) {
                 abuf[((size_t)b * H + h) * dv + row] = d2;
-                if (abuf16) abuf16[((size_t)b * H + h) * dv + row] = __float2bfloat16_rn(d2);
+                if (abuf16) {
+                    const int f = h * dv + row;
+                    abuf16[(size_t)b * H * dv + (perm ? perm16(f) : f)] = __float2bfloat16_rn(perm ? d2 * kOperandScale : d2);
+                }
             }
         }
     }

@@ -84,7 +84,7 @@ int run_attn(void* scratch, const void* kpool, const void* vpool, int kv_dtype, 
     c.tok_src = nullptr; c.host_out = nullptr; c.host_err = nullptr; c.dev_err = nullptr;
     AttnParams p;
     p.kpool = kpool; p.vpool = vpool; p.page_table = page_table; p.pt_stride = pt_stride;
-    p.qbuf = q; p.gbuf = gate; p.abuf = out; p.abuf16 = nullptr; p.part = sc.part; p.ticket = sc.ticket;
+    p.qbuf = q; p.gbuf = gate; p.abuf = out; p.abuf16 = nullptr; p.perm = 0; p.part = sc.part; p.ticket = sc.ticket;
     p.heads = heads; p.kv_heads = kv_heads; p.hg = 1;
     p.num_pages = num_pages; p.err = sc.err; p.min_pages_per_split = 1;
     const int G = heads / kv_heads;

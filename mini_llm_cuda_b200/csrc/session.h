@@ -1,6 +1,7 @@
 // Model and session of the decode path, and what the host files share: the launch chains of one step (chain.cuh, one
 // translation unit per weight type) and everything around them (engine.cu).
 #pragma once
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -11,6 +12,7 @@
 #include "errors.h"
 #include "kernels.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_dec.cuh"
 #include "tc_host.h"
 #include "grid_params.h"
 #include "lean_params.h"
@@ -153,6 +155,7 @@ struct mlb_session {
     mlb::LeanParams lean;
     // tensor-core projections (bf16 weights, batch >= 16)
     bool use_tc = false;
+    bool use_dec = false;                     // the step's projections on mma.sync tiles (gemm_dec.cuh) instead of tcgen05 ones
     int tc_nb = 0, tc_stages = 0, tc_stages_swiglu = 0;
     int tc_max_split = 8;                     // largest cluster that may split a GEMM's k-blocks
     bool tc_split_forced = false;             // MLB_TC_SPLIT given: take it as the limit without the k-blocks-per-CTA rule
@@ -167,7 +170,8 @@ struct mlb_session {
     mlb::bf16_t* tple16 = nullptr;           // [layers][B][ple] per-layer embedding rows of the step's tokens
     std::vector<TcLayerMaps> tc_maps;
     // activation operand maps per batch tile 16, 32, 64, 128, 256 (index log2(Nb/16))
-    struct alignas(64) TcGlobalMaps { CUtensorMap E, xn[5], a_attn[5], a_dn[5], h[5]; } tc_g;
+    // (decode GEMMs of gemm_dec.cuh: per tile of 16, 32, 64 sequences and 1, 2, 4 k-blocks, index gd_index)
+    struct alignas(64) TcGlobalMaps { CUtensorMap E, xn[9], a_attn[9], a_dn[9], h[9]; } tc_g;
     int* pinned_err = nullptr;
     // prompt columns: further sets of step buffers, `B` columns wide, that share this session's KV pool, page table,
     // delta-net state and stream; a column is one prompt token of one sequence. A set per power of two of columns,
@@ -257,6 +261,41 @@ static TcShape tc_pick_shape(const mlb_session* s, int B, int N, int nkb_all, in
         }
     }
     return best;
+}
+// Launch shape of a decode GEMM (gemm_dec.cuh).
+struct GdShape { int np, split, g, stages, w_bytes; size_t smem; };
+static int gd_index(int np, int g) { return (np >> 1) * 3 + (g >> 1); }       // np, g in {1, 2, 4}
+// mma.sync multiplies at about 512 a cycle and SM here (k-loop times against sequences per CTA), tcgen05 eight times as fast, so what
+// gemm_dec_kernel saves around the products it pays back in them once they are many. Measured per step, tcgen05 -> mma.sync: cfg1 372
+// -> 195 us at 4 sequences, 534 -> 455 at 256; cfg4 (gate/up 2 x 5632 x 2048) 2338 -> 1677 at 4, 3112 -> 2760 at 48 (7.5 M products
+// per SM in the gate/up projection, the largest), 2735 -> 2739 and behind long prompts 3385 -> 3440 at 64 (10 M). The line lies between.
+constexpr long kGdMostProducts = 8L << 20;
+static bool gd_small_enough(const mlb_session* s) {
+    return s->B <= 256 && 2L * s->m->cfg.ffn_dim * s->m->cfg.dim * s->B / s->sm_count <= kGdMostProducts;
+}
+// The k-ranges are those of the tcgen05 launch of the same batch (the results are the same bits). Sequences per CTA: the most
+// that still leaves 96 CTAs, two thirds of the SMs - fewer CTAs read the activations less often, more of them share the epilogue.
+static GdShape gd_pick(const mlb_session* s, int N, int nkb, int mode, bool w8, bool ext) {
+    GdShape g;
+    const int na = mode == TC_SWIGLU ? 2 : 1;
+    const bool ext2 = w8 && mode == TC_RESID;
+    g.split = std::max(1, tc_pick_shape(s, s->B, N, nkb, na, w8, na == 2 || ext2 ? 2 : 1).split);
+    g.np = 4;
+    while (g.np > 1 && (16 * (g.np / 2) >= s->B || (long)((N + kGdF - 1) / kGdF) * ((s->B + 16 * g.np - 1) / (16 * g.np)) < 96)) g.np >>= 1;
+    g.w_bytes = kGdF * (w8 && !ext ? 64 : 128);
+    const int ct = 16 * g.np;
+    // k-blocks per copy: as many as leave two stages
+    size_t stage = 0;
+    int n_iter = 1;
+    for (g.g = 4;; g.g >>= 1) {
+        stage = (size_t)g.split * g.g * (na * g.w_bytes + ct * 128);
+        n_iter = ((nkb + g.split - 1) / g.split + g.g - 1) / g.g + (ext ? 1 : 0);
+        if (g.g == 1 || stage * std::min(2, n_iter) <= kGdRing) break;
+    }
+    g.stages = (int)std::max<size_t>(1, std::min<size_t>(std::min(n_iter, kGdMaxStages), kGdRing / stage));
+    const size_t part = (size_t)g.split * (ext2 ? 2 : 1) * ct * (32 * na + 4) * 4;
+    g.smem = 1024 + std::max((size_t)g.stages * stage, part);
+    return g;
 }
 static int nb_index(int nb) { return nb == 16 ? 0 : nb == 32 ? 1 : nb == 64 ? 2 : nb == 128 ? 3 : 4; }
 

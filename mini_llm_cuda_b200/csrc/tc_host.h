@@ -41,6 +41,21 @@ static inline int make_u8_map(EncodeTiledFn enc, CUtensorMap* out, const void* b
     return MLB_OK;
 }
 
+// 3-D map over the same kind of matrix, bf16 (128-byte swizzle) or e4m3 codes (64-byte swizzle): (64 elements, rows, k-blocks of 64),
+// box = [g k-blocks][box_rows][64]. `cols` is a multiple of 64: a k-block that ended inside the row would run on into the next.
+static inline int make_kblock_map(EncodeTiledFn enc, CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t g, bool codes) {
+    const uint64_t esz = codes ? 1 : 2;
+    cuuint64_t dims[3] = {64, rows, cols / 64};
+    cuuint64_t strides[2] = {cols * esz, 64 * esz};
+    cuuint32_t box[3] = {64, box_rows, g};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(out, codes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, codes ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(MLB_E_CUDA, "cuTensorMapEncodeTiled (k-blocks) failed with code %d", (int)r);
+    return MLB_OK;
+}
+
 static inline EncodeTiledFn get_encode_tiled() {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
