@@ -714,26 +714,34 @@ cudaError_t embed_cols_launch(bool w8, bool pdl, cudaStream_t st, const StepCtl&
 // ------------------------------------------------------------------------------------------------
 // Projections (gemm_cols.cuh)
 // ------------------------------------------------------------------------------------------------
-template <int MODE, typename KVT>
+template <int MODE, typename KVT, bool SUMS>
 static cudaError_t gemm_cols_one(bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w, const CUtensorMap& w2,
                                  const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c, const QkvPostParams& q) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_cols_kernel<MODE, KVT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGcSmem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_cols_kernel<MODE, KVT, SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGcSmem);
     if (e != cudaSuccess) return e;
     const size_t smem = 1024 + (size_t)p.stages * (kGcM + p.BN) * 128;
-    return launch_pdl(pdl, gemm_cols_kernel<MODE, KVT>, dim3(ctas), dim3(kGcThreads), smem, st, x, w, w2, xx, wx, p, c, q);
+    return launch_pdl(pdl, gemm_cols_kernel<MODE, KVT, SUMS>, dim3(ctas), dim3(kGcThreads), smem, st, x, w, w2, xx, wx, p, c, q);
 }
 
-cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
+template <bool SUMS>
+static cudaError_t gemm_cols_mode(int mode, int kv_dtype, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
+                                  const CUtensorMap& w2, const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c,
+                                  const QkvPostParams& q) {
+    switch (mode) {
+        case TC_RAW: return gemm_cols_one<TC_RAW, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+        case TC_RESID: return gemm_cols_one<TC_RESID, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+        case TC_SWIGLU: return gemm_cols_one<TC_SWIGLU, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+        default:
+            if (kv_dtype == MLB_DT_F32) return gemm_cols_one<TC_QKV, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+            return gemm_cols_one<TC_QKV, bf16_t, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+    }
+}
+
+cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
                              const CUtensorMap& w2, const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c,
                              const QkvPostParams& q) {
-    switch (mode) {
-        case TC_RAW: return gemm_cols_one<TC_RAW, float>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-        case TC_RESID: return gemm_cols_one<TC_RESID, float>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-        case TC_SWIGLU: return gemm_cols_one<TC_SWIGLU, float>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-        default:
-            if (kv_dtype == MLB_DT_F32) return gemm_cols_one<TC_QKV, float>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-            return gemm_cols_one<TC_QKV, bf16_t>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-    }
+    if (sums) return gemm_cols_mode<true>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+    return gemm_cols_mode<false>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
 }
 
 static __global__ void __launch_bounds__(256) widen_e4m3_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n16) {

@@ -372,7 +372,7 @@ static int run_cols(mlb_session* s, int kind, int* n_launches) {
         p.y = y; p.h16 = h16; p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = parts; p.eps = cfg.rms_eps;
         p.xg16 = s->xn16; p.gain_next = next_gain; p.ssq_out = s->tc_ssq;
         p.s1 = s1; p.s2 = s2; p.err = s->dev_err;
-        CU(gemm_cols_launch(mode, cfg.kv_dtype, s->use_pdl, g.ctas, s->stream, X, W, W2, ext ? ext->pleT : X, ext ? ext->pleP : W, p, c, q ? *q : q0));
+        CU(gemm_cols_launch(mode, cfg.kv_dtype, g.sums, s->use_pdl, g.ctas, s->stream, X, W, W2, ext ? ext->pleT : X, ext ? ext->pleP : W, p, c, q ? *q : q0));
         ++launches;
         return MLB_OK;
     };
@@ -863,8 +863,9 @@ static int model_widen(mlb_model* m, cudaStream_t st) {
 // operand pair (`exts_apart`: with accumulators of its own), in `split` ranges. Tensor memory (512 columns) bounds BN x
 // accumulators x buffers. A 128 x BN x 64 k-block takes about 0.30 / 0.19 / 0.14 us at BN = 256 / 128 / 64 (the MMA's own
 // rate at 256, operand reads below), an epilogue 3 us at 256, hidden under the next tile's k-loop where there are two
-// buffers; the cheapest in the sum over a CTA's tiles wins.
-static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode, bool exts_apart, int split, int min_bn) {
+// buffers; the cheapest in the sum over a CTA's tiles wins. More ranges than one: sums in registers (64 a thread: BN <= 128) over
+// four accumulators in turn, except under a QK norm, which looks a head's features up in tensor memory.
+static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode, bool exts_apart, int split, int min_bn, bool qk_norm) {
     ColsGemm best{};
     double best_cost = -1.0;
     static const int bns[3] = {256, 128, 64};
@@ -875,10 +876,11 @@ static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode
         if (exts_apart ? lo < nkb - nkb_x : hi > lo) ++mains;
         if (exts_apart && hi > nkb - nkb_x) ++exts;
     }
-    for (int i = 0; i < 3; ++i) {
+    const bool sums = mains + exts > 1 && !(mode == TC_QKV && qk_norm) && exts < kGcMaxBufs;
+    for (int i = sums ? 1 : 0; i < 3; ++i) {
         const int bn = bns[i];
         for (int nbuf = 2; nbuf >= 1; --nbuf) {
-            if (bn < min_bn || bn * (mains + exts) * nbuf > 512) continue;
+            if (bn < min_bn || (!sums && bn * (mains + exts) * nbuf > 512)) continue;
             const int bn_out = mode == TC_SWIGLU ? bn / 2 : bn;
             const long tiles = (long)((T + kGcM - 1) / kGcM) * ((N + bn_out - 1) / bn_out);
             const long waves = (tiles + sm_count - 1) / sm_count;
@@ -890,9 +892,10 @@ static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode
                 best.bn = bn;
                 best.stages = (int)std::min<long>(std::min(fit, kGcMaxStages), std::max<long>(2, nkb * waves));
                 best.ctas = (int)std::min<long>(tiles, sm_count);
-                best.split = split; best.mains = mains; best.exts = exts; best.nbuf = nbuf;
+                best.split = split; best.mains = mains; best.exts = exts; best.sums = sums;
+                best.nbuf = sums ? kGcMaxBufs : nbuf;
                 best.tmem_cols = 32;
-                while (best.tmem_cols < (uint32_t)(bn * (mains + exts) * nbuf)) best.tmem_cols <<= 1;
+                while (best.tmem_cols < (uint32_t)(bn * (sums ? kGcMaxBufs : (mains + exts) * nbuf))) best.tmem_cols <<= 1;
             }
             break;
         }
@@ -927,7 +930,7 @@ static int setup_cols_path(mlb_session* s) {
         const bool resid8 = w8 && mode == TC_RESID;
         const TcShape ref = tc_pick_shape(s, kTcRefCols, N, nkb, mode == TC_SWIGLU ? 2 : 1, w8, mode == TC_SWIGLU || resid8 ? 2 : 1);
         const ColsGemm g = gc_pick(s->sm_count, T, N, nkb, nkb_x, mode, apart, std::max(1, ref.split),
-                                    mode == TC_QKV && c.qk_norm ? c.head_dim : 64);       // a tile holds whole heads for their norm
+                                    mode == TC_QKV && c.qk_norm ? c.head_dim : 64, c.qk_norm != 0);       // a tile holds whole heads for their norm
         fits = fits && g.bn > 0;
         return g;
     };

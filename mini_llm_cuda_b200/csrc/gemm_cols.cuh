@@ -18,7 +18,10 @@
 // in another order end, some layers later, in other roundings and now and then in another token. That kernel splits the
 // k-blocks of a tile over the CTAs of a cluster and adds their partial accumulators in order; here the same ranges of
 // k-blocks go to accumulators of their own (`split`), and the sums of squares are taken over 32 features at a time in the
-// order of its warp shuffles.
+// order of its warp shuffles. SUMS: the ranges take turns with four accumulators of 128 columns, and the epilogue's threads
+// add each finished one to sums in registers (64 per thread), so the MMAs go on whatever the number of ranges. Holding all
+// of a tile's accumulators in tensor memory until its epilogue left five of them BN = 64 and no second set: cfg4's O and
+// down projections at 32768 prompt tokens took 75 ms.
 // Every mbarrier wait is bounded; one that runs out records a code and the CTA drains without waiting further.
 #pragma once
 #include "gemm_tc.cuh"
@@ -29,6 +32,7 @@ constexpr int kGcM = 128;
 constexpr int kGcEpiWarps = 8;
 constexpr int kGcThreads = 64 + 32 * kGcEpiWarps;
 constexpr int kGcMaxStages = 8;
+constexpr int kGcMaxBufs = 4;
 constexpr size_t kGcSmem = 224 * 1024;
 
 struct GemmColsParams {
@@ -36,7 +40,7 @@ struct GemmColsParams {
     int stages, nkb_x;             // ring depth; k-blocks taken from the second operand pair
     int split, mains, exts;        // ranges of k-blocks; of them, how many hold k-blocks of the main pair / of a second pair that
                                    // accumulates separately (scaled weights; 0: it shares the main accumulators)
-    int nbuf;                      // sets of accumulators in tensor memory: 2 = epilogue under the next k-loop
+    int nbuf;                      // sets of accumulators in tensor memory: 2 = epilogue under the next k-loop; SUMS: accumulators, used in turn
     uint32_t tmem_cols;
     int early_w;                   // weight tiles may be fetched before the predecessor kernel has finished
     float* y;                      // RAW: fp32 [c][N]; RESID: residual stream, updated in place
@@ -81,7 +85,7 @@ __device__ __forceinline__ void ld_feat16(const float* p, float* v) {
     }
 }
 
-template <int MODE, typename KVT>
+template <int MODE, typename KVT, bool SUMS>
 __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                                                                   const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmXx,
                                                                   const __grid_constant__ CUtensorMap tmWx, const __grid_constant__ GemmColsParams p,
@@ -93,20 +97,20 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
     const int n_tiles = n_m * n_n;
     if ((int)blockIdx.x >= n_tiles) return;
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t bars[2 * kGcMaxStages + 4];
+    __shared__ __align__(8) uint64_t bars[2 * kGcMaxStages + 2 * kGcMaxBufs];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8u * kGcMaxStages;
-    const uint32_t tfull0 = empty0 + 8u * kGcMaxStages, tempty0 = tfull0 + 16u;
+    const uint32_t tfull0 = empty0 + 8u * kGcMaxStages, tempty0 = tfull0 + 8u * kGcMaxBufs;
     const int a_bytes = kGcM * 128, stage_bytes = a_bytes + p.BN * 128;
     const int nkb1 = (p.K + kTcKB - 1) / kTcKB, nkb = nkb1 + p.nkb_x;
-    const uint32_t acc_cols = (uint32_t)((p.mains + p.exts) * p.BN);
+    const uint32_t acc_cols = (uint32_t)((SUMS ? 1 : p.mains + p.exts) * p.BN);
     if (tid == 0) {
         for (int i = 0; i < p.stages; ++i) {
             mbar_init(full0 + 8u * i, 1);
             mbar_init(empty0 + 8u * i, 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kGcMaxBufs; ++i) {
             mbar_init(tfull0 + 8u * i, 1);
             mbar_init(tempty0 + 8u * i, kGcEpiWarps);
         }
@@ -170,8 +174,10 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
             uint32_t ph = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++i) {
-                if (i >= p.nbuf && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
-                tc_fence_after();
+                if (!SUMS) {
+                    if (i >= p.nbuf && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
+                    tc_fence_after();
+                }
                 const uint32_t acc = tmem + buf * acc_cols;
                 int r = 0, hi = nkb / p.split;           // range of k-blocks: [nkb r / split, nkb (r + 1) / split)
                 bool fresh = true, xfresh = true;        // the next MMA starts its accumulator
@@ -186,8 +192,17 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                     const uint32_t base = ring + (uint32_t)(s * stage_bytes);
                     const uint64_t ad = umma_desc_sw128(base), bd = umma_desc_sw128(base + a_bytes);
                     const bool ext = p.exts > 0 && kb >= nkb1;
+                    if (SUMS && (ext ? xfresh : fresh)) {
+                        // the next accumulator in turn; the one before it is complete
+                        if (kb > 0) {
+                            umma_commit(tfull0 + 8u * buf);
+                            if (++buf == p.nbuf) { buf = 0; ++use; }
+                        }
+                        if (use > 0 && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
+                        tc_fence_after();
+                    }
                     // the separate accumulators of the second pair lie behind the main ones, its ranges are the last ones
-                    const uint32_t dst = acc + (uint32_t)((ext ? p.mains + r - (p.split - p.exts) : r) * p.BN);
+                    const uint32_t dst = SUMS ? tmem + (uint32_t)(buf * p.BN) : acc + (uint32_t)((ext ? p.mains + r - (p.split - p.exts) : r) * p.BN);
                     const bool first = ext ? xfresh : fresh;
 #pragma unroll
                     for (int j = 0; j < kTcKB / 16; ++j) umma_bf16(dst, ad + 2u * j, bd + 2u * j, idesc, (first && j == 0) ? 0u : 1u);
@@ -238,7 +253,48 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                 }
             };
             if (MODE == TC_RESID) load_resid(f_begin);
-            if (!tc_wait(tfull0 + 8u * buf, (uint32_t)use & 1u, p.err, 24)) { ok = false; break; }
+            // SUMS: the ranges' accumulators arrive one after another and are added up here, in their order, each given back at once.
+            // 64 sums per thread: BN = 128 (SWIGLU: 32 of gate, 32 of up)
+            float sums[SUMS ? 64 : 1];
+            if (SUMS) {
+                for (int r = 0; r < p.mains && ok; ++r) {
+                    ok = tc_wait(tfull0 + 8u * buf, (uint32_t)use & 1u, p.err, 24);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a = tmem + (uint32_t)(buf * p.BN) + lane_base;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t ta[2][16];
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int ch = 2 * h + k;
+                            const bool here = MODE == TC_SWIGLU ? 16 * k < span : 16 * ch < span;
+                            if (here) tmem_ld16_issue(a + (uint32_t)(MODE == TC_SWIGLU ? h * bn_out + half * span + 16 * k : half * span + 16 * ch), ta[k]);
+                        }
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                float& o = sums[SUMS ? 16 * (2 * h + k) + j : 0];
+                                o = r == 0 ? __uint_as_float(ta[k][j]) : __fadd_rn(o, __uint_as_float(ta[k][j]));
+                            }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty0 + 8u * buf);
+                    if (++buf == p.nbuf) { buf = 0; ++use; }
+                }
+                // accumulators of the second pair stay where they are until the element-wise work below has read them
+                for (int r = 0, b = buf, u = use; r < p.exts && ok; ++r) {
+                    ok = tc_wait(tfull0 + 8u * b, (uint32_t)u & 1u, p.err, 24);
+                    if (++b == p.nbuf) { b = 0; ++u; }
+                }
+                if (!ok) break;
+            } else if (!tc_wait(tfull0 + 8u * buf, (uint32_t)use & 1u, p.err, 24)) {
+                ok = false;
+                break;
+            }
             tc_fence_after();
             const uint32_t acc = tmem + buf * acc_cols + lane_base;
             float head_sc = 1.0f, sqp[16];
@@ -275,6 +331,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                     for (int j = 0; j < w; ++j) t[j] += t[j + w];
                 return t[0];
             };
+#pragma unroll 1
             for (int cc = 0; cc < span; cc += 16) {
                 const int f0 = f_begin + cc, col = half * span + cc;
                 if (f0 >= p.N) {                       // uniform for the warp; the sums of squares behind the last feature are zero
@@ -293,9 +350,35 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                 const bool whole = f0 + 16 <= p.N;
                 __syncwarp();                          // tcgen05.ld is a warp-wide instruction
                 float v[16], w2[16];
-                load_acc(acc + (uint32_t)col, p.mains, v);
-                if (MODE == TC_SWIGLU) load_acc(acc + (uint32_t)(bn_out + col), p.mains, w2);
-                if (MODE == TC_RESID && p.exts > 0) load_acc(acc + (uint32_t)(p.mains * p.BN + col), p.exts, w2);
+                if constexpr (SUMS) {
+                    // the front 16 of the sums; the others move up, so that a rolled loop names registers
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        v[j] = sums[j];
+                        sums[j] = sums[16 + j];
+                        if (MODE == TC_SWIGLU) {
+                            w2[j] = sums[32 + j];
+                            sums[32 + j] = sums[48 + j];
+                        } else {
+                            sums[16 + j] = sums[32 + j];
+                            sums[32 + j] = sums[48 + j];
+                        }
+                    }
+                    if (MODE == TC_RESID && p.exts > 0) {
+                        load_acc(acc + (uint32_t)col, 1, w2);
+                        for (int r = 1, b = buf; r < p.exts; ++r) {
+                            if (++b == p.nbuf) b = 0;
+                            float e[16];
+                            load_acc(tmem + (uint32_t)(b * p.BN + col) + lane_base, 1, e);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) w2[j] = __fadd_rn(w2[j], e[j]);
+                        }
+                    }
+                } else {
+                    load_acc(acc + (uint32_t)col, p.mains, v);
+                    if (MODE == TC_SWIGLU) load_acc(acc + (uint32_t)(bn_out + col), p.mains, w2);
+                    if (MODE == TC_RESID && p.exts > 0) load_acc(acc + (uint32_t)(p.mains * p.BN + col), p.exts, w2);
+                }
                 if (MODE == TC_SWIGLU) {
                     float sa[16], sb[16];
                     if (p.s1 != nullptr && whole) {
@@ -402,7 +485,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                     const int e0 = fs % q.hd, head = fs / q.hd;
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] *= rinv;
-                    if (seg < 2 && q.qk_norm) {
+                    if (!SUMS && seg < 2 && q.qk_norm) {
                         // per-head RMS norm (inference.cu:52-81, :97-111): the head's other features come from tensor memory
                         if (e0 == 0 || cc == 0) {
                             float ss = 0.f;
@@ -453,8 +536,10 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(tempty0 + 8u * buf);
-            if (++buf == p.nbuf) { buf = 0; ++use; }
+            for (int r = 0; r < (SUMS ? p.exts : 1); ++r) {
+                if (lane == 0) mbar_arrive(tempty0 + 8u * buf);
+                if (++buf == p.nbuf) { buf = 0; ++use; }
+            }
         }
     }
     __syncthreads();
