@@ -224,32 +224,63 @@ struct RowsJob {
     int* ocnt;                     // how many of them are finished (shared memory, zero between phases)
 };
 
-template <typename T>
-__device__ __forceinline__ float smem_row_dot(const T* row, int nvec, const float* xs, int lane) {
+// Dot products of N rows with x, every one in the order of a single row's; one read of x serves all of them. With FP8 weights x is
+// four bytes to a byte of weights: 15 warps with a row each read 75 x 16 bytes per lane and 512 columns, and the shared-memory
+// pipe (300 cycles) was what an iteration took.
+template <typename T, int N>
+__device__ __forceinline__ void smem_rows_dot(const T* const (&row)[N], int nvec, const float* xs, int lane, float (&v)[N]) {
     constexpr int EPV = Elem<T>::EPV;
     const float4* xp = reinterpret_cast<const float4*>(xs);
-    float a0 = 0.f, a1 = 0.f;
+    float a0[N], a1[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) a0[i] = a1[i] = 0.f;
 #pragma unroll 1
     for (int vi = lane; vi < nvec; vi += 32) {
-        float w[EPV];
-        Elem<T>::unpack(*reinterpret_cast<const uint4*>(row + (size_t)vi * EPV), w);
+        uint4 raw[N];
 #pragma unroll
-        for (int q = 0; q < EPV / 4; ++q) {
-            const float4 t = xp[q * nvec + vi];
-            a0 = fmaf(w[4 * q], t.x, a0); a1 = fmaf(w[4 * q + 1], t.y, a1);
-            a0 = fmaf(w[4 * q + 2], t.z, a0); a1 = fmaf(w[4 * q + 3], t.w, a1);
+        for (int i = 0; i < N; ++i) raw[i] = *reinterpret_cast<const uint4*>(row[i] + (size_t)vi * EPV);
+        float4 t[EPV / 4];
+#pragma unroll
+        for (int q = 0; q < EPV / 4; ++q) t[q] = xp[q * nvec + vi];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            float w[EPV];
+            Elem<T>::unpack(raw[i], w);
+#pragma unroll
+            for (int q = 0; q < EPV / 4; ++q) {
+                a0[i] = fmaf(w[4 * q], t[q].x, a0[i]); a1[i] = fmaf(w[4 * q + 1], t[q].y, a1[i]);
+                a0[i] = fmaf(w[4 * q + 2], t[q].z, a0[i]); a1[i] = fmaf(w[4 * q + 3], t[q].w, a1[i]);
+            }
         }
     }
-    return warp_sum(a0 + a1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = warp_sum(a0[i] + a1[i]);
+}
+
+// Local row of a warp's i-th unit (a row, or two neighbouring ones): units go round the warps.
+__device__ __forceinline__ int unit_row(int warp, int i, int two) { return (warp + kRingWarps * i) << two; }
+// Two rows to a unit: with FP8 weights for what they save in reads of x, otherwise where rows outnumber the warps (else idle warps
+// would be the price: 3 to 14 rows of a phase in the fp32 models). The chunks of the ring then hold whole units.
+template <typename T>
+__device__ __forceinline__ int rows_two(const Ring& r, int rows, int K) {
+    const int rpc = max(1, r.stage_bytes / (K * (int)sizeof(T)));
+    return (sizeof(T) == 1 || rows > kRingWarps) && (rpc % 2 == 0 || rows <= rpc) && rows > 1 ? 1 : 0;
+}
+// Scale of the row that lane `lane` stands for among the warp's units i .. i + 31 (15 with two rows): a warp asks for all of its scales before
+// it waits for the phase's input. They come from HBM, 1700 cycles a row where they were asked for with the row.
+__device__ __forceinline__ float lane_scale(const float* scale, int r0, int rows, int warp, int lane, int i, int two) {
+    const int row = unit_row(warp, i + (lane >> two), two) + (two ? lane & 1 : 0);
+    return scale != nullptr && row < rows ? __ldg(scale + r0 + row) : 1.0f;
 }
 
 template <typename T>
-__device__ __forceinline__ void consume_rows(Ring& r, const RowsJob& j, bool pair, int warp, int lane, float& bv, int& bi, long long* tm) {
+__device__ __forceinline__ void consume_rows(Ring& r, const RowsJob& j, bool pair, int warp, int lane, float sl, float sl2, float& bv, int& bi, long long* tm) {
     (void)tm;
     constexpr int EPV = Elem<T>::EPV;
     constexpr int NW = kRingWarps;
     const int K = j.K, rows = j.rows, nvec = K / EPV;
     const int rpc = max(1, r.stage_bytes / (K * (int)sizeof(T)));
+    const int two = rows_two<T>(r, rows, K);
     // the norm of the input (inference.cu:24-50, :83-95): every warp adds up the threads' sums of squares
     float rn = 1.0f;
     if (j.norm_n > 0) {
@@ -258,7 +289,8 @@ __device__ __forceinline__ void consume_rows(Ring& r, const RowsJob& j, bool pai
         for (int i = 0; i < NW; ++i) t += j.red[lane + 32 * i];
         rn = rsqrtf(__fdividef(warp_sum(t), (float)j.norm_n) + j.eps);
     }
-    int wrow = warp;                       // this warp's next local row
+    int unit = 0;                          // this warp's next unit
+    int wrow = unit_row(warp, 0, two);     // and its first local row
 #pragma unroll 1
     for (int c0 = 0; c0 < rows; c0 += rpc) {
         const int n = min(rpc, rows - c0);
@@ -274,41 +306,70 @@ __device__ __forceinline__ void consume_rows(Ring& r, const RowsJob& j, bool pai
         const T* A = reinterpret_cast<const T*>(r.stages + (size_t)ia * r.stage_bytes);
         const T* Bm = reinterpret_cast<const T*>(r.stages + (size_t)ib * r.stage_bytes);
 #pragma unroll 1
-        for (; wrow < c0 + n; wrow += NW) {
-            const size_t off = (size_t)(wrow - c0) * K;
-            const int row = j.r0 + wrow;
-            // the row's scales come from global memory: asked for before the dot products, used after
-            const float sv = j.scale ? j.scale[row] : 1.0f;
-            const float su = j.scale2 ? j.scale2[row] : 1.0f;
-            float v = smem_row_dot<T>(A + off, nvec, j.xs, lane);
-            float u = 0.f;
-            if (pair) u = smem_row_dot<T>(Bm + off, nvec, j.xs, lane);
+        for (; wrow < c0 + n; wrow = unit_row(warp, ++unit, two)) {
+            const int nr = two ? min(2, rows - wrow) : 1;      // rows of this unit
+            const int at = (unit << two) & 31;                 // lane with the scale of its first row
+            if (at == 0 && unit > 0) {
+                sl = lane_scale(j.scale, j.r0, rows, warp, lane, unit, two);
+                sl2 = lane_scale(j.scale2, j.r0, rows, warp, lane, unit, two);
+            }
+            const T* a0 = A + (size_t)(wrow - c0) * K;
+            const T* a1 = nr == 2 ? a0 + K : a0;
+            float v0, v1 = 0.f, u0 = 0.f, u1 = 0.f;
+            if (pair) {
+                const T* b0 = Bm + (size_t)(wrow - c0) * K;
+                if (two) {
+                    const T* const rw[4] = {a0, a1, b0, nr == 2 ? b0 + K : b0};
+                    float o[4];
+                    smem_rows_dot<T, 4>(rw, nvec, j.xs, lane, o);
+                    v0 = o[0]; v1 = o[1]; u0 = o[2]; u1 = o[3];
+                } else {
+                    const T* const rw[2] = {a0, b0};
+                    float o[2];
+                    smem_rows_dot<T, 2>(rw, nvec, j.xs, lane, o);
+                    v0 = o[0]; u0 = o[1];
+                }
+            } else if (two) {
+                const T* const rw[2] = {a0, a1};
+                float o[2];
+                smem_rows_dot<T, 2>(rw, nvec, j.xs, lane, o);
+                v0 = o[0]; v1 = o[1];
+            } else {
+                const T* const rw[1] = {a0};
+                float o[1];
+                smem_rows_dot<T, 1>(rw, nvec, j.xs, lane, o);
+                v0 = o[0];
+            }
             // The finished rows are collected in shared memory and the warp that finishes the CTA's last
             // one publishes the whole slot with one store instruction per 32 rows: a line that every CTA
             // polls must change once. (Measured on B200: rows stored one by one by their warps, a few
             // dozen cycles apart, make an exchange cost 3-4 us instead of 1.2 us.)
+            // Lane 0 finishes the unit's first row, lane 1 its second.
+            const float sv = __shfl_sync(0xffffffffu, sl, at + (lane & 1)), su = __shfl_sync(0xffffffffu, sl2, at + (lane & 1));
+            float v = lane == 0 ? v0 : v1;
+            const float u = lane == 0 ? u0 : u1;
+            const int lrow = wrow + (lane & 1), row = j.r0 + lrow;
             int last = 0;
-            if (lane == 0) {
+            if (lane < nr) {
                 v = (v * sv) * rn;
                 if (j.mode == RJ_SWIGLU) {
                     // applySiluToFFN + hadamardMultiplyFFN, inference.cu:262-281
                     v = __fdividef(v, 1.0f + __expf(-v)) * ((u * su) * rn);
                 } else if (j.mode == RJ_RESID) {
-                    if (j.pacc) v += j.pacc[wrow];
+                    if (j.pacc) v += j.pacc[lrow];
                     v += j.resid[row];
                 }
                 if (j.mode == RJ_LM) {
                     j.logits[row] = v;
                     if (v > bv || (v == bv && row < bi)) { bv = v; bi = row; }
                 } else {
-                    j.obuf[wrow] = v;
+                    j.obuf[lrow] = v;
                     __threadfence_block();
                     last = atomicAdd(j.ocnt, 1) == rows - 1;
                 }
             }
             if (j.mode != RJ_LM) {
-                last = __shfl_sync(0xffffffffu, last, 0);
-                if (last) {
+                if (__any_sync(0xffffffffu, last)) {
                     __threadfence_block();
 #pragma unroll 1
                     for (int q = lane; q < rows; q += 32) ll_store(j.dst + q, j.obuf[q], j.epoch);
@@ -824,17 +885,38 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
     // One warp per (layer, row of this CTA); all layers at once, before the first exchange.
     if (p.ple > 0) {
         const int n = p.n_layers * xrows;
+        // Four of them at a time, four columns per lane each: 32 loads from HBM in flight instead of two (24 layers x 14 rows of 128
+        // columns took 37 us of a 980 us step).
 #pragma unroll 1
-        for (int i = warp; i < n; i += kRingWarps) {
-            const int l = i / xrows, j = i - l * xrows;
-            const StepLayer& L = k.layers[l];
-            const T2* Pm = reinterpret_cast<const T2*>(L.pleP) + (size_t)(xr0 + j) * p.ple;
-            const T2* Tb = reinterpret_cast<const T2*>(L.pleT) + (size_t)tok * p.ple;
-            float a = 0.f;
+        for (int i0 = warp; i0 < n; i0 += 4 * kRingWarps) {
+            float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-            for (int q = lane; q < p.ple; q += 32) a = fmaf(Elem<T2>::get(Pm, q), Elem<T2>::get(Tb, q), a);
-            a = warp_sum(a);
-            if (lane == 0) pacc[l * pacc_stride + j] = a;
+            for (int q0 = lane; q0 < p.ple; q0 += 128) {
+                float x[4][4], y[4][4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int i = min(i0 + u * kRingWarps, n - 1), l = i / xrows, j = i - l * xrows;
+                    const StepLayer& L = k.layers[l];
+                    const T2* Pm = reinterpret_cast<const T2*>(L.pleP) + (size_t)(xr0 + j) * p.ple;
+                    const T2* Tb = reinterpret_cast<const T2*>(L.pleT) + (size_t)tok * p.ple;
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        const int q = q0 + 32 * w;
+                        x[u][w] = q < p.ple ? Elem<T2>::get(Pm, q) : 0.f;
+                        y[u][w] = q < p.ple ? Elem<T2>::get(Tb, q) : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) a[u] = fmaf(x[u][w], y[u][w], a[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * kRingWarps, l = i / xrows, j = i - l * xrows;
+                const float t = warp_sum(a[u]);
+                if (lane == 0 && i < n) pacc[l * pacc_stride + j] = t;
+            }
         }
         consumer_sync();
     }
@@ -928,6 +1010,19 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
             gain = p.g_final;
             job.mode = RJ_LM; job.scale = p.Es;
         }
+        // ---- this CTA's rows, and their scales: asked for here, used after the dot products -----------------------------
+        int r0, r1;
+        if (vout) {
+            vec_rows(*vout, k.tabs, rank, r0, r1);
+            job.dst = vec_slot(*vout, rank);
+        } else {
+            r0 = k.tabs[p.vocab_tab + rank];
+            r1 = k.tabs[p.vocab_tab + rank + 1];
+            job.dst = nullptr;
+        }
+        job.rows = r1 - r0; job.K = K; job.r0 = r0; job.xs = xs;
+        const int two = rows_two<T>(ring, job.rows, K);
+        const float sl = lane_scale(job.scale, r0, job.rows, warp, lane, 0, two), sl2 = lane_scale(job.scale2, r0, job.rows, warp, lane, 0, two);
         // ---- fetch the input; the RMS norm's sum of squares goes along ----------------------------------------------
         float* red = redb[ri];
         if (gain) ri ^= 1;
@@ -936,30 +1031,26 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
         if (gain) red[tid] = ss;
         consumer_sync();
         grid_mark(k, tslot);
-        // ---- this CTA's rows ------------------------------------------------------------------------------------------
-        int r0, r1;
-        if (vout) {
-            vec_rows(*vout, k.tabs, rank, r0, r1);
-            job.dst = vec_slot(*vout, rank);
-            job.epoch = ++e;
-        } else {
-            r0 = k.tabs[p.vocab_tab + rank];
-            r1 = k.tabs[p.vocab_tab + rank + 1];
-            job.dst = nullptr;
-            job.epoch = 0;
-        }
-        job.rows = r1 - r0; job.K = K; job.r0 = r0; job.xs = xs;
+        job.epoch = vout ? ++e : 0;
         job.norm_n = gain ? d : 0; job.red = red;
-        consume_rows<T>(ring, job, pair, warp, lane, bv, bi, k.tm);
+        consume_rows<T>(ring, job, pair, warp, lane, sl, sl2, bv, bi, k.tm);
         e_in = e;
         if (ph == PH_PROJ) e_proj = e;
         grid_mark(k, tslot + 1);
     }
 
     if (p.with_lm_head) {
-        // reduce the warps' argmax picks (lane 0 of each warp holds them), then (in CTA 0) the grid's
+        // reduce the warps' argmax picks (lanes 0 and 1 of each warp hold them), then (in CTA 0) the grid's
         float* tmp = smem + p.off_mix;
-        if (lane == 0) { tmp[2 * warp] = bv; tmp[2 * warp + 1] = __int_as_float(bi); }
+        {
+            const float v1 = __shfl_sync(0xffffffffu, bv, 1);
+            const int i1 = __shfl_sync(0xffffffffu, bi, 1);
+            if (lane == 0) {
+                if (v1 > bv || (v1 == bv && i1 < bi)) { bv = v1; bi = i1; }
+                tmp[2 * warp] = bv;
+                tmp[2 * warp + 1] = __int_as_float(bi);
+            }
+        }
         consumer_sync();
         ++e;
         if (tid == 0) {
