@@ -104,18 +104,18 @@ __device__ __forceinline__ void vec_rows(const GridVec& v, const int* tabs, int 
 }
 __device__ __forceinline__ unsigned long long* vec_slot(const GridVec& v, int rank) { return v.buf + (size_t)rank * v.slotw; }
 
-// Poll until the four words carry epoch `e`; at most kGridSpinLimit rounds. The caller passes
-// four valid addresses (a thread with fewer words repeats one).
-__device__ __forceinline__ void ll_poll4(const unsigned long long* s0, const unsigned long long* s1, const unsigned long long* s2,
-                                         const unsigned long long* s3, unsigned long long (&w)[4], uint32_t e, volatile int* dead, int* err) {
+// Poll until the N words carry epoch `e`; at most kGridSpinLimit rounds. The caller passes
+// N valid addresses (a thread with fewer words repeats one).
+template <int N>
+__device__ __forceinline__ void ll_poll(const unsigned long long* const (&src)[N], unsigned long long (&w)[N], uint32_t e, volatile int* dead, int* err) {
     uint32_t spins = 0;
 #pragma unroll 1
     for (;;) {
-        w[0] = ll_load(s0);
-        w[1] = ll_load(s1);
-        w[2] = ll_load(s2);
-        w[3] = ll_load(s3);
-        const bool ok = (uint32_t)(w[0] >> 32) == e && (uint32_t)(w[1] >> 32) == e && (uint32_t)(w[2] >> 32) == e && (uint32_t)(w[3] >> 32) == e;
+        bool ok = true;
+#pragma unroll
+        for (int u = 0; u < N; ++u) w[u] = ll_load(src[u]);
+#pragma unroll
+        for (int u = 0; u < N; ++u) ok = ok && (uint32_t)(w[u] >> 32) == e;
         if (ok) break;
         if (*dead) break;
         __nanosleep(MLB_POLL_SLEEP);
@@ -130,8 +130,8 @@ __device__ __forceinline__ void ll_poll4(const unsigned long long* s0, const uns
 // The whole vector. Row r goes to lin[r] (if lin) and, multiplied by gain[r] (if gain), to the GEMV
 // layout of nvec weight vectors at xs. Returns the sum of squares of what this thread fetched.
 // The gains are asked for before the polls start. `tabs`: shared memory seen as ints.
-template <int EPV>
-__device__ __noinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* lin, float* xs, int nvec,
+template <int EPV, int U>
+__device__ __noinline__ float ll_gather_vec_u(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* lin, float* xs, int nvec,
                                             const int* tabs, volatile int* dead, int* err) {
     const int P = vp->P, rpc = vp->rpc, slotw = vp->slotw, tab = vp->tab;
     const unsigned magic = vp->magic;
@@ -139,13 +139,13 @@ __device__ __noinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const
     const int n = P * rpc;
     float ss = 0.f;
 #pragma unroll 1
-    for (int q0 = threadIdx.x; q0 < n; q0 += kRingConsumers * 4) {
-        const unsigned long long* src[4];
-        unsigned long long w[4];
-        int row[4];
-        float g[4];
+    for (int q0 = threadIdx.x; q0 < n; q0 += kRingConsumers * U) {
+        const unsigned long long* src[U];
+        unsigned long long w[U];
+        int row[U];
+        float g[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             // slot q of the vector: producer c, its j-th word. A thread past the end, or on the unused last
             // word of a producer with one row less, repeats the producer's first word and drops it.
             const int q = min(q0 + u * kRingConsumers, n - 1);
@@ -157,9 +157,9 @@ __device__ __noinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const
             src[u] = buf + (size_t)c * slotw + (valid ? j : 0);
             g[u] = (gain != nullptr && valid) ? gain[r0 + j] : 1.0f;
         }
-        ll_poll4(src[0], src[1], src[2], src[3], w, e, dead, err);
+        ll_poll(src, w, e, dead, err);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             if (row[u] >= 0) {
                 const float val = __uint_as_float((uint32_t)w[u]);
                 if (lin) lin[row[u]] = val;
@@ -171,19 +171,37 @@ __device__ __noinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const
     return ss;
 }
 
-// Rows [row0, row0 + n) of a vector to dst[0..n).
-static __device__ __noinline__ void ll_gather_rows(const GridVec* vp, int row0, int n, uint32_t e, float* dst, const int* tabs, volatile int* dead,
-                                            int* err) {
+// U words of a thread in flight, whatever it needs for one round trip (0.6 us under 148 polling CTAs), up to five: 960, 1920, 2400 rows.
+// Not more: the code of eight is fetched cold every time (a cfg4 step took 1470 us with it, 912 with four, 881 with five), and words
+// asked for twice cost too (cfg0 87 us with four, 91 with five).
+template <int EPV>
+__device__ __forceinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* lin, float* xs, int nvec,
+                                               const int* tabs, volatile int* dead, int* err) {
+    const int n = vp->P * vp->rpc;
+    if (n <= 2 * kRingConsumers) return ll_gather_vec_u<EPV, 2>(vp, e, gain, lin, xs, nvec, tabs, dead, err);
+    if (n <= 4 * kRingConsumers) return ll_gather_vec_u<EPV, 4>(vp, e, gain, lin, xs, nvec, tabs, dead, err);
+    return ll_gather_vec_u<EPV, 5>(vp, e, gain, lin, xs, nvec, tabs, dead, err);
+}
+
+// n rows of a vector to dst[0..n): entry i is row ri + i - si of the last of the segments (ri, si) with si <= i, the first being
+// (r0, 0). A mixer's pieces of a projection arrive together, in one round trip.
+static __device__ __noinline__ void ll_gather_rows(const GridVec* vp, int n, int r0, int r1, int s1, int r2, int s2, int r3, int s3, int r4, int s4,
+                                                   uint32_t e, float* dst, const int* tabs, volatile int* dead, int* err) {
     const int P = vp->P, slotw = vp->slotw, tab = vp->tab;
     const float pn = (float)P * vp->inv_n;
     const unsigned long long* buf = vp->buf;
 #pragma unroll 1
-    for (int i0 = threadIdx.x; i0 < n; i0 += kRingConsumers * 4) {
-        const unsigned long long* src[4];
-        unsigned long long w[4];
+    for (int i0 = threadIdx.x; i0 < n; i0 += kRingConsumers * 2) {
+        const unsigned long long* src[2];
+        unsigned long long w[2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int row = row0 + min(i0 + u * kRingConsumers, n - 1);
+        for (int u = 0; u < 2; ++u) {
+            const int i = min(i0 + u * kRingConsumers, n - 1);
+            int row = r0 + i;
+            if (i >= s1) row = r1 + i - s1;
+            if (i >= s2) row = r2 + i - s2;
+            if (i >= s3) row = r3 + i - s3;
+            if (i >= s4) row = r4 + i - s4;
             // owner of a row under r0(c) = floor(c N / P) is floor(((row + 1) P - 1) / N): estimated in
             // floating point (off by one at most), settled against the row table
             int c = min(P - 1, (int)(((float)row + 0.5f) * pn));
@@ -191,12 +209,13 @@ static __device__ __noinline__ void ll_gather_rows(const GridVec* vp, int row0, 
             else if (tabs[tab + c + 1] <= row) ++c;
             src[u] = buf + (size_t)c * slotw + (row - tabs[tab + c]);
         }
-        ll_poll4(src[0], src[1], src[2], src[3], w, e, dead, err);
+        ll_poll(src, w, e, dead, err);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 2; ++u)
             if (i0 + u * kRingConsumers < n) dst[i0 + u * kRingConsumers] = __uint_as_float((uint32_t)w[u]);
     }
 }
+constexpr int kNoSeg = 0x7fffffff;
 
 template <typename KVT> __device__ __forceinline__ float round_kv(float v);
 template <> __device__ __forceinline__ float round_kv<float>(float v) { return v; }
@@ -439,11 +458,8 @@ __device__ __forceinline__ void grid_attention(const GridParams& p, const StepLa
     Ring& ring = k.ring;
 
     // (a) raw projections of the item's query heads (+ this step's key and value row)
-    ll_gather_rows(&p.vproj_attn, h0 * HD, G * HD, e_proj, tq, k.tabs, k.dead, k.err);
-    if (it.cur_here) {
-        ll_gather_rows(&p.vproj_attn, L.nq + kvh * HD, HD, e_proj, tk, k.tabs, k.dead, k.err);
-        ll_gather_rows(&p.vproj_attn, L.nq + L.nk + kvh * HD, HD, e_proj, tv, k.tabs, k.dead, k.err);
-    }
+    ll_gather_rows(&p.vproj_attn, (G + (it.cur_here ? 2 : 0)) * HD, h0 * HD, L.nq + kvh * HD, G * HD, L.nq + L.nk + kvh * HD, (G + 1) * HD, 0, kNoSeg, 0, kNoSeg,
+                   e_proj, tq, k.tabs, k.dead, k.err);
     consumer_sync();
     grid_mark(k, 4);
     // (b) per-head RMS norm (inference.cu:52-81, :97-111) and RoPE on adjacent pairs
@@ -514,25 +530,38 @@ __device__ __forceinline__ void grid_attention(const GridParams& p, const StepLa
             const int cnt = min(ppc * kKvBlock, it.n_prev - c0 * kKvBlock);      // earlier positions in this chunk
             if (scanner) {
 #pragma unroll 1
-                for (int j0 = sub * PPI; j0 < cnt; j0 += WPH * PPI) {
-                    const int j = j0 + grp;
-                    const bool valid = j < cnt;
-                    const int jj = valid ? j : 0;
-                    float kv[EPL], vv[EPL];
-                    Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(Ks + (size_t)jj * HD + lr * EPL), kv);
-                    Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(Vs + (size_t)jj * HD + lr * EPL), vv);
-                    float s = 0.f;
+                for (int j0 = sub * PPI; j0 < cnt; j0 += 2 * WPH * PPI) {
+                    // two scores side by side, their updates one after the other (a position behind the last one changes nothing)
+                    float s[2];
 #pragma unroll
-                    for (int e = 0; e < EPL; ++e) s = fmaf(q[e], kv[e], s);
+                    for (int u = 0; u < 2; ++u) {
+                        const int j = j0 + u * WPH * PPI + grp;
+                        float kv[EPL];
+                        Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(Ks + (size_t)(j < cnt ? j : 0) * HD + lr * EPL), kv);
+                        s[u] = 0.f;
 #pragma unroll
-                    for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    s = valid ? s : kNegBig;
-                    const float mn = fmaxf(m, s);
-                    const float sc = __expf(m - mn), pe = valid ? __expf(s - mn) : 0.f;
-                    l = l * sc + pe;
+                        for (int e = 0; e < EPL; ++e) s[u] = fmaf(q[e], kv[e], s[u]);
+                    }
 #pragma unroll
-                    for (int e = 0; e < EPL; ++e) acc[e] = fmaf(pe, vv[e], acc[e] * sc);
-                    m = mn;
+                    for (int o = LPR / 2; o > 0; o >>= 1) {
+                        const float s0 = __shfl_xor_sync(0xffffffffu, s[0], o), s1 = __shfl_xor_sync(0xffffffffu, s[1], o);
+                        s[0] += s0;
+                        s[1] += s1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int j = j0 + u * WPH * PPI + grp;
+                        const bool valid = j < cnt;
+                        float vv[EPL];
+                        Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(Vs + (size_t)(valid ? j : 0) * HD + lr * EPL), vv);
+                        const float su = valid ? s[u] : kNegBig;
+                        const float mn = fmaxf(m, su);
+                        const float sc = __expf(m - mn), pe = valid ? __expf(su - mn) : 0.f;
+                        l = l * sc + pe;
+#pragma unroll
+                        for (int e = 0; e < EPL; ++e) acc[e] = fmaf(pe, vv[e], acc[e] * sc);
+                        m = mn;
+                    }
                 }
             }
             __syncwarp();
@@ -612,6 +641,8 @@ __device__ __forceinline__ void grid_combine(const GridParams& p, const StepLaye
     const int hd = p.hd, tid = k.tid, lane = k.lane, warp = k.warp, W = hd + 2, S = k.plan->S, G = p.heads / p.kv_heads;
     float* parts = k.smem + p.off_parts;           // [h_count][S][hd+2]
     float* gate = k.smem + p.off_gate;             // [h_count][hd]
+    // (the gates have arrived long before the partials)
+    if (L.ng) ll_gather_rows(&p.vproj_attn, h_count * hd, L.nq + L.nk + L.nv + h_first * hd, 0, kNoSeg, 0, kNoSeg, 0, kNoSeg, 0, kNoSeg, e_proj, gate, k.tabs, k.dead, k.err);
     // partial (hl, sp): hd + 2 words of item (kv head, sp); 5 words per lane cover hd = 128
     int hl = warp / S, sp = warp - hl * S;
 #pragma unroll 1
@@ -619,22 +650,17 @@ __device__ __forceinline__ void grid_combine(const GridParams& p, const StepLaye
         const int h = h_first + hl;
         const unsigned long long* src = p.parts + (size_t)((h / G) * S + sp) * p.parts_slotw + (h % G) * W;
         float* out = parts + (size_t)pi * W;
-        unsigned long long w[4];
-        const int e0 = lane, e1 = lane + 32, e2 = min(lane + 64, W - 1), e3 = min(lane + 96, W - 1);
-        ll_poll4(src + e0, src + e1, src + e2, src + e3, w, e_parts, k.dead, k.err);
-        out[e0] = __uint_as_float((uint32_t)w[0]);
-        out[e1] = __uint_as_float((uint32_t)w[1]);
-        out[e2] = __uint_as_float((uint32_t)w[2]);
-        out[e3] = __uint_as_float((uint32_t)w[3]);
-        if (lane + 128 < W) {
-            ll_poll4(src + lane + 128, src + lane + 128, src + lane + 128, src + lane + 128, w, e_parts, k.dead, k.err);
-            out[lane + 128] = __uint_as_float((uint32_t)w[0]);
-        }
+        const unsigned long long* at[5];
+        unsigned long long w[5];
+#pragma unroll
+        for (int u = 0; u < 5; ++u) at[u] = src + min(lane + 32 * u, W - 1);
+        ll_poll(at, w, e_parts, k.dead, k.err);
+#pragma unroll
+        for (int u = 0; u < 5; ++u) out[min(lane + 32 * u, W - 1)] = __uint_as_float((uint32_t)w[u]);
         // next partial of this warp
         sp += kRingWarps;
         while (sp >= S) { sp -= S; ++hl; }
     }
-    if (L.ng) ll_gather_rows(&p.vproj_attn, L.nq + L.nk + L.nv + h_first * hd, h_count * hd, e_proj, gate, k.tabs, k.dead, k.err);
     consumer_sync();
 #pragma unroll 1
     for (int i = tid; i < h_count * hd; i += kRingConsumers) {
@@ -672,13 +698,10 @@ __device__ __forceinline__ void grid_delta_net(const GridParams& p, const StepLa
     float* qn = mix;                        // [nh][dk]
     float* kn = qn + nh * dk;               // [nh][dk]
     float* rv = kn + nh * dk;               // [rows]
-    float* gates = rv + ((rows + 3) & ~3);  // beta[nh] then alpha[nh]
+    float* gates = rv + rows;               // beta[nh] then alpha[nh]
     const int seg_k = H * dk, seg_v = 2 * H * dk, seg_b = seg_v + H * dv, seg_a = seg_b + H;
-    ll_gather_rows(&p.vproj_dn, h_lo * dk, nh * dk, e_proj, qn, k.tabs, k.dead, k.err);
-    ll_gather_rows(&p.vproj_dn, seg_k + h_lo * dk, nh * dk, e_proj, kn, k.tabs, k.dead, k.err);
-    ll_gather_rows(&p.vproj_dn, seg_v + r0, rows, e_proj, rv, k.tabs, k.dead, k.err);
-    ll_gather_rows(&p.vproj_dn, seg_b + h_lo, nh, e_proj, gates, k.tabs, k.dead, k.err);
-    ll_gather_rows(&p.vproj_dn, seg_a + h_lo, nh, e_proj, gates + nh, k.tabs, k.dead, k.err);
+    ll_gather_rows(&p.vproj_dn, 2 * nh * dk + rows + 2 * nh, h_lo * dk, seg_k + h_lo * dk, nh * dk, seg_v + r0, 2 * nh * dk, seg_b + h_lo, 2 * nh * dk + rows,
+                   seg_a + h_lo, 2 * nh * dk + rows + nh, e_proj, mix, k.tabs, k.dead, k.err);
     consumer_sync();
     grid_mark(k, 10);
     // L2-normalise q and k of the heads this CTA touches: one warp per vector
@@ -1073,7 +1096,7 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
     if (rank == 0) {
         if (p.with_lm_head) {
             float* lm = smem + p.off_parts;          // free by now
-            ll_gather_rows(&p.vlm, 0, 2 * C, e, lm, k.tabs, k.dead, k.err);
+            ll_gather_rows(&p.vlm, 2 * C, 0, 0, kNoSeg, 0, kNoSeg, 0, kNoSeg, 0, kNoSeg, e, lm, k.tabs, k.dead, k.err);
             consumer_sync();
             if (warp == 0 && p.do_pick) {
                 // lowest index among the largest values (the host loop of inference_orchestrator.cu:77-84 keeps the first)
