@@ -107,6 +107,7 @@ struct mlb_session {
     int *pos = nullptr, *tok = nullptr, *limit_prefill = nullptr, *limit_decode = nullptr;
     int *prompt = nullptr, *out_ring = nullptr, *out_idx = nullptr, *page_table = nullptr;
     unsigned long long* seeds = nullptr;
+    std::vector<unsigned long long> h_seeds;      // what `seeds` holds (empty: nothing yet)
     float *x = nullptr, *qbuf = nullptr, *gbuf = nullptr, *abuf = nullptr, *hbuf = nullptr, *raw = nullptr;
     float *logits = nullptr, *part = nullptr, *part_val = nullptr, *probe = nullptr;
     int *part_idx = nullptr, *attn_ticket = nullptr, *lm_ticket = nullptr;
