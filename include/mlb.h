@@ -112,8 +112,8 @@ void mlb_session_free(mlb_session* s);
  * With bf16 or FP8 weights and 64 prompt tokens or more the prompt is consumed as columns of
  * tensor-core steps, up to 4096 tokens at a time (bf16 activations: the cache equals the token loop's
  * within the low-precision tolerance; an FP8 model gets its codes as bf16 on the device
- * the first time, 2 bytes per weight). With fp32 weights and 5 tokens or more it is consumed as columns of the
- * fp32 GEMV chain; otherwise, or with MLB_PREFILL=step in the environment,
+ * the first time, 2 bytes per weight). With fp32 weights and 5 tokens or more, and with the others where one to
+ * three sequences bring 8 to 63 tokens, it is consumed as columns of the fp32 GEMV chain; otherwise, or with MLB_PREFILL=step in the environment,
  * one token per step and sequence. MLB_PREFILL=chunk asks for the columns and fails with
  * MLB_E_UNSUPPORTED where they cannot run. */
 int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t* lens, int stride);

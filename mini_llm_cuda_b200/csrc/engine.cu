@@ -320,6 +320,7 @@ static void free_session(mlb_session* s) {
     cudaSetDevice(s->m->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (auto* cs : s->cols) free_session(cs);
+    free_session(s->cols_gemv);
     for (auto& e : s->plan_free) if (e) cudaEventDestroy(e);
     if (s->plan_host) cudaFreeHost(s->plan_host);
     for (auto& g : s->graphs) if (g) cudaGraphExecDestroy(g);
@@ -1107,7 +1108,7 @@ static int apply_sampling(mlb_session* s, const mlb_sampling* sp, int* kind) {
 
 // A session, or (parent != null) the column set of one: `batch` columns of step buffers on the
 // parent's KV pool, delta-net state and stream, always on the tensor-core step.
-static int session_create(mlb_model* m, int batch, int max_context, int kv_block, int kv_pages, mlb_session* parent, mlb_session** out) {
+static int session_create(mlb_model* m, int batch, int max_context, int kv_block, int kv_pages, mlb_session* parent, mlb_session** out, bool gemv_cols = false) {
     if (!m || !out) return fail(MLB_E_INVALID, "null argument");
     *out = nullptr;
     if (batch < 1) return fail(MLB_E_INVALID, "batch must be >= 1");
@@ -1162,7 +1163,7 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     if (c.query_gating || !parent) SA(sess_alloc(s, (void**)&s->gbuf, B * nq * 4, true));
     SA(sess_alloc(s, (void**)&s->abuf, B * a_dim * 4, true));
     if (has_dn || !parent) SA(sess_alloc(s, (void**)&s->raw, B * s->raw_stride * 4, true));
-    if (!parent || c.weight_dtype == MLB_DT_F32) SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
+    if (!parent || gemv_cols) SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
     if (!parent) {
         SA(sess_alloc(s, (void**)&s->logits, B * c.vocab * 4, true));        // a column set's are made when a text is scored
         SA(sess_alloc(s, (void**)&s->probe, (size_t)c.vocab * 4, true));
@@ -1246,7 +1247,7 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
         SA(setup_lean_path(s));
         if (!s->use_lean) SA(setup_grid_path(s));
     }
-    if (parent && c.weight_dtype != MLB_DT_F32) {        // columns in fp32 run the GEMV chain
+    if (parent && !gemv_cols) {        // columns in fp32 run the GEMV chain
         SA(setup_cols_path(s));
         if (!s->use_cols) SA(setup_tc_path(s));
         if (!s->use_cols && !s->use_tc) {
@@ -1306,7 +1307,8 @@ extern "C" void mlb_session_free(mlb_session* s) { free_session(s); }
 // chunk: auto takes this path from 64 prompt tokens on (its activations are bf16, so the cache
 // differs from the token loop's within the low-precision tolerance); `*done` tells whether it ran.
 // Models with fp32 weights run their columns through the GEMV chain instead, eight to a CTA, in fp32 like the token loop,
-// wherever that loop would take kF32ColSteps steps or more.
+// wherever that loop would take kF32ColSteps steps or more. So do shorter prompts of the other models where the token loop
+// has fp32 activations (one to three sequences, which have no tensor-core step), from kGemvColumns columns on.
 //
 // Width of a step: a column set of 256 leaves most SMs without a tile (d = 512: 4 row tiles of 128) and pays the
 // step's ~45 launches once per 256 tokens; at 4096 columns the same launches carry 16 times the work.
@@ -1314,13 +1316,17 @@ extern "C" void mlb_session_free(mlb_session* s) { free_session(s); }
 // A step of columns costs 3.3 token steps of one sequence (0.27 and 0.59 ms on the two fp32 configurations, 8 or 12 columns), fewer
 // of several sequences.
 constexpr int kF32ColSteps = 4;
+// bf16 / FP8 models, in columns: token loop -> columns, cfg1 553 -> 546 us at 6, 719 -> 537 at 8, 1394 -> 620 at 16, 5180 -> 1097 at 61;
+// cfg3 2037 -> 1430 at 8; cfg4 5.0 -> 5.3 ms at 6, 6.6 -> 4.9 at 8, 51 -> 24 at 61. Several sequences share the loop's steps: three
+// of 8 tokens 1427 -> 635 us on cfg1, so there a column set also has to replace kF32ColSteps of them.
+constexpr int kGemvColumns = 8;
 
 // The narrowest column set that holds `n` columns (n <= kColMax).
 static int cols_get(mlb_session* s, int n, mlb_session** out) {
     int i = 0;
     while ((kColMin << i) < n) ++i;
     if (!s->cols[i]) {
-        int rc = session_create(s->m, kColMin << i, s->max_ctx, 0, 0, s, &s->cols[i]);
+        int rc = session_create(s->m, kColMin << i, s->max_ctx, 0, 0, s, &s->cols[i], s->m->cfg.weight_dtype == MLB_DT_F32);
         if (rc) { s->cols[i] = nullptr; return rc; }
     }
     *out = s->cols[i];
@@ -1344,11 +1350,21 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     if (f32 && mode == "chunk") return fail(MLB_E_UNSUPPORTED, "MLB_PREFILL=chunk needs bf16 or FP8 weights");
     int longest = 0;
     for (int b = 0; b < B; ++b) longest = std::max(longest, lens[b] - keep);
-    if (total < 1 || (mode == "auto" && (f32 ? longest < kF32ColSteps : total < 64))) return MLB_OK;
+    const bool gemv = !f32 && mode == "auto" && !s->use_tc && total < kColMin;      // fewer columns than the narrowest set holds
+    if (total < 1 || (mode == "auto" && (f32 ? longest < kF32ColSteps : gemv ? (total < kGemvColumns || longest < kF32ColSteps) : total < kColMin))) return MLB_OK;
     int rc;
     mlb_session* cs = nullptr;
     if (s->cols_failed && mode != "chunk") return MLB_OK;
-    if ((rc = cols_get(s, (int)std::min<long>(total, kColMax), &cs))) {
+    auto get = [&](int n) {
+        if (!gemv) return cols_get(s, n, &cs);
+        if (!s->cols_gemv) {
+            const int r = session_create(s->m, kColMin, s->max_ctx, 0, 0, s, &s->cols_gemv, true);
+            if (r) { s->cols_gemv = nullptr; return r; }
+        }
+        cs = s->cols_gemv;
+        return (int)MLB_OK;
+    };
+    if ((rc = get((int)std::min<long>(total, kColMax)))) {
         s->cols_failed = true;
         return mode == "chunk" ? rc : (int)MLB_OK;
     }
@@ -1367,7 +1383,7 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     long left = total;
     for (int slot = 0, used = 0; left > 0; slot = (slot + 1) % kPlanSlots, ++used) {
         const int want = (int)std::min<long>(left, kColMax);
-        if ((rc = cols_get(s, want, &cs))) return rc;
+        if ((rc = get(want))) return rc;
         if (kind == CHAIN_GREEDY && !cs->logits && (rc = sess_alloc(cs, (void**)&cs->logits, (size_t)cs->B * V * 4, false))) return rc;
         if ((rc = ensure_graph(cs, kind))) return rc;
         // the largest equal share that fits; what is left over goes to the first sequences
@@ -1429,7 +1445,7 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     *done = true;
     for (auto* c2 : s->cols)
         if (c2 && (rc = check_err_readback(c2))) return rc;
-    return MLB_OK;
+    return s->cols_gemv ? check_err_readback(s->cols_gemv) : (int)MLB_OK;
 }
 
 extern "C" int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t* lens, int stride) {

@@ -179,6 +179,7 @@ struct mlb_session {
     // made when first needed.
     mlb_session* cols[mlb::kColSets] = {};  // owned by the session they serve
     bool cols_failed = false;
+    mlb_session* cols_gemv = nullptr;       // column set of kColMin columns on the GEMV chain, for short prompts of bf16 / FP8 models
     mlb_session* parent = nullptr;          // set in a column set
     int* seq_of = nullptr;                  // [B] in a column set: column -> sequence of the parent
     bool use_cols = false;                  // column set: persistent column GEMMs (else, without memory for the bf16 codes, run_tc)

@@ -91,3 +91,29 @@ def test_fp32_prompt_columns_match_oracle(api, tmp_path, name, lens):
         assert logits_error(logits[b], want[-1]) < TOL_FP32, b
     sess.close()
     model.close()
+
+
+@pytest.mark.parametrize("name", ["mha64", "gqa4_128", "gqa8_64", "dn_odd", "fp8"])
+@pytest.mark.parametrize("lens", [[8], [9], [63], [5, 5, 1], [30, 3]])
+def test_short_prompts_in_fp32_activations(api, tmp_path, monkeypatch, name, lens):
+    """bf16 / FP8 models, one to three sequences, 8 to 63 columns: the GEMV chain; the oracle's logits, and the token
+    loop's up to the rounding of single K/V entries."""
+    spec = dataclasses.replace(SPECS[name], max_context=96)
+    path = write_model(tmp_path, spec, seed=57)
+    oracle = load_oracle(path)
+    prompts = random_prompts(spec.vocab, lens, seed=59)
+    model = api.Model(path)
+    got = []
+    for mode in ("auto", "step"):
+        monkeypatch.setenv("MLB_PREFILL", mode)
+        sess = api.Session(model, len(lens))
+        sess.prefill(prompts)
+        assert sess.positions().tolist() == [n - 1 for n in lens]
+        sess.decode_step()
+        got.append(sess.logits())
+        sess.close()
+    model.close()
+    assert logits_error(got[0], got[1]) < 2e-3
+    for b in range(len(lens)):
+        _, want = oracle_rollout(oracle, prompts[b], 1)
+        assert logits_error(got[0][b], want[0]) < TOL_LOWP, b
