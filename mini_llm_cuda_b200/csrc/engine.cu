@@ -28,6 +28,8 @@ int fail(int code, const char* fmt, ...) {
     vsnprintf(buf, sizeof buf, fmt, ap);
     va_end(ap);
     g_err = buf;
+    // The runtime keeps a failed call's code for this thread's next cudaGetLastError, which a later, healthy launch would report as its own.
+    if (code == MLB_E_CUDA || code == MLB_E_NOMEM) cudaGetLastError();
     return code;
 }
 
