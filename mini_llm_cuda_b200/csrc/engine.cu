@@ -292,10 +292,22 @@ extern "C" void mlb_model_free(mlb_model* m) { free_model(m); }
 // --------------------------------------------------------------------------------------
 namespace mlb {
 
+// The most device memory that the column sets of a session may hold together, in bytes (MLB_COLUMNS_MB).
+static size_t cols_limit() {
+    const char* v = std::getenv("MLB_COLUMNS_MB");
+    return v ? (size_t)std::max(0, std::atoi(v)) << 20 : SIZE_MAX;
+}
+
 static int sess_alloc(mlb_session* s, void** p, size_t bytes, bool zero) {
+    if (s->parent && s->parent->cols_bytes + bytes > cols_limit())
+        return fail(MLB_E_NOMEM, "%zu bytes more for prompt columns exceed MLB_COLUMNS_MB (%zu bytes held)", bytes, s->parent->cols_bytes);
     cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
     if (e != cudaSuccess) return fail(MLB_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     s->allocs.push_back(*p);
+    if (s->parent) {
+        s->own_bytes += bytes;
+        s->parent->cols_bytes += bytes;
+    }
     if (zero) CU(cudaMemset(*p, 0, bytes ? bytes : 16));
     return MLB_OK;
 }
@@ -328,6 +340,7 @@ static void free_session(mlb_session* s) {
     for (auto& g : s->graphs) if (g) cudaGraphExecDestroy(g);
     for (auto& g : s->tgraphs) if (g) cudaGraphExecDestroy(g);
     for (void* p : s->allocs) cudaFree(p);
+    if (s->parent) s->parent->cols_bytes -= s->own_bytes;
     if (s->pinned_tok) cudaFreeHost(s->pinned_tok);
     if (s->pinned_out) cudaFreeHost(s->pinned_out);
     if (s->pinned_err) cudaFreeHost(s->pinned_err);
@@ -1128,7 +1141,7 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     s->parent = parent;
     if (parent) s->kv_pages = parent->kv_pages;
 #define SA(expr) do { int r__ = (expr); if (r__) { free_session(s); return r__; } } while (0)
-#define SCU(expr) do { cudaError_t e__ = (expr); if (e__ != cudaSuccess) { free_session(s); return fail(MLB_E_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e__)); } } while (0)
+#define SCU(expr) do { cudaError_t e__ = (expr); if (e__ != cudaSuccess) { free_session(s); return fail(e__ == cudaErrorMemoryAllocation ? MLB_E_NOMEM : MLB_E_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e__)); } } while (0)
     if (parent) s->stream = parent->stream;
     else SCU(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     const size_t B = batch;
@@ -1323,15 +1336,45 @@ constexpr int kF32ColSteps = 4;
 // of 8 tokens 1427 -> 635 us on cfg1, so there a column set also has to replace kF32ColSteps of them.
 constexpr int kGemvColumns = 8;
 
-// The narrowest column set that holds `n` columns (n <= kColMax).
-static int cols_get(mlb_session* s, int n, mlb_session** out) {
-    int i = 0;
-    while ((kColMin << i) < n) ++i;
-    if (!s->cols[i]) {
-        int rc = session_create(s->m, kColMin << i, s->max_ctx, 0, 0, s, &s->cols[i], s->m->cfg.weight_dtype == MLB_DT_F32);
-        if (rc) { s->cols[i] = nullptr; return rc; }
+// The column set of kColMin << i columns, with room for their logits if they are `scored`. A set whose logits are refused is given back:
+// a narrower one may fit in its place.
+static int cols_make(mlb_session* s, int i, bool scored) {
+    mlb_session*& cs = s->cols[i];
+    int rc = MLB_OK;
+    if (!cs) rc = session_create(s->m, kColMin << i, s->max_ctx, 0, 0, s, &cs, s->m->cfg.weight_dtype == MLB_DT_F32);
+    if (rc) cs = nullptr;
+    else if (scored && !cs->logits && (rc = sess_alloc(cs, (void**)&cs->logits, (size_t)cs->B * s->m->cfg.vocab * 4, false))) {
+        free_session(cs);
+        cs = nullptr;
     }
-    *out = s->cols[i];
+    return rc;
+}
+
+// A column set for the next `n` columns: the narrowest that holds them, or, without memory for it, a wider one that exists or a
+// narrower one, which takes fewer of them. `cap`: the widest that this call still asks for.
+static int cols_get(mlb_session* s, long n, bool scored, int* cap, mlb_session** out) {
+    for (;;) {
+        int i = 0;
+        while ((kColMin << i) < std::min<long>(n, *cap)) ++i;
+        const int rc = cols_make(s, i, scored);
+        *out = s->cols[i];
+        if (rc != MLB_E_NOMEM) return rc;
+        for (int j = i + 1; j < kColSets; ++j) {
+            *out = s->cols[j];
+            if (*out && (!scored || (*out)->logits)) return MLB_OK;
+        }
+        if (i == 0) return rc;
+        *cap = kColMin << (i - 1);
+    }
+}
+
+// Pinned ring of the chunks' plans.
+static int plan_ring(mlb_session* s) {
+    if (s->plan_host) return MLB_OK;
+    for (auto& e : s->plan_free)
+        if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    s->plan_host_ints = cols_layout(s->m->cfg, s->B, kColMax).ints;
+    CU(cudaMallocHost((void**)&s->plan_host, kPlanSlots * s->plan_host_ints * 4));
     return MLB_OK;
 }
 
@@ -1354,11 +1397,11 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     for (int b = 0; b < B; ++b) longest = std::max(longest, lens[b] - keep);
     const bool gemv = !f32 && mode == "auto" && !s->use_tc && total < kColMin;      // fewer columns than the narrowest set holds
     if (total < 1 || (mode == "auto" && (f32 ? longest < kF32ColSteps : gemv ? (total < kGemvColumns || longest < kF32ColSteps) : total < kColMin))) return MLB_OK;
-    int rc;
+    int rc, cap = kColMax;
     mlb_session* cs = nullptr;
     if (s->cols_failed && mode != "chunk") return MLB_OK;
-    auto get = [&](int n) {
-        if (!gemv) return cols_get(s, n, &cs);
+    auto get = [&](long n) {
+        if (!gemv) return cols_get(s, n, score_out != nullptr, &cap, &cs);
         if (!s->cols_gemv) {
             const int r = session_create(s->m, kColMin, s->max_ctx, 0, 0, s, &s->cols_gemv, true);
             if (r) { s->cols_gemv = nullptr; return r; }
@@ -1366,14 +1409,9 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
         cs = s->cols_gemv;
         return (int)MLB_OK;
     };
-    if ((rc = get((int)std::min<long>(total, kColMax)))) {
-        s->cols_failed = true;
+    if ((rc = get(total)) || (rc = plan_ring(s))) {
+        s->cols_failed = rc != MLB_E_NOMEM;        // memory may come back: asked for again by the next prompt
         return mode == "chunk" ? rc : (int)MLB_OK;
-    }
-    if (!s->plan_host) {
-        s->plan_host_ints = cols_layout(cfg, s->B, kColMax).ints;
-        CU(cudaMallocHost((void**)&s->plan_host, kPlanSlots * s->plan_host_ints * 4));
-        for (auto& e : s->plan_free) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     const size_t V = (size_t)cfg.vocab;
     const int qt = attn_cols_queries(cfg.heads / cfg.kv_heads);
@@ -1384,10 +1422,8 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     std::vector<int> cursor(B, 0);
     long left = total;
     for (int slot = 0, used = 0; left > 0; slot = (slot + 1) % kPlanSlots, ++used) {
-        const int want = (int)std::min<long>(left, kColMax);
-        if ((rc = get(want))) return rc;
-        if (kind == CHAIN_GREEDY && !cs->logits && (rc = sess_alloc(cs, (void**)&cs->logits, (size_t)cs->B * V * 4, false))) return rc;
-        if ((rc = ensure_graph(cs, kind))) return rc;
+        if ((rc = get(left)) || (rc = ensure_graph(cs, kind))) return rc;
+        const int want = (int)std::min<long>(left, cs->B);
         // the largest equal share that fits; what is left over goes to the first sequences
         int lo = 0, hi = want;
         auto filled = [&](int share) {
@@ -1445,9 +1481,10 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     }
     CU(cudaStreamSynchronize(s->stream));
     *done = true;
+    rc = s->cols_gemv ? check_err_readback(s->cols_gemv) : (int)MLB_OK;
     for (auto* c2 : s->cols)
-        if (c2 && (rc = check_err_readback(c2))) return rc;
-    return s->cols_gemv ? check_err_readback(s->cols_gemv) : (int)MLB_OK;
+        if (const int r = c2 ? check_err_readback(c2) : (int)MLB_OK) rc = r;
+    return rc;
 }
 
 extern "C" int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t* lens, int stride) {

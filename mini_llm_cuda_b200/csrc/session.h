@@ -178,7 +178,8 @@ struct mlb_session {
     // delta-net state and stream; a column is one prompt token of one sequence. A set per power of two of columns,
     // made when first needed.
     mlb_session* cols[mlb::kColSets] = {};  // owned by the session they serve
-    bool cols_failed = false;
+    size_t cols_bytes = 0, own_bytes = 0;   // device memory of the column sets; in a column set, its own
+    bool cols_failed = false;               // they cannot be had here, for another reason than memory
     mlb_session* cols_gemv = nullptr;       // column set of kColMin columns on the GEMV chain, for short prompts of bf16 / FP8 models
     mlb_session* parent = nullptr;          // set in a column set
     int* seq_of = nullptr;                  // [B] in a column set: column -> sequence of the parent
