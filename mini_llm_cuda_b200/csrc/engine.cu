@@ -1421,7 +1421,7 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     // sequence, positions ascending.
     std::vector<int> cursor(B, 0);
     long left = total;
-    for (int slot = 0, used = 0; left > 0; slot = (slot + 1) % kPlanSlots, ++used) {
+    for (int slot = 0; left > 0; slot = (slot + 1) % kPlanSlots) {
         if ((rc = get(left)) || (rc = ensure_graph(cs, kind))) return rc;
         const int want = (int)std::min<long>(left, cs->B);
         // the largest equal share that fits; what is left over goes to the first sequences
@@ -1438,7 +1438,7 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
         int extra = want - (int)filled(lo);
         const ColsLayout lay = cols_layout(cfg, s->B, cs->B);
         int* pl = s->plan_host + slot * s->plan_host_ints;
-        if (used >= kPlanSlots) CU(cudaEventSynchronize(s->plan_free[slot]));
+        CU(cudaEventSynchronize(s->plan_free[slot]));      // the slot's last plan has left it, also one of a call that failed half-way
         int n = 0, runs = 0, tiles = 0;
         for (int b = 0; b < B; ++b) {
             const int rest = lens[b] - keep - cursor[b];
@@ -1515,7 +1515,10 @@ extern "C" int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t*
         if ((rc = sync_page_table(s))) return rc;
     }
     bool by_columns = false;
-    if ((rc = prefill_columns(s, tokens, lens, stride, &by_columns))) return rc;
+    if ((rc = prefill_columns(s, tokens, lens, stride, &by_columns))) {
+        cudaStreamSynchronize(s->stream);          // chunks may be under way
+        return rc;
+    }
     if (!by_columns) {
         std::vector<int> hp((size_t)B * s->max_ctx, 0), first(B), lim(B);
         for (int b = 0; b < B; ++b) {
