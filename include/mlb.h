@@ -97,10 +97,9 @@ int mlb_file_inspect(const char* path, const mlb_config* override_or_null, mlb_c
 /* Replaces the activation half of allocateMemory (memory_allocation.cu:500-552): instead of
  * maxL-sized scratch per op it owns a paged KV cache (pages of kv_block positions),
  * fp32 delta-net state and one decode step's scratch. kv_pages = 0 sizes the pool for
- * batch * max_context. A session of 4 sequences or more on an FP8 model runs its steps as
- * tensor-core GEMMs on a bf16 copy of the weights that the model builds on the device the first
- * time (2 bytes per weight, shared by all its sessions); MLB_GEMM=simt in the environment keeps
- * the FP8 GEMV kernels. */
+ * batch * max_context. A session of 4 sequences or more on a bf16 or FP8 model runs its steps as
+ * tensor-core GEMMs (FP8 codes are widened inside the kernel); MLB_GEMM=simt in the environment keeps
+ * the GEMV kernels. Prompt columns add to a session's memory on first use, see mlb_prefill. */
 int mlb_session_new(mlb_model* m, int batch, int max_context, int kv_block, int kv_pages,
                     mlb_session** out);
 int mlb_session_reset(mlb_session* s);
@@ -111,8 +110,10 @@ void mlb_session_free(mlb_session* s);
  * it, position lens[b]-1 holds the last prompt token as the pending input of the next step.
  * With bf16 or FP8 weights and 64 prompt tokens or more the prompt is consumed as columns of
  * tensor-core steps, up to 4096 tokens at a time (bf16 activations: the cache equals the token loop's
- * within the low-precision tolerance; an FP8 model gets its codes as bf16 on the device
- * the first time, 2 bytes per weight). With fp32 weights and 5 tokens or more, and with the others where one to
+ * within the low-precision tolerance; an FP8 model gets a copy of its codes as bf16 on the device
+ * the first time, 2 bytes per weight, kept until the model is freed and shared by its sessions; without
+ * room for it, or with MLB_FP8_COPY=0, the codes are widened inside the GEMMs). The columns' buffers are made
+ * when a width is first needed and stay with the session (MLB_COLUMNS_MB limits them). With fp32 weights and 5 tokens or more, and with the others where one to
  * three sequences bring 8 to 63 tokens, it is consumed as columns of the fp32 GEMV chain; otherwise, or with MLB_PREFILL=step in the environment,
  * one token per step and sequence. MLB_PREFILL=chunk asks for the columns and fails with
  * MLB_E_UNSUPPORTED where they cannot run. */
@@ -188,6 +189,10 @@ int mlb_session_step_bytes(mlb_session* s, uint64_t* weights, uint64_t* kv, uint
                            uint64_t* rows);
 /* Kernels launched per decode step by the current configuration. */
 int mlb_session_launches_per_step(mlb_session* s);
+/* Which kernels serve: of a decode step (columns = 0) "lean", "grid" (whole-GPU kernels), "gemv", "mma" or "tcgen05" (launch
+ * chains by their projections); of a prompt chunk of `columns` tokens "cols" (column GEMMs), "tcgen05" (FP8 without the bf16
+ * copy of its codes) or "gemv", "none" while no prompt has needed that width. */
+const char* mlb_session_path(const mlb_session* s, int columns);
 /* Diagnostics of the batch-1 single-kernel step (no counterpart in the reference). When the
  * session was created with MLB_GRID_TIMERS=1 in the environment, mlb_session_grid_timers copies
  * 32 cycle counters per CTA (summed over the steps since the last call; what each one covers is

@@ -93,6 +93,7 @@ def lib() -> C.CDLL:
         "mlb_session_positions": (C.c_int, [vp, i32p]),
         "mlb_session_step_bytes": (C.c_int, [vp, u64p, u64p, u64p, u64p]),
         "mlb_session_launches_per_step": (C.c_int, [vp]),
+        "mlb_session_path": (C.c_char_p, [vp, C.c_int]),
         "mlb_session_grid_timers": (C.c_int, [vp, C.POINTER(C.c_longlong), C.c_int]),
         "mlb_session_grid_trace": (C.c_int, [vp, C.POINTER(C.c_longlong), C.c_int]),
         "mlb_op_wait_probe": (C.c_int, [C.c_int, C.c_uint32]),
@@ -319,6 +320,10 @@ class Session:
 
     def launches_per_step(self) -> int:
         return check(lib().mlb_session_launches_per_step(self._h))
+
+    def path(self, columns: int = 0) -> str:
+        """Which kernels serve a decode step, or a prompt chunk of that many columns (mlb.h)."""
+        return lib().mlb_session_path(self._h, columns).decode()
 
     def grid_trace(self) -> np.ndarray:
         """[CTAs][256] trace events of the last single-kernel step (MLB_GRID_TIMERS=1), else empty."""

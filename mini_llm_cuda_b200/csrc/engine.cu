@@ -833,11 +833,20 @@ static int setup_tc_path(mlb_session* s) {
     return MLB_OK;
 }
 
-// The FP8 codes of a model as bf16. Leaves `wide` empty where there is no memory for them.
-static int model_widen(mlb_model* m, cudaStream_t st) {
+// The FP8 codes of a model as bf16, made on first use; false where there is no memory for them (asked for again by the next caller) or
+// MLB_FP8_COPY=0 refuses them.
+static int model_widen(mlb_model* m, cudaStream_t st, bool* have) {
     std::lock_guard<std::mutex> hold(m->wide_mutex);
-    if (!m->wide.empty() || m->wide_failed) return MLB_OK;
+    const char* env = std::getenv("MLB_FP8_COPY");
+    *have = false;
+    if (env && env[0] == '0') return MLB_OK;
+    *have = !m->wide.empty();
+    if (*have) return MLB_OK;
     const mlb_config& c = m->cfg;
+    size_t need = (size_t)c.vocab * c.dim * 2, free_bytes = 0, all = 0;
+    for (const DevLayer& L : m->layers) need += ((size_t)L.n_qkv * c.dim + (size_t)c.dim * L.o_in + 3 * (size_t)c.ffn_dim * c.dim) * 2;
+    CU(cudaMemGetInfo(&free_bytes, &all));
+    if (free_bytes < need) return MLB_OK;
     std::vector<void*> made;
     int rc = MLB_OK;
     auto widen = [&](const void* codes, size_t n) -> void* {
@@ -865,13 +874,13 @@ static int model_widen(mlb_model* m, cudaStream_t st) {
     const cudaError_t e = cudaStreamSynchronize(st);      // sessions on other streams read them from here on
     if (rc || e != cudaSuccess) {
         for (void* p : made) cudaFree(p);
-        m->wide_failed = true;
         if (rc == MLB_E_NOMEM && e == cudaSuccess) return MLB_OK;
         return fail(MLB_E_CUDA, "widening of the FP8 weights failed: %s", cudaGetErrorString(e));
     }
     m->allocs.insert(m->allocs.end(), made.begin(), made.end());
     m->wide_E = we;
     m->wide.swap(w);
+    *have = true;
     return MLB_OK;
 }
 
@@ -929,8 +938,9 @@ static int setup_cols_path(mlb_session* s) {
     const bool w8 = c.weight_dtype == MLB_DT_FP8_E4M3;
     int rc;
     if (w8) {
-        if ((rc = model_widen(s->m, s->stream))) return rc;
-        if (m->wide.empty()) return MLB_OK;
+        bool have = false;
+        if ((rc = model_widen(s->m, s->stream, &have))) return rc;
+        if ((s->no_copy = !have)) return MLB_OK;
     }
     if ((rc = build_step_layers(s))) return rc;
     const int T = s->B, nq = c.heads * c.head_dim, a_dn = c.heads * c.dn_value_dim;
@@ -1341,6 +1351,15 @@ constexpr int kGemvColumns = 8;
 static int cols_make(mlb_session* s, int i, bool scored) {
     mlb_session*& cs = s->cols[i];
     int rc = MLB_OK;
+    if (cs && cs->no_copy) {
+        // made without the bf16 codes of an FP8 model: made again where they can be had by now
+        bool have = false;
+        if ((rc = model_widen(s->m, s->stream, &have))) return rc;
+        if (have) {
+            free_session(cs);
+            cs = nullptr;
+        }
+    }
     if (!cs) rc = session_create(s->m, kColMin << i, s->max_ctx, 0, 0, s, &cs, s->m->cfg.weight_dtype == MLB_DT_F32);
     if (rc) cs = nullptr;
     else if (scored && !cs->logits && (rc = sess_alloc(cs, (void**)&cs->logits, (size_t)cs->B * s->m->cfg.vocab * 4, false))) {
@@ -1880,6 +1899,18 @@ extern "C" int mlb_session_launches_per_step(mlb_session* s) {
     int rc = ensure_graph(s, CHAIN_GREEDY);
     if (rc) return rc;
     return s->launches_per_step[CHAIN_GREEDY];
+}
+
+extern "C" const char* mlb_session_path(const mlb_session* s, int columns) {
+    if (!s || columns < 0) return "none";
+    if (columns > 0) {
+        int i = 0;
+        while (i + 1 < kColSets && (kColMin << i) < columns) ++i;
+        const mlb_session* cs = s->cols[i] ? s->cols[i] : (i == 0 ? s->cols_gemv : nullptr);
+        return !cs ? "none" : (cs->use_cols ? "cols" : (cs->use_tc ? "tcgen05" : "gemv"));
+    }
+    if (s->use_lean || s->use_grid) return s->use_lean ? "lean" : "grid";
+    return !s->use_tc ? "gemv" : (s->use_dec ? "mma" : "tcgen05");
 }
 
 // ---- host-only allocator entry points --------------------------------------------------

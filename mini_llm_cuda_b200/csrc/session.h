@@ -62,7 +62,6 @@ struct mlb_model {
     struct Wide { void *Wqkv = nullptr, *Wo = nullptr, *W1a = nullptr, *W1b = nullptr, *W2 = nullptr; };
     std::vector<Wide> wide;
     void* wide_E = nullptr;
-    bool wide_failed = false;
     std::mutex wide_mutex;
 };
 
@@ -183,7 +182,8 @@ struct mlb_session {
     mlb_session* cols_gemv = nullptr;       // column set of kColMin columns on the GEMV chain, for short prompts of bf16 / FP8 models
     mlb_session* parent = nullptr;          // set in a column set
     int* seq_of = nullptr;                  // [B] in a column set: column -> sequence of the parent
-    bool use_cols = false;                  // column set: persistent column GEMMs (else, without memory for the bf16 codes, run_tc)
+    bool use_cols = false;                  // column set: persistent column GEMMs (else, without the bf16 codes, run_tc)
+    bool no_copy = false;                   // column set of an FP8 model that was made without them
     ColsGemm cg_qkv{}, cg_dn{}, cg_o_attn{}, cg_o_dn{}, cg_up{}, cg_down{}, cg_last{}, cg_head{};      // cg_last: the last layer's down projection
     mlb::ColsPlan plan;                     // column set: what the columns of the current chunk are (one array, plan_dev)
     int* plan_dev = nullptr;

@@ -117,3 +117,32 @@ def test_short_prompts_in_fp32_activations(api, tmp_path, monkeypatch, name, len
     for b in range(len(lens)):
         _, want = oracle_rollout(oracle, prompts[b], 1)
         assert logits_error(got[0][b], want[0]) < TOL_LOWP, b
+
+
+def test_fp8_columns_without_the_bf16_copy(api, tmp_path, monkeypatch):
+    """An FP8 model whose bf16 codes cannot be had: its columns run on the decode step's kernels, codes widened tile by tile. At 129
+    to 256 columns their k-ranges are those of the column GEMMs, hence the same bits; the copy is used once it can be had."""
+    spec = dataclasses.replace(SPECS["fp8"], max_context=700)
+    path = write_model(tmp_path, spec, seed=63)
+    oracle = load_oracle(path)
+    tokens = random_prompts(spec.vocab, [600], seed=65)[0]
+    st = oracle.new_state()
+    want = np.stack([np.asarray(oracle.step(st, int(t))) for t in tokens])
+    model = api.Model(path)
+    monkeypatch.setenv("MLB_FP8_COPY", "0")
+    sess = api.Session(model, 1)
+    got = {}
+    for length in (1, 64, 65, 129, 256, 600):
+        got[length] = sess.score(tokens[:length])
+        assert sess.path(length) == "tcgen05"
+        worst = max(logits_error(got[length][i], want[i]) for i in range(length))
+        assert worst < TOL_LOWP, (length, worst)
+    monkeypatch.delenv("MLB_FP8_COPY")
+    copied = {}
+    for length in got:
+        copied[length] = sess.score(tokens[:length])
+        assert sess.path(length) == "cols"
+    for length in (129, 256):
+        assert np.array_equal(got[length], copied[length]), length
+    sess.close()
+    model.close()
