@@ -1179,14 +1179,16 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     }
     const int nq = c.heads * c.head_dim;
     const int a_dim = std::max(nq, c.heads * c.dn_value_dim);
-    bool has_dn = false;
-    for (int i = 0; i < c.layers; ++i) has_dn = has_dn || c.layer_types[i] == MLB_LAYER_DELTA_NET;
+    bool has_dn = false, has_attn = false;
+    for (int i = 0; i < c.layers; ++i) (c.layer_types[i] == MLB_LAYER_DELTA_NET ? has_dn : has_attn) = true;
+    // a column set's attention over a bf16 cache (attn_cols_kernel) has no splits and writes the next operand only
+    const bool split_attn = !parent || gemv_cols || c.kv_dtype == MLB_DT_F32;
     s->max_q = nq;
     s->raw_stride = 2 * c.heads * c.dn_key_dim + c.heads * c.dn_value_dim + 2 * c.heads;
     SA(sess_alloc(s, (void**)&s->x, B * c.dim * 4, true));
-    SA(sess_alloc(s, (void**)&s->qbuf, B * nq * 4, true));
-    if (c.query_gating || !parent) SA(sess_alloc(s, (void**)&s->gbuf, B * nq * 4, true));
-    SA(sess_alloc(s, (void**)&s->abuf, B * a_dim * 4, true));
+    if (has_attn || !parent) SA(sess_alloc(s, (void**)&s->qbuf, B * nq * 4, true));
+    if ((c.query_gating && has_attn) || !parent) SA(sess_alloc(s, (void**)&s->gbuf, B * nq * 4, true));
+    if (split_attn) SA(sess_alloc(s, (void**)&s->abuf, B * a_dim * 4, true));
     if (has_dn || !parent) SA(sess_alloc(s, (void**)&s->raw, B * s->raw_stride * 4, true));
     if (!parent || gemv_cols) SA(sess_alloc(s, (void**)&s->hbuf, B * c.ffn_dim * 4, true));
     if (!parent) {
@@ -1206,15 +1208,19 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     // beat two of 18 and four of 9 (63 vs 78 and 74 us).
     s->attn_min_pps = 11;
     if (const char* v = std::getenv("MLB_ATTN_MIN_PAGES")) s->attn_min_pps = std::max(1, std::atoi(v));
-    SA(sess_alloc(s, (void**)&s->part, B * c.heads * s->splits * (c.head_dim + 2) * 4, true));
-    SA(sess_alloc(s, (void**)&s->attn_ticket, B * c.heads * 4, true));
+    if (split_attn) {
+        SA(sess_alloc(s, (void**)&s->part, B * c.heads * s->splits * (c.head_dim + 2) * 4, true));
+        SA(sess_alloc(s, (void**)&s->attn_ticket, B * c.heads * 4, true));
+    }
     s->lm_rows = 16;
     // argmax partials per sequence: one per LM-head CTA of either GEMV form (the streamed form
     // launches up to one CTA per SM, whatever the vocabulary size)
     s->lm_parts = std::max((c.vocab + s->lm_rows - 1) / s->lm_rows, 2 * sm_count);
-    SA(sess_alloc(s, (void**)&s->part_val, B * s->lm_parts * 4, true));
-    SA(sess_alloc(s, (void**)&s->part_idx, B * s->lm_parts * 4, true));
-    SA(sess_alloc(s, (void**)&s->lm_ticket, (B + 7) / 1 * 4, true));
+    if (!parent) {         // columns pick nothing
+        SA(sess_alloc(s, (void**)&s->part_val, B * s->lm_parts * 4, true));
+        SA(sess_alloc(s, (void**)&s->part_idx, B * s->lm_parts * 4, true));
+        SA(sess_alloc(s, (void**)&s->lm_ticket, (B + 7) / 1 * 4, true));
+    }
     s->kpool.assign(c.layers, nullptr);
     s->vpool.assign(c.layers, nullptr);
     s->state.assign(c.layers, nullptr);

@@ -1,4 +1,6 @@
 """Device memory that is not to be had: what fails, what goes on, and what the calls after it see."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -101,5 +103,18 @@ def test_prompts_go_on_without_memory_for_their_columns(api, tmp_path, monkeypat
     assert np.array_equal(logits(sess, long), by_columns[0])
     monkeypatch.setenv("MLB_COLUMNS_MB", "1")              # no room beside the wide set: it serves
     assert np.array_equal(logits(sess, short), by_columns[1])
+    sess.close()
+    model.close()
+
+
+def test_column_sets_hold_what_their_kernels_use(api, tmp_path, monkeypatch):
+    """4096 columns of this model need per column: x and q (512 bytes each), the raw delta-net projection (1552), bf16 operands (256 +
+    256 + 512), sums of squares, plan: 15 MB. Partial results of attention splits and of the LM head's pick would add 37 MB."""
+    spec = dataclasses.replace(WIDE, max_context=4200)
+    model = api.Model(write_model(tmp_path, spec, seed=86))
+    sess = api.Session(model, 1)
+    monkeypatch.setenv("MLB_COLUMNS_MB", "16")
+    sess.prefill(random_prompts(spec.vocab, [4097], seed=87))
+    assert sess.path(4096) == "cols"
     sess.close()
     model.close()
