@@ -2,6 +2,7 @@
 // paged K/V rows, and the gated delta-net recurrence over a sequence's columns. Everything else of a column step is
 // the decode step's own kernels with a column in the place of a sequence.
 #include <cstring>
+#include <type_traits>
 
 #include "cols_host.h"
 #include "../../include/mlb.h"
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
     const int rbase = (HD == 64 ? 0 : (warp & 1) * 16) + lane / L * 4;          // this thread's rows: rbase .. rbase + 3
     const int own = HD == 64 ? a : a >> 1;                                      // the row of them whose softmax it keeps
     const int own_pos = pos0 + min((rbase + own) / G, nq - 1);
+    const int warp_first = pos0 + min((HD == 64 ? 0 : (warp & 1) * 16) / G, nq - 1);
     const int warp_last = pos0 + min(((HD == 64 ? 0 : (warp & 1) * 16) + (HD == 64 ? 31 : 15)) / G, nq - 1);
     const uint32_t sm0 = smem_u32(sm);
     auto load = [&](int pass, int t, int st) {
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
             const int idx = tid + i * kAcThreads, row = idx / (HD / 8), ch = idx % (HD / 8);
             const int sl = row / kKvBlock;           // slot: w_local * 2 + k
             const int pg = 2 * pass + (sl >> 1) + 4 * (2 * t + (sl & 1));
-            const bool ok = pg < np;
+            const bool ok = pg < np && pg * kKvBlock + row % kKvBlock <= last;      // rows behind the tile's last position read as zeros
             const int page = ok ? pt[pg] : 0;
             const size_t off = (((size_t)page * p.kv_heads + kvh) * kKvBlock + (row % kKvBlock)) * HD + ch * 8;
             cp_async16(sm0 + (uint32_t)(st * 2 * TILE + row * HD * 2 + ch * 16), p.kpool + off, ok);
@@ -168,6 +170,88 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
             for (int e = 0; e < 8; ++e) acc[r][e] = 0ull;
         float m = kNegBig, l = 0.f;
         if (pass == 1 && n_t > 0) load(1, 0, 0);
+        // One page of the warp's stream. `later`: the page may hold positions behind some row of the warp. Their probability is 0, but 0
+        // times a value that is no number is none: their products are left out.
+        auto use_page = [&](auto later, const unsigned char* kt, const unsigned char* vt, int cnt) {
+#pragma unroll 1
+            for (int c = 0; c < CPP; ++c) {
+                float s[16];                      // [row][u]
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    f32x2 kp[8];
+                    unpack(kt + ((c * 4 + u) * NG + grp) * HD * 2, kp);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        f32x2 d = 0ull;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) d = fma2(q[r][e], kp[e], d);
+                        float x, y;
+                        unpack2(d, x, y);
+                        s[r * 4 + u] = x + y;
+                    }
+                }
+                {
+                    const bool up = (a & (L / 2)) != 0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float send = up ? s[j] : s[j + 8], keep = up ? s[j + 8] : s[j];
+                        s[j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 2);
+                    }
+                }
+                {
+                    const bool up = (a & (L / 4)) != 0;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float send = up ? s[j] : s[j + 4], keep = up ? s[j + 4] : s[j];
+                        s[j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 4);
+                    }
+                }
+                if (HD == 128) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], 1);
+                }
+                // softmax of the own row
+                float mn = m;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool valid = !decltype(later)::value || (c * 4 + u) * NG + grp < cnt;
+                    s[u] = valid ? s[u] / inv_div : kNegBig;
+                    mn = fmaxf(mn, s[u]);
+                }
+                const float sc = expf(m - mn);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool valid = !decltype(later)::value || (c * 4 + u) * NG + grp < cnt;
+                    s[u] = valid ? expf(s[u] - mn) : 0.f;
+                }
+                l = __fadd_rn(__fmul_rn(l, sc), s[0]);         // (not one fma: the other kernel's roundings)
+                l = __fadd_rn(__fadd_rn(__fadd_rn(l, s[1]), s[2]), s[3]);
+                m = mn;
+                const int src = lane - a;
+                if (__any_sync(0xffffffffu, sc != 1.0f)) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const float x = __shfl_sync(0xffffffffu, sc, src + (HD == 64 ? r : 2 * r));
+                        const f32x2 xx = pack2(x, x);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) acc[r][e] = mul2(acc[r][e], xx);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    f32x2 vp[8];
+                    unpack(vt + ((c * 4 + u) * NG + grp) * HD * 2, vp);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const float x = __shfl_sync(0xffffffffu, s[u], src + (HD == 64 ? r : 2 * r));
+                        if (decltype(later)::value && x == 0.f) continue;
+                        const f32x2 xx = pack2(x, x);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) acc[r][e] = fma2(xx, vp[e], acc[r][e]);
+                    }
+                }
+            }
+        };
 #pragma unroll 1
         for (int t = 0; t < n_t; ++t) {
             const int st = t & 1;
@@ -185,83 +269,8 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
                 const unsigned char* kt = sm + st * 2 * TILE + (wl * 2 + k) * kKvBlock * HD * 2;
                 const unsigned char* vt = kt + TILE;
                 const int cnt = own_pos + 1 - pg * kKvBlock;
-#pragma unroll 1
-                for (int c = 0; c < CPP; ++c) {
-                    float s[16];                      // [row][u]
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        f32x2 kp[8];
-                        unpack(kt + ((c * 4 + u) * NG + grp) * HD * 2, kp);
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            f32x2 d = 0ull;
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) d = fma2(q[r][e], kp[e], d);
-                            float x, y;
-                            unpack2(d, x, y);
-                            s[r * 4 + u] = x + y;
-                        }
-                    }
-                    {
-                        const bool up = (a & (L / 2)) != 0;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float send = up ? s[j] : s[j + 8], keep = up ? s[j + 8] : s[j];
-                            s[j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 2);
-                        }
-                    }
-                    {
-                        const bool up = (a & (L / 4)) != 0;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float send = up ? s[j] : s[j + 4], keep = up ? s[j + 4] : s[j];
-                            s[j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 4);
-                        }
-                    }
-                    if (HD == 128) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], 1);
-                    }
-                    // softmax of the own row
-                    float mn = m;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const bool valid = (c * 4 + u) * NG + grp < cnt;
-                        s[u] = valid ? s[u] / inv_div : kNegBig;
-                        mn = fmaxf(mn, s[u]);
-                    }
-                    const float sc = expf(m - mn);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const bool valid = (c * 4 + u) * NG + grp < cnt;
-                        s[u] = valid ? expf(s[u] - mn) : 0.f;
-                    }
-                    l = __fadd_rn(__fmul_rn(l, sc), s[0]);         // (not one fma: the other kernel's roundings)
-                    l = __fadd_rn(__fadd_rn(__fadd_rn(l, s[1]), s[2]), s[3]);
-                    m = mn;
-                    const int src = lane - a;
-                    if (__any_sync(0xffffffffu, sc != 1.0f)) {
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const float x = __shfl_sync(0xffffffffu, sc, src + (HD == 64 ? r : 2 * r));
-                            const f32x2 xx = pack2(x, x);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) acc[r][e] = mul2(acc[r][e], xx);
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        f32x2 vp[8];
-                        unpack(vt + ((c * 4 + u) * NG + grp) * HD * 2, vp);
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const float x = __shfl_sync(0xffffffffu, s[u], src + (HD == 64 ? r : 2 * r));
-                            const f32x2 xx = pack2(x, x);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) acc[r][e] = fma2(xx, vp[e], acc[r][e]);
-                        }
-                    }
-                }
+                if (pg * kKvBlock + kKvBlock - 1 > warp_first) use_page(std::true_type(), kt, vt, cnt);
+                else use_page(std::false_type(), kt, vt, cnt);
             }
             __syncthreads();                         // the stage is refilled in the next round
         }

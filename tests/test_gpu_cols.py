@@ -1,12 +1,13 @@
 """Prompt columns at the edges of their tiles: column sets of 64 to 4096, attention tiles of 64 (query, head) rows over
 64-position K/V tiles, delta-net chunks of 4 columns in groups of 16, GEMM tiles of 128 columns; against the oracle."""
 import dataclasses
+import os
 
 import numpy as np
 import pytest
 
 from helpers import TOL_FP32, TOL_LOWP, load_oracle, logits_error, oracle_rollout, random_prompts, write_model
-from mini_llm_cuda_b200.model_file import ModelSpec, periodic_layer_types
+from mini_llm_cuda_b200.model_file import ModelSpec, periodic_layer_types, synth_weights, write_model_bin
 
 pytestmark = pytest.mark.gpu
 
@@ -144,5 +145,42 @@ def test_fp8_columns_without_the_bf16_copy(api, tmp_path, monkeypatch):
         assert sess.path(length) == "cols"
     for length in (129, 256):
         assert np.array_equal(got[length], copied[length]), length
+    sess.close()
+    model.close()
+
+
+@pytest.mark.parametrize("name", ["mha64", "gqa4_128", "gqa8_64", "gqa2_128", "fp8"])
+def test_columns_do_not_see_later_positions_that_are_no_numbers(api, tmp_path, name):
+    """A token whose embedding is infinite makes its K/V rows NaN. Neither the tokens before it in the same chunk nor a later request
+    that gets its pages may see them (the token's own logit, from the same row of the tied table, is left out)."""
+    spec = dataclasses.replace(SPECS[name], max_context=400, layer_types=["attention"] * SPECS[name].layers)
+    weights = synth_weights(spec, seed=67)
+    bad = 7
+    weights["tokenEmbeddings"][bad] = np.inf
+    path = os.path.join(str(tmp_path), "m.bin")
+    write_model_bin(path, spec, weights)
+    model = api.Model(path)
+    text = [t for t in random_prompts(spec.vocab, [320], seed=69)[0] if t != bad]
+    fresh = api.Session(model, 1)
+    others = np.arange(spec.vocab) != bad
+    want = fresh.score(text)[:, others]
+    assert np.isfinite(want).all()
+    for at in (1, 15, 16, 33, 70, 131, 200):
+        got = fresh.score(text[:at] + [bad] * 3 + text[at:])[:, others]
+        assert np.array_equal(got[:at], want[:at]), at
+        assert np.isnan(got[at]).all()
+    fresh.close()
+    sess = api.Session(model, 1, max_context=352)
+    sess.prefill([[bad] * 350])                               # every page of the pool
+    for n in (65, 70, 81, 255):
+        sess.prefill([text[:n]])
+        sess.decode_step()
+        used = sess.logits()[:, others]
+        other = api.Session(model, 1, max_context=352)
+        other.prefill([text[:n]])
+        other.decode_step()
+        assert np.isfinite(used).all() and np.array_equal(used, other.logits()[:, others]), n
+        other.close()
+        sess.prefill([[bad] * 350])
     sess.close()
     model.close()
