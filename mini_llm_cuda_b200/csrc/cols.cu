@@ -87,7 +87,8 @@ constexpr int kAcRows = 32;      // (query, head) rows per CTA
 constexpr int kAcThreads = 256;
 constexpr int kAcPages = 4;      // pages of a K/V tile: two for each of the two w of a pass
 
-int attn_cols_queries(int group) { return kAcRows / group; }
+// (a model without attention layers may state any number of heads per kv head)
+int attn_cols_queries(int group) { return group <= kAcRows ? kAcRows / group : 1; }
 
 template <int HD>
 constexpr size_t attn_cols_smem() {

@@ -184,3 +184,20 @@ def test_columns_do_not_see_later_positions_that_are_no_numbers(api, tmp_path, n
         sess.prefill([[bad] * 350])
     sess.close()
     model.close()
+
+
+@pytest.mark.parametrize("weight_dtype", ["bfloat16", "float32"])
+def test_prompt_of_a_model_without_attention_whose_heads_state_no_group(api, tmp_path, weight_dtype):
+    """64 heads, one kv head, delta-net layers only: no attention tile holds 64 heads, and none is needed."""
+    spec = ModelSpec(dim=128, layers=2, heads=64, kv_heads=1, head_dim=64, ffn_dim=256, vocab=128, max_context=96, rms_eps=1e-5, dn_key_dim=64,
+                     dn_value_dim=8, layer_types=["delta_net"] * 2, weight_dtype=weight_dtype, kv_dtype="bfloat16")
+    path = write_model(tmp_path, spec, seed=71)
+    prompt = random_prompts(spec.vocab, [80], seed=73)[0]
+    _, want = oracle_rollout(load_oracle(path), prompt, 1)
+    model = api.Model(path)
+    sess = api.Session(model, 1)
+    sess.prefill([prompt])
+    sess.decode_step()
+    assert logits_error(sess.logits()[0], want[0]) < (TOL_FP32 if weight_dtype == "float32" else TOL_LOWP)
+    sess.close()
+    model.close()
