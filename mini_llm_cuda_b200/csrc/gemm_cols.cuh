@@ -222,6 +222,8 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
         pdl_wait();
         int buf = 0, use = 0;
         bool ok = true;
+        // (tcgen05.ld is a warp-wide instruction: the lanes go on or give up together)
+        auto arrived = [&](int b, int u) { return (bool)__all_sync(0xffffffffu, tc_wait(tfull0 + 8u * b, (uint32_t)u & 1u, p.err, 24)); };
         for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
             const int m0 = t % n_m * kGcM, n0 = t / n_m * bn_out;
             const int tok = m0 + quarter * 32 + lane;
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
             float sums[SUMS ? 64 : 1];
             if (SUMS) {
                 for (int r = 0; r < p.mains && ok; ++r) {
-                    ok = tc_wait(tfull0 + 8u * buf, (uint32_t)use & 1u, p.err, 24);
+                    ok = arrived(buf, use);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a = tmem + (uint32_t)(buf * p.BN) + lane_base;
@@ -287,12 +289,11 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                 }
                 // accumulators of the second pair stay where they are until the element-wise work below has read them
                 for (int r = 0, b = buf, u = use; r < p.exts && ok; ++r) {
-                    ok = tc_wait(tfull0 + 8u * b, (uint32_t)u & 1u, p.err, 24);
+                    ok = arrived(b, u);
                     if (++b == p.nbuf) { b = 0; ++u; }
                 }
                 if (!ok) break;
-            } else if (!tc_wait(tfull0 + 8u * buf, (uint32_t)use & 1u, p.err, 24)) {
-                ok = false;
+            } else if (!(ok = arrived(buf, use))) {
                 break;
             }
             tc_fence_after();

@@ -17,7 +17,9 @@
 //   other warps     one per 16 rows and range: ldmatrix, mma; partial sums to shared memory; epilogue
 // e4m3 weights: ldmatrix on codes hands lane q of a row the codes 4q .. 4q + 3 of sixteen, so the activation operand of such
 // models is written with its features permuted to match inside every sixteen (perm16), and times 2^64 (gd_widen).
-// Every mbarrier wait is bounded.
+// Every mbarrier wait is bounded. A consumer whose wait ran out hands no stage back, so no copy starts behind the last wait of the
+// CTA's last consumer, and those under way have had that wait's time to land when the CTA ends. (Stages handed back by a consumer that
+// no longer waits were refilled into a block about to end.)
 #pragma once
 #include "gemm_tc.cuh"
 
@@ -69,7 +71,7 @@ constexpr float kGdScaleBack = 72057594037927936.0f;       // 2^56
 
 // grid = (ceil(N / 32), ceil(B / (16 NP))), block = 32 (RT split + 1) with RT = 2 (4 for SWIGLU) row tiles of 16.
 template <int MODE, typename KVT, typename WT, int NP>
-__global__ void __launch_bounds__(32 * ((MODE == TC_SWIGLU ? 4 : 2) * kGdMaxSplit + 1)) gemm_dec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
+__global__ void __launch_bounds__(32 * ((MODE == TC_SWIGLU ? 4 : 2) * kGdMaxSplit + 1), MODE == TC_QKV && sizeof(WT) == 2 && NP == 1 ? 3 : 0) gemm_dec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                                                                                   const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWx,
                                                                                   const __grid_constant__ CUtensorMap tmXx, const __grid_constant__ GemmDecParams p,
                                                                                   const __grid_constant__ StepCtl c, const __grid_constant__ QkvPostParams q) {
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(32 * ((MODE == TC_SWIGLU ? 4 : 2) * kGdMaxSpli
         }
         if (i + p.stages < n_iter) {
             __syncwarp();
-            if (lane == 0) mbar_arrive(empty0 + 8u * st);
+            if (lane == 0 && ok) mbar_arrive(empty0 + 8u * st);
         }
         if (++st == p.stages) { st = 0; ph ^= 1u; }
     }
