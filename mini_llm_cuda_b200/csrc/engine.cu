@@ -317,6 +317,24 @@ static int queue_err_readback(mlb_session* s) {
     CU(cudaMemcpyAsync(s->pinned_err, s->dev_err, 4, cudaMemcpyDeviceToHost, s->stream));
     return MLB_OK;
 }
+// What a code that a kernel left in the error word stands for.
+static const char* wait_text(int code) {
+    switch (code) {
+        case 1: return "producer waiting for a free ring stage";
+        case 2: return "consumer waiting for a weight chunk";
+        case 11: return "tcgen05 GEMM, loader waiting for a free stage";
+        case 12: return "tcgen05 GEMM, MMA issuer waiting for operands";
+        case 13: return "tcgen05 GEMM, epilogue waiting for the accumulators";
+        case 14: return "tcgen05 GEMM, widening warps waiting for codes";
+        case 21: return "column GEMM, loader waiting for a free stage";
+        case 22: return "column GEMM, MMA issuer waiting for a free accumulator";
+        case 23: return "column GEMM, MMA issuer waiting for operands";
+        case 24: return "column GEMM, epilogue waiting for an accumulator";
+        case 31: return "decode GEMM, producer waiting for a free stage";
+        case 32: return "decode GEMM, consumer waiting for operands";
+        default: return "consumer waiting for another CTA's results";
+    }
+}
 // After the synchronisation: a bounded device-side wait ran out somewhere in the step.
 static int check_err_readback(mlb_session* s) {
     if (*s->pinned_err == 0) return MLB_OK;
@@ -324,9 +342,7 @@ static int check_err_readback(mlb_session* s) {
     *s->pinned_err = 0;
     cudaMemsetAsync(s->dev_err, 0, 4, s->stream);
     cudaStreamSynchronize(s->stream);
-    return fail(MLB_E_TIMEOUT, "a bounded device-side wait ran out (code %d: %s); the results of this call are invalid", code,
-                code == 1 ? "producer waiting for a free ring stage"
-                          : (code == 2 ? "consumer waiting for a weight chunk" : "consumer waiting for another CTA's results"));
+    return fail(MLB_E_TIMEOUT, "a bounded device-side wait ran out (code %d: %s); the results of this call are invalid", code, wait_text(code));
 }
 
 static void free_session(mlb_session* s) {
