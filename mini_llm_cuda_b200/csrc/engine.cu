@@ -400,7 +400,7 @@ static int run_cols(mlb_session* s, int kind, int* n_launches) {
                     bool normed, const float* next_gain, const mlb_session::TcLayerMaps* ext, const QkvPostParams* q, const float* s1, const float* s2) -> int {
         GemmColsParams p;
         p.N = N; p.K = K; p.BN = g.bn; p.stages = g.stages; p.nkb_x = ext ? (ple + kTcKB - 1) / kTcKB : 0;
-        p.split = g.split; p.mains = g.mains; p.exts = g.exts; p.nbuf = g.nbuf; p.tmem_cols = g.tmem_cols; p.early_w = 1;
+        p.split = g.split; p.mains = g.mains; p.exts = g.exts; p.nbuf = g.nbuf; p.tmem_cols = g.tmem_cols;
         p.y = y; p.h16 = h16; p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = parts; p.eps = cfg.rms_eps;
         p.xg16 = s->xn16; p.gain_next = next_gain; p.ssq_out = s->tc_ssq;
         p.s1 = s1; p.s2 = s2; p.err = s->dev_err;

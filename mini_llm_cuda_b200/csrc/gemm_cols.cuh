@@ -42,7 +42,6 @@ struct GemmColsParams {
                                    // accumulates separately (scaled weights; 0: it shares the main accumulators)
     int nbuf;                      // sets of accumulators in tensor memory: 2 = epilogue under the next k-loop; SUMS: accumulators, used in turn
     uint32_t tmem_cols;
-    int early_w;                   // weight tiles may be fetched before the predecessor kernel has finished
     float* y;                      // RAW: fp32 [c][N]; RESID: residual stream, updated in place
     bf16_t* h16;                   // SWIGLU: bf16 [c][N]
     const float* ssq_in; int ssq_parts; float eps;      // deferred RMS norm, as in GemmTcParams
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
             const uint32_t ring = smem_u32(smem);
             // the first tile's first weight tiles depend on nothing: on their way before the predecessor is waited for
             const int first = blockIdx.x;
-            const int pre = p.early_w ? min(p.stages, nkb) : 0;
+            const int pre = min(p.stages, nkb);
             for (int kb = 0; kb < pre; ++kb) {
                 mbar_expect_tx(full0 + 8u * kb, (uint32_t)stage_bytes);
                 load_w(kb, first / n_m * bn_out, ring + (uint32_t)(kb * stage_bytes), full0 + 8u * kb);

@@ -70,6 +70,8 @@ __device__ __forceinline__ void gd_widen(uint32_t w, uint32_t& lo, uint32_t& hi)
 constexpr float kGdScaleBack = 72057594037927936.0f;       // 2^56
 
 // grid = (ceil(N / 32), ceil(B / (16 NP))), block = 32 (RT split + 1) with RT = 2 (4 for SWIGLU) row tiles of 16.
+// Three CTAs an SM asked for where the compiler would otherwise take 56 registers for a fourth (cfg1 at 4 sequences: 186 us a step with
+// 56, 178 with 72).
 template <int MODE, typename KVT, typename WT, int NP>
 __global__ void __launch_bounds__(32 * ((MODE == TC_SWIGLU ? 4 : 2) * kGdMaxSplit + 1), MODE == TC_QKV && sizeof(WT) == 2 && NP == 1 ? 3 : 0) gemm_dec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                                                                                   const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWx,
