@@ -336,7 +336,7 @@ struct Chain {
                 q.kpool = s->kpool[i]; q.vpool = s->vpool[i]; q.page_table = s->page_table; q.pt_stride = s->max_pages;
                 q.qbuf = s->qbuf; q.gbuf = s->gbuf;
                 if ((rc = gemm_tc<TC_QKV>(s, c, M.qkv, M.qkv, s->tc_g.xn, L.n_qkv, d, nullptr, nullptr, true, nullptr, nullptr, &q, L.Sqkv, nullptr, rec,
-                                          "qkv_gemm_tcgen05_norm_rope_kvappend")))
+                                          s->use_dec ? "qkv_gemm_mma_norm_rope_kvappend" : "qkv_gemm_tcgen05_norm_rope_kvappend")))
                     return rc;
                 ++launches;
                 AttnParams a;
@@ -355,7 +355,7 @@ struct Chain {
                     if ((rc = rec->begin("attn_flash_decode_paged", kvb, fl))) return rc;
                 }
                 const int G = cfg.heads / cfg.kv_heads;
-                if (s->parent && std::is_same<KVT, bf16_t>::value) {
+                if (s->parent && !s->as_steps && std::is_same<KVT, bf16_t>::value) {
                     AttnColsParams ac;
                     ac.kpool = static_cast<const bf16_t*>(s->kpool[i]); ac.vpool = static_cast<const bf16_t*>(s->vpool[i]);
                     ac.page_table = s->page_table; ac.pt_stride = s->max_pages;
@@ -371,7 +371,7 @@ struct Chain {
                 ++launches;
             } else {
                 if ((rc = gemm_tc<TC_RAW>(s, c, M.qkv, M.qkv, s->tc_g.xn, L.n_qkv, d, s->raw, nullptr, true, nullptr, nullptr, nullptr, L.Sqkv, nullptr, rec,
-                                          "deltanet_proj_gemm_tcgen05")))
+                                          s->use_dec ? "deltanet_proj_gemm_mma" : "deltanet_proj_gemm_tcgen05")))
                     return rc;
                 ++launches;
                 const int dk = cfg.dn_key_dim, dv = cfg.dn_value_dim, H = cfg.heads;
@@ -389,17 +389,17 @@ struct Chain {
             }
             const CUtensorMap* amap = L.type == MLB_LAYER_ATTENTION ? s->tc_g.a_attn : s->tc_g.a_dn;
             if ((rc = gemm_tc<TC_RESID>(s, c, M.o, M.o, amap, d, L.o_in, s->x, nullptr, false, L.g2, nullptr, nullptr, L.So, nullptr, rec,
-                                        "oproj_gemm_tcgen05_residual_norm")))
+                                        s->use_dec ? "oproj_gemm_mma_residual_norm" : "oproj_gemm_tcgen05_residual_norm")))
                 return rc;
             ++launches;
             if ((rc = gemm_tc<TC_SWIGLU>(s, c, M.w1a, M.w1b, s->tc_g.xn, F, d, nullptr, s->h16, true, nullptr, nullptr, nullptr, L.S1a, L.S1b, rec,
-                                         "ffn_gateup_gemm_tcgen05_swiglu")))
+                                         s->use_dec ? "ffn_gateup_gemm_mma_swiglu" : "ffn_gateup_gemm_tcgen05_swiglu")))
                 return rc;
             ++launches;
             const bool last = i + 1 == cfg.layers;
             const float* g_next = last ? m->g_final : m->layers[i + 1].g1;
             if ((rc = gemm_tc<TC_RESID>(s, c, M.w2, M.w2, s->tc_g.h, d, F, s->x, nullptr, false, g_next,
-                                        (!last && ple > 0) ? &s->tc_maps[i + 1] : nullptr, nullptr, L.S2, nullptr, rec, "ffn_down_gemm_tcgen05_residual_ple_norm")))
+                                        (!last && ple > 0) ? &s->tc_maps[i + 1] : nullptr, nullptr, L.S2, nullptr, rec, s->use_dec ? "ffn_down_gemm_mma_residual_ple_norm" : "ffn_down_gemm_tcgen05_residual_ple_norm")))
                 return rc;
             ++launches;
         }
@@ -412,7 +412,7 @@ struct Chain {
             ++launches;
         } else {
             if ((rc = gemm_tc<TC_RAW>(s, c, s->tc_g.E, s->tc_g.E, s->tc_g.xn, cfg.vocab, d, s->logits, nullptr, true, nullptr, nullptr, nullptr, static_cast<const float*>(m->Es), nullptr, rec,
-                                      "lmhead_gemm_tcgen05")))
+                                      s->use_dec ? "lmhead_gemm_mma" : "lmhead_gemm_tcgen05")))
                 return rc;
             ++launches;
             if (s->parent) {

@@ -755,7 +755,14 @@ static int tc_probe_clusters(mlb_session* s) {
     return MLB_OK;
 }
 
-// Tensor-core projections for batches of 4 sequences or more with bf16 weights (MLB_GEMM=simt turns it off).
+// MLB_GEMM=tcgen05: every tensor-core projection on gemm_tc.cuh, and prompt columns as steps of the decode kernels, whose results those of
+// gemm_dec.cuh, gemm_cols.cuh and attn_cols_kernel have to equal bit for bit.
+static bool gemm_tcgen05_only() {
+    const char* v = std::getenv("MLB_GEMM");
+    return v && std::string(v) == "tcgen05";
+}
+
+// Tensor-core projections for batches of 4 sequences or more with bf16 or FP8 weights (MLB_GEMM=simt turns them off).
 static int setup_tc_path(mlb_session* s) {
     const mlb_config& c = s->m->cfg;
     s->use_tc = false;
@@ -763,7 +770,7 @@ static int setup_tc_path(mlb_session* s) {
     const std::string mode = env ? env : "auto";
     if (!s->parent && (mode == "simt" || s->use_grid || s->use_lean)) return MLB_OK;
     if (c.weight_dtype != MLB_DT_BF16 && c.weight_dtype != MLB_DT_FP8_E4M3) {
-        if (mode == "tc") return fail(MLB_E_UNSUPPORTED, "MLB_GEMM=tc needs bf16 or FP8 weights");
+        if (mode != "auto") return fail(MLB_E_UNSUPPORTED, "MLB_GEMM=%s needs bf16 or FP8 weights", mode.c_str());
         return MLB_OK;
     }
     const bool w8 = c.weight_dtype == MLB_DT_FP8_E4M3;
@@ -773,7 +780,7 @@ static int setup_tc_path(mlb_session* s) {
     if (!s->parent && mode == "auto" && s->B < 4) return MLB_OK;
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) {
-        if (mode == "tc") return fail(MLB_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+        if (mode != "auto") return fail(MLB_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
         return MLB_OK;
     }
     const int B = s->B;
@@ -791,13 +798,14 @@ static int setup_tc_path(mlb_session* s) {
     const auto kb = [](int k) { return (k + kTcKB - 1) / kTcKB; };
     // mma.sync tiles for the projections, or tcgen05 ones: gd_small_enough. The QK norm needs whole heads in a tile, the k-block maps
     // whole k-blocks, the ranges of a tile a warp each: other models stay on gemm_tc.cuh.
-    s->use_dec = !s->parent && !c.qk_norm && gd_small_enough(s) && c.dim % kTcKB == 0 && c.ffn_dim % kTcKB == 0 && c.ple_dim % kTcKB == 0 &&
+    s->use_dec = !s->parent && mode != "tcgen05" && !c.qk_norm && (mode == "mma" ? B <= 256 : gd_small_enough(s)) && c.dim % kTcKB == 0 && c.ffn_dim % kTcKB == 0 && c.ple_dim % kTcKB == 0 &&
                  nq % kTcKB == 0 && a_dn % kTcKB == 0;
     const auto ranges_fit = [&](int n, int nkb, int mode, bool ext) { return gd_pick(s, n, nkb, mode, w8, ext).split <= kGdMaxSplit; };
     for (int i = 0; i < c.layers && s->use_dec; ++i)
         s->use_dec = ranges_fit(s->m->layers[i].n_qkv, kb(c.dim), TC_QKV, false) && ranges_fit(c.dim, kb(s->m->layers[i].o_in), TC_RESID, false);
     s->use_dec = s->use_dec && ranges_fit(c.ffn_dim, kb(c.dim), TC_SWIGLU, false) && ranges_fit(c.vocab, kb(c.dim), TC_RAW, false) &&
                  ranges_fit(c.dim, kb(c.ffn_dim) + kb(c.ple_dim), TC_RESID, c.ple_dim > 0) && ranges_fit(c.dim, kb(c.ffn_dim), TC_RESID, false);
+    if (mode == "mma" && !s->use_dec && !s->parent) return fail(MLB_E_UNSUPPORTED, "MLB_GEMM=mma: a QK norm, a width or the batch rules its tiles out");
     s->tc_shape_down = tc_pick_shape(s, B, c.dim, (c.ffn_dim + kTcKB - 1) / kTcKB + (c.ple_dim + kTcKB - 1) / kTcKB, 1, w8, w8 ? 2 : 1);
     const int parts = (c.dim + kTcM - 1) / kTcM * 4;
     if ((rc = sess_alloc(s, (void**)&s->xn16, (size_t)B * c.dim * 2, true))) return rc;
@@ -1198,7 +1206,8 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
     bool has_dn = false, has_attn = false;
     for (int i = 0; i < c.layers; ++i) (c.layer_types[i] == MLB_LAYER_DELTA_NET ? has_dn : has_attn) = true;
     // a column set's attention over a bf16 cache (attn_cols_kernel) has no splits and writes the next operand only
-    const bool split_attn = !parent || gemv_cols || c.kv_dtype == MLB_DT_F32;
+    s->as_steps = parent && !gemv_cols && gemm_tcgen05_only();
+    const bool split_attn = !parent || gemv_cols || s->as_steps || c.kv_dtype == MLB_DT_F32;
     s->max_q = nq;
     s->raw_stride = 2 * c.heads * c.dn_key_dim + c.heads * c.dn_value_dim + 2 * c.heads;
     SA(sess_alloc(s, (void**)&s->x, B * c.dim * 4, true));
@@ -1295,7 +1304,7 @@ static int session_create(mlb_model* m, int batch, int max_context, int kv_block
         if (!s->use_lean) SA(setup_grid_path(s));
     }
     if (parent && !gemv_cols) {        // columns in fp32 run the GEMV chain
-        SA(setup_cols_path(s));
+        if (!s->as_steps) SA(setup_cols_path(s));
         if (!s->use_cols) SA(setup_tc_path(s));
         if (!s->use_cols && !s->use_tc) {
             free_session(s);

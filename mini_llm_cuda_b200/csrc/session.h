@@ -153,7 +153,7 @@ struct mlb_session {
     int lean_idx = -1;
     size_t lean_smem = 0;
     mlb::LeanParams lean;
-    // tensor-core projections (bf16 weights, batch >= 16)
+    // tensor-core projections (bf16 or FP8 weights, batch >= 4)
     bool use_tc = false;
     bool use_dec = false;                     // the step's projections on mma.sync tiles (gemm_dec.cuh) instead of tcgen05 ones
     int tc_nb = 0, tc_stages = 0, tc_stages_swiglu = 0;
@@ -183,6 +183,7 @@ struct mlb_session {
     mlb_session* parent = nullptr;          // set in a column set
     int* seq_of = nullptr;                  // [B] in a column set: column -> sequence of the parent
     bool use_cols = false;                  // column set: persistent column GEMMs (else, without the bf16 codes, run_tc)
+    bool as_steps = false;                  // column set: on the decode step's kernels throughout (MLB_GEMM=tcgen05)
     bool no_copy = false;                   // column set of an FP8 model that was made without them
     ColsGemm cg_qkv{}, cg_dn{}, cg_o_attn{}, cg_o_dn{}, cg_up{}, cg_down{}, cg_last{}, cg_head{};      // cg_last: the last layer's down projection
     mlb::ColsPlan plan;                     // column set: what the columns of the current chunk are (one array, plan_dev)

@@ -1,0 +1,93 @@
+"""Kernels that are built to return the bits of the kernel they replaced, held to it on one model: the projections of a step on mma.sync
+and on tcgen05 tiles, the column GEMMs and the column attention against the decode step's kernels, the column form of the delta-net
+recurrence (one row of the state per lane group, or four) against the step's."""
+import numpy as np
+import pytest
+
+from helpers import random_prompts, write_model
+from mini_llm_cuda_b200.model_file import ModelSpec, periodic_layer_types
+
+pytestmark = pytest.mark.gpu
+
+COMMON = dict(kv_dtype="bfloat16", rms_eps=1e-5, max_context=320)
+SPECS = {
+    # 21 + 1 k-blocks in ranges; a vocabulary that ends inside a tile
+    "bf16": ModelSpec(dim=256, layers=4, heads=4, head_dim=64, ffn_dim=1344, ple_dim=64, vocab=500, layer_types=periodic_layer_types(4, 2),
+                      weight_dtype="bfloat16", **COMMON),
+    "bf16_gqa_gated": ModelSpec(dim=512, layers=2, heads=8, kv_heads=2, head_dim=128, ffn_dim=1408, vocab=512, query_gating=True, weight_dtype="bfloat16", **COMMON),
+    "fp8": ModelSpec(dim=512, layers=4, heads=4, kv_heads=1, head_dim=128, ffn_dim=1408, ple_dim=64, vocab=512, layer_types=periodic_layer_types(4, 3),
+                     weight_dtype="float8_e4m3", **COMMON),
+}
+QK_NORM = {
+    "bf16_qknorm": ModelSpec(dim=256, layers=2, heads=4, kv_heads=1, head_dim=128, ffn_dim=264, vocab=512, qk_norm=True, query_gating=True,
+                             weight_dtype="bfloat16", **COMMON),
+}
+
+
+@pytest.fixture(scope="module")
+def api(built_lib):
+    from mini_llm_cuda_b200 import api as _api
+    return _api
+
+
+@pytest.mark.parametrize("name", list(SPECS))
+def test_step_projections_on_both_tiles(api, tmp_path, monkeypatch, name):
+    """Token loop of four tokens, then four greedy steps: ids and logits, 4 to 256 sequences."""
+    monkeypatch.setenv("MLB_PREFILL", "step")
+    spec = SPECS[name]
+    model = api.Model(write_model(tmp_path, spec, seed=101))
+    for batch in (4, 17, 37, 64, 130, 256):
+        prompts = random_prompts(spec.vocab, [1 + b % 4 for b in range(batch)], seed=103)
+        got = {}
+        for tiles in ("mma", "tcgen05"):
+            monkeypatch.setenv("MLB_GEMM", tiles)
+            sess = api.Session(model, batch)
+            assert sess.path() == tiles
+            names = [k["name"] for k in sess.profile(1, False) if "gemm" in k["name"]]
+            assert len(names) >= 4 and all(tiles in n for n in names), names
+            sess.prefill(prompts)
+            got[tiles] = sess.decode(4), sess.logits()
+            sess.close()
+        assert np.array_equal(got["mma"][0], got["tcgen05"][0]) and np.array_equal(got["mma"][1], got["tcgen05"][1]), batch
+    model.close()
+
+
+@pytest.mark.parametrize("name", [*SPECS, *QK_NORM])
+def test_columns_against_the_decode_steps_kernels(api, tmp_path, monkeypatch, name):
+    """129 to 256 columns (one set, whose k-ranges are those that every width takes): every position's logits."""
+    spec = {**SPECS, **QK_NORM}[name]
+    model = api.Model(write_model(tmp_path, spec, seed=105))
+    text = random_prompts(spec.vocab, [256], seed=107)[0]
+    got = {}
+    for gemm, path in (("auto", "cols"), ("tcgen05", "tcgen05")):
+        monkeypatch.setenv("MLB_GEMM", gemm)
+        sess = api.Session(model, 1)
+        for n in (129, 200, 256):
+            got[gemm, n] = sess.score(text[:n])
+            assert sess.path(n) == path
+        sess.close()
+    for n in (129, 200, 256):
+        assert np.array_equal(got["auto", n], got["tcgen05", n]), n
+    model.close()
+
+
+@pytest.mark.parametrize("dk,dv,heads,batch", [(64, 72, 3, 1), (128, 128, 4, 1), (64, 64, 4, 48), (128, 72, 3, 48)])
+def test_recurrence_over_columns_against_steps(api, tmp_path, monkeypatch, dk, dv, heads, batch):
+    """fp32 models run prompt columns and steps on the same GEMV chain, so that the recurrence is what differs: one sequence (one row per
+    lane group) and 48 (four rows)."""
+    monkeypatch.setenv("MLB_DECODE_PATH", "chain")
+    spec = ModelSpec(dim=192, layers=2, heads=heads, head_dim=64, ffn_dim=256, dn_key_dim=dk, dn_value_dim=dv, vocab=300, max_context=96, rms_eps=1e-5,
+                     layer_types=["delta_net"] * 2, weight_dtype="float32", kv_dtype="float32")
+    model = api.Model(write_model(tmp_path, spec, seed=109))
+    prompts = random_prompts(spec.vocab, [41 - b % 7 for b in range(batch)], seed=111)
+    got = {}
+    for mode in ("auto", "step"):
+        monkeypatch.setenv("MLB_PREFILL", mode)
+        sess = api.Session(model, batch)
+        sess.prefill(prompts)
+        assert (sess.path(batch * 40) != "none") == (mode == "auto")
+        sess.decode_step()
+        got[mode] = sess.logits()
+        sess.close()
+    assert np.array_equal(got["auto"], got["step"])
+    model.close()
