@@ -1,5 +1,5 @@
-"""Prompt columns at the edges of their tiles: column sets of 64 to 4096, attention tiles of 64 (query, head) rows over
-64-position K/V tiles, delta-net chunks of 4 columns in groups of 16, GEMM tiles of 128 columns; against the oracle."""
+"""Prompt columns at the edges of their tiles: column sets of 64 to 4096, attention tiles of 32 (query, head) rows over
+64-position K/V tiles, delta-net stages of 16 columns, GEMM tiles of 128 columns; against the oracle."""
 import dataclasses
 import os
 
@@ -44,6 +44,7 @@ def test_scored_columns_at_tile_edges(api, tmp_path, name):
     sess = api.Session(model, 1)
     for length in (1, 2, 15, 17, 63, 64, 65, 127, 128, 129, 1025):
         got = sess.score(tokens[:length])
+        assert sess.path(length) == "cols"
         worst = max(logits_error(got[i], want[i]) for i in range(length))
         assert worst < TOL_LOWP, (length, worst)
     sess.close()

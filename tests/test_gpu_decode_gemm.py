@@ -40,6 +40,7 @@ def test_decode_projections_at_tile_edges(api, tmp_path, name):
     model = api.Model(path)
     for batch in (4, 5, 15, 16, 17, 32, 33, 64, 65, 129, 256):
         sess = api.Session(model, batch)
+        assert sess.path() == "mma"
         sess.prefill([texts[b % 11][:1] for b in range(batch)])
         for k in range(4):
             sess.decode_step(in_tokens=np.array([texts[b % 11][k] for b in range(batch)], dtype=np.int32))

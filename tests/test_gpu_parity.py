@@ -191,8 +191,9 @@ def test_ragged_batch_matches_oracle(api, tmp_path, monkeypatch, name, batch, pa
                                                    ("odd_bf16", 21, "auto", 4), ("odd_fp8", 37, "auto", 0), ("odd_fp8", 37, "auto", 2)])
 def test_tensor_core_batch_path_matches_oracle(api, tmp_path, monkeypatch, name, batch, gemm, split):
     """Batch >= 4 with bf16 weights, or FP8 weights widened to bf16 tile by tile inside the kernel, runs the
-    projections as tcgen05 GEMMs on bf16 activations. `split` pins the largest thread-block cluster that may
-    share the k-blocks of an output tile (0: the library's choice).
+    projections as tensor-core GEMMs on bf16 activations: mma.sync tiles where widths and k-ranges allow (a per-layer
+    embedding of 32, odd widths and more than four ranges do not), else tcgen05 ones. `split` pins the largest
+    thread-block cluster that may share the k-blocks of an output tile (0: the library's choice).
     Teacher-forced on the oracle's tokens: logits within 2e-2 at every step; the device pick equals
     the oracle's wherever the oracle's top-2 margin exceeds that bound."""
     monkeypatch.setenv("MLB_GEMM", gemm)
@@ -207,6 +208,7 @@ def test_tensor_core_batch_path_matches_oracle(api, tmp_path, monkeypatch, name,
     rolls = [oracle_rollout(oracle, prompts[b], steps) for b in range(batch)]
     model = api.Model(path)
     sess = api.Session(model, batch)
+    assert sess.path() == ("mma" if name in ("bf16_wide_ple", "bf16_w_f32_kv") and split <= 4 else "tcgen05")
     sess.prefill(prompts)
     worst = 0.0
     checked = 0
@@ -261,7 +263,7 @@ def test_baseline_batched_shapes_match_oracle(api, tmp_path, name):
     model = api.Model(path)
     sess = api.Session(model, batch)
     sess.prefill(prompts)
-    assert sess.launches_per_step() > 1          # the tensor-core chain, not a batch-1 kernel
+    assert sess.path() == ("tcgen05" if name == "cfg4" else "mma")          # cfg4: 10 M products per SM in the gate/up projection
     worst, checked, close_calls = 0.0, 0, 0
     prev = None
     for i in range(steps):
