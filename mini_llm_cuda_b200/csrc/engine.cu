@@ -1668,7 +1668,8 @@ static int decode_impl(mlb_session* s, const mlb_sampling* sp, int n, const int3
     bool any = false;
     for (int b = 0; b < B; ++b) any = any || seq_live(s, b);
     if (!any) return fail(MLB_E_CONTEXT_FULL, "every sequence is at max_context %d or has drawn the stop token", s->max_ctx);
-    if (n > s->max_ctx) n = std::min(n, s->max_ctx);
+    const int n_out = n;                       // ids per sequence in out_tokens; behind max_context steps none is left to take
+    n = std::min(n, s->max_ctx);
     int kind, rc;
     if ((rc = apply_sampling(s, sp, &kind))) return rc;
     if ((rc = grow_pages(s, n))) return rc;
@@ -1679,7 +1680,7 @@ static int decode_impl(mlb_session* s, const mlb_sampling* sp, int n, const int3
             s->pinned_tok[b] = in_tokens[b];
         }
     }
-    if (n == 1 && !step_ms && !s->use_grid && !s->use_lean) {
+    if (n_out == 1 && !step_ms && !s->use_grid && !s->use_lean) {
         // the one-token call: one graph launch, one synchronisation
         if ((rc = ensure_token_graph(s, kind, in_tokens != nullptr))) return rc;
         // The kernel that advances a sequence writes its id to pinned host memory (the error word first, by
@@ -1707,7 +1708,7 @@ static int decode_impl(mlb_session* s, const mlb_sampling* sp, int n, const int3
         s->have_logits = true;
         return check_err_readback(s);
     }
-    if (n == 1 && !step_ms && B == 1 && (s->use_grid || s->use_lean) && seq_live(s, 0)) {
+    if (n_out == 1 && !step_ms && B == 1 && (s->use_grid || s->use_lean) && seq_live(s, 0)) {
         // The one-token call of the single-kernel step: the pending id travels as a launch argument, the
         // kernel that advances the sequence writes the picked id and the error word to pinned host memory,
         // and the host polls that word instead of synchronising the stream (which costs 5-10 us more).
@@ -1756,19 +1757,23 @@ static int decode_impl(mlb_session* s, const mlb_sampling* sp, int n, const int3
         // one id per sequence: gather through the pinned buffer
         CU(cudaMemcpy2DAsync(s->pinned_tok, 4, s->out_ring, (size_t)s->max_ctx * 4, 4, B, cudaMemcpyDeviceToHost, s->stream));
         CU(cudaStreamSynchronize(s->stream));
-        for (int b = 0; b < B; ++b) out_tokens[b] = s->pinned_tok[b];
+        for (int b = 0; b < B; ++b) out_tokens[(size_t)b * n_out] = s->pinned_tok[b];
     } else {
         std::vector<int> ring((size_t)B * n);
         CU(cudaMemcpy2DAsync(ring.data(), (size_t)n * 4, s->out_ring, (size_t)s->max_ctx * 4, (size_t)n * 4, B, cudaMemcpyDeviceToHost, s->stream));
         CU(cudaStreamSynchronize(s->stream));
-        std::memcpy(out_tokens, ring.data(), ring.size() * 4);
+        for (int b = 0; b < B; ++b) std::memcpy(out_tokens + (size_t)b * n_out, &ring[(size_t)b * n], (size_t)n * 4);
     }
     if (step_ms) {
+        std::fill(step_ms + n, step_ms + n_out, 0.f);
         for (int i = 0; i < n; ++i) CU(cudaEventElapsedTime(&step_ms[i], ev[2 * i], ev[2 * i + 1]));
         if (total_ms) CU(cudaEventElapsedTime(total_ms, ev[0], ev[2 * (size_t)n - 1]));
         for (auto& e : ev) cudaEventDestroy(e);
     }
-    for (int b = 0; b < B; ++b) note_outputs(s, b, &out_tokens[(size_t)b * n], n);
+    for (int b = 0; b < B; ++b) {
+        note_outputs(s, b, &out_tokens[(size_t)b * n_out], n);
+        std::fill(&out_tokens[(size_t)b * n_out] + n, &out_tokens[(size_t)b * n_out] + n_out, -1);
+    }
     s->have_logits = true;
     return check_err_readback(s);
 }

@@ -525,6 +525,25 @@ def test_context_limit_and_errors(api, tmp_path):
     model.close()
 
 
+def test_more_steps_than_the_context_holds(api, tmp_path):
+    """mlb_decode_n for more ids than max_context: every sequence's row has the length asked for, -1 behind its end."""
+    spec = small(max_context=20)
+    model = api.Model(write_model(tmp_path, spec, seed=11))
+    prompts = random_prompts(spec.vocab, [5, 12], seed=2)
+    sess = api.Session(model, 2)
+    sess.prefill(prompts)
+    want = sess.decode(20)
+    sess.prefill(prompts)
+    got = sess.decode(33)
+    assert np.array_equal(got[:, :20], want) and (got[:, 20:] == -1).all()
+    sess.prefill(prompts)
+    ms, got = sess.decode_timed(33, False)
+    assert np.array_equal(got[:, :20], want) and (got[:, 20:] == -1).all()
+    assert (ms[:20] > 0).all() and (ms[20:] == 0).all()
+    sess.close()
+    model.close()
+
+
 def test_topk_sampler_matches_oracle_on_device_logits(api, tmp_path):
     """Teacher-forced: at every step the device's draw must equal the oracle's draw from the
     device's own logits (same Philox counter), except where the uniform lands within 1e-5 of a
