@@ -405,8 +405,8 @@ cudaError_t attn_cols_launch(int head_dim, int group, bool pdl, int max_tiles, c
 // share R rows; a lane holds the elements of four of that kernel's lanes (a, a + 8, a + 16, a + 24), as packed pairs, so
 // that the first two steps of a row's 32-lane sum are its own additions and three shuffle steps are left, on values halved from
 // step to step; k^ and q^ of a column are read from shared memory once for R rows. The inputs of 16 columns at a time come
-// through a three-stage cp.async ring and are L2-normalised there. R = 4 where the sequences fill the SMs (fewest
-// instructions per row), else R = 1 (a quarter of the rows, and of the instructions in the chain, per warp).
+// through a three-stage cp.async ring and are L2-normalised there. R = 4 where the chunk's runs fill the SMs (fewest
+// instructions per row), else R = 1 (a quarter of the rows, and of the instructions in the chain, per warp): delta_cols_serial.
 // ------------------------------------------------------------------------------------------------
 constexpr int kDcCols = 16;       // columns per ring stage
 constexpr int kDcStages = 3;
@@ -632,8 +632,14 @@ static cudaError_t delta_cols_one(bool pdl, int max_runs, cudaStream_t st, const
     return launch_pdl(pdl, delta_cols_kernel<DK, R>, dim3((p.dv + rows - 1) / rows, p.H, max_runs), dim3(kDcThreads), smem, st, p);
 }
 
-cudaError_t delta_cols_launch(int dk, bool pdl, int max_runs, cudaStream_t st, const DeltaColsParams& p) {
-    const bool few = (long)max_runs * p.H * p.dv < 148L * 16 * kDcWarps;
+// One row per lane group where a chunk is a serial chain rather than a load: columns / longest run sequences side by side, each of H dv rows,
+// do not give every SM a CTA of 64 rows. Measured per launch, one row -> four: one run of 3000 columns (dk 128, 16 heads) 2074 -> 3494 us,
+// of 899 (dk 64, 8 heads) 318 -> 424.
+bool delta_cols_serial(int sm_count, int H, int dv, int columns, int longest) {
+    return (long)columns * H * dv < (long)longest * sm_count * 16 * kDcWarps;
+}
+
+cudaError_t delta_cols_launch(int dk, bool few, bool pdl, int max_runs, cudaStream_t st, const DeltaColsParams& p) {
     if (dk == 64) return few ? delta_cols_one<64, 1>(pdl, max_runs, st, p) : delta_cols_one<64, 4>(pdl, max_runs, st, p);
     return few ? delta_cols_one<128, 1>(pdl, max_runs, st, p) : delta_cols_one<128, 4>(pdl, max_runs, st, p);
 }

@@ -40,7 +40,9 @@ struct DeltaColsParams {
     float l2_eps;
     const int* hdr; const int4* runs;
 };
-cudaError_t delta_cols_launch(int dk, bool pdl, int max_runs, cudaStream_t st, const DeltaColsParams& p);
+// Which form a chunk of `columns`, the longest run of `longest`, takes: `few` of delta_cols_launch.
+bool delta_cols_serial(int sm_count, int H, int dv, int columns, int longest);
+cudaError_t delta_cols_launch(int dk, bool few, bool pdl, int max_runs, cudaStream_t st, const DeltaColsParams& p);
 
 // ---- embedding of a chunk ------------------------------------------------------------------------
 struct EmbedColsParams {

@@ -354,6 +354,7 @@ static void free_session(mlb_session* s) {
     for (auto& e : s->plan_free) if (e) cudaEventDestroy(e);
     if (s->plan_host) cudaFreeHost(s->plan_host);
     for (auto& g : s->graphs) if (g) cudaGraphExecDestroy(g);
+    for (auto& g : s->other_graphs) if (g) cudaGraphExecDestroy(g);
     for (auto& g : s->tgraphs) if (g) cudaGraphExecDestroy(g);
     for (void* p : s->allocs) cudaFree(p);
     if (s->parent) s->parent->cols_bytes -= s->own_bytes;
@@ -1463,6 +1464,8 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
         s->cols_failed = rc != MLB_E_NOMEM;        // memory may come back: asked for again by the next prompt
         return mode == "chunk" ? rc : (int)MLB_OK;
     }
+    bool has_dn = false;
+    for (int i = 0; i < cfg.layers; ++i) has_dn = has_dn || cfg.layer_types[i] == MLB_LAYER_DELTA_NET;
     const size_t V = (size_t)cfg.vocab;
     const int qt = attn_cols_queries(cfg.heads / cfg.kv_heads);
     size_t scored = 0;
@@ -1472,7 +1475,7 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     std::vector<int> cursor(B, 0);
     long left = total;
     for (int slot = 0; left > 0; slot = (slot + 1) % kPlanSlots) {
-        if ((rc = get(left)) || (rc = ensure_graph(cs, kind))) return rc;
+        if ((rc = get(left))) return rc;
         const int want = (int)std::min<long>(left, cs->B);
         // the largest equal share that fits; what is left over goes to the first sequences
         int lo = 0, hi = want;
@@ -1489,12 +1492,13 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
         const ColsLayout lay = cols_layout(cfg, s->B, cs->B);
         int* pl = s->plan_host + slot * s->plan_host_ints;
         CU(cudaEventSynchronize(s->plan_free[slot]));      // the slot's last plan has left it, also one of a call that failed half-way
-        int n = 0, runs = 0, tiles = 0;
+        int n = 0, runs = 0, tiles = 0, longest = 0;
         for (int b = 0; b < B; ++b) {
             const int rest = lens[b] - keep - cursor[b];
             int take = std::min(rest, lo);
             if (extra > 0 && take < rest) { ++take; --extra; }
             if (take <= 0) continue;
+            longest = std::max(longest, take);
             int* r = pl + lay.runs + 4 * (size_t)runs++;
             r[0] = n; r[1] = take; r[2] = b; r[3] = cursor[b];
             for (int q = 0; q < take; q += qt) {
@@ -1513,6 +1517,12 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
         for (int i = n; i < cs->B; ++i) pl[lay.tok + i] = pl[lay.pos + i] = pl[lay.lim + i] = pl[lay.seq + i] = 0;      // idle columns
         pl[0] = n; pl[1] = runs; pl[2] = tiles; pl[3] = 0;
         left -= n;
+        const bool few = has_dn && delta_cols_serial(s->sm_count, cfg.heads, cfg.dn_value_dim, n, longest);
+        if (cs->few_runs != few) {
+            std::swap(cs->graphs, cs->other_graphs);
+            cs->few_runs = few;
+        }
+        if ((rc = ensure_graph(cs, kind))) return rc;
         CU(cudaMemcpyAsync(cs->plan_dev, pl, lay.ints * 4, cudaMemcpyHostToDevice, s->stream));
         CU(cudaEventRecord(s->plan_free[slot], s->stream));
         CU(cudaGraphLaunch(cs->graphs[kind], s->stream));

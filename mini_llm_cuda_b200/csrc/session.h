@@ -186,6 +186,8 @@ struct mlb_session {
     bool as_steps = false;                  // column set: on the decode step's kernels throughout (MLB_GEMM=tcgen05)
     bool no_copy = false;                   // column set of an FP8 model that was made without them
     ColsGemm cg_qkv{}, cg_dn{}, cg_o_attn{}, cg_o_dn{}, cg_up{}, cg_down{}, cg_last{}, cg_head{};      // cg_last: the last layer's down projection
+    bool few_runs = false;                  // column set: form of the delta-net recurrence in `graphs`; the other form's are other_graphs
+    cudaGraphExec_t other_graphs[3] = {nullptr, nullptr, nullptr};
     mlb::ColsPlan plan;                     // column set: what the columns of the current chunk are (one array, plan_dev)
     int* plan_dev = nullptr;
     int* plan_host = nullptr;               // session: pinned ring of kPlanSlots plans of the widest set
@@ -310,7 +312,7 @@ static inline cudaError_t delta_cols(const mlb_session* s, int i, float* out, bf
     dc.raw = s->raw; dc.raw_stride = s->raw_stride; dc.state = s->state[i]; dc.H = cfg.heads; dc.dv = cfg.dn_value_dim;
     dc.out = out; dc.out16 = out16; dc.l2_eps = 1e-6f;
     dc.hdr = s->plan.hdr; dc.runs = reinterpret_cast<const int4*>(s->plan.runs);
-    return delta_cols_launch(cfg.dn_key_dim, s->use_pdl, s->plan.max_runs, s->stream, dc);
+    return delta_cols_launch(cfg.dn_key_dim, s->few_runs, s->use_pdl, s->plan.max_runs, s->stream, dc);
 }
 
 // ---- the launch chains (chain_f32.cu, chain_bf16.cu, chain_fp8.cu) ------------------------------------

@@ -71,23 +71,28 @@ def test_columns_against_the_decode_steps_kernels(api, tmp_path, monkeypatch, na
     model.close()
 
 
-@pytest.mark.parametrize("dk,dv,heads,batch", [(64, 72, 3, 1), (128, 128, 4, 1), (64, 64, 4, 48), (128, 72, 3, 48)])
-def test_recurrence_over_columns_against_steps(api, tmp_path, monkeypatch, dk, dv, heads, batch):
+@pytest.mark.parametrize("dk,dv,heads,batch,uneven", [(64, 72, 3, 1, 0), (128, 128, 4, 1, 0), (64, 64, 4, 48, 0), (128, 72, 3, 48, 0), (64, 64, 4, 48, 1),
+                                                      (128, 72, 3, 48, 1)])
+def test_recurrence_over_columns_against_steps(api, tmp_path, monkeypatch, dk, dv, heads, batch, uneven):
     """fp32 models run prompt columns and steps on the same GEMV chain, so that the recurrence is what differs: one sequence (one row per
-    lane group) and 48 (four rows)."""
+    lane group), 48 (four rows), 48 of which one has a long prompt (one row again); twice, in one order and in the other."""
     monkeypatch.setenv("MLB_DECODE_PATH", "chain")
     spec = ModelSpec(dim=192, layers=2, heads=heads, head_dim=64, ffn_dim=256, dn_key_dim=dk, dn_value_dim=dv, vocab=300, max_context=96, rms_eps=1e-5,
                      layer_types=["delta_net"] * 2, weight_dtype="float32", kv_dtype="float32")
     model = api.Model(write_model(tmp_path, spec, seed=109))
-    prompts = random_prompts(spec.vocab, [41 - b % 7 for b in range(batch)], seed=111)
+    even, one_long = [41 - b % 7 for b in range(batch)], [90 if b == 3 else 2 for b in range(batch)]
+    asked = [random_prompts(spec.vocab, lens, seed=111) for lens in ([one_long, even, one_long] if uneven else [even])]
     got = {}
     for mode in ("auto", "step"):
         monkeypatch.setenv("MLB_PREFILL", mode)
         sess = api.Session(model, batch)
-        sess.prefill(prompts)
-        assert (sess.path(batch * 40) != "none") == (mode == "auto")
-        sess.decode_step()
-        got[mode] = sess.logits()
+        got[mode] = []
+        for prompts in asked:
+            sess.prefill(prompts)
+            assert (sess.path(sum(len(p) - 1 for p in prompts)) != "none") == (mode == "auto")
+            sess.decode_step()
+            got[mode].append(sess.logits())
         sess.close()
-    assert np.array_equal(got["auto"], got["step"])
+    for a, b in zip(got["auto"], got["step"]):
+        assert np.array_equal(a, b)
     model.close()
