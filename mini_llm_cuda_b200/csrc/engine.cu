@@ -798,7 +798,8 @@ static int setup_tc_path(mlb_session* s) {
     if ((rc = tc_probe_clusters(s))) return rc;
     const auto kb = [](int k) { return (k + kTcKB - 1) / kTcKB; };
     // mma.sync tiles for the projections, or tcgen05 ones: gd_small_enough. The QK norm needs whole heads in a tile, the k-block maps
-    // whole k-blocks, the ranges of a tile a warp each: other models stay on gemm_tc.cuh.
+    // whole k-blocks, the ranges of a tile a warp each: other models stay on gemm_tc.cuh (cfg1 with QK norm 361 / 380 / 532 us a step at
+    // 4 / 37 / 256 sequences, 178 / 224 / 424 without).
     s->use_dec = !s->parent && mode != "tcgen05" && !c.qk_norm && (mode == "mma" ? B <= 256 : gd_small_enough(s)) && c.dim % kTcKB == 0 && c.ffn_dim % kTcKB == 0 && c.ple_dim % kTcKB == 0 &&
                  nq % kTcKB == 0 && a_dn % kTcKB == 0;
     const auto ranges_fit = [&](int n, int nkb, int mode, bool ext) { return gd_pick(s, n, nkb, mode, w8, ext).split <= kGdMaxSplit; };

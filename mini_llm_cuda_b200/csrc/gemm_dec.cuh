@@ -7,9 +7,9 @@
 // epilogue, unrolled over accumulator registers, is fetched cold by every CTA (3.5 - 5.6 us). Here a CTA takes 32
 // features and 16, 32 or 64 sequences: five to ten times the CTAs, the k-ranges are warps of one CTA and meet in shared
 // memory, and the epilogue is a rolled loop over sequences with a feature per lane. mma.sync m16n8k16 and
-// tcgen05.mma kind::f16 return the same bits for the same sixteen products and accumulator (checked over random
-// operands, whatever the order inside the sixteen), and k-ranges, their sum and the epilogue's operations are gemm_tc_kernel's, so
-// the results are too.
+// tcgen05.mma kind::f16 return the same bits for the same sixteen products and accumulator, whatever the order inside the sixteen (an
+// observation, not documented: the tests compare whole steps on both tiles bit for bit), and k-ranges, their sum and the epilogue's
+// operations are gemm_tc_kernel's, so the results are too.
 //   producer warp   TMA: per stage G 64-wide k-blocks of every range, weights [G][32 x 64] (two for gate/up) and activations
 //                   [G][CT x 64], each one copy of a three-dimensional map (k-block, row, 64 elements): a copy costs the
 //                   TMA unit about 300 cycles however small it is, which bound the kernel at one k-block per copy. The weights of
