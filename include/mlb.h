@@ -116,7 +116,8 @@ void mlb_session_free(mlb_session* s);
  * when a width is first needed and stay with the session (MLB_COLUMNS_MB limits them). With fp32 weights and 5 tokens or more, and with the others where one to
  * three sequences bring 8 to 63 tokens, it is consumed as columns of the fp32 GEMV chain; otherwise, or with MLB_PREFILL=step in the environment,
  * one token per step and sequence. MLB_PREFILL=chunk asks for the columns and fails with
- * MLB_E_UNSUPPORTED where they cannot run. */
+ * MLB_E_UNSUPPORTED where they cannot run, with MLB_E_NOMEM without memory for them (otherwise the token loop
+ * takes the prompt then). */
 int mlb_prefill(mlb_session* s, const int32_t* tokens, const int32_t* lens, int stride);
 
 /* ---- several GPUs of one box ---------------------------------------------------------------------
@@ -147,7 +148,8 @@ int mlb_pool_decode_n(mlb_pool* p, const mlb_sampling* sampling, int n, int32_t*
  * weights; activations are bf16, i.e. the logits agree with the fp32 forward within the low-precision
  * tolerance). With fp32 weights, or with MLB_SCORE=step in the environment, the tokens run through the
  * token loop instead (fp32 activations, the fp32 bound of the decode path; about 0.2 ms per token).
- * Uses sequence 0 of the session; the session is reset before and after. */
+ * Logits of a chunk are kept on the device (4 bytes x vocabulary x up to 4096 columns, narrower chunks where that
+ * is refused; MLB_E_NOMEM without room for 64 columns). Uses sequence 0 of the session; the session is reset before and after. */
 int mlb_score_tokens(mlb_session* s, const int32_t* tokens, int len, float* logits_out);
 
 /* Replaces one iteration of the while loop of runInferenceLoop
