@@ -7,6 +7,7 @@
 #include "grid_host.h"
 #include "lean_host.h"
 #include "sgemv.cuh"
+#include "attn_decode.cuh"
 
 namespace mlb {
 
@@ -180,13 +181,18 @@ struct Chain {
         // few CTAs (small batch): two query heads per CTA, G/2 CTAs per kv head (cfg4 at batch 1: 1.28 -> 1.14 ms
         // per step); with the GPU already full the extra CTAs only re-read K/V (62 -> 69 us at 64 sequences)
         if (G >= 4 && G % 2 == 0 && s->splits * p.kv_heads * s->B < 2 * s->sm_count) { p.hg = G / 2; G = 2; }
-        dim3 grid(s->splits, p.kv_heads * p.hg, s->B);
+        p.splits = s->splits;
+        const dim3 grid = attn_grid(p, s->B);
+        auto launch = [&](auto kernel, size_t smem, int threads) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            return e == cudaSuccess ? launch_chain(s->use_pdl, kernel, grid, dim3(threads), smem, s->stream, c, p) : e;
+        };
         cudaError_t e;
         switch (G) {
-            case 1: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 1>, grid, dim3(128), 0, s->stream, c, p); break;
-            case 2: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 2>, grid, dim3(128), 0, s->stream, c, p); break;
-            case 4: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 4>, grid, dim3(128), 0, s->stream, c, p); break;
-            default: e = launch_chain(s->use_pdl, attn_decode_kernel<KVT, HD, 8>, grid, dim3(128), 0, s->stream, c, p); break;
+            case 1: e = launch(attn_decode_kernel<KVT, HD, 1>, attn_decode_smem<KVT, HD, 1>(), attn_threads<1>()); break;
+            case 2: e = launch(attn_decode_kernel<KVT, HD, 2>, attn_decode_smem<KVT, HD, 2>(), attn_threads<2>()); break;
+            case 4: e = launch(attn_decode_kernel<KVT, HD, 4>, attn_decode_smem<KVT, HD, 4>(), attn_threads<4>()); break;
+            default: e = launch(attn_decode_kernel<KVT, HD, 8>, attn_decode_smem<KVT, HD, 8>(), attn_threads<8>()); break;
         }
         if (e != cudaSuccess) return fail(MLB_E_CUDA, "attention launch failed: %s", cudaGetErrorString(e));
         return MLB_OK;
@@ -321,7 +327,8 @@ struct Chain {
         const int perm = s->use_dec && sizeof(T) == 1 ? 1 : 0;       // operand order of the FP8 decode GEMMs
         int launches = 0, rc;
         if (rec && (rc = rec->begin("embed_ple_gather_norm", (uint64_t)B * d * 8 + (uint64_t)B * ple * 2 * cfg.layers, 0))) return rc;
-        CU(launch_chain(s->use_pdl, embed_tc_kernel<T>, dim3(B, (d + kTcM - 1) / kTcM), dim3(128), (size_t)ple * 4, s->stream, c,
+        // (without overlap: what the step's kernels read before they wait for their predecessor was written by earlier steps)
+        CU(launch_chain(false, embed_tc_kernel<T>, dim3(B, (d + kTcM - 1) / kTcM), dim3(128), (size_t)ple * 4, s->stream, c,
                         static_cast<const T*>(m->E), static_cast<const float*>(m->Es), d, static_cast<const StepLayer*>(s->step_layers), cfg.layers, ple,
                         static_cast<const float*>(m->layers[0].g1), s->x, s->xn16, s->tc_ssq, s->tple16, perm));
         if (rec && (rc = rec->end())) return rc;
@@ -344,7 +351,7 @@ struct Chain {
                 a.page_table = s->page_table; a.pt_stride = s->max_pages;
                 a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16; a.perm = perm;
                 a.part = s->part; a.ticket = s->attn_ticket;
-                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
+                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = s->dev_err; a.min_pages_per_split = s->attn_min_pps; a.early = 1;
                 if (rec) {
                     uint64_t kvb = 0, fl = 0;
                     for (int b = 0; b < B; ++b) {
@@ -445,7 +452,8 @@ struct Chain {
         if (s->use_tc) return run_tc(s, kind, c, rec, n_launches);
 
         if (rec && (rc = rec->begin("embed_ple_gather", (uint64_t)B * (d * sizeof(T) + (uint64_t)p * sizeof(T2) + (uint64_t)d * 4) + (uint64_t)d * p * sizeof(T2), 0))) return rc;
-        CU(launch_chain(s->use_pdl, embed_kernel<T, T2>, embed_grid(B, d, p), embed_block(B, d, p), (size_t)p * 4, s->stream, c,
+        // (without overlap: what the step's kernels read before they wait for their predecessor was written by earlier steps)
+        CU(launch_chain(false, embed_kernel<T, T2>, embed_grid(B, d, p), embed_block(B, d, p), (size_t)p * 4, s->stream, c,
                         static_cast<const T*>(m->E), static_cast<const float*>(m->Es), d, static_cast<const T2*>(m->layers[0].pleT),
                         static_cast<const T2*>(m->layers[0].pleP), p, s->x));
         if (rec && (rc = rec->end())) return rc;
@@ -472,7 +480,7 @@ struct Chain {
                 a.page_table = s->page_table; a.pt_stride = s->max_pages;
                 a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = nullptr; a.perm = 0;
                 a.part = s->part; a.ticket = s->attn_ticket;
-                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
+                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = s->dev_err; a.min_pages_per_split = s->attn_min_pps; a.early = 1;
                 if (rec) {
                     uint64_t kvb = 0, fl = 0;
                     for (int b = 0; b < B; ++b) {

@@ -322,6 +322,7 @@ static const char* wait_text(int code) {
     switch (code) {
         case 1: return "producer waiting for a free ring stage";
         case 2: return "consumer waiting for a weight chunk";
+        case 6: return "attention waiting for K/V pages";
         case 11: return "tcgen05 GEMM, loader waiting for a free stage";
         case 12: return "tcgen05 GEMM, MMA issuer waiting for operands";
         case 13: return "tcgen05 GEMM, epilogue waiting for the accumulators";
@@ -433,7 +434,7 @@ static int run_cols(mlb_session* s, int kind, int* n_launches) {
                 AttnParams a;
                 a.kpool = s->kpool[i]; a.vpool = s->vpool[i]; a.page_table = s->page_table; a.pt_stride = s->max_pages;
                 a.qbuf = s->qbuf; a.gbuf = L.ng ? s->gbuf : nullptr; a.abuf = s->abuf; a.abuf16 = s->a16; a.perm = 0; a.part = s->part; a.ticket = s->attn_ticket;
-                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = nullptr; a.min_pages_per_split = s->attn_min_pps;
+                a.heads = cfg.heads; a.kv_heads = cfg.kv_heads; a.num_pages = 0; a.err = s->dev_err; a.min_pages_per_split = s->attn_min_pps; a.early = 0;
                 rc = chain_attn_f32kv(s, c, a);
                 if (rc) return rc;
             }

@@ -88,6 +88,35 @@ __device__ __forceinline__ int perm16(int f) {
 // and its factor, a power of two (kernels that serve both kinds of operand take `perm` for the pair)
 constexpr float kOperandScale = 18446744073709551616.0f;        // 2^64
 
+// ---- packed pairs of fp32 (two independent IEEE operations per instruction) ------------------------
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 pack2u(uint32_t a, uint32_t b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -657,289 +686,6 @@ __global__ void __launch_bounds__(256) gemv_kernel(StepCtl c, GemvParams p) {
             if (tid == 0) p.ticket[blockIdx.y] = 0;        // ready for the next step
         }
     }
-}
-
-// ------------------------------------------------------------------------------------
-// Split-K flash-decode over the paged KV cache, with the split combine and the query
-// gating folded into the last-arriving CTA of each (sequence, kv head).
-//
-// Reference ops replaced: K^T Q GEMM, getHeadDimScaledMaskedAttn, the max / sum / apply
-// softmax kernels, V P GEMM, applyGatingToValueScaledAttnPostSoftmax
-// (inference.cu:510-579, kernels :136-250). Scores are divided by sqrtf(head_dim) as there.
-// grid = (splits, kv_heads, B), block = 128.
-// ------------------------------------------------------------------------------------
-struct AttnParams {
-    const void* kpool; const void* vpool;     // [page][kv_heads][16][hd]
-    const int* page_table; int pt_stride;
-    const float* qbuf;      // [B][heads*hd]
-    const float* gbuf;      // [B][heads*hd] sigmoid gates or null
-    float* abuf;            // [B][heads*hd]
-    bf16_t* abuf16;         // same values as the bf16 operand of a tensor-core O projection, or null
-    int perm;               // features of abuf16 in perm16 order
-    float* part;            // [B][heads][splits][hd+2]
-    int* ticket;            // [B * gridDim.y]
-    int heads, kv_heads;
-    int hg;                 // CTAs per kv head along grid.y: each takes G of the kv head's query heads
-    // A caller-owned page table (the operator entry points) is not trusted: with num_pages > 0 a sequence
-    // whose position needs more than pt_stride pages is skipped (code 4 in *err) and a page id outside
-    // [0, num_pages) is replaced by page 0 (code 5), so that nothing outside the caller's buffers is read.
-    // The session passes 0: its own allocator filled the table.
-    int num_pages;
-    int* err;
-    // A split is worth its partials and the combine only with enough positions in it: a sequence uses
-    // min(grid splits, pages / min_pages_per_split) of them. 1 = every page may be a split.
-    int min_pages_per_split;
-};
-
-template <typename KVT, int HD, int G>
-__global__ void __launch_bounds__(128) attn_decode_kernel(StepCtl c, AttnParams p) {
-    constexpr int EPL = 16 / sizeof(KVT);          // elements per lane per row
-    constexpr int LPR = HD / EPL;                  // lanes per row
-    constexpr int PPI = 32 / LPR;                  // positions per warp iteration
-    constexpr int NW = 4;
-    static_assert(LPR <= 32 && PPI >= 1, "head_dim too large for one warp row");
-    // With many query heads per kv head one CTA would hold all their accumulators (160+ registers,
-    // no room for a second chunk of loads in flight): hg CTAs share a kv head instead, G heads each;
-    // the K/V rows they re-read come from L2.
-    const int b = blockIdx.z, kvh = blockIdx.y / p.hg, split = blockIdx.x;
-    const int tslot = b * (int)gridDim.y + (int)blockIdx.y;
-    pdl_launch_dependents();
-    pdl_wait();                                    // q and this step's K/V row come from the projection kernel
-    if (!seq_active(c, b)) return;                 // uniform for all CTAs of this sequence
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lr = lane % LPR, grp = lane / LPR;
-    const int pos = c.pos[b];
-    const int ctx = pos + 1;
-    const int npages = (ctx + kKvBlock - 1) / kKvBlock;
-    // The grid is sized for the longest context; a split needs at least one page, and the CTAs
-    // beyond the page count leave at once (fewer partials for the combine to read). Every CTA of a
-    // (sequence, kv head) computes the same S.
-    if (p.num_pages > 0 && npages > p.pt_stride) {   // uniform for all CTAs of this sequence
-        if (threadIdx.x == 0) atomicExch(p.err, 4);
-        return;
-    }
-    const int S = max(1, min((int)gridDim.x, npages / max(1, p.min_pages_per_split)));
-    const int SG = (int)gridDim.x;                 // stride of the partial buffer: fixed by the grid, not by S
-    if (split >= S) return;
-    const int pps = (npages + S - 1) / S;
-    const int pg_begin = split * pps, pg_end = min(npages, pg_begin + pps);
-
-    __shared__ float sq[G][HD];
-    __shared__ float sred[NW][G][HD + 2];
-    const int h0 = kvh * G * p.hg + ((int)blockIdx.y % p.hg) * G;
-    for (int i = tid; i < G * HD; i += blockDim.x)
-        sq[i / HD][i % HD] = p.qbuf[((size_t)b * p.heads + h0) * HD + i];
-    __syncthreads();
-
-    float q[G][EPL];
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) q[g][e] = sq[g][lr * EPL + e];
-
-    float m[G], l[G], acc[G][EPL];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        m[g] = kNegBig; l[g] = 0.f;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) acc[g][e] = 0.f;
-    }
-    const float inv_div = sqrtf((float)HD);
-    const KVT* kpool = reinterpret_cast<const KVT*>(p.kpool);
-    const KVT* vpool = reinterpret_cast<const KVT*>(p.vpool);
-
-    // This warp's pages: pg_begin + warp + NW * i. Lane i holds the pool index of the i-th one
-    // (refreshed every 32 pages), so that the page loop does not start with a dependent load.
-    constexpr int ITERS = kKvBlock / PPI;
-    constexpr int CH = ITERS < 4 ? ITERS : 4;      // positions per lane group handled together
-    const int* pt = p.page_table + kv_seq(c, b) * p.pt_stride;
-    const int span = pg_end - pg_begin - warp;
-    const int npw = span > 0 ? (span + NW - 1) / NW : 0;
-    int pidx = 0;
-    constexpr int CPP = ITERS / CH;                // chunks per page
-    const int nq = npw * CPP;                      // this warp's chunks, in order
-    // All loads of a chunk first, then the scores of its positions (independent of one another), one
-    // rescale of the running sums and one exponential per position.
-    auto load_chunk = [&](int qi, uint4* kk, uint4* vv4, int& cnt, int& c0) {
-        const int i = qi / CPP;
-        c0 = (qi - i * CPP) * CH;
-        if (c0 == 0 && (i & 31) == 0) {
-            const int ii = i + lane;
-            pidx = ii < npw ? pt[pg_begin + warp + NW * ii] : 0;
-            if (p.num_pages > 0 && (unsigned)pidx >= (unsigned)p.num_pages) {
-                atomicExch(p.err, 5);
-                pidx = 0;
-            }
-        }
-        const int pg = pg_begin + warp + NW * i;
-        const int page = __shfl_sync(0xffffffffu, pidx, i & 31);
-        cnt = min(kKvBlock, ctx - pg * kKvBlock);
-        const size_t base = ((size_t)page * p.kv_heads + kvh) * kKvBlock * HD;
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int j = (c0 + u) * PPI + grp;
-            kk[u] = make_uint4(0, 0, 0, 0);
-            vv4[u] = make_uint4(0, 0, 0, 0);
-            if (j < cnt) {
-                kk[u] = __ldcg(reinterpret_cast<const uint4*>(kpool + base + (size_t)j * HD + lr * EPL));
-                vv4[u] = __ldcg(reinterpret_cast<const uint4*>(vpool + base + (size_t)j * HD + lr * EPL));
-            }
-        }
-    };
-    auto use_chunk = [&](const uint4* kk, const uint4* vv4, int cnt, int c0) {
-        float sv[G][CH];
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const bool valid = (c0 + u) * PPI + grp < cnt;
-            float kv[EPL];
-            Elem<KVT>::unpack(kk[u], kv);
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                float sdot = 0.f;
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) sdot = fmaf(q[g][e], kv[e], sdot);
-#pragma unroll
-                for (int o = LPR / 2; o > 0; o >>= 1) sdot += __shfl_xor_sync(0xffffffffu, sdot, o);
-                sv[g][u] = valid ? sdot / inv_div : kNegBig;
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float mn = m[g];
-#pragma unroll
-            for (int u = 0; u < CH; ++u) mn = fmaxf(mn, sv[g][u]);
-            const float sc = expf(m[g] - mn);
-            l[g] *= sc;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) acc[g][e] *= sc;
-#pragma unroll
-            for (int u = 0; u < CH; ++u) {
-                const bool valid = (c0 + u) * PPI + grp < cnt;
-                sv[g][u] = valid ? expf(sv[g][u] - mn) : 0.f;
-                l[g] += sv[g][u];
-            }
-            m[g] = mn;
-        }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            float vv[EPL];
-            Elem<KVT>::unpack(vv4[u], vv);
-#pragma unroll
-            for (int g = 0; g < G; ++g)
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) acc[g][e] = fmaf(sv[g][u], vv[e], acc[g][e]);
-        }
-    };
-    if (G <= 2) {
-        // few heads per CTA leave registers for a second chunk: the next chunk's loads are in flight
-        // while the current one is used (twice the bytes in flight per warp)
-        uint4 ka[CH], va[CH], kb[CH], vb[CH];
-        int cnt_a = 0, c0_a = 0, cnt_b = 0, c0_b = 0;
-        if (nq > 0) load_chunk(0, ka, va, cnt_a, c0_a);
-        for (int qi = 0; qi < nq; qi += 2) {
-            if (qi + 1 < nq) load_chunk(qi + 1, kb, vb, cnt_b, c0_b);
-            use_chunk(ka, va, cnt_a, c0_a);
-            if (qi + 1 < nq) {
-                if (qi + 2 < nq) load_chunk(qi + 2, ka, va, cnt_a, c0_a);
-                use_chunk(kb, vb, cnt_b, c0_b);
-            }
-        }
-    } else {
-        uint4 ka[CH], va[CH];
-        int cnt_a = 0, c0_a = 0;
-        for (int qi = 0; qi < nq; ++qi) {
-            load_chunk(qi, ka, va, cnt_a, c0_a);
-            use_chunk(ka, va, cnt_a, c0_a);
-        }
-    }
-    // merge the PPI lane groups of the warp
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-#pragma unroll
-        for (int o = LPR; o < 32; o <<= 1) {
-            float mo = __shfl_xor_sync(0xffffffffu, m[g], o);
-            float lo = __shfl_xor_sync(0xffffffffu, l[g], o);
-            float mn = fmaxf(m[g], mo);
-            float sa = expf(m[g] - mn), sb = expf(mo - mn);
-            l[g] = l[g] * sa + lo * sb;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) {
-                float ao = __shfl_xor_sync(0xffffffffu, acc[g][e], o);
-                acc[g][e] = acc[g][e] * sa + ao * sb;
-            }
-            m[g] = mn;
-        }
-        if (grp == 0) {
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) sred[warp][g][lr * EPL + e] = acc[g][e];
-            if (lr == 0) { sred[warp][g][HD] = m[g]; sred[warp][g][HD + 1] = l[g]; }
-        }
-    }
-    __syncthreads();
-    // merge the warps; thread t < HD owns output dim t
-    for (int i = tid; i < G * HD; i += blockDim.x) {
-        int g = i / HD, e = i % HD;
-        float mn = kNegBig;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) mn = fmaxf(mn, sred[w][g][HD]);
-        float lt = 0.f, at = 0.f;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-            float sc = expf(sred[w][g][HD] - mn);
-            lt += sred[w][g][HD + 1] * sc;
-            at += sred[w][g][e] * sc;
-        }
-        int h = h0 + g;
-        if (S == 1) {
-            float o = at / lt;
-            if (p.gbuf) o *= p.gbuf[((size_t)b * p.heads + h) * HD + e];
-            p.abuf[((size_t)b * p.heads + h) * HD + e] = o;
-            if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
-        } else {
-            float* pp = p.part + (((size_t)b * p.heads + h) * SG + split) * (HD + 2);
-            pp[e] = at;
-            if (e == 0) { pp[HD] = mn; pp[HD + 1] = lt; }
-        }
-    }
-    if (S == 1) return;
-    __shared__ int is_last;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        int t = atomicAdd(&p.ticket[tslot], 1);
-        is_last = (t == S - 1);
-    }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    // Combine: one warp per head turns the splits' (max, sum) pairs into normalised weights once;
-    // then every thread accumulates its output elements with independent loads.
-    __shared__ float wsm[G][64];
-    for (int g = warp; g < G; g += NW) {
-        const float* pp = p.part + ((size_t)b * p.heads + h0 + g) * SG * (HD + 2);
-        float m0 = kNegBig, l0 = 0.f, m1 = kNegBig, l1 = 0.f;
-        if (lane < S) { m0 = __ldcg(pp + (size_t)lane * (HD + 2) + HD); l0 = __ldcg(pp + (size_t)lane * (HD + 2) + HD + 1); }
-        if (lane + 32 < S) { m1 = __ldcg(pp + (size_t)(lane + 32) * (HD + 2) + HD); l1 = __ldcg(pp + (size_t)(lane + 32) * (HD + 2) + HD + 1); }
-        float mx = fmaxf(m0, m1);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float w0 = expf(m0 - mx), w1 = expf(m1 - mx);
-        const float lt = warp_sum(l0 * w0 + l1 * w1);
-        wsm[g][lane] = w0 / lt;
-        wsm[g][lane + 32] = w1 / lt;
-    }
-    __syncthreads();
-    for (int i = tid; i < G * HD; i += blockDim.x) {
-        int g = i / HD, e = i % HD, h = h0 + g;
-        const float* pp = p.part + ((size_t)b * p.heads + h) * SG * (HD + 2) + e;
-        float o = 0.f;
-#pragma unroll 4
-        for (int s = 0; s < S; ++s) o = fmaf(wsm[g][s], __ldcg(pp + (size_t)s * (HD + 2)), o);
-        if (p.gbuf) o *= p.gbuf[((size_t)b * p.heads + h) * HD + e];
-        p.abuf[((size_t)b * p.heads + h) * HD + e] = o;
-        if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
-    }
-    if (tid == 0) p.ticket[tslot] = 0;
 }
 
 // ------------------------------------------------------------------------------------

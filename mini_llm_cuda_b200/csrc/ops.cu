@@ -5,6 +5,7 @@
 
 #include "../../include/mlb.h"
 #include "errors.h"
+#include "attn_decode.cuh"
 #include "kernels.cuh"
 #include "ring.cuh"
 #include "tc_host.h"
@@ -59,15 +60,20 @@ int check_attn_args(const void* kpool, const void* vpool, int kv_dtype, const in
 }
 
 template <typename KVT, int HD>
-cudaError_t launch_attn(const StepCtl& c, const AttnParams& p, int G, int splits, int B, cudaStream_t st) {
-    dim3 grid(splits, p.kv_heads, B);
+cudaError_t launch_attn(const StepCtl& c, AttnParams p, int G, int B, cudaStream_t st) {
+    const dim3 grid = attn_grid(p, B);
+    auto launch = [&](auto kernel, size_t smem, int threads) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<grid, threads, smem, st>>>(c, p);
+        return cudaGetLastError();
+    };
     switch (G) {
-        case 1: attn_decode_kernel<KVT, HD, 1><<<grid, 128, 0, st>>>(c, p); break;
-        case 2: attn_decode_kernel<KVT, HD, 2><<<grid, 128, 0, st>>>(c, p); break;
-        case 4: attn_decode_kernel<KVT, HD, 4><<<grid, 128, 0, st>>>(c, p); break;
-        default: attn_decode_kernel<KVT, HD, 8><<<grid, 128, 0, st>>>(c, p); break;
+        case 1: return launch(attn_decode_kernel<KVT, HD, 1>, attn_decode_smem<KVT, HD, 1>(), attn_threads<1>());
+        case 2: return launch(attn_decode_kernel<KVT, HD, 2>, attn_decode_smem<KVT, HD, 2>(), attn_threads<2>());
+        case 4: return launch(attn_decode_kernel<KVT, HD, 4>, attn_decode_smem<KVT, HD, 4>(), attn_threads<4>());
+        default: return launch(attn_decode_kernel<KVT, HD, 8>, attn_decode_smem<KVT, HD, 8>(), attn_threads<8>());
     }
-    return cudaGetLastError();
 }
 
 // Clears the part of the scratch that must start at zero, then launches. No allocation.
@@ -86,13 +92,13 @@ int run_attn(void* scratch, const void* kpool, const void* vpool, int kv_dtype, 
     p.kpool = kpool; p.vpool = vpool; p.page_table = page_table; p.pt_stride = pt_stride;
     p.qbuf = q; p.gbuf = gate; p.abuf = out; p.abuf16 = nullptr; p.perm = 0; p.part = sc.part; p.ticket = sc.ticket;
     p.heads = heads; p.kv_heads = kv_heads; p.hg = 1;
-    p.num_pages = num_pages; p.err = sc.err; p.min_pages_per_split = 1;
+    p.num_pages = num_pages; p.err = sc.err; p.min_pages_per_split = 1; p.early = 0; p.splits = splits;
     const int G = heads / kv_heads;
     cudaError_t e;
     if (kv_dtype == MLB_DT_F32)
-        e = head_dim == 64 ? launch_attn<float, 64>(c, p, G, splits, batch, st) : launch_attn<float, 128>(c, p, G, splits, batch, st);
+        e = head_dim == 64 ? launch_attn<float, 64>(c, p, G, batch, st) : launch_attn<float, 128>(c, p, G, batch, st);
     else
-        e = head_dim == 64 ? launch_attn<bf16_t, 64>(c, p, G, splits, batch, st) : launch_attn<bf16_t, 128>(c, p, G, splits, batch, st);
+        e = head_dim == 64 ? launch_attn<bf16_t, 64>(c, p, G, batch, st) : launch_attn<bf16_t, 128>(c, p, G, batch, st);
     if (e != cudaSuccess) return fail(MLB_E_CUDA, "attention op launch failed: %s", cudaGetErrorString(e));
     return MLB_OK;
 }
@@ -100,6 +106,7 @@ int run_attn(void* scratch, const void* kpool, const void* vpool, int kv_dtype, 
 }  // namespace
 
 static const char* attn_err_text(int code) {
+    if (code == 6) return "a bounded wait for K/V pages ran out";
     return code == 4 ? "a position needs more pages than pt_stride (that sequence was skipped)"
                      : "the page table names a page outside [0, num_pages) (page 0 was read instead)";
 }

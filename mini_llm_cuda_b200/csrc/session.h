@@ -10,7 +10,7 @@
 
 #include "../../include/mlb.h"
 #include "errors.h"
-#include "kernels.cuh"
+#include "attn_decode.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_dec.cuh"
 #include "tc_host.h"

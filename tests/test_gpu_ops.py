@@ -79,6 +79,33 @@ def test_attention_op_matches_fp64(api, heads, kv_heads, hd, dtype_name, splits,
     assert err < 2e-5, err
 
 
+@pytest.mark.parametrize("group,hd,dtype_name", [(1, 64, "bfloat16"), (2, 64, "float32"), (4, 64, "bfloat16"), (8, 64, "float32"), (1, 128, "float32"),
+                                                 (2, 128, "bfloat16"), (4, 128, "bfloat16"), (8, 128, "bfloat16")])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_attention_op_many_sequences(api, group, hd, dtype_name, splits):
+    """Sequences enough that one CTA takes a sequence's splits in turn: contexts at the edges of pages, of the four streams of pages and of a
+    stream's ring; rows behind a context hold no numbers; queries on a 4-byte boundary."""
+    import torch
+    dtype = getattr(torch, dtype_name)
+    kv_heads, batch = 2, 76
+    heads = kv_heads * group
+    edges = [1, 15, 16, 17, 63, 64, 65, 128, 129, 192, 193, 257, 400]
+    ctx_list = [edges[b % len(edges)] for b in range(batch)]
+    case = make_attention_case(torch, batch, heads, kv_heads, hd, ctx_list, dtype, 5, True)
+    for b, ctx in enumerate(ctx_list):
+        if ctx % 16:
+            page = int(case["table"][b, ctx // 16])
+            case["kpool"][page, :, ctx % 16:] = float("nan")
+            case["vpool"][page, :, ctx % 16:] = float("inf")
+    shifted = torch.empty(batch * heads * hd + 1, device="cuda:0")
+    shifted[1:] = case["q"].flatten()
+    case["q"] = shifted[1:]
+    rc, out = call_attention(api, torch, "mlb_op_attn_decode", case, batch, heads, kv_heads, hd, splits, dtype)
+    assert rc == 0, api.lib().mlb_last_error()
+    err = (out.cpu().double() - case["want"]).abs().max().item()
+    assert err < 2e-5, err
+
+
 def test_attention_op_rejects_bad_arguments(api):
     import torch
     case = make_attention_case(torch, 1, 4, 4, 64, [5], torch.float32, 1, False)
