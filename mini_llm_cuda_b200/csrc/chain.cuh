@@ -235,7 +235,7 @@ struct Chain {
             SampleParams sp;
             sp.logits = s->logits; sp.V = s->m->cfg.vocab; sp.top_k = s->cur_topk; sp.temperature = s->cur_temp; sp.seeds = s->seeds;
             if (rec && (rc = rec->begin("sample_topk_philox", (uint64_t)s->B * s->m->cfg.vocab * 4 * 5, 0))) return rc;
-            CU(launch_chain(false, sample_topk_kernel, dim3(s->B), dim3(256), 0, s->stream, c, sp));
+            CU(launch_chain(false, sample_topk_kernel, dim3(s->B), dim3(kPickThreads), 0, s->stream, c, sp));
             if (rec && (rc = rec->end())) return rc;
             ++launches;
         }
@@ -426,13 +426,13 @@ struct Chain {
                 // columns that are scored: their logits are the result
             } else if (kind == CHAIN_GREEDY) {
                 if (rec && (rc = rec->begin("argmax_pick", (uint64_t)B * cfg.vocab * 4, 0))) return rc;
-                CU(launch_chain(s->use_pdl, argmax_advance_kernel, dim3(B), dim3(256), 0, s->stream, c, static_cast<const float*>(s->logits), cfg.vocab));
+                CU(launch_chain(s->use_pdl, argmax_advance_kernel, dim3(B), dim3(kPickThreads), 0, s->stream, c, static_cast<const float*>(s->logits), cfg.vocab));
                 if (rec && (rc = rec->end())) return rc;
             } else {
                 SampleParams sp;
                 sp.logits = s->logits; sp.V = cfg.vocab; sp.top_k = s->cur_topk; sp.temperature = s->cur_temp; sp.seeds = s->seeds;
                 if (rec && (rc = rec->begin("sample_topk_philox", (uint64_t)B * cfg.vocab * 4 * 5, 0))) return rc;
-                CU(launch_chain(s->use_pdl, sample_topk_kernel, dim3(B), dim3(256), 0, s->stream, c, sp));
+                CU(launch_chain(s->use_pdl, sample_topk_kernel, dim3(B), dim3(kPickThreads), 0, s->stream, c, sp));
                 if (rec && (rc = rec->end())) return rc;
             }
             ++launches;
@@ -548,7 +548,7 @@ struct Chain {
                 SampleParams sp;
                 sp.logits = s->logits; sp.V = cfg.vocab; sp.top_k = s->cur_topk; sp.temperature = s->cur_temp; sp.seeds = s->seeds;
                 if (rec && (rc = rec->begin("sample_topk_philox", (uint64_t)B * cfg.vocab * 4 * 5, 0))) return rc;
-                CU(launch_chain(s->use_pdl, sample_topk_kernel, dim3(B), dim3(256), 0, s->stream, c, sp));
+                CU(launch_chain(s->use_pdl, sample_topk_kernel, dim3(B), dim3(kPickThreads), 0, s->stream, c, sp));
                 if (rec && (rc = rec->end())) return rc;
                 ++launches;
             }

@@ -713,40 +713,69 @@ __global__ void __launch_bounds__(128) embed_tc_kernel(StepCtl c, const WT* __re
     pdl_wait();                      // pos / tok come from the last kernel of the previous step
     const int b = blockIdx.x;
     if (!seq_active(c, b)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = blockIdx.y * 128 + tid;
+    // Everything that does not need the token is asked for before it is read: 64 columns of this feature's projection row, the table
+    // pointer of this thread's first piece of the later layers' rows.
+    constexpr int PRE = 8;
+    const int pieces = ple / 8, n_pieces = (n_layers - 1) * pieces;
+    uint4 pre[PRE];
+    const bf16_t* prow = nullptr;
+    int piece = blockIdx.y * 128 + tid, layer = 0;
+    const uint4* table = nullptr;
+    if (ple > 0) {
+        prow = static_cast<const bf16_t*>(layers[0].pleP) + (size_t)min(i, d - 1) * ple;
+#pragma unroll
+        for (int j = 0; j < PRE; ++j) pre[j] = __ldg(reinterpret_cast<const uint4*>(prow) + min(j, pieces - 1));
+        layer = 1 + piece / pieces;
+        if (piece < n_pieces) table = static_cast<const uint4*>(layers[layer].pleT);
+    }
+    const float gi = gain[min(i, d - 1)];
     int t = c.tok[b];
     if (c.tok_src != nullptr) {
         t = c.tok_src[b];
         if (blockIdx.y == 0 && threadIdx.x == 0) c.tok[b] = t;
     }
     extern __shared__ __align__(16) float trow[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float e = i < d ? __fmul_rn(Elem<WT>::get(E, (size_t)t * d + i), escale ? escale[t] : 1.0f) : 0.f;
     if (ple > 0) {
         const bf16_t* T0 = static_cast<const bf16_t*>(layers[0].pleT);
         for (int j = tid; j < ple; j += 128) trow[j] = __bfloat162float(T0[(size_t)t * ple + j]);
-        for (int l = 1 + blockIdx.y; l < n_layers; l += gridDim.y) {
-            const bf16_t* Tl = static_cast<const bf16_t*>(layers[l].pleT);
-            for (int j = tid; j < ple; j += 128) tple16[((size_t)l * c.B + b) * ple + j] = Tl[(size_t)t * ple + j];
+        // 16-byte pieces of the later layers' rows, a piece per thread
+        while (piece < n_pieces) {
+            const int j = piece % pieces;
+            reinterpret_cast<uint4*>(tple16)[((size_t)layer * c.B + b) * pieces + j] = __ldg(table + (size_t)t * pieces + j);
+            piece += gridDim.y * 128;
+            layer = 1 + piece / pieces;
+            if (piece < n_pieces) table = static_cast<const uint4*>(layers[layer].pleT);
         }
         __syncthreads();
     }
-    const int i = blockIdx.y * 128 + tid;
     float v = 0.f;
     if (i < d) {
-        v = Elem<WT>::get(E, (size_t)t * d + i) * (escale ? escale[t] : 1.0f);
+        v = e;
         if (ple > 0) {
             float a = 0.f;
-            const bf16_t* prow = static_cast<const bf16_t*>(layers[0].pleP) + (size_t)i * ple;
+#pragma unroll
+            for (int j = 0; j < PRE; ++j) {
+                if (j < pieces) {
+                    float w[8];
+                    Elem<bf16_t>::unpack(pre[j], w);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) a = fmaf(w[k], trow[8 * j + k], a);
+                }
+            }
 #pragma unroll 4
-            for (int j = 0; j < ple; j += 8) {
+            for (int j = 8 * PRE; j < ple; j += 8) {
                 float w[8];
                 Elem<bf16_t>::load_vec(prow + j, w);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) a = fmaf(w[e], trow[j + e], a);
+                for (int k = 0; k < 8; ++k) a = fmaf(w[k], trow[j + k], a);
             }
             v += a;
         }
         x[(size_t)b * d + i] = v;
-        xg16[(size_t)b * d + (perm ? perm16(i) : i)] = __float2bfloat16_rn(v * gain[i] * (perm ? kOperandScale : 1.0f));
+        xg16[(size_t)b * d + (perm ? perm16(i) : i)] = __float2bfloat16_rn(v * gi * (perm ? kOperandScale : 1.0f));
     }
     const float ss = warp_sum(v * v);
     if (lane == 0) ssq[((size_t)b * gridDim.y + blockIdx.y) * 4 + warp] = ss;
@@ -754,7 +783,8 @@ __global__ void __launch_bounds__(128) embed_tc_kernel(StepCtl c, const WT* __re
 
 // Greedy pick over the fp32 logits of a batched LM-head GEMM: argmax, lowest index on ties
 // (inference_orchestrator.cu:77-84, :112), then append. One CTA per sequence.
-static __global__ void __launch_bounds__(256) argmax_advance_kernel(StepCtl c, const float* __restrict__ logits, int V) {
+// (Eight logits per thread in flight: 37 sequences of 8192 took 16.2 us with 256 threads and one at a time.)
+static __global__ void __launch_bounds__(kPickThreads) argmax_advance_kernel(StepCtl c, const float* __restrict__ logits, int V) {
     pdl_launch_dependents();
     pdl_wait();
     const int b = blockIdx.x;
@@ -762,9 +792,18 @@ static __global__ void __launch_bounds__(256) argmax_advance_kernel(StepCtl c, c
     const float* lg = logits + (size_t)b * V;
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float v = lg[i];
-        if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
+    for (int base = 0; base < V; base += 8 * kPickThreads) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = base + u * kPickThreads + (int)threadIdx.x;
+            v[u] = __ldcg(lg + min(i, V - 1));
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = base + u * kPickThreads + (int)threadIdx.x;
+            if (i < V && (v[u] > bv || (v[u] == bv && i < bi))) { bv = v[u]; bi = i; }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -772,14 +811,21 @@ static __global__ void __launch_bounds__(256) argmax_advance_kernel(StepCtl c, c
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
-    __shared__ float sv[8];
-    __shared__ int si[8];
+    static_assert(kPickThreads == 32 * 32, "one warp reduces the warps' picks");
+    __shared__ float sv[32];
+    __shared__ int si[32];
     if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = bv; si[threadIdx.x >> 5] = bi; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            if (sv[w] > bv || (sv[w] == bv && si[w] < bi)) { bv = sv[w]; bi = si[w]; }
-        advance_seq(c, b, bi);
+    if (threadIdx.x < 32) {
+        bv = sv[threadIdx.x];
+        bi = si[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+        }
+        if (threadIdx.x == 0) advance_seq(c, b, bi);
     }
 }
 

@@ -814,197 +814,185 @@ __device__ __forceinline__ uint32_t float_order_key(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);   // larger float -> larger key
 }
 
-constexpr int kSampleCap = 1024;       // max candidates kept in shared memory
-constexpr int kSampleKeys = 8192;      // order keys of the first logits kept in shared memory between the passes
+constexpr int kPickThreads = 1024;     // greedy pick and sampler: a CTA per sequence, eight logits per thread in flight
+constexpr int kSampleCap = 1024;       // most candidates that are sorted
+constexpr int kSampleRank = 256;       // up to so many are sorted by counting
 
 __device__ __forceinline__ float float_from_order_key(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
 
 // Temperature / top-k / Philox pick of one sequence per CTA (no counterpart in the reference, whose loop
-// is greedy: inference_orchestrator.cu:77-84). The k largest logits are found by a radix select over
-// order-preserving keys, most significant byte first. The keys of the first kSampleKeys logits are computed
-// once (one division each) and kept in shared memory; a warp adds to a histogram bin once per distinct bin
-// (__match_any_sync) - logits share their leading byte, and 8192 atomics on three or four words were most of
-// the kernel's 52 us at 256 sequences.
-static __global__ void __launch_bounds__(256) sample_topk_kernel(StepCtl c, SampleParams p) {
+// is greedy: inference_orchestrator.cu:77-84). The k largest logits are found by a radix select over order-preserving keys, kept in
+// registers for the first 8192: 12 bits first (sign, exponent, three bits of mantissa), which leave few more than k
+// candidates; further digits only where more than kSampleCap share the bin of the k-th. Candidates are sorted by (key descending,
+// index ascending), up to kSampleRank of them by counting how many come before each. The sums of the exponentials
+// are taken by one thread in that order (the order is part of the result), the pick is looked for by all.
+// Bound by latencies: 256 sequences of 8192 logits 36.6 us with four 8-bit digits and 256 threads.
+static __global__ void __launch_bounds__(kPickThreads) sample_topk_kernel(StepCtl c, SampleParams p) {
+    constexpr int NT = kPickThreads, U = 8;
     const int b = blockIdx.x;
     pdl_launch_dependents();
     pdl_wait();
     if (!seq_active(c, b)) return;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const float* lg = p.logits + (size_t)b * p.V;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, V = p.V;
+    const float* lg = p.logits + (size_t)b * V;
     const float T = p.temperature;
-    const int k = min(p.top_k, min(p.V, kSampleCap));
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t s_prefix, s_mask, s_need;
-    __shared__ uint32_t skey[kSampleKeys];
-    __shared__ float cval[kSampleCap];
-    __shared__ int cidx[kSampleCap];
-    __shared__ int s_count, s_overflow;
-    if (tid == 0) { s_prefix = 0; s_mask = 0; s_need = (uint32_t)k; }
-    __syncthreads();
-    // after the four passes s_prefix is the key of the k-th largest element
-    for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 24 - 8 * pass;
-        hist[tid] = 0;
-        __syncthreads();
-        const uint32_t prefix = s_prefix, mask = s_mask;
-        // The first digit (sign and exponent bits) is shared by most logits: lanes with the same bin add once
-        // (__match_any_sync). From the second digit on only the few keys under the chosen prefix count and their
-        // bins differ: plain atomics, no warp-wide exchange.
-        auto count = [&](int i, uint32_t key) {
-            const bool ok = i < p.V && (key & mask) == prefix;
-            const uint32_t bin = (key >> shift) & 0xffu;
-            if (pass == 0) {
-                const unsigned act = __ballot_sync(0xffffffffu, ok);
-                if (ok) {
-                    const unsigned peers = __match_any_sync(act, bin);
-                    if (lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
-                }
-            } else if (ok) {
-                atomicAdd(&hist[bin], 1u);
-            }
-        };
-        // logits from global memory eight at a time per thread: one L2 latency per eight values instead of
-        // one per value (the ballot below consumes a value as soon as it is there); keys of later passes come
-        // from shared memory
-        for (int base = 0; base < p.V; base += 8 * 256) {
-            const bool from_global = pass == 0 || base + 8 * 256 > kSampleKeys;
-            float v[8];
-            if (from_global) {
+    const int k = min(p.top_k, min(V, kSampleCap));
+    __shared__ __align__(16) unsigned char area[16384];
+    uint32_t* hist = reinterpret_cast<uint32_t*>(area);                                  // [4096], then over it
+    unsigned long long* cand = reinterpret_cast<unsigned long long*>(area);              // [kSampleCap] and
+    unsigned long long* ranked = cand + kSampleCap;                                      // [kSampleRank]
+    __shared__ __align__(16) float cum[kSampleCap];
+    __shared__ uint32_t wsum[NT / 32];
+    __shared__ uint32_t s_prefix, s_mask, s_need, s_cand;
+    __shared__ int s_count, s_pick;
+    auto key_of = [&](float v) { return float_order_key(T == 1.0f ? v : v / T); };
+    uint32_t key[U];
+    {
+        float v[U];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int i = base + u * 256 + tid;
-                    v[u] = i < p.V ? lg[i] : 0.f;
-                }
-            }
+        for (int u = 0; u < U; ++u) v[u] = u * NT + tid < V ? lg[u * NT + tid] : 0.f;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = base + u * 256 + tid;
-                uint32_t key = 0;
-                if (from_global) {
-                    key = float_order_key(v[u] / T);
-                    if (pass == 0 && i < p.V && i < kSampleKeys) skey[i] = key;
-                } else if (i < p.V) {
-                    key = skey[i];
-                }
-                count(i, key);
-            }
-        }
-        __syncthreads();
-        if (tid < 32) {
-            // the bin that holds the `need`-th largest key of this digit: lane l sums bins 255 - 8l .. 248 - 8l,
-            // an exclusive scan over the lanes finds the lane, which then walks its eight bins
-            const uint32_t need = s_need;
-            uint32_t mine = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) mine += hist[255 - 8 * lane - j];
-            uint32_t incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += up;
-            }
-            const uint32_t before = incl - mine;
-            // the last lane also takes the case of fewer than `need` candidates in all bins (k > count)
-            const bool here = (before < need && need <= incl) || (lane == 31 && incl < need);
-            if (here) {
-                uint32_t left = need - before, bin = 255 - 8 * lane;
-                for (int j = 0; j < 8; ++j, --bin) {
-                    const uint32_t h = hist[bin];
-                    if (h >= left || bin == 0) break;
-                    left -= h;
-                }
-                s_need = left;
-                s_prefix = prefix | (bin << shift);
-                s_mask = mask | (0xffu << shift);
-            }
-        }
-        __syncthreads();
+        for (int u = 0; u < U; ++u) key[u] = key_of(v[u]);
     }
-    const uint32_t kth = s_prefix;
-    if (tid == 0) { s_count = 0; s_overflow = 0; }
-    __syncthreads();
-    for (int i = tid; i < p.V; i += blockDim.x) {
-        const uint32_t key = i < kSampleKeys ? skey[i] : float_order_key(lg[i] / T);
-        if (key >= kth) {
-            int slot = atomicAdd(&s_count, 1);
-            if (slot < kSampleCap) { cval[slot] = float_from_order_key(key); cidx[slot] = i; } else s_overflow = 1;
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u * NT + tid < V) f(u * NT + tid, key[u]);
+        for (int base = U * NT; base < V; base += U * NT) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = base + u * NT + tid < V ? lg[base + u * NT + tid] : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (base + u * NT + tid < V) f(base + u * NT + tid, key_of(v[u]));
         }
+    };
+    if (tid == 0) { s_prefix = 0; s_mask = 0; s_need = (uint32_t)k; s_count = 0; s_pick = 0x7fffffff; }
+    // s_prefix ends as a lower bound of the k-th largest key with at most kSampleCap keys on or above it, or as that key itself
+#pragma unroll 1
+    for (int pass = 0; pass < 3; ++pass) {
+        const int shift = pass == 0 ? 20 : (pass == 1 ? 8 : 0), nb = pass == 2 ? 256 : 4096;
+        for (int i = tid; i < nb; i += NT) hist[i] = 0;
+        __syncthreads();
+        const uint32_t prefix = s_prefix, mask = s_mask, need = s_need;
+        each([&](int, uint32_t x) {
+            if ((x & mask) == prefix) atomicAdd(&hist[(x >> shift) & (uint32_t)(nb - 1)], 1u);
+        });
+        __syncthreads();
+        // the bin that holds the `need`-th largest key of this digit: thread t sums bins nb - 1 - 4t .. nb - 4 - 4t, a scan
+        // over the threads finds the one, which then walks its four bins
+        uint32_t mine = 0;
+        if (4 * tid < nb) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mine += hist[nb - 1 - 4 * tid - j];
+        }
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        const uint32_t below = __reduce_add_sync(0xffffffffu, lane < warp ? wsum[lane] : 0u);
+        const uint32_t before = below + incl - mine;
+        if (before < need && need <= before + mine) {
+            uint32_t left = need - before, bin = (uint32_t)(nb - 1 - 4 * tid);
+            for (int j = 0; j < 3 && hist[bin] < left; ++j) left -= hist[bin--];
+            s_need = left;
+            s_cand = (uint32_t)k - left + hist[bin];
+            s_prefix = prefix | (bin << shift);
+            s_mask = mask | ((uint32_t)(nb - 1) << shift);
+        }
+        __syncthreads();
+        if (s_cand <= (uint32_t)kSampleCap) break;
     }
+    const uint32_t least = s_prefix;
+    auto entry = [](uint32_t x, int i) { return ((unsigned long long)x << 32) | (uint32_t)~i; };      // larger: comes first
+    each([&](int i, uint32_t x) {
+        if (x >= least) {
+            const int slot = atomicAdd(&s_count, 1);
+            if (slot < kSampleCap) cand[slot] = entry(x, i);
+        }
+    });
     __syncthreads();
     int n = min(s_count, kSampleCap);
-    if (s_overflow) {
+    if (s_count > kSampleCap) {
         // More than kSampleCap values tie at the threshold: keep the strictly larger ones and
         // refill ties in index order with one thread (degenerate inputs only).
+        __syncthreads();
         if (tid == 0) {
             int w = 0;
-            for (int i = 0; i < p.V && w < kSampleCap; ++i) {
-                float v = lg[i] / T;
-                if (float_order_key(v) > kth) { cval[w] = v; cidx[w] = i; ++w; }
-            }
-            for (int i = 0; i < p.V && w < kSampleCap; ++i) {
-                float v = lg[i] / T;
-                if (float_order_key(v) == kth) { cval[w] = v; cidx[w] = i; ++w; }
-            }
+            for (int ties = 0; ties < 2; ++ties)
+                for (int i = 0; i < V && w < kSampleCap; ++i) {
+                    const uint32_t x = key_of(lg[i]);
+                    if (ties ? x == least : x > least) cand[w++] = entry(x, i);
+                }
             s_count = w;
         }
         __syncthreads();
         n = s_count;
     }
-    // pad to a power of two and bitonic sort: value descending, index ascending
-    int np2 = 1;
-    while (np2 < n) np2 <<= 1;
-    for (int i = n + tid; i < np2; i += blockDim.x) { cval[i] = -INFINITY; cidx[i] = 0x7fffffff; }
-    __syncthreads();
-    for (int sz = 2; sz <= np2; sz <<= 1) {
-        for (int st = sz >> 1; st > 0; st >>= 1) {
-            for (int i = tid; i < np2; i += blockDim.x) {
-                int j = i ^ st;
-                if (j > i) {
-                    bool up = ((i & sz) == 0);
-                    float vi = cval[i], vj = cval[j];
-                    int ii = cidx[i], ij = cidx[j];
-                    bool i_first = (vi > vj) || (vi == vj && ii < ij);   // i belongs before j
-                    if (i_first != up) { cval[i] = vj; cval[j] = vi; cidx[i] = ij; cidx[j] = ii; }
+    const unsigned long long* sorted = ranked;
+    if (n <= kSampleRank) {
+        constexpr int PER = NT / kSampleRank;          // threads per candidate
+        const int i = tid / PER;
+        const unsigned long long me = i < n ? cand[i] : 0ull;
+        int r = 0;
+        for (int j = tid % PER; j < n; j += PER) r += cand[j] > me ? 1 : 0;
+#pragma unroll
+        for (int o = 1; o < PER; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (tid % PER == 0 && i < n) ranked[r] = me;
+        __syncthreads();
+    } else {
+        // padded to a power of two and bitonic sorted
+        sorted = cand;
+        int np2 = 1;
+        while (np2 < n) np2 <<= 1;
+        for (int i = n + tid; i < np2; i += NT) cand[i] = 0ull;
+        __syncthreads();
+        for (int sz = 2; sz <= np2; sz <<= 1) {
+            for (int st = sz >> 1; st > 0; st >>= 1) {
+                for (int i = tid; i < np2; i += NT) {
+                    const int j = i ^ st;
+                    if (j > i) {
+                        const unsigned long long x = cand[i], y = cand[j];
+                        if ((x > y) != ((i & sz) == 0)) { cand[i] = y; cand[j] = x; }
+                    }
                 }
+                __syncthreads();
             }
-            __syncthreads();
         }
     }
     // the exponentials in parallel, their sums by one thread in descending order (the order is part of the result)
     const int kk = min(k, n);
-    {
-        const float v0 = cval[0];
-        float e[(kSampleCap + 255) / 256];
-#pragma unroll
-        for (int r = 0; r < (kSampleCap + 255) / 256; ++r) {
-            const int j = tid + 256 * r;
-            e[r] = j < kk ? expf(cval[j] - v0) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < (kSampleCap + 255) / 256; ++r) {
-            const int j = tid + 256 * r;
-            if (j < kk) cval[j] = e[r];
-        }
-        __syncthreads();
-    }
+    const float v0 = float_from_order_key((uint32_t)(sorted[0] >> 32));
+    for (int j = tid; j < kk; j += NT) cum[j] = expf(float_from_order_key((uint32_t)(sorted[j] >> 32)) - v0);
+    __syncthreads();
     if (tid == 0) {
         float total = 0.f;
-        for (int j = 0; j < kk; ++j) total += cval[j];
-        unsigned long long seed = p.seeds[b];
-        uint32_t w0 = philox_first_word((uint32_t)(c.pos[b] + 1), (uint32_t)(seed & 0xffffffffull), (uint32_t)(seed >> 32));
-        float u = (float)(w0 >> 8) * (1.0f / 16777216.0f);
-        float target = u * total, cum = 0.f;
-        int pick = kk - 1;
-        for (int j = 0; j < kk; ++j) {
-            cum += cval[j];
-            if (cum > target) { pick = j; break; }
+        int j = 0;
+        for (; j + 8 <= kk; j += 8) {
+            const float4 x = *reinterpret_cast<const float4*>(cum + j), y = *reinterpret_cast<const float4*>(cum + j + 4);
+            float4 o, q;
+            o.x = total += x.x; o.y = total += x.y; o.z = total += x.z; o.w = total += x.w;
+            q.x = total += y.x; q.y = total += y.y; q.z = total += y.z; q.w = total += y.w;
+            *reinterpret_cast<float4*>(cum + j) = o;
+            *reinterpret_cast<float4*>(cum + j + 4) = q;
         }
-        advance_seq(c, b, cidx[pick]);
+        for (; j < kk; ++j) cum[j] = total += cum[j];
     }
+    __syncthreads();
+    const unsigned long long seed = p.seeds[b];
+    const uint32_t w0 = philox_first_word((uint32_t)(c.pos[b] + 1), (uint32_t)(seed & 0xffffffffull), (uint32_t)(seed >> 32));
+    const float u = (float)(w0 >> 8) * (1.0f / 16777216.0f);
+    const float target = u * cum[kk - 1];
+    for (int j = tid; j < kk; j += NT)
+        if (cum[j] > target) atomicMin(&s_pick, j);
+    __syncthreads();
+    if (tid == 0) advance_seq(c, b, (int)~(uint32_t)sorted[min(s_pick, kk - 1)]);
 }
 
 // Column softmax of the logits for the probability probe (getVocabMaxByCol_softmax,

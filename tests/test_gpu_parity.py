@@ -11,7 +11,7 @@ import pytest
 
 from helpers import (TOL_FP32, TOL_LOWP, load_oracle, logits_error, oracle_rollout, random_prompts,
                      write_model)
-from mini_llm_cuda_b200.model_file import ModelSpec, named_spec, periodic_layer_types
+from mini_llm_cuda_b200.model_file import ModelSpec, named_spec, periodic_layer_types, synth_weights, write_model_bin
 from oracle.decode_oracle import sample_top_k
 
 pytestmark = pytest.mark.gpu
@@ -540,6 +540,38 @@ def test_more_steps_than_the_context_holds(api, tmp_path):
     ms, got = sess.decode_timed(33, False)
     assert np.array_equal(got[:, :20], want) and (got[:, 20:] == -1).all()
     assert (ms[:20] > 0).all() and (ms[20:] == 0).all()
+    sess.close()
+    model.close()
+
+
+@pytest.mark.parametrize("vocab,top_k,tied", [(300, 1024, False), (1000, 257, False), (9001, 200, False), (40003, 1000, False), (2048, 50, True), (700, 3, True)])
+def test_topk_sampler_sizes(api, tmp_path, vocab, top_k, tied):
+    """Vocabularies beside the 8192 logits that stay in registers, k at the whole vocabulary, behind the 256 candidates that are sorted by
+    counting and near the 1024 that are kept; all logits equal (an all-zero embedding): the k lowest ids are the candidates."""
+    spec = small(vocab=vocab)
+    weights = synth_weights(spec, seed=14)
+    if tied:
+        weights["tokenEmbeddings"][:] = 0
+    path = str(tmp_path / "m.bin")
+    write_model_bin(path, spec, weights)
+    model = api.Model(path)
+    sess = api.Session(model, 3)
+    prompts = random_prompts(spec.vocab, [4, 1, 6], seed=5)
+    sess.prefill(prompts)
+    seeds = [3, 2**33 + 1, 77]
+    close_calls = 0
+    for step in range(12):
+        out = sess.decode_step({"mode": "top_k", "top_k": top_k, "temperature": 0.7, "seeds": seeds})
+        lg = sess.logits()
+        for b in range(3):
+            want, margin = sample_top_k(lg[b], 0.7, min(top_k, vocab), seeds[b], len(prompts[b]) + step, return_margin=True)
+            if int(out[b]) != want:
+                assert margin < 1e-5, f"step {step} seq {b}: got {out[b]} want {want} margin {margin}"
+                close_calls += 1
+    assert close_calls <= 2
+    if tied:
+        sess.prefill(prompts)
+        assert (sess.decode(3) == 0).all()
     sess.close()
     model.close()
 
