@@ -89,18 +89,25 @@ struct Chain {
             grid_x = (p.N + g.rows_per_cta - 1) / g.rows_per_cta;
         }
         auto up4 = [](int v) { return (v + 3) / 4 * 4; };
-        int off = 0;
-        g.off_xs = off; off += up4(p.K);
-        g.off_xs2 = off; off += up4(std::max(p.Kp, 4));
-        g.off_outs = off; off += up4(std::max(p.hd, 64));
-        g.off_pacc = off; off += up4(g.rows_per_cta + 4);
-        g.off_red = off; off += 64;
-        off = (off + 31) / 32 * 32;
-        g.off_bar = off; off += 8 * 4;
-        off = (off + 31) / 32 * 32;
-        g.off_ring = off;
-        const size_t fixed = (size_t)off * 4;
-        if (fixed + 3 * (size_t)g.stage_bytes > 210 * 1024) return MLB_OK;
+        g.xs_stride = up4(p.K); g.xs2_stride = up4(std::max(p.Kp, 4)); g.outs_stride = up4(std::max(p.hd, 64)); g.pacc_stride = up4(g.rows_per_cta + 4);
+        // as many sequences per CTA (three at most) as leave three stages; without room for one the other GEMV serves
+        int bt = std::min(s->B, 3);
+        size_t fixed = 0;
+        for (;; --bt) {
+            if (bt == 0) return MLB_OK;
+            int off = 0;
+            g.off_xs = off; off += bt * g.xs_stride;
+            g.off_xs2 = off; off += bt * g.xs2_stride;
+            g.off_outs = off; off += bt * g.outs_stride;
+            g.off_pacc = off; off += bt * g.pacc_stride;
+            g.off_red = off; off += 64;
+            off = (off + 31) / 32 * 32;
+            g.off_bar = off; off += 8 * 4;
+            off = (off + 31) / 32 * 32;
+            g.off_ring = off;
+            fixed = (size_t)off * 4;
+            if (fixed + 3 * (size_t)g.stage_bytes <= 210 * 1024) break;
+        }
         g.n_stages = (int)std::min<size_t>(s->sg_max_stages, (210 * 1024 - fixed) / g.stage_bytes);
         g.err = s->dev_err;
         const size_t smem = fixed + (size_t)g.n_stages * g.stage_bytes;
@@ -111,8 +118,13 @@ struct Chain {
             int rc = rec->begin(name, wbytes + abytes, 2ull * p.N * (p.K + p.Kp) * s->B * (MODE == GEMV_SWIGLU ? 2 : 1));
             if (rc) return rc;
         }
-        cudaError_t e = launch_chain(s->use_pdl, sgemv_kernel<T, T2, KVT, MODE>, dim3(grid_x, s->B), dim3(kSgThreads), smem,
-                                     s->stream, c, p, g);
+        const dim3 grid(grid_x, (s->B + bt - 1) / bt), block(kSgThreads);
+        cudaError_t e;
+        switch (bt) {
+            case 1: e = launch_chain(s->use_pdl, sgemv_kernel<T, T2, KVT, 1, MODE>, grid, block, smem, s->stream, c, p, g); break;
+            case 2: e = launch_chain(s->use_pdl, sgemv_kernel<T, T2, KVT, 2, MODE>, grid, block, smem, s->stream, c, p, g); break;
+            default: e = launch_chain(s->use_pdl, sgemv_kernel<T, T2, KVT, 3, MODE>, grid, block, smem, s->stream, c, p, g); break;
+        }
         if (e != cudaSuccess) return fail(MLB_E_CUDA, "launch of %s (streamed) failed: %s", name, cudaGetErrorString(e));
         *done = true;
         if (rec) return rec->end();
@@ -157,7 +169,9 @@ struct Chain {
     template <int MODE>
     static int configure_mode() {
         const int big = 200 * 1024;
-        CU(cudaFuncSetAttribute(sgemv_kernel<T, T2, KVT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
+        CU(cudaFuncSetAttribute(sgemv_kernel<T, T2, KVT, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
+        CU(cudaFuncSetAttribute(sgemv_kernel<T, T2, KVT, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
+        CU(cudaFuncSetAttribute(sgemv_kernel<T, T2, KVT, 3, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024));
         CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CU(cudaFuncSetAttribute(gemv_kernel<T, T2, KVT, 4, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));

@@ -1,6 +1,5 @@
 // Shared pieces of the kernels that stream weights through shared memory: mbarrier / TMA-bulk
-// wrappers, the ring of shared-memory stages with its bounded waits, the producer's slab issue
-// and the consumers' dot products out of a stage. Used by the streamed GEMV (sgemv.cuh), the
+// wrappers, the ring of shared-memory stages with its bounded waits and the producer's slab issue. Used by the streamed GEMV (sgemv.cuh), the
 // whole-GPU batch-1 step (grid.cuh), the tcgen05 GEMM (gemm_tc.cuh) and the operator tests (ops.cu).
 #pragma once
 #include "kernels.cuh"
@@ -133,97 +132,6 @@ __device__ __forceinline__ void issue_slab_pair(Ring& r, const unsigned char* a,
         }
     }
     __syncwarp();
-}
-
-// ---- consumer side ------------------------------------------------------------------------------
-// Two rows at a time against the activation vector in shared memory: one read of x serves both
-// rows, so shared-memory traffic is 2 bytes per weight byte (fp32 x, bf16 weights) instead of 3.
-template <typename T, bool PERM = false>
-__device__ __forceinline__ void smem_rows_dot2(const T* row0, const T* row1, int nvec, const float* xs, int lane, float& a0,
-                                               float& a1) {
-    // PERM: xs is stored as [EPV/4][nvec] float4s (xs_f4_index), else linearly
-    constexpr int EPV = Elem<T>::EPV;
-    a0 = 0.f;
-    a1 = 0.f;
-#pragma unroll 2
-    for (int vi = lane; vi < nvec; vi += 32) {
-        float w0[EPV], w1[EPV];
-        Elem<T>::unpack(*reinterpret_cast<const uint4*>(row0 + (size_t)vi * EPV), w0);
-        Elem<T>::unpack(*reinterpret_cast<const uint4*>(row1 + (size_t)vi * EPV), w1);
-        const float4* xp = reinterpret_cast<const float4*>(xs);
-#pragma unroll
-        for (int q = 0; q < EPV / 4; ++q) {
-            const float4 t = PERM ? xp[q * nvec + vi] : xp[vi * (EPV / 4) + q];
-            a0 = fmaf(w0[4 * q], t.x, a0); a0 = fmaf(w0[4 * q + 1], t.y, a0);
-            a0 = fmaf(w0[4 * q + 2], t.z, a0); a0 = fmaf(w0[4 * q + 3], t.w, a0);
-            a1 = fmaf(w1[4 * q], t.x, a1); a1 = fmaf(w1[4 * q + 1], t.y, a1);
-            a1 = fmaf(w1[4 * q + 2], t.z, a1); a1 = fmaf(w1[4 * q + 3], t.w, a1);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    }
-}
-
-// Consume a slab of `rows` rows of K elements: f(local_row, dot) runs in every lane of the warp
-// that owns the row, with the full dot product.
-template <typename T, int NW = kRingWarps, bool PERM = false, typename F>
-__device__ __forceinline__ void consume_slab(Ring& r, int rows, int K, const float* xs, int warp, int lane, F&& f) {
-    const int nvec = K / Elem<T>::EPV;
-    const int row_bytes = K * (int)sizeof(T);
-    const int rpc = max(1, r.stage_bytes / row_bytes);
-    for (int r0 = 0; r0 < rows; r0 += rpc) {
-        const int n = min(rpc, rows - r0);
-        r.wait(r.full0 + 8u * r.idx, r.phase, 2);
-        const T* base = reinterpret_cast<const T*>(r.stages + (size_t)r.idx * r.stage_bytes);
-        if (n >= 2 * NW) {
-            for (int i = 2 * warp; i < n; i += 2 * NW) {
-                const bool two = i + 1 < n;
-                float a0, a1;
-                smem_rows_dot2<T, PERM>(base + (size_t)i * K, base + (size_t)(two ? i + 1 : i) * K, nvec, xs, lane, a0, a1);
-                f(r0 + i, a0);
-                if (two) f(r0 + i + 1, a1);
-            }
-        } else {
-            // few long rows in the chunk: one row per warp keeps more warps busy
-            for (int i = warp; i < n; i += NW) {
-                float a0, a1;
-                smem_rows_dot2<T, PERM>(base + (size_t)i * K, base + (size_t)i * K, nvec, xs, lane, a0, a1);
-                f(r0 + i, a0);
-            }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(r.empty0 + 8u * r.idx);
-        r.advance();
-    }
-}
-
-// Chunk-interleaved pair of slabs: f(local_row, dot_a, dot_b).
-template <typename T, int NW = kRingWarps, bool PERM = false, typename F>
-__device__ __forceinline__ void consume_slab_pair(Ring& r, int rows, int K, const float* xs, int warp, int lane, F&& f) {
-    const int nvec = K / Elem<T>::EPV;
-    const int row_bytes = K * (int)sizeof(T);
-    const int rpc = max(1, r.stage_bytes / row_bytes);
-    for (int r0 = 0; r0 < rows; r0 += rpc) {
-        const int n = min(rpc, rows - r0);
-        const int ia = r.idx;
-        r.wait(r.full0 + 8u * r.idx, r.phase, 2);
-        r.advance();
-        const int ib = r.idx;
-        r.wait(r.full0 + 8u * r.idx, r.phase, 2);
-        r.advance();
-        const T* A = reinterpret_cast<const T*>(r.stages + (size_t)ia * r.stage_bytes);
-        const T* Bm = reinterpret_cast<const T*>(r.stages + (size_t)ib * r.stage_bytes);
-        for (int i = warp; i < n; i += NW) {
-            float a0, a1;
-            smem_rows_dot2<T, PERM>(A + (size_t)i * K, Bm + (size_t)i * K, nvec, xs, lane, a0, a1);
-            f(r0 + i, a0, a1);
-        }
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(r.empty0 + 8u * ia); mbar_arrive(r.empty0 + 8u * ib); }
-    }
 }
 
 // Sum over the consumer threads; every consumer gets the total. `red` holds kRingWarps floats.

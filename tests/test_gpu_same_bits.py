@@ -96,3 +96,29 @@ def test_recurrence_over_columns_against_steps(api, tmp_path, monkeypatch, dk, d
     for a, b in zip(got["auto"], got["step"]):
         assert np.array_equal(a, b)
     model.close()
+
+
+@pytest.mark.parametrize("name", ["fp8", "bf16", "fp32_qknorm_gated"])
+def test_streamed_gemv_of_several_sequences(api, tmp_path, monkeypatch, name):
+    """A CTA of the streamed GEMV takes up to three sequences: each gets the ids and logits that it gets alone. Two to seven
+    sequences: whole and ragged groups of three; down projections whose input leaves room for fewer (ffn_dim 9216: 108 KB for three)."""
+    for key, value in (("MLB_PREFILL", "step"), ("MLB_DECODE_PATH", "chain"), ("MLB_GEMV", "stream"), ("MLB_GEMM", "simt")):
+        monkeypatch.setenv(key, value)
+    spec = {**SPECS, "fp32_qknorm_gated": ModelSpec(dim=256, layers=2, heads=4, kv_heads=2, head_dim=64, ffn_dim=9216, vocab=500, qk_norm=True, query_gating=True,
+                                                    rms_eps=1e-5, max_context=64)}[name]
+    model = api.Model(write_model(tmp_path, spec, seed=113))
+    prompts = random_prompts(spec.vocab, [3 + b % 4 for b in range(7)], seed=115)
+    sess = api.Session(model, 1)
+    want = []
+    for p in prompts:
+        sess.prefill([p])
+        want.append((sess.decode(4)[0], sess.logits()[0]))
+    sess.close()
+    for batch in (2, 3, 4, 7):
+        sess = api.Session(model, batch)
+        sess.prefill(prompts[:batch])
+        ids, logits = sess.decode(4), sess.logits()
+        for b in range(batch):
+            assert np.array_equal(ids[b], want[b][0]) and np.array_equal(logits[b], want[b][1]), (batch, b)
+        sess.close()
+    model.close()
