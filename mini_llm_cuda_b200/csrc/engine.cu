@@ -590,13 +590,17 @@ static GridVec grid_vec(int N, int P, int tab) {
     v.slotw = (v.rpc + 15) / 16 * 16;
     v.tab = tab;
     v.inv_n = 1.0f / (float)N;
-    v.magic = 0;
-    if (v.rpc > 1) {
-        // q / rpc as one multiply-high, exact over the range the kernel uses (q < P * rpc < 2^16 * rpc)
-        v.magic = (unsigned)(((1ull << 32) + (unsigned)v.rpc - 1) / (unsigned)v.rpc);
-        for (unsigned q = 0; q < (unsigned)(P * v.rpc); ++q)
-            if ((unsigned)(((unsigned long long)q * v.magic) >> 32) != q / (unsigned)v.rpc) { v.N = -1; break; }     // never seen; the caller refuses
-    }
+    v.wpp = (v.rpc + 2) / 3;
+    // q / d as one multiply-high, exact over the range the kernel uses (q < P * d < 2^16 * d)
+    auto magic = [&](int d) {
+        if (d == 1) return 0u;
+        const unsigned m = (unsigned)(((1ull << 32) + (unsigned)d - 1) / (unsigned)d);
+        for (unsigned q = 0; q < (unsigned)(P * d); ++q)
+            if ((unsigned)(((unsigned long long)q * m) >> 32) != q / (unsigned)d) { v.N = -1; break; }     // never seen; the caller refuses
+        return m;
+    };
+    v.magic = magic(v.rpc);
+    v.magic3 = magic(v.wpp);
     return v;
 }
 
@@ -660,12 +664,13 @@ static int setup_grid_path(mlb_session* s) {
     const int tab_lm = off; off += up4(C + 1);
     gp.vocab_tab = off; off += up4(C + 1);
     gp.off_tabs = 0;
-    gp.xs_stride = up4(std::max(std::max(c.dim, c.ffn_dim), a_dim));
-    gp.off_xs = off; off += 2 * gp.xs_stride;
-    gp.off_xa = off; off += up4(c.dim);
-    gp.off_xb = off; off += up4(c.dim);
+    // two input buffers in turn: phases whose input is the residual stream, and the others (output and down projection)
+    gp.xs_stride = up4(c.dim);
+    gp.off_xs = off; off += gp.xs_stride + up4(std::max(c.ffn_dim, a_dim));
+    gp.off_xa = off; off += up4(rpc_d);
+    gp.off_xb = off; off += up4(rpc_d);
     gp.off_parts = off; off += up4(std::max(has_attn ? std::max(gp.s_max * (c.head_dim + 2), kGridDirectWords) : 0, 2 * C));
-    gp.off_gate = off; off += up4(has_attn ? c.heads * c.head_dim : 4);
+    gp.off_gate = off; off += up4(has_attn && c.query_gating ? c.heads * c.head_dim : 4);
     {
         const int attn_n = has_attn ? G * c.head_dim + 2 * c.head_dim + kRingWarps * (c.head_dim + 2) : 0;
         const int comb_n = has_attn ? std::max(c.heads * gp.s_direct, gp.s_max) : 0;
@@ -684,15 +689,15 @@ static int setup_grid_path(mlb_session* s) {
     gp.off_bar = off; off += max_stages * 2 * 2;              // 8-byte barriers: full[] then empty[]
     off = (off + 31) / 32 * 32;
     gp.off_ring = off;
-    // ring: stages of whole rows (and whole KV pages), 16 KB unless a row is longer, as many as fit below ~208 KB
+    // ring: stages of whole rows (and whole KV pages), 16 KB unless a row is longer, as many as fit below 226 KB
     size_t widest = (size_t)std::max(std::max(c.dim, c.ffn_dim), a_dim) * elt_size(c.weight_dtype);
     if (has_attn) widest = std::max(widest, (size_t)kKvBlock * c.head_dim * elt_size(c.kv_dtype));
     if (has_dn) widest = std::max(widest, (size_t)c.dn_key_dim * 4);
     gp.stage_bytes = (int)std::max<size_t>(16 * 1024, (widest + 1023) / 1024 * 1024);
     if (const char* v = std::getenv("MLB_GRID_STAGE_KB")) gp.stage_bytes = std::max(gp.stage_bytes, std::min(64, std::atoi(v)) * 1024);
     const size_t fixed = (size_t)off * 4;
-    if (fixed + 3 * (size_t)gp.stage_bytes > 208 * 1024) return no("the activations leave too little shared memory for the weight ring");
-    gp.n_stages = (int)std::min<size_t>(max_stages, (208 * 1024 - fixed) / gp.stage_bytes);
+    if (fixed + 3 * (size_t)gp.stage_bytes > 226 * 1024) return no("the activations leave too little shared memory for the weight ring");
+    gp.n_stages = (int)std::min<size_t>(max_stages, (226 * 1024 - fixed) / gp.stage_bytes);
     const size_t smem = fixed + (size_t)gp.n_stages * gp.stage_bytes;
     int per_sm = 0, rc;
     if ((rc = grid_kernel_probe(c.weight_dtype, c.kv_dtype, smem, &per_sm))) return rc;

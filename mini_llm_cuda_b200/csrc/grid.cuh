@@ -8,8 +8,9 @@
 //     shared-memory stages. The producer depends on nothing but free stages, so it runs phases
 //     ahead of the consumers: weights, the K/V pages of the CTA's attention item and its rows of
 //     the delta-net state are in shared memory before the activations that need them arrive.
-//   * Activations cross CTAs as 8-byte {value, epoch} words. A reader polls the words themselves
-//     until they carry the epoch of the phase it waits for: no grid barrier, no flag, no fence.
+//   * Activations cross CTAs as 8-byte {value, epoch} words, or three to a 16-byte {value, value, value, epoch} word where no sum of
+//     squares goes with them. A reader polls the words themselves until they carry the epoch of the phase it waits for: no
+//     grid barrier, no flag, no fence.
 //     Every producer writes into a slot of its own (whole 128-byte lines): a line polled by all
 //     CTAs has exactly one writer. (Measured on B200: an all-to-all of 512 words among 148 CTAs
 //     costs 2.4 us with densely packed words, 1.2 us with one slot per writer; the hop from one
@@ -62,6 +63,23 @@ __device__ __forceinline__ unsigned long long ll_load(const unsigned long long* 
     unsigned long long w;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
     return w;
+}
+// Three values and their epoch, 16 bytes that are written and read as one.
+__device__ __forceinline__ void ll_store3(uint4* p, float a, float b, float c, uint32_t e) {
+    const unsigned long long lo = ((unsigned long long)__float_as_uint(b) << 32) | __float_as_uint(a);
+    const unsigned long long hi = ((unsigned long long)e << 32) | __float_as_uint(c);
+    asm volatile("{\n.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ uint4 ll_load3(const uint4* p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;\n}\n" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+// `n` values in shared memory to a slot of 16-byte words, by one warp: one store instruction per 96 values.
+__device__ __forceinline__ void ll_publish3(unsigned long long* slot, const float* v, int n, uint32_t e, int lane) {
+    uint4* d = reinterpret_cast<uint4*>(slot);
+#pragma unroll 1
+    for (int q = lane; 3 * q < n; q += 32) ll_store3(d + q, v[3 * q], v[min(3 * q + 1, n - 1)], v[min(3 * q + 2, n - 1)], e);
 }
 __device__ __forceinline__ float fast_sigmoid(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
 
@@ -127,16 +145,16 @@ __device__ __forceinline__ void ll_poll(const unsigned long long* const (&src)[N
     }
 }
 
-// The whole vector. Row r goes to lin[r] (if lin) and, multiplied by gain[r] (if gain), to the GEMV
-// layout of nvec weight vectors at xs. Returns the sum of squares of what this thread fetched.
+// The whole vector. Row r goes, multiplied by gain[r], to the GEMV layout of nvec weight vectors at xs; this CTA's own rows
+// (rank's of the vector) also to own, by local row. Returns the sum of squares of what this thread fetched.
 // The gains are asked for before the polls start. `tabs`: shared memory seen as ints.
 template <int EPV, int U>
-__device__ __noinline__ float ll_gather_vec_u(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* lin, float* xs, int nvec,
+__device__ __noinline__ float ll_gather_vec_u(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* own, int rank, float* xs, int nvec,
                                             const int* tabs, volatile int* dead, int* err) {
     const int P = vp->P, rpc = vp->rpc, slotw = vp->slotw, tab = vp->tab;
     const unsigned magic = vp->magic;
     const unsigned long long* buf = vp->buf;
-    const int n = P * rpc;
+    const int n = P * rpc, own0 = tabs[tab + rank], own1 = tabs[tab + rank + 1];
     float ss = 0.f;
 #pragma unroll 1
     for (int q0 = threadIdx.x; q0 < n; q0 += kRingConsumers * U) {
@@ -155,14 +173,14 @@ __device__ __noinline__ float ll_gather_vec_u(const GridVec* vp, uint32_t e, con
             const bool valid = q0 + u * kRingConsumers < n && r0 + j < r1;
             row[u] = valid ? r0 + j : -1;
             src[u] = buf + (size_t)c * slotw + (valid ? j : 0);
-            g[u] = (gain != nullptr && valid) ? gain[r0 + j] : 1.0f;
+            g[u] = valid ? gain[r0 + j] : 1.0f;
         }
         ll_poll(src, w, e, dead, err);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (row[u] >= 0) {
                 const float val = __uint_as_float((uint32_t)w[u]);
-                if (lin) lin[row[u]] = val;
+                if (row[u] >= own0 && row[u] < own1) own[row[u] - own0] = val;
                 xs[xs_index<EPV>(row[u], nvec)] = val * g[u];
                 ss = fmaf(val, val, ss);
             }
@@ -175,12 +193,66 @@ __device__ __noinline__ float ll_gather_vec_u(const GridVec* vp, uint32_t e, con
 // Not more: the code of eight is fetched cold every time (a cfg4 step took 1470 us with it, 912 with four, 881 with five), and words
 // asked for twice cost too (cfg0 87 us with four, 91 with five).
 template <int EPV>
-__device__ __forceinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* lin, float* xs, int nvec,
+__device__ __forceinline__ float ll_gather_vec(const GridVec* vp, uint32_t e, const float* __restrict__ gain, float* own, int rank, float* xs, int nvec,
                                                const int* tabs, volatile int* dead, int* err) {
     const int n = vp->P * vp->rpc;
-    if (n <= 2 * kRingConsumers) return ll_gather_vec_u<EPV, 2>(vp, e, gain, lin, xs, nvec, tabs, dead, err);
-    if (n <= 4 * kRingConsumers) return ll_gather_vec_u<EPV, 4>(vp, e, gain, lin, xs, nvec, tabs, dead, err);
-    return ll_gather_vec_u<EPV, 5>(vp, e, gain, lin, xs, nvec, tabs, dead, err);
+    if (n <= 2 * kRingConsumers) return ll_gather_vec_u<EPV, 2>(vp, e, gain, own, rank, xs, nvec, tabs, dead, err);
+    if (n <= 4 * kRingConsumers) return ll_gather_vec_u<EPV, 4>(vp, e, gain, own, rank, xs, nvec, tabs, dead, err);
+    return ll_gather_vec_u<EPV, 5>(vp, e, gain, own, rank, xs, nvec, tabs, dead, err);
+}
+
+// The whole vector in words of three rows, to the GEMV layout at xs. (Five words are one round trip for 5632 rows, which took three as
+// single words; the order of a sum of squares hangs on who fetches what, so vectors that are normed stay with those.)
+template <int EPV, int U>
+__device__ __noinline__ void ll_gather_vec3_u(const GridVec* vp, uint32_t e, float* xs, int nvec, const int* tabs, volatile int* dead, int* err) {
+    const int P = vp->P, wpp = vp->wpp, slotw = vp->slotw, tab = vp->tab;
+    const unsigned magic = vp->magic3;
+    const unsigned long long* buf = vp->buf;
+    const int n = P * wpp;
+#pragma unroll 1
+    for (int q0 = threadIdx.x; q0 < n; q0 += kRingConsumers * U) {
+        const uint4* src[U];
+        uint4 w[U];
+        int row[U], rows[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int q = min(q0 + u * kRingConsumers, n - 1);
+            const int c = magic ? (int)__umulhi((unsigned)q, magic) : q;
+            const int j = q - c * wpp;
+            const int r0 = tabs[tab + c], r1 = tabs[tab + c + 1];
+            row[u] = r0 + 3 * j;
+            rows[u] = q0 + u * kRingConsumers < n ? min(3, r1 - row[u]) : 0;       // 0 or less: this producer's first word once more, dropped
+            src[u] = reinterpret_cast<const uint4*>(buf + (size_t)c * slotw) + (rows[u] > 0 ? j : 0);
+        }
+        uint32_t spins = 0;
+#pragma unroll 1
+        for (;;) {
+            bool ok = true;
+#pragma unroll
+            for (int u = 0; u < U; ++u) w[u] = ll_load3(src[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) ok = ok && w[u].w == e;
+            if (ok) break;
+            if (*dead) break;
+            __nanosleep(MLB_POLL_SLEEP);
+            if (++spins > kGridSpinLimit) {
+                *dead = 1;
+                atomicExch(err, 3);
+                break;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (rows[u] > 0) xs[xs_index<EPV>(row[u], nvec)] = __uint_as_float(w[u].x);
+            if (rows[u] > 1) xs[xs_index<EPV>(row[u] + 1, nvec)] = __uint_as_float(w[u].y);
+            if (rows[u] > 2) xs[xs_index<EPV>(row[u] + 2, nvec)] = __uint_as_float(w[u].z);
+        }
+    }
+}
+template <int EPV>
+__device__ __forceinline__ void ll_gather_vec3(const GridVec* vp, uint32_t e, float* xs, int nvec, const int* tabs, volatile int* dead, int* err) {
+    if (vp->P * vp->wpp <= 2 * kRingConsumers) ll_gather_vec3_u<EPV, 2>(vp, e, xs, nvec, tabs, dead, err);
+    else ll_gather_vec3_u<EPV, 5>(vp, e, xs, nvec, tabs, dead, err);
 }
 
 // n rows of a vector to dst[0..n): entry i is row ri + i - si of the last of the segments (ri, si) with si <= i, the first being
@@ -233,7 +305,7 @@ struct RowsJob {
     const float* scale2;           // the up matrix's scale (RJ_SWIGLU)
     unsigned long long* dst;       // this CTA's slot of the output vector, by local row
     uint32_t epoch;
-    const float* resid;            // RJ_RESID: residual stream in shared memory, by global row
+    const float* resid;            // RJ_RESID: this CTA's rows of the residual stream in shared memory, by local row
     const float* pacc;             // RJ_RESID: addend per local row, or null
     float* logits;                 // RJ_LM
     int norm_n;                    // > 0: scale by 1 / sqrt(sum(red[0..479]) / norm_n + eps) (the RMS norm, applied late)
@@ -249,16 +321,16 @@ struct RowsJob {
 template <typename T, int N>
 __device__ __forceinline__ void smem_rows_dot(const T* const (&row)[N], int nvec, const float* xs, int lane, float (&v)[N]) {
     constexpr int EPV = Elem<T>::EPV;
-    const float4* xp = reinterpret_cast<const float4*>(xs);
-    float a0[N], a1[N];
+    const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(xs);
+    f32x2 a[N];                                    // sums over the even and the odd columns
 #pragma unroll
-    for (int i = 0; i < N; ++i) a0[i] = a1[i] = 0.f;
-#pragma unroll 1
+    for (int i = 0; i < N; ++i) a[i] = 0ull;
+#pragma unroll (N <= 2 ? 2 : 1)
     for (int vi = lane; vi < nvec; vi += 32) {
         uint4 raw[N];
 #pragma unroll
         for (int i = 0; i < N; ++i) raw[i] = *reinterpret_cast<const uint4*>(row[i] + (size_t)vi * EPV);
-        float4 t[EPV / 4];
+        ulonglong2 t[EPV / 4];
 #pragma unroll
         for (int q = 0; q < EPV / 4; ++q) t[q] = xp[q * nvec + vi];
 #pragma unroll
@@ -267,13 +339,17 @@ __device__ __forceinline__ void smem_rows_dot(const T* const (&row)[N], int nvec
             Elem<T>::unpack(raw[i], w);
 #pragma unroll
             for (int q = 0; q < EPV / 4; ++q) {
-                a0[i] = fmaf(w[4 * q], t[q].x, a0[i]); a1[i] = fmaf(w[4 * q + 1], t[q].y, a1[i]);
-                a0[i] = fmaf(w[4 * q + 2], t[q].z, a0[i]); a1[i] = fmaf(w[4 * q + 3], t[q].w, a1[i]);
+                a[i] = fma2(pack2(w[4 * q], w[4 * q + 1]), t[q].x, a[i]);
+                a[i] = fma2(pack2(w[4 * q + 2], w[4 * q + 3]), t[q].y, a[i]);
             }
         }
     }
 #pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = warp_sum(a0[i] + a1[i]);
+    for (int i = 0; i < N; ++i) {
+        float x, y;
+        unpack2(a[i], x, y);
+        v[i] = warp_sum(x + y);
+    }
 }
 
 // Local row of a warp's i-th unit (a row, or two neighbouring ones): units go round the warps.
@@ -376,7 +452,7 @@ __device__ __forceinline__ void consume_rows(Ring& r, const RowsJob& j, bool pai
                     v = __fdividef(v, 1.0f + __expf(-v)) * ((u * su) * rn);
                 } else if (j.mode == RJ_RESID) {
                     if (j.pacc) v += j.pacc[lrow];
-                    v += j.resid[row];
+                    v += j.resid[lrow];
                 }
                 if (j.mode == RJ_LM) {
                     j.logits[row] = v;
@@ -391,7 +467,8 @@ __device__ __forceinline__ void consume_rows(Ring& r, const RowsJob& j, bool pai
                 if (__any_sync(0xffffffffu, last)) {
                     __threadfence_block();
 #pragma unroll 1
-                    for (int q = lane; q < rows; q += 32) ll_store(j.dst + q, j.obuf[q], j.epoch);
+                    for (int q = lane; q < rows && j.mode != RJ_SWIGLU; q += 32) ll_store(j.dst + q, j.obuf[q], j.epoch);
+                    if (j.mode == RJ_SWIGLU) ll_publish3(j.dst, j.obuf, rows, j.epoch, lane);
                     if (lane == 0) *j.ocnt = 0;
                 }
             }
@@ -637,7 +714,7 @@ __device__ __forceinline__ void grid_attention(const GridParams& p, const StepLa
 // One warp per (head, split) partial fetches it; one thread per output element combines.
 template <int EPV>
 __device__ __forceinline__ void grid_combine(const GridParams& p, const StepLayer& L, GridCtx& k, int h_first, int h_count, uint32_t e_proj,
-                                             uint32_t e_parts, float* xs, int nvec, unsigned long long* dst, uint32_t e_out) {
+                                             uint32_t e_parts, float* xs, int nvec, float* obuf, unsigned long long* dst, uint32_t e_out) {
     const int hd = p.hd, tid = k.tid, lane = k.lane, warp = k.warp, W = hd + 2, S = k.plan->S, G = p.heads / p.kv_heads;
     float* parts = k.smem + p.off_parts;           // [h_count][S][hd+2]
     float* gate = k.smem + p.off_gate;             // [h_count][hd]
@@ -680,7 +757,11 @@ __device__ __forceinline__ void grid_combine(const GridParams& p, const StepLaye
         float o = __fdividef(at, lt);
         if (L.ng) o *= fast_sigmoid(gate[i]);      // sigmoid of the gate projection (inference.cu:248)
         if (xs) xs[xs_index<EPV>(i, nvec)] = o;
-        else ll_store(dst + i, o, e_out);
+        else obuf[i] = o;
+    }
+    if (!xs) {
+        consumer_sync();
+        if (warp == 0) ll_publish3(dst, obuf, h_count * hd, e_out, lane);
     }
 }
 
@@ -765,8 +846,7 @@ __device__ __forceinline__ void grid_delta_net(const GridParams& p, const StepLa
             last = __shfl_sync(0xffffffffu, last, 0);
             if (last) {
                 __threadfence_block();
-#pragma unroll 1
-                for (int q = lane; q < rows; q += 32) ll_store(dst + q, obuf[q], e_out);
+                ll_publish3(dst, obuf, rows, e_out, lane);
                 if (lane == 0) *ocnt = 0;
             }
         }
@@ -886,10 +966,10 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
     // Input of a projection (GEMV layout) and the threads' sums of squares, two buffers each, used in
     // turn: a warp that is done with its rows of one phase fills the next phase's input while slower
     // warps still read the previous one; the block barrier after a gather is the only one of a phase.
-    float* xsb[2] = {smem + p.off_xs, smem + p.off_xs + p.xs_stride};
+    float* xsb[2] = {smem + p.off_xs, smem + p.off_xs + p.xs_stride};      // the first of the residual stream's size: projections, gate/up, LM head
     float* redb[2] = {smem + p.off_red, smem + p.off_red + kRingConsumers};
-    float* xa = smem + p.off_xa;        // residual stream after the FFN (linear)
-    float* xb = smem + p.off_xb;        // residual stream after the mixer (linear)
+    float* xa = smem + p.off_xa;        // this CTA's rows of the residual stream after the FFN
+    float* xb = smem + p.off_xb;        // and after the mixer
     float* pacc = smem + p.off_pacc;    // [layer][local row]: per-layer-embedding contribution to this CTA's rows of x
     Ring& ring = k.ring;
     const int d = p.d;
@@ -974,14 +1054,14 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
         const GridVec* vin = &p.vx;
         const GridVec* vout = nullptr;
         const float* gain = nullptr;
-        float* lin = nullptr;
+        float* own = nullptr;
         int K = d, tslot = 2;
         bool pair = false, do_gather = true;
         job.scale2 = nullptr;
         job.resid = nullptr;
         job.pacc = nullptr;
         if (ph == PH_PROJ) {
-            gain = L.g1; lin = xa;
+            gain = L.g1; own = xa;
             vout = attn ? &p.vproj_attn : &p.vproj_dn;
             job.mode = RJ_STORE; job.scale = L.Sqkv;
         } else if (ph == PH_OPROJ) {
@@ -1001,7 +1081,7 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
                 // head combines it and publishes the result (a second exchange, but nobody fetches heads * S partials)
                 if (plan.direct || rank < p.heads) {
                     grid_combine<EPV>(p, L, k, plan.direct ? 0 : rank, plan.direct ? p.heads : 1, e_proj, e_parts, plan.direct ? xs : nullptr,
-                                      K / EPV, vec_slot(p.va_head, rank), e_parts + 1);
+                                      K / EPV, smem + p.off_mix, vec_slot(p.va_head, rank), e_parts + 1);
                     if (!plan.direct) grid_mark(k, 7);
                 }
                 if (plan.direct) {
@@ -1018,7 +1098,7 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
             }
         } else if (ph == PH_GATEUP) {
             tslot = 12;
-            vin = &p.vxb; gain = L.g2; lin = xb;
+            vin = &p.vxb; gain = L.g2; own = xb;
             vout = &p.vh;
             pair = true;
             job.mode = RJ_SWIGLU; job.scale = L.S1a; job.scale2 = L.S1b;
@@ -1030,7 +1110,7 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
             if (p.ple > 0 && li + 1 < p.n_layers) job.pacc = pacc + (li + 1) * pacc_stride;
         } else {
             tslot = 16;
-            gain = p.g_final;
+            gain = p.g_final; own = xa;
             job.mode = RJ_LM; job.scale = p.Es;
         }
         // ---- this CTA's rows, and their scales: asked for here, used after the dot products -----------------------------
@@ -1050,7 +1130,8 @@ __device__ __forceinline__ void grid_consumer(const StepCtl& c, const GridParams
         float* red = redb[ri];
         if (gain) ri ^= 1;
         float ss = 0.f;
-        if (do_gather) ss = ll_gather_vec<EPV>(vin, e_in, gain, lin, xs, K / EPV, k.tabs, k.dead, k.err);
+        if (gain) ss = ll_gather_vec<EPV>(vin, e_in, gain, own, rank, xs, K / EPV, k.tabs, k.dead, k.err);
+        else if (do_gather) ll_gather_vec3<EPV>(vin, e_in, xs, K / EPV, k.tabs, k.dead, k.err);
         if (gain) red[tid] = ss;
         consumer_sync();
         grid_mark(k, tslot);

@@ -20,6 +20,8 @@ struct GridVec {
     unsigned magic;        // q / rpc == __umulhi(q, magic) for every q < P * rpc (checked on the host); 0: rpc == 1
     int tab;               // shared-memory float offset of the row table r0[0..P] (ints, filled by the kernel)
     float inv_n;           // 1 / N
+    int wpp;               // 16-byte words per producer where a word carries three rows, ceil(rpc / 3)
+    unsigned magic3;       // q / wpp, as magic; 0: wpp == 1
     int pad;
 };
 constexpr int kGridVecs = 8;   // the vectors of GridParams, vx first, stand one after the other
