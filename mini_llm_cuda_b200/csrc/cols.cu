@@ -52,10 +52,11 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // fp32 pairs, K/V read as bf16 and unpacked once for four rows. The partial scores of the four rows are summed by a butterfly
 // that leaves each lane one row, whose exponentials it takes alone and hands to the others. Half of the streams are
 // live at a time: the pages of w = 0, 1 first, then those of w = 2, 3.
-// What bounds it: the chain of a chunk of four positions - scores, butterfly, maximum, exponentials, shuffles, P V, one after the other
-// under two warps a scheduler - not its FMAs (1 and 2 cycles per SM, row and position at HD = 64 and 128): 3001 tokens of 16 heads of 128
-// take 1351 us a layer, 5.4 cycles; 256 x 256 tokens of 8 heads of 64, 16 columns of a sequence to a chunk and so half of every tile
-// padding, 185 us a chunk, 13 cycles.
+// What bounds it: 11 instructions per warp, row and position share of 64 under two warps a scheduler (IPC 2.2 an SM, FMA pipe half busy;
+// 64 q and 64 accumulator registers a thread leave room for no more warps), not its FMAs (1 and 2 cycles per SM, row and position at
+// HD = 64 and 128): 3001 tokens of 16 heads of 128 take 1290 us a layer, 5.2 cycles (1351 with the chunks of a page one after the other and
+// a division per score). At HD = 64 a page is one chunk; two pages at once wasted more on odd numbers of pages (256 x 256 tokens of 8
+// heads: 185 -> 212 us a launch of 16 columns each).
 // ------------------------------------------------------------------------------------------------
 constexpr int kAcRows = 32;      // (query, head) rows per CTA
 constexpr int kAcThreads = 256;
@@ -134,7 +135,10 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
         q[r][0] = pack2(x0.x, y0.x); q[r][1] = pack2(x0.y, y0.y); q[r][2] = pack2(x0.z, y0.z); q[r][3] = pack2(x0.w, y0.w);
         q[r][4] = pack2(x1.x, y1.x); q[r][5] = pack2(x1.y, y1.y); q[r][6] = pack2(x1.z, y1.z); q[r][7] = pack2(x1.w, y1.w);
     }
-    const float inv_div = sqrtf((float)HD);
+    // x / sqrtf(HD), correctly rounded, without a division's branches: by its reciprocal (HD 64: a power of two), for HD 128 by the two-word
+    // reciprocal zh + zl of sqrtf(128) (Brisebarre, Muller, Raina 2004: division by a divisor known in advance; all 2^23 significands
+    // compared with the division). Infinities stay, as zl > 0; below 2^-90 a last place may differ, which no exponential sees.
+    auto scaled = [](float x) { return HD == 64 ? x * 0.125f : fmaf(x, 0x1.6a09e6p-4f, __fmul_rn(x, 0x1.9fcef4p-29f)); };
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
         const int n_t = np > 2 * pass ? ((np - 2 * pass + 3) / 4 + 1) / 2 : 0;         // tiles: of the pass's first w, which has the most pages
@@ -145,16 +149,19 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
             for (int e = 0; e < 8; ++e) acc[r][e] = 0ull;
         float m = kNegBig, l = 0.f;
         if (pass == 1 && n_t > 0) load(1, 0, 0);
-        // One page of the warp's stream. `later`: the page may hold positions behind some row of the warp. Their probability is 0, but 0
-        // times a value that is no number is none: their products are left out.
+        // One page of the warp's stream: one or two chunks of four positions. The products, butterflies and exponentials of two chunks
+        // depend on one another only by the running maximum and fill one another's waits. `later`: the page may hold positions behind some
+        // row of the warp. Their probability is 0, but 0 times a value that is no number is none: their products are left out.
         auto use_page = [&](auto later, const unsigned char* kt, const unsigned char* vt, int cnt) {
-#pragma unroll 1
-            for (int c = 0; c < CPP; ++c) {
-                float s[16];                      // [row][u]
+            auto row_of = [&](int c, int u) { return (c * 4 + u) * NG + grp; };
+            auto valid = [&](int c, int u) { return !decltype(later)::value || row_of(c, u) < cnt; };
+            float s[CPP][16];                     // [chunk][row][u]
+#pragma unroll
+            for (int c = 0; c < CPP; ++c)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     f32x2 kp[8];
-                    unpack(kt + ((c * 4 + u) * NG + grp) * HD * 2, kp);
+                    unpack(kt + row_of(c, u) * HD * 2, kp);
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
                         f32x2 d = 0ull;
@@ -162,51 +169,55 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
                         for (int e = 0; e < 8; ++e) d = fma2(q[r][e], kp[e], d);
                         float x, y;
                         unpack2(d, x, y);
-                        s[r * 4 + u] = x + y;
+                        s[c][r * 4 + u] = x + y;
                     }
                 }
-                {
-                    const bool up = (a & (L / 2)) != 0;
+            const bool up1 = (a & (L / 2)) != 0, up2 = (a & (L / 4)) != 0;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float send = up ? s[j] : s[j + 8], keep = up ? s[j + 8] : s[j];
-                        s[j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 2);
-                    }
-                }
-                {
-                    const bool up = (a & (L / 4)) != 0;
+            for (int c = 0; c < CPP; ++c)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float send = up ? s[j] : s[j + 4], keep = up ? s[j + 4] : s[j];
-                        s[j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 4);
-                    }
+                for (int j = 0; j < 8; ++j) {
+                    const float send = up1 ? s[c][j] : s[c][j + 8], keep = up1 ? s[c][j + 8] : s[c][j];
+                    s[c][j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 2);
                 }
-                if (HD == 128) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], 1);
+            for (int c = 0; c < CPP; ++c)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float send = up2 ? s[c][j] : s[c][j + 4], keep = up2 ? s[c][j + 4] : s[c][j];
+                    s[c][j] = keep + __shfl_xor_sync(0xffffffffu, send, L / 4);
                 }
-                // softmax of the own row
+            if (HD == 128) {
+#pragma unroll
+                for (int c = 0; c < CPP; ++c)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[c][j] += __shfl_xor_sync(0xffffffffu, s[c][j], 1);
+            }
+            // softmax of the own row
+            float sc[CPP];
+#pragma unroll
+            for (int c = 0; c < CPP; ++c) {
                 float mn = m;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const bool valid = !decltype(later)::value || (c * 4 + u) * NG + grp < cnt;
-                    s[u] = valid ? s[u] / inv_div : kNegBig;
-                    mn = fmaxf(mn, s[u]);
+                    s[c][u] = valid(c, u) ? scaled(s[c][u]) : kNegBig;
+                    mn = fmaxf(mn, s[c][u]);
                 }
-                const float sc = expf(m - mn);
+                sc[c] = expf(m - mn);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool valid = !decltype(later)::value || (c * 4 + u) * NG + grp < cnt;
-                    s[u] = valid ? expf(s[u] - mn) : 0.f;
-                }
-                l = __fadd_rn(__fmul_rn(l, sc), s[0]);         // (not one fma: the other kernel's roundings)
-                l = __fadd_rn(__fadd_rn(__fadd_rn(l, s[1]), s[2]), s[3]);
+                for (int u = 0; u < 4; ++u) s[c][u] = valid(c, u) ? expf(s[c][u] - mn) : 0.f;
+                l = __fadd_rn(__fmul_rn(l, sc[c]), s[c][0]);         // (not one fma: the other kernel's roundings)
+                l = __fadd_rn(__fadd_rn(__fadd_rn(l, s[c][1]), s[c][2]), s[c][3]);
                 m = mn;
-                const int src = lane - a;
-                if (__any_sync(0xffffffffu, sc != 1.0f)) {
+            }
+            const int src = lane - a;
+            const bool moved = __any_sync(0xffffffffu, sc[0] != 1.0f || sc[CPP - 1] != 1.0f);
+#pragma unroll
+            for (int c = 0; c < CPP; ++c) {
+                if (moved) {
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
-                        const float x = __shfl_sync(0xffffffffu, sc, src + (HD == 64 ? r : 2 * r));
+                        const float x = __shfl_sync(0xffffffffu, sc[c], src + (HD == 64 ? r : 2 * r));
                         const f32x2 xx = pack2(x, x);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) acc[r][e] = mul2(acc[r][e], xx);
@@ -215,10 +226,10 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     f32x2 vp[8];
-                    unpack(vt + ((c * 4 + u) * NG + grp) * HD * 2, vp);
+                    unpack(vt + row_of(c, u) * HD * 2, vp);
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
-                        const float x = __shfl_sync(0xffffffffu, s[u], src + (HD == 64 ? r : 2 * r));
+                        const float x = __shfl_sync(0xffffffffu, s[c][u], src + (HD == 64 ? r : 2 * r));
                         if (decltype(later)::value && x == 0.f) continue;
                         const f32x2 xx = pack2(x, x);
 #pragma unroll
