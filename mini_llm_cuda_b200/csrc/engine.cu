@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <numeric>
 
 #include "session.h"
 #include "cols_host.h"
@@ -1471,15 +1472,15 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
         s->cols_failed = rc != MLB_E_NOMEM;        // memory may come back: asked for again by the next prompt
         return mode == "chunk" ? rc : (int)MLB_OK;
     }
-    bool has_dn = false;
-    for (int i = 0; i < cfg.layers; ++i) has_dn = has_dn || cfg.layer_types[i] == MLB_LAYER_DELTA_NET;
+    bool has_dn = false, has_attn = false;
+    for (int i = 0; i < cfg.layers; ++i) (cfg.layer_types[i] == MLB_LAYER_DELTA_NET ? has_dn : has_attn) = true;
     const size_t V = (size_t)cfg.vocab;
     const int qt = attn_cols_queries(cfg.heads / cfg.kv_heads);
     size_t scored = 0;
     // A chunk takes the next tokens of as many sequences as it can, an equal share each: the
     // delta-net recurrence is serial along a sequence and parallel across sequences. Columns stay grouped by
     // sequence, positions ascending.
-    std::vector<int> cursor(B, 0);
+    std::vector<int> cursor(B, 0), take(B), order(B);
     long left = total;
     for (int slot = 0; left > 0; slot = (slot + 1) % kPlanSlots) {
         if ((rc = get(left))) return rc;
@@ -1496,30 +1497,51 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
             if (filled(mid) <= want) lo = mid; else hi = mid - 1;
         }
         int extra = want - (int)filled(lo);
+        // A share that ends inside an attention tile leaves the tile's other rows idle (256 sequences: 16 of 32 rows of every tile). It
+        // is rounded up to whole tiles, for as many of the sequences furthest behind as then fit; the others come with the next chunk
+        // (request of 256 prompts of 256 tokens, 8 heads of 64: 104.7 -> 95.5 ms).
+        std::fill(take.begin(), take.end(), 0);
+        bool all = true;
+        for (int b = 0; b < B; ++b) all = all && lens[b] - keep - cursor[b] <= lo;
+        if (has_attn && !f32 && !all && lo > 0 && (lo % qt || extra > 0)) {
+            const int share = (lo + qt - 1) / qt * qt;
+            std::iota(order.begin(), order.end(), 0);
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cursor[x] < cursor[y]; });
+            int room = want;
+            for (const int b : order) {
+                const int most = std::min(lens[b] - keep - cursor[b], share);
+                const int t = most <= room ? most : room / qt * qt;
+                take[b] = t;
+                room -= t;
+            }
+        } else {
+            for (int b = 0; b < B; ++b) {
+                const int rest = lens[b] - keep - cursor[b];
+                take[b] = std::min(rest, lo);
+                if (extra > 0 && take[b] < rest) { ++take[b]; --extra; }
+            }
+        }
         const ColsLayout lay = cols_layout(cfg, s->B, cs->B);
         int* pl = s->plan_host + slot * s->plan_host_ints;
         CU(cudaEventSynchronize(s->plan_free[slot]));      // the slot's last plan has left it, also one of a call that failed half-way
         int n = 0, runs = 0, tiles = 0, longest = 0;
         for (int b = 0; b < B; ++b) {
-            const int rest = lens[b] - keep - cursor[b];
-            int take = std::min(rest, lo);
-            if (extra > 0 && take < rest) { ++take; --extra; }
-            if (take <= 0) continue;
-            longest = std::max(longest, take);
+            if (take[b] <= 0) continue;
+            longest = std::max(longest, take[b]);
             int* r = pl + lay.runs + 4 * (size_t)runs++;
-            r[0] = n; r[1] = take; r[2] = b; r[3] = cursor[b];
-            for (int q = 0; q < take; q += qt) {
+            r[0] = n; r[1] = take[b]; r[2] = b; r[3] = cursor[b];
+            for (int q = 0; q < take[b]; q += qt) {
                 int* t = pl + lay.tiles + 4 * (size_t)tiles++;
-                t[0] = n + q; t[1] = std::min(qt, take - q); t[2] = b; t[3] = cursor[b] + q;
+                t[0] = n + q; t[1] = std::min(qt, take[b] - q); t[2] = b; t[3] = cursor[b] + q;
             }
-            for (int i = 0; i < take; ++i, ++n) {
+            for (int i = 0; i < take[b]; ++i, ++n) {
                 const int t = cursor[b] + i;
                 pl[lay.tok + n] = tokens[(size_t)b * stride + t];
                 pl[lay.pos + n] = t;
                 pl[lay.lim + n] = t + 1;        // active: pos < limit
                 pl[lay.seq + n] = b;
             }
-            cursor[b] += take;
+            cursor[b] += take[b];
         }
         for (int i = n; i < cs->B; ++i) pl[lay.tok + i] = pl[lay.pos + i] = pl[lay.lim + i] = pl[lay.seq + i] = 0;      // idle columns
         pl[0] = n; pl[1] = runs; pl[2] = tiles; pl[3] = 0;

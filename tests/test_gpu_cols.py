@@ -51,9 +51,10 @@ def test_scored_columns_at_tile_edges(api, tmp_path, name):
     model.close()
 
 
-@pytest.mark.parametrize("name,lens", [("mha64", [2100, 1, 2050]), ("dn_odd", [2048, 2049, 3]), ("gqa4_128", [4099]), ("fp8", [65] * 70)])
+@pytest.mark.parametrize("name,lens", [("mha64", [2100, 1, 2050]), ("dn_odd", [2048, 2049, 3]), ("gqa4_128", [4099]), ("fp8", [65] * 70), ("mha64", [70, 33, 101] * 29)])
 def test_prompts_longer_than_one_chunk(api, tmp_path, monkeypatch, name, lens):
-    """More than 4096 prompt tokens: the sequences continue across chunks, in equal shares; many short ones share a chunk."""
+    """More than 4096 prompt tokens: the sequences continue across chunks, in equal shares; many short ones share a chunk, in whole
+    attention tiles (87 sequences: shares of 47 become 64, and the last of them wait for the next chunk)."""
     monkeypatch.setenv("MLB_PREFILL", "chunk")
     spec = dataclasses.replace(SPECS[name], max_context=max(lens) + 8)
     path = write_model(tmp_path, spec, seed=45)
