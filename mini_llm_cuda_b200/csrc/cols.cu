@@ -11,19 +11,32 @@
 namespace mlb {
 
 template <typename... KArgs>
-static cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, KArgs... args) {
+static cudaError_t launch_pdl_cluster(bool pdl, int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, KArgs... args) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... KArgs>
+static cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, KArgs... args) {
+    return launch_pdl_cluster(pdl, 1, kernel, grid, block, smem, st, args...);
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
@@ -715,34 +728,41 @@ cudaError_t embed_cols_launch(bool w8, bool pdl, cudaStream_t st, const StepCtl&
 // ------------------------------------------------------------------------------------------------
 // Projections (gemm_cols.cuh)
 // ------------------------------------------------------------------------------------------------
-template <int MODE, typename KVT, bool SUMS>
+template <int MODE, typename KVT, bool SUMS, bool PAIR>
 static cudaError_t gemm_cols_one(bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w, const CUtensorMap& w2,
                                  const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c, const QkvPostParams& q) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_cols_kernel<MODE, KVT, SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGcSmem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_cols_kernel<MODE, KVT, SUMS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGcSmem);
     if (e != cudaSuccess) return e;
-    const size_t smem = 1024 + (size_t)p.stages * (kGcM + p.BN) * 128;
-    return launch_pdl(pdl, gemm_cols_kernel<MODE, KVT, SUMS>, dim3(ctas), dim3(kGcThreads), smem, st, x, w, w2, xx, wx, p, c, q);
+    if (SUMS) {
+        cudaFuncAttributes a;
+        if ((e = cudaFuncGetAttributes(&a, gemm_cols_kernel<MODE, KVT, SUMS, PAIR>)) != cudaSuccess) return e;
+        if (a.numRegs != kGcRegsLaunch) return cudaErrorInvalidConfiguration;      // its register shares would not add up
+    }
+    const size_t smem = 1024 + (size_t)p.stages * (kGcM + (PAIR ? p.BN / 2 : p.BN)) * 128 + gc_staging(MODE);
+    return launch_pdl_cluster(pdl, PAIR ? 2 : 1, gemm_cols_kernel<MODE, KVT, SUMS, PAIR>, dim3(ctas), dim3(kGcThreads), smem, st, x, w, w2, xx, wx, p, c, q);
 }
 
-template <bool SUMS>
+template <bool SUMS, bool PAIR>
 static cudaError_t gemm_cols_mode(int mode, int kv_dtype, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
                                   const CUtensorMap& w2, const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c,
                                   const QkvPostParams& q) {
     switch (mode) {
-        case TC_RAW: return gemm_cols_one<TC_RAW, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-        case TC_RESID: return gemm_cols_one<TC_RESID, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-        case TC_SWIGLU: return gemm_cols_one<TC_SWIGLU, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+        case TC_RAW: return gemm_cols_one<TC_RAW, float, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+        case TC_RESID: return gemm_cols_one<TC_RESID, float, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+        case TC_SWIGLU: return gemm_cols_one<TC_SWIGLU, float, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
         default:
-            if (kv_dtype == MLB_DT_F32) return gemm_cols_one<TC_QKV, float, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-            return gemm_cols_one<TC_QKV, bf16_t, SUMS>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+            if (kv_dtype == MLB_DT_F32) return gemm_cols_one<TC_QKV, float, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+            return gemm_cols_one<TC_QKV, bf16_t, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
     }
 }
 
-cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
+cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pair, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
                              const CUtensorMap& w2, const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c,
                              const QkvPostParams& q) {
-    if (sums) return gemm_cols_mode<true>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
-    return gemm_cols_mode<false>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+    if (pair) return sums ? gemm_cols_mode<true, true>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q)
+                          : gemm_cols_mode<false, true>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
+    return sums ? gemm_cols_mode<true, false>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q)
+                : gemm_cols_mode<false, false>(mode, kv_dtype, pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
 }
 
 static __global__ void __launch_bounds__(256) widen_e4m3_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n16) {

@@ -59,7 +59,7 @@ cudaError_t embed_cols_launch(bool w8, bool pdl, cudaStream_t st, const StepCtl&
 struct GemmColsParams;
 struct QkvPostParams;
 // `mode` a GemmTcMode; raises the kernel's shared-memory limit on first use.
-cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
+cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pair, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
                              const CUtensorMap& w2, const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c,
                              const QkvPostParams& q);
 // e4m3 codes -> the same values as bf16 (exact), n a multiple of 16

@@ -407,7 +407,7 @@ static int run_cols(mlb_session* s, int kind, int* n_launches) {
         p.y = y; p.h16 = h16; p.ssq_in = normed ? s->tc_ssq : nullptr; p.ssq_parts = parts; p.eps = cfg.rms_eps;
         p.xg16 = s->xn16; p.gain_next = next_gain; p.ssq_out = s->tc_ssq;
         p.s1 = s1; p.s2 = s2; p.err = s->dev_err;
-        CU(gemm_cols_launch(mode, cfg.kv_dtype, g.sums, s->use_pdl, g.ctas, s->stream, X, W, W2, ext ? ext->pleT : X, ext ? ext->pleP : W, p, c, q ? *q : q0));
+        CU(gemm_cols_launch(mode, cfg.kv_dtype, g.sums, g.pair, s->use_pdl, g.ctas, s->stream, X, W, W2, ext ? ext->pleT : X, ext ? ext->pleP : W, p, c, q ? *q : q0));
         ++launches;
         return MLB_OK;
     };
@@ -919,15 +919,16 @@ static int model_widen(mlb_model* m, cudaStream_t st, bool* have) {
 
 // Launch shape of a column GEMM: `T` columns, `N` output features, `nkb` k-blocks of 64, the last `nkb_x` of a second
 // operand pair (`exts_apart`: with accumulators of its own), in `split` ranges. Tensor memory (512 columns) bounds BN x
-// accumulators x buffers. A 128 x BN x 64 k-block takes about 0.30 / 0.19 / 0.14 us at BN = 256 / 128 / 64 (the MMA's own
-// rate at 256, operand reads below), an epilogue 3 us at 256, hidden under the next tile's k-loop where there are two
-// buffers; the cheapest in the sum over a CTA's tiles wins. More ranges than one: sums in registers (64 a thread: BN <= 128) over
-// four accumulators in turn, except under a QK norm, which looks a head's features up in tensor memory.
+// accumulators x buffers. A 128 x BN x 64 k-block takes about 0.43 / 0.36 / 0.26 us at BN = 256 / 128 / 64 with every SM at it: its
+// operand bytes (48 / 32 / 24 KB) at what an SM gets from L2. A pair of CTAs has one of 256 x 256 in 0.42 (32 KB each). An epilogue takes 3 us
+// at 256, hidden under the next tile's k-loop where there are two buffers; the cheapest in the sum over a CTA's tiles wins. More ranges than
+// one: sums in registers (64 a thread, 128 in a pair) over accumulators in turn, except under a QK norm, which looks a head's features up in
+// tensor memory. A pair's two accumulators leave room for one range of a second pair. MLB_COLS_PAIR=0|1: never | wherever it can run.
 static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode, bool exts_apart, int split, int min_bn, bool qk_norm) {
     ColsGemm best{};
     double best_cost = -1.0;
     static const int bns[3] = {256, 128, 64};
-    static const double t_kb[3] = {0.30, 0.19, 0.14};
+    static const double t_kb[3] = {0.43, 0.36, 0.26};
     int mains = 0, exts = 0;
     for (int r = 0; r < split; ++r) {
         const int lo = (int)((long)nkb * r / split), hi = (int)((long)nkb * (r + 1) / split);
@@ -935,28 +936,37 @@ static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode
         if (exts_apart && hi > nkb - nkb_x) ++exts;
     }
     const bool sums = mains + exts > 1 && !(mode == TC_QKV && qk_norm) && exts < kGcMaxBufs;
+    auto consider = [&](int bn, bool pair, int nbuf, double t_kb) {
+        const int bn_out = mode == TC_SWIGLU ? bn / 2 : bn, rows = pair ? 2 * kGcM : kGcM, teams = pair ? sm_count / 2 : sm_count;
+        const long tiles = (long)((T + rows - 1) / rows) * ((N + bn_out - 1) / bn_out);
+        const long waves = (tiles + teams - 1) / teams;
+        const double loop = nkb * t_kb, epi = 3.0 * bn / 256 + 0.5;
+        const double cost = 1.5 + loop + epi + (waves - 1) * (nbuf >= 2 ? std::max(loop, epi) : loop + epi);
+        if (best_cost >= 0 && cost >= best_cost) return;
+        best_cost = cost;
+        const int fit = (int)((kGcSmem - 1024 - gc_staging(mode)) / ((size_t)(kGcM + (pair ? bn / 2 : bn)) * 128));
+        best.bn = bn; best.pair = pair;
+        best.w_rows = mode == TC_SWIGLU || pair ? bn / 2 : bn;
+        best.stages = (int)std::min<long>(std::min(fit, kGcMaxStages), std::max<long>(2, nkb * waves));
+        best.ctas = (int)std::min<long>(tiles, teams) * (pair ? 2 : 1);
+        best.split = split; best.mains = mains; best.exts = exts; best.sums = sums;
+        best.nbuf = nbuf;
+        best.tmem_cols = 32;
+        while (best.tmem_cols < (uint32_t)(bn * nbuf * (sums ? 1 : mains + exts))) best.tmem_cols <<= 1;
+    };
     for (int i = sums ? 1 : 0; i < 3; ++i) {
-        const int bn = bns[i];
-        for (int nbuf = 2; nbuf >= 1; --nbuf) {
-            if (bn < min_bn || (!sums && bn * (mains + exts) * nbuf > 512)) continue;
-            const int bn_out = mode == TC_SWIGLU ? bn / 2 : bn;
-            const long tiles = (long)((T + kGcM - 1) / kGcM) * ((N + bn_out - 1) / bn_out);
-            const long waves = (tiles + sm_count - 1) / sm_count;
-            const double loop = nkb * t_kb[i], epi = 3.0 * bn / 256 + 0.5;
-            const double cost = 1.5 + loop + epi + (waves - 1) * (nbuf == 2 ? std::max(loop, epi) : loop + epi);
-            if (best_cost < 0 || cost < best_cost) {
-                best_cost = cost;
-                const int fit = (int)((kGcSmem - 1024) / ((size_t)(kGcM + bn) * 128));
-                best.bn = bn;
-                best.stages = (int)std::min<long>(std::min(fit, kGcMaxStages), std::max<long>(2, nkb * waves));
-                best.ctas = (int)std::min<long>(tiles, sm_count);
-                best.split = split; best.mains = mains; best.exts = exts; best.sums = sums;
-                best.nbuf = sums ? kGcMaxBufs : nbuf;
-                best.tmem_cols = 32;
-                while (best.tmem_cols < (uint32_t)(bn * (sums ? kGcMaxBufs : (mains + exts) * nbuf))) best.tmem_cols <<= 1;
-            }
-            break;
+        if (bns[i] < min_bn) continue;
+        if (sums) {
+            consider(bns[i], false, kGcMaxBufs, t_kb[i]);
+        } else {
+            const int acc = bns[i] * (mains + exts);
+            if (acc <= 512) consider(bns[i], false, 2 * acc <= 512 ? 2 : 1, t_kb[i]);
         }
+    }
+    const char* env = std::getenv("MLB_COLS_PAIR");
+    if (T >= 2 * kGcM && (sums ? exts < 2 : mains + exts == 1) && !(env && env[0] == '0')) {
+        if (env) best_cost = -1.0;
+        consider(256, true, 2, 0.42);
     }
     return best;
 }
@@ -1013,18 +1023,18 @@ static int setup_cols_path(mlb_session* s) {
         auto& M = s->tc_maps[i];
         const void *wqkv = L.Wqkv, *wo = L.Wo, *w1a = L.W1a, *w1b = L.W1b, *w2 = L.W2;
         if (w8) { const auto& w = m->wide[i]; wqkv = w.Wqkv; wo = w.Wo; w1a = w.W1a; w1b = w.W1b; w2 = w.W2; }
-        const int bn_qkv = L.type == MLB_LAYER_ATTENTION ? s->cg_qkv.bn : s->cg_dn.bn;
-        if ((rc = make_bf16_map(enc, &M.qkv, wqkv, L.n_qkv, c.dim, bn_qkv))) return rc;
-        if ((rc = make_bf16_map(enc, &M.o, wo, c.dim, L.o_in, L.type == MLB_LAYER_ATTENTION ? s->cg_o_attn.bn : s->cg_o_dn.bn))) return rc;
-        if ((rc = make_bf16_map(enc, &M.w1a, w1a, c.ffn_dim, c.dim, s->cg_up.bn / 2))) return rc;
-        if ((rc = make_bf16_map(enc, &M.w1b, w1b, c.ffn_dim, c.dim, s->cg_up.bn / 2))) return rc;
-        if ((rc = make_bf16_map(enc, &M.w2, w2, c.dim, c.ffn_dim, (i + 1 < c.layers && c.ple_dim > 0) ? s->cg_down.bn : s->cg_last.bn))) return rc;
+        const int rows_qkv = L.type == MLB_LAYER_ATTENTION ? s->cg_qkv.w_rows : s->cg_dn.w_rows;
+        if ((rc = make_bf16_map(enc, &M.qkv, wqkv, L.n_qkv, c.dim, rows_qkv))) return rc;
+        if ((rc = make_bf16_map(enc, &M.o, wo, c.dim, L.o_in, L.type == MLB_LAYER_ATTENTION ? s->cg_o_attn.w_rows : s->cg_o_dn.w_rows))) return rc;
+        if ((rc = make_bf16_map(enc, &M.w1a, w1a, c.ffn_dim, c.dim, s->cg_up.w_rows))) return rc;
+        if ((rc = make_bf16_map(enc, &M.w1b, w1b, c.ffn_dim, c.dim, s->cg_up.w_rows))) return rc;
+        if ((rc = make_bf16_map(enc, &M.w2, w2, c.dim, c.ffn_dim, (i + 1 < c.layers && c.ple_dim > 0) ? s->cg_down.w_rows : s->cg_last.w_rows))) return rc;
         if (c.ple_dim > 0) {
-            if ((rc = make_bf16_map(enc, &M.pleP, L.pleP, c.dim, c.ple_dim, s->cg_down.bn))) return rc;
+            if ((rc = make_bf16_map(enc, &M.pleP, L.pleP, c.dim, c.ple_dim, s->cg_down.w_rows))) return rc;
             if ((rc = make_bf16_map(enc, &M.pleT, s->tple16 + (size_t)i * T * c.ple_dim, T, c.ple_dim, kGcM))) return rc;
         }
     }
-    if ((rc = make_bf16_map(enc, &s->tc_g.E, w8 ? m->wide_E : m->E, c.vocab, c.dim, s->cg_head.bn))) return rc;
+    if ((rc = make_bf16_map(enc, &s->tc_g.E, w8 ? m->wide_E : m->E, c.vocab, c.dim, s->cg_head.w_rows))) return rc;
     if ((rc = make_bf16_map(enc, &s->tc_g.xn[0], s->xn16, T, c.dim, kGcM))) return rc;
     if ((rc = make_bf16_map(enc, &s->tc_g.a_attn[0], s->a16, T, nq, kGcM))) return rc;
     if ((rc = make_bf16_map(enc, &s->tc_g.a_dn[0], s->a16, T, a_dn, kGcM))) return rc;

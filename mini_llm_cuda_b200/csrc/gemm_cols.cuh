@@ -8,7 +8,12 @@
 // pieces of its token's row.
 //   warp 0     TMA loader: [128 x 64] activation tile and [BN x 64] weight tile (gate and up halves for SwiGLU) per stage
 //   warp 1     MMA issuer: tcgen05.mma M128 x BN x K16, four per stage, into one of two accumulators
-//   warps 2-9  epilogue of the other accumulator: two warps per TMEM lane quarter, half of the columns each
+//   warps 2, 3 nothing: they complete the warpgroup that gives its registers to the epilogue's
+//   warps 4-11 epilogue of the other accumulator: two warps per TMEM lane quarter, half of the columns each
+// PAIR: two CTAs (the SMs of a TPC) share a tile of 256 columns x 256 features (tcgen05 cta_group::2): each loads its own 128 columns and half of
+// the weight rows, so that a k-block costs an SM 32 KB for 128 x 256 products where a lone CTA loads 32 KB for 128 x 128 or 48 KB for 128 x 256;
+// what an SM gets from L2 (about 100 GB/s with all of them at it) bounds the k-loop. 4096 columns, 2048 features: O 94 -> 61 us, down (K 5632)
+// 177 -> 105, QKV (3072) 88 -> 77, delta-net projections (6176) 142 -> 94 with pairs, the register shares below and staged residuals.
 // One CTA per SM walks tiles of the output; the epilogue of a tile runs under the k-loop of the next one where tensor
 // memory holds the accumulators twice.
 // FP8 weights come as an exact bf16 copy of their codes; their row scales are applied to the accumulator, and the bf16
@@ -18,8 +23,8 @@
 // in another order end, some layers later, in other roundings and now and then in another token. That kernel splits the
 // k-blocks of a tile over the CTAs of a cluster and adds their partial accumulators in order; here the same ranges of
 // k-blocks go to accumulators of their own (`split`), and the sums of squares are taken over 32 features at a time in the
-// order of its warp shuffles. SUMS: the ranges take turns with four accumulators of 128 columns, and the epilogue's threads
-// add each finished one to sums in registers (64 per thread), so the MMAs go on whatever the number of ranges. Holding all
+// order of its warp shuffles. SUMS: the ranges take turns with four accumulators of 128 columns (PAIR: two of 256), and the epilogue's threads
+// add each finished one to sums in registers (64 per thread, 128), so the MMAs go on whatever the number of ranges. Holding all
 // of a tile's accumulators in tensor memory until its epilogue left five of them BN = 64 and no second set: cfg4's O and
 // down projections at 32768 prompt tokens took 75 ms.
 // Every mbarrier wait is bounded; one that runs out records a code and the CTA drains without waiting further.
@@ -30,10 +35,17 @@ namespace mlb {
 
 constexpr int kGcM = 128;
 constexpr int kGcEpiWarps = 8;
-constexpr int kGcThreads = 64 + 32 * kGcEpiWarps;
+constexpr int kGcThreads = 128 + 32 * kGcEpiWarps;
+// Registers of a thread of a kernel with sums (SUMS), at launch (what 384 threads leave each), then of warps 0 - 3 and of the epilogue's:
+// 128 sums and an epilogue's values do not fit 168. The shares add up to what the block was launched with (checked before the launch: a
+// share that the block does not own would be waited for without end).
+constexpr int kGcRegsLaunch = 168, kGcRegsFew = 40, kGcRegsMany = 232;
+static_assert(128 * kGcRegsFew + 32 * kGcEpiWarps * kGcRegsMany <= kGcThreads * kGcRegsLaunch, "register shares");
 constexpr int kGcMaxStages = 8;
 constexpr int kGcMaxBufs = 4;
-constexpr size_t kGcSmem = 224 * 1024;
+constexpr int kGcStgRow = 36;                  // floats from one token's staging row to the next: 16-byte accesses by rows and by columns without conflicts
+constexpr size_t gc_staging(int mode) { return mode == TC_RESID ? (size_t)kGcEpiWarps * 32 * kGcStgRow * 4 : 0; }
+constexpr size_t kGcSmem = 216 * 1024;         // of 227 KB; the factors and barriers take 8.5
 
 struct GemmColsParams {
     int N, K, BN;                  // output features (SWIGLU: of h), width of the main operands, MMA N
@@ -56,11 +68,8 @@ __device__ __forceinline__ void st_f32x8(float* p, const float* v) {
                  "f"(v[5]), "f"(v[6]), "f"(v[7])
                  : "memory");
 }
-__device__ __forceinline__ void ld_f32x8(const float* p, float* v) {
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                 : "l"(p)
-                 : "memory");
+__device__ __forceinline__ void gc_cp_async16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ uint32_t gc_pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -84,7 +93,32 @@ __device__ __forceinline__ void ld_feat16(const float* p, float* v) {
     }
 }
 
-template <int MODE, typename KVT, bool SUMS>
+// ---- two CTAs on one tile (cta_group::2): rank 0 issues the MMAs and owns the barriers of operands and free accumulators -----------
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// arrives on the barrier at this offset in both CTAs
+__device__ __forceinline__ void umma_commit_pair(uint32_t mbar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(mbar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
+template <int MODE, typename KVT, bool SUMS, bool PAIR>
 __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                                                                   const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmXx,
                                                                   const __grid_constant__ CUtensorMap tmWx, const __grid_constant__ GemmColsParams p,
@@ -92,16 +126,20 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
     extern __shared__ unsigned char smem_raw[];
     const int n_cols = *c.n_cols;                                  // in place before the step's first kernel starts
     const int bn_out = MODE == TC_SWIGLU ? p.BN / 2 : p.BN;
-    const int n_m = (n_cols + kGcM - 1) / kGcM, n_n = (p.N + bn_out - 1) / bn_out;
+    constexpr int TM = PAIR ? 2 * kGcM : kGcM;                     // columns of a tile
+    const int rank = PAIR ? (int)cluster_rank() : 0, team = PAIR ? blockIdx.x / 2 : blockIdx.x, n_teams = PAIR ? gridDim.x / 2 : gridDim.x;
+    const int n_m = (n_cols + TM - 1) / TM, n_n = (p.N + bn_out - 1) / bn_out;
     const int n_tiles = n_m * n_n;
-    if ((int)blockIdx.x >= n_tiles) return;
+    if (team >= n_tiles) return;                                   // (the CTAs of a pair alike)
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2 * kGcMaxStages + 2 * kGcMaxBufs];
     __shared__ uint32_t tmem_slot;
+    __shared__ float feat[kGcEpiWarps][2][128];                    // per-feature factors of a warp's part of the tile
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8u * kGcMaxStages;
     const uint32_t tfull0 = empty0 + 8u * kGcMaxStages, tempty0 = tfull0 + 8u * kGcMaxBufs;
-    const int a_bytes = kGcM * 128, stage_bytes = a_bytes + p.BN * 128;
+    const int b_rows = PAIR ? p.BN / 2 : p.BN;                      // of the weight tile, in this CTA
+    const int a_bytes = kGcM * 128, stage_bytes = a_bytes + b_rows * 128;
     const int nkb1 = (p.K + kTcKB - 1) / kTcKB, nkb = nkb1 + p.nkb_x;
     const uint32_t acc_cols = (uint32_t)((SUMS ? 1 : p.mains + p.exts) * p.BN);
     if (tid == 0) {
@@ -111,123 +149,179 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
         }
         for (int i = 0; i < kGcMaxBufs; ++i) {
             mbar_init(tfull0 + 8u * i, 1);
-            mbar_init(tempty0 + 8u * i, kGcEpiWarps);
+            mbar_init(tempty0 + 8u * i, PAIR ? 2 * kGcEpiWarps : kGcEpiWarps);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(p.tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(p.tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(p.tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync_all();                                  // the other CTA's barriers are set up
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     pdl_launch_dependents();
 
-    if (warp == 0) {
-        if (lane == 0) {
-            auto load_w = [&](int kb, int n0, uint32_t base, uint32_t bar) {
-                if (kb < nkb1) {
-                    tma_load_2d(base + a_bytes, &tmW, kb * kTcKB, n0, bar);
-                    if (MODE == TC_SWIGLU) tma_load_2d(base + a_bytes + bn_out * 128, &tmW2, kb * kTcKB, n0, bar);
-                } else {
-                    tma_load_2d(base + a_bytes, &tmWx, (kb - nkb1) * kTcKB, n0, bar);
-                }
-            };
-            auto load_x = [&](int kb, int m0, uint32_t base, uint32_t bar) {
-                if (kb < nkb1) tma_load_2d(base, &tmX, kb * kTcKB, m0, bar);
-                else tma_load_2d(base, &tmXx, (kb - nkb1) * kTcKB, m0, bar);
-            };
-            const uint32_t ring = smem_u32(smem);
-            // the first tile's first weight tiles depend on nothing: on their way before the predecessor is waited for
-            const int first = blockIdx.x;
-            const int pre = min(p.stages, nkb);
-            for (int kb = 0; kb < pre; ++kb) {
-                mbar_expect_tx(full0 + 8u * kb, (uint32_t)stage_bytes);
-                load_w(kb, first / n_m * bn_out, ring + (uint32_t)(kb * stage_bytes), full0 + 8u * kb);
-            }
-            pdl_wait();
-            int s = 0;
-            uint32_t ph = 1;
-            bool ok = true;
-            for (int t = first; t < n_tiles && ok; t += gridDim.x) {
-                const int m0 = t % n_m * kGcM, n0 = t / n_m * bn_out;
-                for (int kb = 0; kb < nkb; ++kb) {
-                    const uint32_t bar = full0 + 8u * s, base = ring + (uint32_t)(s * stage_bytes);
-                    if (t != first || kb >= pre) {
-                        if (!tc_wait(empty0 + 8u * s, ph, p.err, 21)) { ok = false; break; }
-                        mbar_expect_tx(bar, (uint32_t)stage_bytes);
-                        load_w(kb, n0, base, bar);
-                    }
-                    load_x(kb, m0, base, bar);
-                    if (++s == p.stages) { s = 0; ph ^= 1u; }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16(kGcM, p.BN);
-            const uint32_t ring = smem_u32(smem);
-            int s = 0, i = 0, buf = 0, use = 0;        // use: how often this buffer has been filled before
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++i) {
-                if (!SUMS) {
-                    if (i >= p.nbuf && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
-                    tc_fence_after();
-                }
-                const uint32_t acc = tmem + buf * acc_cols;
-                int r = 0, hi = nkb / p.split;           // range of k-blocks: [nkb r / split, nkb (r + 1) / split)
-                bool fresh = true, xfresh = true;        // the next MMA starts its accumulator
-                for (int kb = 0; kb < nkb; ++kb) {
-                    while (kb >= hi) {
-                        ++r;
-                        hi = (int)((long)nkb * (r + 1) / p.split);
-                        fresh = xfresh = true;
-                    }
-                    if (!tc_wait(full0 + 8u * s, ph, p.err, 23)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t base = ring + (uint32_t)(s * stage_bytes);
-                    const uint64_t ad = umma_desc_sw128(base), bd = umma_desc_sw128(base + a_bytes);
-                    const bool ext = p.exts > 0 && kb >= nkb1;
-                    if (SUMS && (ext ? xfresh : fresh)) {
-                        // the next accumulator in turn; the one before it is complete
-                        if (kb > 0) {
-                            umma_commit(tfull0 + 8u * buf);
-                            if (++buf == p.nbuf) { buf = 0; ++use; }
+    if (warp < 4) {
+        if (SUMS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kGcRegsFew));
+        if (warp == 0) {
+            if (lane == 0) {
+                // of a pair, rank r loads columns 128 r .. of the tile and weight rows BN / 2 r .. (SWIGLU: gate | up); all bytes of a
+                // stage count on rank 0's barrier, which rank 0 arms for both
+                const uint32_t bytes = (uint32_t)(PAIR ? 2 * stage_bytes : stage_bytes);
+                const uint32_t lfull0 = PAIR ? cluster_map(full0, 0) : full0;
+                auto tma = [&](uint32_t dst, const CUtensorMap* map, int k, int row, uint32_t bar) {
+                    if (PAIR) tma_load_2d_pair(dst, map, k, row, bar);
+                    else tma_load_2d(dst, map, k, row, bar);
+                };
+                auto load_w = [&](int kb, int n0, uint32_t base, uint32_t bar) {
+                    if (kb < nkb1) {
+                        if (PAIR && MODE == TC_SWIGLU) {
+                            tma(base + a_bytes, rank ? &tmW2 : &tmW, kb * kTcKB, n0, bar);
+                        } else {
+                            tma(base + a_bytes, &tmW, kb * kTcKB, n0 + rank * b_rows, bar);
+                            if (MODE == TC_SWIGLU) tma(base + a_bytes + bn_out * 128, &tmW2, kb * kTcKB, n0, bar);
                         }
-                        if (use > 0 && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
+                    } else {
+                        tma(base + a_bytes, &tmWx, (kb - nkb1) * kTcKB, n0 + rank * b_rows, bar);
+                    }
+                };
+                auto load_x = [&](int kb, int m0, uint32_t base, uint32_t bar) {
+                    if (kb < nkb1) tma(base, &tmX, kb * kTcKB, m0, bar);
+                    else tma(base, &tmXx, (kb - nkb1) * kTcKB, m0, bar);
+                };
+                auto arm = [&](int st) { if (rank == 0) mbar_expect_tx(full0 + 8u * st, bytes); };
+                const uint32_t ring = smem_u32(smem);
+                // the first tile's first weight tiles depend on nothing: on their way before the predecessor is waited for
+                const int first = team;
+                const int pre = min(p.stages, nkb);
+                for (int kb = 0; kb < pre; ++kb) {
+                    arm(kb);
+                    load_w(kb, first / n_m * bn_out, ring + (uint32_t)(kb * stage_bytes), lfull0 + 8u * kb);
+                }
+                pdl_wait();
+                int s = 0;
+                uint32_t ph = 1;
+                bool ok = true;
+                for (int t = first; t < n_tiles && ok; t += n_teams) {
+                    const int m0 = t % n_m * TM + rank * kGcM, n0 = t / n_m * bn_out;
+                    for (int kb = 0; kb < nkb; ++kb) {
+                        const uint32_t bar = lfull0 + 8u * s, base = ring + (uint32_t)(s * stage_bytes);
+                        if (t != first || kb >= pre) {
+                            if (!tc_wait(empty0 + 8u * s, ph, p.err, 21)) { ok = false; break; }
+                            arm(s);
+                            load_w(kb, n0, base, bar);
+                        }
+                        load_x(kb, m0, base, bar);
+                        if (++s == p.stages) { s = 0; ph ^= 1u; }
+                    }
+                }
+            }
+        } else if (warp == 1) {
+            if (lane == 0 && rank == 0) {
+                auto commit = [](uint32_t bar) {
+                    if (PAIR) umma_commit_pair(bar);
+                    else umma_commit(bar);
+                };
+                const uint32_t idesc = umma_idesc_bf16(TM, p.BN);
+                const uint32_t ring = smem_u32(smem);
+                int s = 0, i = 0, buf = 0, use = 0;        // use: how often this buffer has been filled before
+                uint32_t ph = 0;
+                bool ok = true;
+                for (int t = team; t < n_tiles && ok; t += n_teams, ++i) {
+                    if (!SUMS) {
+                        if (i >= p.nbuf && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
                         tc_fence_after();
                     }
-                    // the separate accumulators of the second pair lie behind the main ones, its ranges are the last ones
-                    const uint32_t dst = SUMS ? tmem + (uint32_t)(buf * p.BN) : acc + (uint32_t)((ext ? p.mains + r - (p.split - p.exts) : r) * p.BN);
-                    const bool first = ext ? xfresh : fresh;
+                    const uint32_t acc = tmem + buf * acc_cols;
+                    int r = 0, hi = nkb / p.split;           // range of k-blocks: [nkb r / split, nkb (r + 1) / split)
+                    bool fresh = true, xfresh = true;        // the next MMA starts its accumulator
+                    for (int kb = 0; kb < nkb; ++kb) {
+                        while (kb >= hi) {
+                            ++r;
+                            hi = (int)((long)nkb * (r + 1) / p.split);
+                            fresh = xfresh = true;
+                        }
+                        if (!tc_wait(full0 + 8u * s, ph, p.err, 23)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t base = ring + (uint32_t)(s * stage_bytes);
+                        const uint64_t ad = umma_desc_sw128(base), bd = umma_desc_sw128(base + a_bytes);
+                        const bool ext = p.exts > 0 && kb >= nkb1;
+                        if (SUMS && (ext ? xfresh : fresh)) {
+                            // the next accumulator in turn; the one before it is complete
+                            if (kb > 0) {
+                                commit(tfull0 + 8u * buf);
+                                if (++buf == p.nbuf) { buf = 0; ++use; }
+                            }
+                            if (use > 0 && !tc_wait(tempty0 + 8u * buf, (uint32_t)(use - 1) & 1u, p.err, 22)) { ok = false; break; }
+                            tc_fence_after();
+                        }
+                        // the separate accumulators of the second pair lie behind the main ones, its ranges are the last ones
+                        const uint32_t dst = SUMS ? tmem + (uint32_t)(buf * p.BN) : acc + (uint32_t)((ext ? p.mains + r - (p.split - p.exts) : r) * p.BN);
+                        const bool first = ext ? xfresh : fresh;
 #pragma unroll
-                    for (int j = 0; j < kTcKB / 16; ++j) umma_bf16(dst, ad + 2u * j, bd + 2u * j, idesc, (first && j == 0) ? 0u : 1u);
-                    if (ext) xfresh = false; else fresh = false;
-                    umma_commit(empty0 + 8u * s);
-                    if (++s == p.stages) { s = 0; ph ^= 1u; }
+                        for (int j = 0; j < kTcKB / 16; ++j) {
+                            if (PAIR) umma_bf16_pair(dst, ad + 2u * j, bd + 2u * j, idesc, (first && j == 0) ? 0u : 1u);
+                            else umma_bf16(dst, ad + 2u * j, bd + 2u * j, idesc, (first && j == 0) ? 0u : 1u);
+                        }
+                        if (ext) xfresh = false; else fresh = false;
+                        commit(empty0 + 8u * s);
+                        if (++s == p.stages) { s = 0; ph ^= 1u; }
+                    }
+                    commit(tfull0 + 8u * buf);      // also after a wait that ran out: the epilogue must not hang on it
+                    if (++buf == p.nbuf) { buf = 0; ++use; }
                 }
-                umma_commit(tfull0 + 8u * buf);      // also after a wait that ran out: the epilogue must not hang on it
-                if (++buf == p.nbuf) { buf = 0; ++use; }
             }
         }
     } else {
+        if (SUMS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kGcRegsMany));
         // ---- epilogue: one token per thread, half of the tile's columns per warp ---------------------------------
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int quarter = warp & 3, half = (warp - 4) >> 2;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        const int span = bn_out / 2;                  // features of this thread per tile, in chunks of 16
+        // features of this thread per tile, in chunks of 16 (a pair's tile has BN = 256)
+        const int span = !PAIR ? bn_out / 2 : (MODE == TC_SWIGLU ? 64 : 128);
+        // a pair's sums leave registers for the rest only if those of finished chunks are given up: no rolled loop there
+        constexpr int UNROLL = PAIR && SUMS && MODE == TC_RESID ? 4 : 1;
         pdl_wait();
         int buf = 0, use = 0;
         bool ok = true;
         // (tcgen05.ld is a warp-wide instruction: the lanes go on or give up together)
+        // an accumulator is free once the warps of both CTAs have read it
+        const uint32_t lempty0 = PAIR ? cluster_map(tempty0, 0) : tempty0;
+        auto release = [&](int b) {
+            if (lane != 0) return;
+            if (PAIR) mbar_arrive_cluster(lempty0 + 8u * b);
+            else mbar_arrive(tempty0 + 8u * b);
+        };
+        float (&fw)[2][128] = feat[warp - 4];
+        // RESID: staging rows of the warp, [32 tokens][32 features]. A thread computes its token's features; the residual stream, which is read and
+        // written, crosses four tokens at a time, eight lanes to 32 consecutive features, and without a register (sums and 16 prefetched
+        // residual values spilled: O / down projections of 4096 columns, 2048 features: 75 / 119 us with the spills, 67 / 109 with a lane per
+        // token and no prefetch, 61 / 105 staged. The other modes only write, and lose: QKV 77 -> 88 - 99 us.)
+        float* stg = reinterpret_cast<float*>(smem + (size_t)p.stages * stage_bytes) + (warp - 4) * 32 * kGcStgRow;
+        const int piece = lane & 7, trow = lane >> 3;
         auto arrived = [&](int b, int u) { return (bool)__all_sync(0xffffffffu, tc_wait(tfull0 + 8u * b, (uint32_t)u & 1u, p.err, 24)); };
-        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-            const int m0 = t % n_m * kGcM, n0 = t / n_m * bn_out;
-            const int tok = m0 + quarter * 32 + lane;
+        for (int t = team; t < n_tiles && ok; t += n_teams) {
+            const int m0 = t % n_m * TM + rank * kGcM, n0 = t / n_m * bn_out;
+            const int tok0 = m0 + quarter * 32, tok = tok0 + lane;
             const bool live = tok < n_cols;
             const int f_begin = n0 + half * span;
+            // the warp's per-feature factors, asked for before the accumulator is waited for: row scales; gains, or scales of the second matrix
+            float ff[2][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int f = min(f_begin + lane + 32 * i, p.N - 1);
+                ff[0][i] = p.s1 != nullptr ? __ldg(p.s1 + f) : 1.0f;
+                if (MODE == TC_RESID) ff[1][i] = __ldg(p.gain_next + f);
+                if (MODE == TC_SWIGLU) ff[1][i] = p.s2 != nullptr ? __ldg(p.s2 + f) : 1.0f;
+            }
             float rinv = 1.0f;
             if (p.ssq_in != nullptr && live) {
                 float tot = 0.f;
@@ -245,18 +339,28 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                 const int page = q.page_table[kv_seq(c, tok) * q.pt_stride + pos / kKvBlock];
                 kv_row = (size_t)page * q.kv_heads * kKvBlock + (pos % kKvBlock);
             }
-            float rnext[16];
-            auto load_resid = [&](int f0) {
-                if (live && f0 < p.N) {               // N is a multiple of 8, chunks end inside it only at 8
-                    const float* r = p.y + (size_t)tok * p.N + f0;
-                    ld_f32x8(r, rnext);
-                    if (f0 + 8 < p.N) ld_f32x8(r + 8, rnext + 8);
+            // residual values of 32 features into the warp's staging rows
+            auto fetch_resid = [&](int fg) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int row = trow + 4 * i, f = fg + 4 * piece;
+                    const bool in = tok0 + row < n_cols && f < p.N;
+                    gc_cp_async16(smem_u32(stg + row * kGcStgRow + 4 * piece), in ? p.y + (size_t)(tok0 + row) * p.N + f : p.y, in);
                 }
+                asm volatile("cp.async.commit_group;" ::: "memory");
             };
-            if (MODE == TC_RESID) load_resid(f_begin);
+            if (MODE == TC_RESID) fetch_resid(f_begin);
+            __syncwarp();                             // the last tile's factors have been read
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                fw[0][lane + 32 * i] = ff[0][i];
+                if (MODE == TC_RESID || MODE == TC_SWIGLU) fw[1][lane + 32 * i] = ff[1][i];
+            }
+            __syncwarp();
             // SUMS: the ranges' accumulators arrive one after another and are added up here, in their order, each given back at once.
-            // 64 sums per thread: BN = 128 (SWIGLU: 32 of gate, 32 of up)
-            float sums[SUMS ? 64 : 1];
+            // A sum per thread for half of the tile's BN <= 16 CH features (SWIGLU: the first half of them of gate, the second of up)
+            constexpr int CH = PAIR ? 8 : 4;
+            float sums[SUMS ? 16 * CH : 1];
             if (SUMS) {
                 for (int r = 0; r < p.mains && ok; ++r) {
                     ok = arrived(buf, use);
@@ -264,13 +368,12 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                     tc_fence_after();
                     const uint32_t a = tmem + (uint32_t)(buf * p.BN) + lane_base;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
+                    for (int h = 0; h < CH / 2; ++h) {
                         uint32_t ta[2][16];
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
-                            const int ch = 2 * h + k;
-                            const bool here = MODE == TC_SWIGLU ? 16 * k < span : 16 * ch < span;
-                            if (here) tmem_ld16_issue(a + (uint32_t)(MODE == TC_SWIGLU ? h * bn_out + half * span + 16 * k : half * span + 16 * ch), ta[k]);
+                            const int ch = MODE == TC_SWIGLU ? (2 * h + k) % (CH / 2) : 2 * h + k, up = MODE == TC_SWIGLU ? (2 * h + k) / (CH / 2) : 0;
+                            if (16 * ch < span) tmem_ld16_issue(a + (uint32_t)(up * bn_out + half * span + 16 * ch), ta[k]);
                         }
                         tmem_ld_wait();
 #pragma unroll
@@ -283,7 +386,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                     }
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(tempty0 + 8u * buf);
+                    release(buf);
                     if (++buf == p.nbuf) { buf = 0; ++use; }
                 }
                 // accumulators of the second pair stay where they are until the element-wise work below has read them
@@ -331,172 +434,107 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                     for (int j = 0; j < w; ++j) t[j] += t[j + w];
                 return t[0];
             };
-#pragma unroll 1
-            for (int cc = 0; cc < span; cc += 16) {
-                const int f0 = f_begin + cc, col = half * span + cc;
-                if (f0 >= p.N) {                       // uniform for the warp; the sums of squares behind the last feature are zero
-                    if (MODE == TC_RESID) {
-                        if ((f0 & 16) && live) {
-                            float z[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) z[j] = 0.f;
-                            p.ssq_out[(size_t)tok * p.ssq_parts + f0 / 32] = sum32(sqp, z);
-                        }
-                        if (live)
-                            for (int g = (f0 + 16) / 32; g < (f_begin + span) / 32 && g < p.ssq_parts; ++g) p.ssq_out[(size_t)tok * p.ssq_parts + g] = 0.f;
-                    }
+#pragma unroll UNROLL
+            for (int cg = 0; cg < span; cg += 32) {
+                const int fg = f_begin + cg;
+                if (fg >= p.N) {                       // uniform for the warp; the sums of squares behind the last feature are zero
+                    if (MODE == TC_RESID && live)
+                        for (int g = fg / 32; g < (f_begin + span) / 32 && g < p.ssq_parts; ++g) p.ssq_out[(size_t)tok * p.ssq_parts + g] = 0.f;
                     break;
                 }
-                const bool whole = f0 + 16 <= p.N;
-                __syncwarp();                          // tcgen05.ld is a warp-wide instruction
-                float v[16], w2[16];
-                if constexpr (SUMS) {
-                    // the front 16 of the sums; the others move up, so that a rolled loop names registers
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        v[j] = sums[j];
-                        sums[j] = sums[16 + j];
-                        if (MODE == TC_SWIGLU) {
-                            w2[j] = sums[32 + j];
-                            sums[32 + j] = sums[48 + j];
-                        } else {
-                            sums[16 + j] = sums[32 + j];
-                            sums[32 + j] = sums[48 + j];
-                        }
-                    }
-                    if (MODE == TC_RESID && p.exts > 0) {
-                        load_acc(acc + (uint32_t)col, 1, w2);
-                        for (int r = 1, b = buf; r < p.exts; ++r) {
-                            if (++b == p.nbuf) b = 0;
-                            float e[16];
-                            load_acc(tmem + (uint32_t)(b * p.BN + col) + lane_base, 1, e);
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) w2[j] = __fadd_rn(w2[j], e[j]);
-                        }
-                    }
-                } else {
-                    load_acc(acc + (uint32_t)col, p.mains, v);
-                    if (MODE == TC_SWIGLU) load_acc(acc + (uint32_t)(bn_out + col), p.mains, w2);
-                    if (MODE == TC_RESID && p.exts > 0) load_acc(acc + (uint32_t)(p.mains * p.BN + col), p.exts, w2);
+                // q | k | v | gate: whole heads of 64 or 128 features each
+                const int seg_k = q.nq, seg_v = q.nq + q.nk, seg_g = seg_v + q.nv;
+                const int seg = MODE != TC_QKV ? 0 : (fg < seg_k ? 0 : (fg < seg_v ? 1 : (fg < seg_g ? 2 : 3)));
+                const int fs = fg - (seg == 0 ? 0 : (seg == 1 ? seg_k : (seg == 2 ? seg_v : seg_g)));     // feature inside its segment
+                const int e0 = MODE == TC_QKV ? fs % q.hd : 0, head = MODE == TC_QKV ? fs / q.hd : 0;
+                if (MODE == TC_RESID) {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                    __syncwarp();
                 }
-                if (MODE == TC_SWIGLU) {
-                    float sa[16], sb[16];
-                    if (p.s1 != nullptr && whole) {
-                        ld_feat16(p.s1 + f0, sa);
-                        ld_feat16(p.s2 + f0, sb);
-                    } else {
+                // ---- a thread's token: two chunks of 16 features -> memory, or (RESID) staging row
+                float4* own = reinterpret_cast<float4*>(stg + lane * kGcStgRow);
+#pragma unroll (UNROLL > 1 ? 2 : 1)
+                for (int h = 0; h < 2; ++h) {
+                    const int cc = cg + 16 * h, f0 = f_begin + cc, col = half * span + cc;
+                    if (cc >= span || (MODE != TC_RESID && f0 >= p.N)) break;             // (a group of 16: SWIGLU with BN = 64)
+                    const bool whole = f0 + 16 <= p.N;
+                    __syncwarp();                      // tcgen05.ld is a warp-wide instruction
+                    float v[16], w2[16];
+                    if constexpr (SUMS) {
+                        // the front 16 of the sums; the others move up, so that a rolled loop names registers
+                        constexpr int HALF = MODE == TC_SWIGLU ? CH / 2 : CH;
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
-                            const int f = min(f0 + j, p.N - 1);
-                            sa[j] = p.s1 != nullptr ? __ldg(p.s1 + f) : 1.0f;
-                            sb[j] = p.s2 != nullptr ? __ldg(p.s2 + f) : 1.0f;
-                        }
-                    }
+                            v[j] = sums[UNROLL > 1 ? cc + j : j];
+                            if (MODE == TC_SWIGLU) w2[j] = sums[16 * (CH / 2) + j];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float g = v[j] * sa[j] * rinv, u = w2[j] * sb[j] * rinv;
-                        v[j] = __fdividef(g, 1.0f + __expf(-g)) * u;            // inference.cu:262-281
+                            for (int g = 0; g < (UNROLL > 1 ? 0 : CH - 1); ++g)
+                                if (g != HALF - 1) sums[16 * g + j] = sums[16 * (g + 1) + j];
+                        }
+                        if (MODE == TC_RESID && p.exts > 0) {
+                            load_acc(acc + (uint32_t)col, 1, w2);
+                            for (int r = 1, b = buf; !PAIR && r < p.exts; ++r) {          // (a pair's two accumulators leave room for one)
+                                if (++b == p.nbuf) b = 0;
+                                float e[16];
+                                load_acc(tmem + (uint32_t)(b * p.BN + col) + lane_base, 1, e);
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) w2[j] = __fadd_rn(w2[j], e[j]);
+                            }
+                        }
+                    } else {
+                        load_acc(acc + (uint32_t)col, p.mains, v);
+                        if (MODE == TC_SWIGLU) load_acc(acc + (uint32_t)(bn_out + col), p.mains, w2);
+                        if (MODE == TC_RESID && p.exts > 0) load_acc(acc + (uint32_t)(p.mains * p.BN + col), p.exts, w2);
                     }
-                    if (live) {
-                        bf16_t* o = p.h16 + (size_t)tok * p.N + f0;
-                        if (whole) {
-                            st_bf16x16(o, v);
+                    if (MODE == TC_SWIGLU) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const float g = v[j] * fw[0][cc + j] * rinv, u = w2[j] * fw[1][cc + j] * rinv;
+                            v[j] = __fdividef(g, 1.0f + __expf(-g)) * u;            // inference.cu:262-281
+                        }
+                    } else if (MODE == TC_RESID) {
+                        // (roundings as in gemm_tc_kernel: scale and second pair in one fma, then the residual)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 r = own[4 * h + i];
+                            const float rr[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                const int j = 4 * i + k;
+                                if (p.s1 != nullptr) v[j] = fmaf(v[j], fw[0][cc + j], p.exts > 0 ? w2[j] : 0.f);
+                                v[j] = __fadd_rn(v[j], rr[k]);                      // inference.cu:252-260, :283-291
+                            }
+                        }
+                        float sq[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sq[j] = (whole || f0 + j < p.N) ? __fmul_rn(v[j], v[j]) : 0.f;
+                        if (h == 1) {
+                            if (live) p.ssq_out[(size_t)tok * p.ssq_parts + f0 / 32] = sum32(sqp, sq);
                         } else {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (f0 + j < p.N) o[j] = __float2bfloat16_rn(v[j]);
+                            for (int j = 0; j < 16; ++j) sqp[j] = sq[j];
                         }
-                    }
-                    continue;
-                }
-                float sa[16];
-                if (p.s1 != nullptr) {
-                    if (whole) {
-                        ld_feat16(p.s1 + f0, sa);
                     } else {
+                        if (p.s1 != nullptr) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) sa[j] = __ldg(p.s1 + min(f0 + j, p.N - 1));
-                    }
-                    if (MODE != TC_RESID) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] *= sa[j];
-                    }
-                }
-                if (MODE == TC_RAW) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] *= rinv;
-                    if (live) {
-                        float* o = p.y + (size_t)tok * p.N + f0;
-                        if (whole && (p.N & 7) == 0) {
-                            put16(o, v);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (f0 + j < p.N) o[j] = v[j];
+                            for (int j = 0; j < 16; ++j) v[j] *= fw[0][cc + j];
                         }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] *= rinv;
                     }
-                } else if (MODE == TC_RESID) {
-                    float r[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) r[j] = rnext[j];
-                    if (cc + 16 < span) load_resid(f0 + 16);
-                    // (roundings as in gemm_tc_kernel: scale and second pair in one fma, then the residual)
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if (p.s1 != nullptr) v[j] = fmaf(v[j], sa[j], p.exts > 0 ? w2[j] : 0.f);
-                        v[j] = __fadd_rn(v[j], r[j]);                           // inference.cu:252-260, :283-291
-                    }
-                    if (live) {
-                        float g[16];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            // N is a multiple of 8: a chunk ends inside the matrix after 8 or 16 features
-                            const float4 t4 = (whole || j < 2) ? __ldg(reinterpret_cast<const float4*>(p.gain_next + f0) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                            g[4 * j] = t4.x; g[4 * j + 1] = t4.y; g[4 * j + 2] = t4.z; g[4 * j + 3] = t4.w;
-                        }
-                        float* o = p.y + (size_t)tok * p.N + f0;
-                        bf16_t* ox = p.xg16 + (size_t)tok * p.N + f0;
-                        st_f32x8(o, v);
-                        uint4 a;
-                        a.x = gc_pack(v[0] * g[0], v[1] * g[1]); a.y = gc_pack(v[2] * g[2], v[3] * g[3]);
-                        a.z = gc_pack(v[4] * g[4], v[5] * g[5]); a.w = gc_pack(v[6] * g[6], v[7] * g[7]);
-                        reinterpret_cast<uint4*>(ox)[0] = a;
-                        if (whole) {
-                            st_f32x8(o + 8, v + 8);
-                            a.x = gc_pack(v[8] * g[8], v[9] * g[9]); a.y = gc_pack(v[10] * g[10], v[11] * g[11]);
-                            a.z = gc_pack(v[12] * g[12], v[13] * g[13]); a.w = gc_pack(v[14] * g[14], v[15] * g[15]);
-                            reinterpret_cast<uint4*>(ox)[1] = a;
-                        }
-                    }
-                    float sq[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) sq[j] = (whole || j < 8) ? __fmul_rn(v[j], v[j]) : 0.f;
-                    if (f0 & 16) {
-                        if (live) p.ssq_out[(size_t)tok * p.ssq_parts + f0 / 32] = sum32(sqp, sq);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) sqp[j] = sq[j];
-                    }
-                } else {
-                    // q | k | v | gate: whole heads of 64 or 128 features each
-                    const int seg_k = q.nq, seg_v = q.nq + q.nk, seg_g = seg_v + q.nv;
-                    const int seg = f0 < seg_k ? 0 : (f0 < seg_v ? 1 : (f0 < seg_g ? 2 : 3));
-                    const int fs = f0 - (seg == 0 ? 0 : (seg == 1 ? seg_k : (seg == 2 ? seg_v : seg_g)));     // feature inside its segment
-                    const int e0 = fs % q.hd, head = fs / q.hd;
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] *= rinv;
-                    if (!SUMS && seg < 2 && q.qk_norm) {
+                    if (MODE == TC_QKV && !SUMS && seg < 2 && q.qk_norm) {
                         // per-head RMS norm (inference.cu:52-81, :97-111): the head's other features come from tensor memory
-                        if (e0 == 0 || cc == 0) {
+                        const int e1 = e0 + 16 * h;
+                        if (e1 == 0 || cc == 0) {
                             float ss = 0.f;
                             for (int e = 0; e < q.hd; e += 32) {
                                 float x[2][16];
 #pragma unroll
                                 for (int b = 0; b < 2; ++b) {
-                                    load_acc(acc + (uint32_t)(col - e0 + e + 16 * b), p.mains, x[b]);
+                                    load_acc(acc + (uint32_t)(col - e1 + e + 16 * b), p.mains, x[b]);
 #pragma unroll
                                     for (int j = 0; j < 16; ++j) {
-                                        if (p.s1 != nullptr) x[b][j] *= __ldg(p.s1 + f0 - e0 + e + 16 * b + j);
+                                        if (p.s1 != nullptr) x[b][j] *= __ldg(p.s1 + f0 - e1 + e + 16 * b + j);
                                         x[b][j] *= rinv;
                                         x[b][j] = __fmul_rn(x[b][j], x[b][j]);
                                     }
@@ -506,16 +544,41 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                             head_sc = rsqrtf(ss * (1.0f / (float)q.hd) + q.eps);
                         }
                         float g[16];
-                        ld_feat16((seg == 0 ? q.gq : q.gk) + fs, g);
+                        ld_feat16((seg == 0 ? q.gq : q.gk) + fs + 16 * h, g);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] *= head_sc * g[j];
                     }
-                    if (live) {
+                    if (MODE == TC_RESID) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) own[4 * h + i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    } else if (MODE == TC_SWIGLU) {
+                        if (live) {
+                            bf16_t* o = p.h16 + (size_t)tok * p.N + f0;
+                            if (whole) {
+                                st_bf16x16(o, v);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    if (f0 + j < p.N) o[j] = __float2bfloat16_rn(v[j]);
+                            }
+                        }
+                    } else if (MODE == TC_RAW) {
+                        if (live) {
+                            float* o = p.y + (size_t)tok * p.N + f0;
+                            if (whole && (p.N & 7) == 0) {
+                                put16(o, v);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    if (f0 + j < p.N) o[j] = v[j];
+                            }
+                        }
+                    } else if (live) {
+                        const int e1 = e0 + 16 * h;
                         if (seg < 2) {
                             // RoPE on adjacent pairs (inference.cu:113-134)
                             float r[16];
-                            const float* rp = q.rope + (size_t)pos * q.hd + e0;
-                            ld_feat16(rp, r);
+                            ld_feat16(q.rope + (size_t)pos * q.hd + e1, r);
 #pragma unroll
                             for (int j = 0; j < 16; j += 2) {
                                 const float a = v[j], b = v[j + 1];
@@ -523,27 +586,49 @@ __global__ void __launch_bounds__(kGcThreads, 1) gemm_cols_kernel(const __grid_c
                                 v[j + 1] = fmaf(r[j + 1], a, r[j] * b);
                             }
                         }
-                        if (seg == 0) put16(q.qbuf + (size_t)tok * q.nq + fs, v);
-                        else if (seg == 1) put16(reinterpret_cast<KVT*>(q.kpool) + (kv_row + (size_t)head * kKvBlock) * q.hd + e0, v);
-                        else if (seg == 2) put16(reinterpret_cast<KVT*>(q.vpool) + (kv_row + (size_t)head * kKvBlock) * q.hd + e0, v);
+                        if (seg == 0) put16(q.qbuf + (size_t)tok * q.nq + fs + 16 * h, v);
+                        else if (seg == 1) put16(reinterpret_cast<KVT*>(q.kpool) + (kv_row + (size_t)head * kKvBlock) * q.hd + e1, v);
+                        else if (seg == 2) put16(reinterpret_cast<KVT*>(q.vpool) + (kv_row + (size_t)head * kKvBlock) * q.hd + e1, v);
                         else {
 #pragma unroll
                             for (int j = 0; j < 16; ++j) v[j] = __fdividef(1.0f, 1.0f + __expf(-v[j]));      // inference.cu:248
-                            put16(q.gbuf + (size_t)tok * q.ng + fs, v);
+                            put16(q.gbuf + (size_t)tok * q.ng + fs + 16 * h, v);
                         }
                     }
                 }
+                if (MODE != TC_RESID) continue;
+                __syncwarp();
+                // ---- staging rows -> residual stream and next operand
+                const int f = fg + 4 * piece;
+                const float* g = fw[1] + cg + 4 * piece;
+#pragma unroll 4
+                for (int i = 0; i < 8; ++i) {
+                    const int row = trow + 4 * i;
+                    if (tok0 + row >= n_cols || f >= p.N) continue;              // N is a multiple of 8
+                    const float4 x = *reinterpret_cast<const float4*>(stg + row * kGcStgRow + 4 * piece);
+                    const size_t at = (size_t)(tok0 + row) * p.N + f;
+                    *reinterpret_cast<float4*>(p.y + at) = x;
+                    *reinterpret_cast<uint2*>(p.xg16 + at) = make_uint2(gc_pack(x.x * g[0], x.y * g[1]), gc_pack(x.z * g[2], x.w * g[3]));
+                }
+                __syncwarp();                          // the staging rows have been read
+                if (cg + 32 < span) fetch_resid(fg + 32);
             }
+            if (MODE == TC_RESID) asm volatile("cp.async.wait_group 0;" ::: "memory");      // (a fetch behind the last feature is not used)
             tc_fence_before();
             __syncwarp();
             for (int r = 0; r < (SUMS ? p.exts : 1); ++r) {
-                if (lane == 0) mbar_arrive(tempty0 + 8u * buf);
+                release(buf);
                 if (++buf == p.nbuf) { buf = 0; ++use; }
             }
         }
+        if (MODE == TC_RESID) asm volatile("cp.async.wait_group 0;" ::: "memory");      // also of a tile that was given up
     }
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
+    if (PAIR) cluster_sync_all();                     // nothing of the other CTA's reads, writes or arrives here any more
+    if (warp == 1) {
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
+    }
 }
 
 }  // namespace mlb

@@ -97,7 +97,7 @@ struct Recorder {
 
 struct TcShape { int nb, split, stages, group; size_t smem; uint32_t tmem_cols; };
 // launch shape of one projection of a column set (gemm_cols.cuh)
-struct ColsGemm { int bn, stages, ctas, split, mains, exts, nbuf; uint32_t tmem_cols; bool sums; };
+struct ColsGemm { int bn, stages, ctas, split, mains, exts, nbuf; uint32_t tmem_cols; bool sums, pair; int w_rows; };      // w_rows: of a CTA's weight tile, one matrix
 
 struct mlb_session {
     mlb_model* m = nullptr;

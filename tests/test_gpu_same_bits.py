@@ -1,6 +1,8 @@
 """Kernels that are built to return the bits of the kernel they replaced, held to it on one model: the projections of a step on mma.sync
 and on tcgen05 tiles, the column GEMMs and the column attention against the decode step's kernels, the column form of the delta-net
 recurrence (one row of the state per lane group, or four) against the step's."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -68,6 +70,27 @@ def test_columns_against_the_decode_steps_kernels(api, tmp_path, monkeypatch, na
         sess.close()
     for n in (129, 200, 256):
         assert np.array_equal(got["auto", n], got["tcgen05", n]), n
+    model.close()
+
+
+@pytest.mark.parametrize("name", [*SPECS, *QK_NORM])
+def test_column_tiles_over_two_ctas(api, tmp_path, monkeypatch, name):
+    """MLB_COLS_PAIR pins the tiles of 256 columns x 256 features of a CTA pair (0: never, 1: wherever they can run): 257 to 1100 columns, the last tile
+    of one column, of one CTA's part and nearly whole; every position's logits."""
+    spec = dataclasses.replace({**SPECS, **QK_NORM}[name], max_context=1200)
+    model = api.Model(write_model(tmp_path, spec, seed=111))
+    text = random_prompts(spec.vocab, [1100], seed=113)[0]
+    lens = (257, 384, 500, 512, 513, 1100)
+    got = {}
+    for pair in "01":
+        monkeypatch.setenv("MLB_COLS_PAIR", pair)
+        sess = api.Session(model, 1)
+        for n in lens:
+            got[pair, n] = sess.score(text[:n])
+            assert sess.path(n) == "cols"
+        sess.close()
+    for n in lens:
+        assert np.array_equal(got["0", n], got["1", n]), n
     model.close()
 
 
