@@ -402,12 +402,17 @@ cudaError_t attn_cols_launch(int head_dim, int group, bool pdl, int max_tiles, c
 // large batch the instructions. There a warp had a row per instruction and 10 shuffles per row and column. Here eight lanes
 // share R rows; a lane holds the elements of four of that kernel's lanes (a, a + 8, a + 16, a + 24), as packed pairs, so
 // that the first two steps of a row's 32-lane sum are its own additions and three shuffle steps are left, on values halved from
-// step to step; k^ and q^ of a column are read from shared memory once for R rows. The inputs of 16 columns at a time come
-// through a three-stage cp.async ring and are L2-normalised there. R = 4 where the chunk's runs fill the SMs (fewest
-// instructions per row), else R = 1 (a quarter of the rows, and of the instructions in the chain, per warp): delta_cols_serial.
+// step to step; k^ and q^ of a column are read from shared memory once for R rows, as the pairs that the products take. The inputs of 16
+// columns at a time come through a cp.async ring and are L2-normalised there, by the walking warps or (R = 1) by others. R = 4 where the
+// chunk's runs fill the SMs (fewest instructions per row), else R = 1 (a quarter of the rows, and of the instructions in the chain, per
+// warp): delta_cols_serial. Per launch, before the pairs, the output sums under the next column and the preparing warps -> with them: one run of
+// 3001 columns, 16 heads of 128 2059 -> 1038 us; 64 runs of 64 columns 363 -> 312, 8 heads of 128 187 -> 164; 128 of 32, 8 heads of 64 54 -> 48.
 // ------------------------------------------------------------------------------------------------
 constexpr int kDcCols = 16;       // columns per ring stage
-constexpr int kDcStages = 3;
+constexpr int dc_stages(int rows) { return rows == 1 ? 4 : 3; }
+// One row per lane group: four more warps copy and normalise the inputs of the next columns under the walk of these, which is then only the
+// recurrence (3001 columns of 16 heads of 128: 1717 -> 1038 us). Where runs fill the SMs other CTAs' walks do that, and the walking warps prepare.
+constexpr int dc_threads(int rows) { return 32 * 4 * (rows == 1 ? 2 : 1); }
 constexpr int kDcWarps = 4;
 constexpr int kDcThreads = 32 * kDcWarps;
 
@@ -433,17 +438,34 @@ __device__ __forceinline__ void delta_pairs(const float* v, int a, f32x2 (&lo)[D
     }
 }
 
+// The same pairs from a column that the kernel has normalised: 16-byte pieces of two pairs, piece i of lane a at i * 8 + a (put together from
+// the elements' own order, a column cost 16 moves per vector).
+template <int DK>
+__device__ __forceinline__ void delta_shared_pairs(const float* v, int a, f32x2* lo, f32x2* hi) {
+    constexpr int H = DK / 64;                      // pieces of lo, and of hi
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(v) + a;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const ulonglong2 x = p[8 * i], y = p[8 * (H + i)];
+        lo[2 * i] = x.x; lo[2 * i + 1] = x.y;
+        hi[2 * i] = y.x; hi[2 * i + 1] = y.y;
+    }
+}
+
 template <int DK, int R>
-__global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams p) {
+__global__ void __launch_bounds__(dc_threads(R)) delta_cols_kernel(DeltaColsParams p) {
     constexpr int EPL = DK / 32;                    // elements per lane of delta_net_kernel
     constexpr int ROWS = 4 * R * kDcWarps;          // rows of S per CTA
+    constexpr int kDcStages = dc_stages(R);
+    constexpr bool APART = R == 1;                  // warps 4 - 7 prepare, 0 - 3 walk
     extern __shared__ __align__(128) unsigned char sm[];
     DeltaStage<DK, R>* ring = reinterpret_cast<DeltaStage<DK, R>*>(sm);
     pdl_launch_dependents();
     if ((int)blockIdx.z >= p.hdr[1]) return;
     const int4 run = p.runs[blockIdx.z];            // first column, columns, sequence, position of the first
     const int h = blockIdx.y, H = p.H, dv = p.dv;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, a = lane & 7;
+    const int tid = threadIdx.x & (kDcThreads - 1), lane = tid & 31, warp = tid >> 5, a = lane & 7;
+    const bool prepares = !APART || threadIdx.x >= kDcThreads, walks = !APART || !prepares;
     const int row0 = blockIdx.x * ROWS, rloc = warp * 4 * R + (lane >> 3) * R;      // this lane's rows: row0 + rloc .. + R - 1
     const int n_rows = min(ROWS, dv - row0);
     const int n_groups = (run.y + kDcCols - 1) / kDcCols;
@@ -481,11 +503,14 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
     f32x2 slo[R][EPL], shi[R][EPL];
     float* Sh = p.state + (((size_t)run.z * H + h) * dv + row0 + rloc) * DK;
     pdl_wait();
-    load(0);
-    load(1);
+    if (prepares) {
+        load(0);
+        load(1);
+        if (APART) load(2);
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        if (rloc + r < n_rows) {
+        if (walks && rloc + r < n_rows) {
             delta_pairs<DK>(Sh + (size_t)r * DK, a, slo[r], shi[r]);
         } else {
 #pragma unroll
@@ -520,13 +545,25 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
         unpack2(add2(l, hh), x, y);
         return x + y;
     };
-    for (int g = 0; g < n_groups; ++g) {
+    // A column's output is summed over the lanes and written under the next column's dot products: in line it was a second chain of shuffles in
+    // a chain that already has one (3001 columns, one row: 1904 -> 1717 us a layer).
+    float od[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) od[r] = 0.f;
+    size_t at = ((size_t)run.x * H + h) * dv + row0 + rloc + own;
+    const bool writes = (R == 4 ? (a & 1) == 0 : a == 0) && rloc + own < n_rows;
+    auto put = [&](float o) {
+        if (writes) {
+            if (p.out) p.out[at] = o;
+            if (p.out16) p.out16[at] = __float2bfloat16_rn(o);
+        }
+        at += (size_t)H * dv;
+    };
+    // L2 norms and gates, as delta_net_kernel takes them
+    auto prepare = [&](int g) {
         DeltaStage<DK, R>& sg = ring[g % kDcStages];
         const int n = min(kDcCols, run.y - g * kDcCols);
-        cp_async_wait<1>();
-        __syncthreads();
         for (int c = warp; c < n; c += kDcWarps) {
-            // L2 norms and gates, as delta_net_kernel takes them
             float q[EPL], k[EPL], x = 0.f, y = 0.f;
 #pragma unroll
             for (int e = 0; e < EPL; ++e) {
@@ -537,22 +574,27 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
             }
             x = sqrtf(warp_sum(x) + p.l2_eps);
             y = sqrtf(warp_sum(y) + p.l2_eps);
+            __syncwarp();                            // every lane has read its part: the column is rewritten as the pairs that the lanes take
 #pragma unroll
             for (int e = 0; e < EPL; ++e) {
-                sg.q[c][lane * EPL + e] = q[e] / x;
-                sg.k[c][lane * EPL + e] = k[e] / y;
+                const int at = (((lane >> 4) * (EPL / 2) + e / 2) * 8 + (lane & 7)) * 4 + (e & 1) * 2 + ((lane >> 3) & 1);
+                sg.q[c][at] = q[e] / x;
+                sg.k[c][at] = k[e] / y;
             }
             if (lane < 2) {
                 float* gt = (lane ? sg.alpha : sg.beta) + c;
                 *gt = 1.0f / (1.0f + expf(-*gt));
             }
         }
-        __syncthreads();
-        load(g + 2);                                 // into the stage whose columns every thread has left behind
+    };
+    auto walk = [&](int g) {
+        DeltaStage<DK, R>& sg = ring[g % kDcStages];
+        const int n = min(kDcCols, run.y - g * kDcCols);
         f32x2 kl[EPL], kh[EPL], ql[EPL], qh[EPL];
-        delta_pairs<DK>(sg.k[0], a, kl, kh);
-        delta_pairs<DK>(sg.q[0], a, ql, qh);
+        delta_shared_pairs<DK>(sg.k[0], a, kl, kh);
+        delta_shared_pairs<DK>(sg.q[0], a, ql, qh);
         float alpha = sg.alpha[0], beta = sg.beta[0], v = sg.v[0][rloc + own];
+#pragma unroll 2
         for (int c = 0; c < n; ++c) {
             const f32x2 al = pack2(alpha, alpha);
             float d[R];
@@ -568,10 +610,11 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
             // next column's inputs, in flight while this one is summed
             const int cn = c + 1 < n ? c + 1 : c;
             f32x2 nkl[EPL], nkh[EPL], nql[EPL], nqh[EPL];
-            delta_pairs<DK>(sg.k[cn], a, nkl, nkh);
-            delta_pairs<DK>(sg.q[cn], a, nql, nqh);
+            delta_shared_pairs<DK>(sg.k[cn], a, nkl, nkh);
+            delta_shared_pairs<DK>(sg.q[cn], a, nql, nqh);
             const float nalpha = sg.alpha[cn], nbeta = sg.beta[cn], nv = sg.v[cn][rloc + own];
-            const float u = beta * (v - reduce(d));
+            const float u = beta * (v - reduce(d)), o = reduce(od);      // (two independent chains of shuffles)
+            if (c + g > 0) put(o);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const float ur = R == 1 ? u : __shfl_sync(0xffffffffu, u, (lane & 24) + 2 * r);
@@ -581,13 +624,7 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
                     slo[r][e] = fma2(uu, kl[e], slo[r][e]);
                     shi[r][e] = fma2(uu, kh[e], shi[r][e]);
                 }
-                d[r] = dot(slo[r], shi[r], ql, qh);
-            }
-            const float o = reduce(d);
-            if ((R == 4 ? (a & 1) == 0 : a == 0) && rloc + own < n_rows) {
-                const size_t at = ((size_t)(run.x + g * kDcCols + c) * H + h) * dv + row0 + rloc + own;
-                if (p.out) p.out[at] = o;
-                if (p.out16) p.out16[at] = __float2bfloat16_rn(o);
+                od[r] = dot(slo[r], shi[r], ql, qh);
             }
 #pragma unroll
             for (int e = 0; e < EPL; ++e) {
@@ -600,7 +637,41 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
             beta = nbeta;
             v = nv;
         }
+    };
+    if (APART) {
+        auto arrived_and_prepared = [&](int g) {     // (each thread has waited for its own copies of the group)
+            asm volatile("bar.sync 1, %0;" ::"n"(kDcThreads) : "memory");
+            prepare(g);
+        };
+        if (prepares && n_groups > 0) {
+            cp_async_wait<2>();
+            arrived_and_prepared(0);
+        }
+        __syncthreads();
+        for (int g = 0; g < n_groups; ++g) {
+            if (walks) {
+                walk(g);
+            } else {
+                if (g + 1 < n_groups) {
+                    cp_async_wait<1>();
+                    arrived_and_prepared(g + 1);
+                }
+                load(g + 3);                         // into the stage that was walked before the last barrier
+            }
+            __syncthreads();
+        }
+    } else {
+        for (int g = 0; g < n_groups; ++g) {
+            cp_async_wait<1>();
+            __syncthreads();
+            prepare(g);
+            __syncthreads();
+            load(g + 2);                             // into the stage whose columns every thread has left behind
+            walk(g);
+        }
     }
+    if (!walks) return;
+    if (n_groups > 0) put(reduce(od));
 #pragma unroll
     for (int r = 0; r < R; ++r)
         if (rloc + r < n_rows) {
@@ -624,15 +695,15 @@ __global__ void __launch_bounds__(kDcThreads) delta_cols_kernel(DeltaColsParams 
 template <int DK, int R>
 static cudaError_t delta_cols_one(bool pdl, int max_runs, cudaStream_t st, const DeltaColsParams& p) {
     constexpr int rows = 4 * R * kDcWarps;
-    const size_t smem = kDcStages * sizeof(DeltaStage<DK, R>);
+    const size_t smem = dc_stages(R) * sizeof(DeltaStage<DK, R>);
     cudaError_t e = cudaFuncSetAttribute(delta_cols_kernel<DK, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_pdl(pdl, delta_cols_kernel<DK, R>, dim3((p.dv + rows - 1) / rows, p.H, max_runs), dim3(kDcThreads), smem, st, p);
+    return launch_pdl(pdl, delta_cols_kernel<DK, R>, dim3((p.dv + rows - 1) / rows, p.H, max_runs), dim3(dc_threads(R)), smem, st, p);
 }
 
 // One row per lane group where a chunk is a serial chain rather than a load: columns / longest run sequences side by side, each of H dv rows,
-// do not give every SM a CTA of 64 rows. Measured per launch, one row -> four: one run of 3000 columns (dk 128, 16 heads) 2074 -> 3494 us,
-// of 899 (dk 64, 8 heads) 318 -> 424.
+// do not give every SM a CTA of 64 rows. Measured per launch, one row -> four, before the former's preparing warps (now 1038 us): one run of 3000
+// columns (dk 128, 16 heads) 2074 -> 3494 us, of 899 (dk 64, 8 heads) 318 -> 424.
 bool delta_cols_serial(int sm_count, int H, int dv, int columns, int longest) {
     return (long)columns * H * dv < (long)longest * sm_count * 16 * kDcWarps;
 }
