@@ -294,47 +294,6 @@ static GdShape gd_pick(const mlb_session* s, int N, int nkb, int mode, bool w8, 
     // than two per SM: a CTA's own chain of barriers, operands and epilogue bounds those, and more of them side by side hide it (LM head of 8192
     // features, 256 sequences, 1024 CTAs of 512: 35.5 us with two per SM, 20.8 with four, 15.3 with eight; of 32000 x 2048, e4m3, 64 sequences:
     // 106 with two, 82 with eight).
-    const long ctas = (long)tiles_m * ((B + nb - 1) / nb) * S;
-            const long resident = S == 1 ? s->sm_count : (long)s->tc_cluster_cap[li] * S;
-            const long waves = (ctas + resident - 1) / resident;
-            const double t_loop = 0.4 * na * kpc;
-            const double t_red = S > 2 ? 2.5 + (double)nacc * nb * 512.0 / 65536.0 : (S > 1 ? 0.5 + (double)nacc * nb * 512.0 / 65536.0 : 0.0);
-            const double t_epi = 0.25 * ((nb / S + 15) / 16);
-            const double cost = (double)waves * (t_loop + t_red + t_epi + 0.5);
-            if (best_cost < 0 || cost < best_cost) {
-                best_cost = cost;
-                uint32_t cols = 32;
-                while (cols < (uint32_t)(nacc * nb)) cols <<= 1;
-                best = TcShape{nb, S, st, g, smem, cols};
-            }
-        }
-    }
-    return best;
-}
-// Launch shape of a decode GEMM (gemm_dec.cuh).
-struct GdShape { int np, split, g, stages, w_bytes; size_t smem; };
-static int gd_index(int np, int g) { return (np >> 1) * 3 + (g >> 1); }       // np, g in {1, 2, 4}
-// mma.sync multiplies at about 512 a cycle and SM here (k-loop times against sequences per CTA), tcgen05 eight times as fast, so what
-// gemm_dec_kernel saves around the products it pays back in them once they are many. Measured per step, tcgen05 -> mma.sync: cfg1 372
-// -> 195 us at 4 sequences, 534 -> 455 at 256; cfg4 (gate/up 2 x 5632 x 2048) 2338 -> 1677 at 4, 3112 -> 2760 at 48 (7.5 M products
-// per SM in the gate/up projection, the largest), 2735 -> 2739 and behind long prompts 3385 -> 3440 at 64 (10 M). The line lies between.
-constexpr long kGdMostProducts = 8L << 20;
-static bool gd_small_enough(const mlb_session* s) {
-    return s->B <= 256 && 2L * s->m->cfg.ffn_dim * s->m->cfg.dim * s->B / s->sm_count <= kGdMostProducts;
-}
-// The k-ranges are those of the tcgen05 launch of the same batch (the results are the same bits). Sequences per CTA: the most
-// that still leaves 96 CTAs, two thirds of the SMs - fewer CTAs read the activations less often, more of them share the epilogue.
-static GdShape gd_pick(const mlb_session* s, int N, int nkb, int mode, bool w8, bool ext) {
-    GdShape g;
-    const int na = mode == TC_SWIGLU ? 2 : 1;
-    const bool ext2 = w8 && mode == TC_RESID;
-    g.split = std::max(1, tc_pick_shape(s, s->B, N, nkb, na, w8, na == 2 || ext2 ? 2 : 1).split);
-    g.np = 4;
-    while (g.np > 1 && (16 * (g.np / 2) >= s->B || (long)((N + kGdF - 1) / kGdF) * ((s->B + 16 * g.np - 1) / (16 * g.np)) < 96)) g.np >>= 1;
-    g.w_bytes = kGdF * (w8 && !ext ? 64 : 128);
-    const int ct = 16 * g.np;
-    // Two CTAs per SM share its shared memory, so that the next launch's weights arrive under this one; four where there are more CTAs than
-    // two per SM: what bounds these is a CTA's own chain (LM head of 8192 features, 256 sequences, 1024 CTAs: RINGFIG).
     const long ctas = (long)((N + kGdF - 1) / kGdF) * ((s->B + 16 * g.np - 1) / (16 * g.np));
     const size_t ring = ctas > 2L * s->sm_count ? kGdRing / 4 : kGdRing;
     // k-blocks per copy: as many as leave two stages
