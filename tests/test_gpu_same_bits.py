@@ -54,10 +54,38 @@ def test_step_projections_on_both_tiles(api, tmp_path, monkeypatch, name):
     model.close()
 
 
-@pytest.mark.parametrize("name", [*SPECS, *QK_NORM])
+# widths that end 8 and 24 features behind a group of 32 (residual stream) and inside a tile
+RAGGED = {
+    "bf16_264": ModelSpec(dim=264, layers=2, heads=4, head_dim=64, ffn_dim=328, ple_dim=64, vocab=500, layer_types=periodic_layer_types(2, 2),
+                          weight_dtype="bfloat16", **COMMON),
+    "bf16_280": ModelSpec(dim=280, layers=2, heads=4, head_dim=64, ffn_dim=1352, vocab=500, weight_dtype="bfloat16", **COMMON),
+}
+
+
+@pytest.mark.parametrize("name", ["bf16", "fp8"])
+def test_step_projections_of_more_ctas_than_two_per_sm(api, tmp_path, monkeypatch, name):
+    """LM head of 125 or 100 x 3 or 4 CTAs, which run on smaller rings, against the tcgen05 tiles."""
+    monkeypatch.setenv("MLB_PREFILL", "step")
+    spec = dataclasses.replace(SPECS[name], vocab=4000 if name == "bf16" else 3200)
+    model = api.Model(write_model(tmp_path, spec, seed=117))
+    for batch in (191, 256):
+        prompts = random_prompts(spec.vocab, [1 + b % 2 for b in range(batch)], seed=119)
+        got = {}
+        for tiles in ("mma", "tcgen05"):
+            monkeypatch.setenv("MLB_GEMM", tiles)
+            sess = api.Session(model, batch)
+            assert sess.path() == tiles
+            sess.prefill(prompts)
+            got[tiles] = sess.decode(2), sess.logits()
+            sess.close()
+        assert np.array_equal(got["mma"][0], got["tcgen05"][0]) and np.array_equal(got["mma"][1], got["tcgen05"][1]), batch
+    model.close()
+
+
+@pytest.mark.parametrize("name", [*SPECS, *QK_NORM, *RAGGED])
 def test_columns_against_the_decode_steps_kernels(api, tmp_path, monkeypatch, name):
     """129 to 256 columns (one set, whose k-ranges are those that every width takes): every position's logits."""
-    spec = {**SPECS, **QK_NORM}[name]
+    spec = {**SPECS, **QK_NORM, **RAGGED}[name]
     model = api.Model(write_model(tmp_path, spec, seed=105))
     text = random_prompts(spec.vocab, [256], seed=107)[0]
     got = {}
@@ -73,11 +101,11 @@ def test_columns_against_the_decode_steps_kernels(api, tmp_path, monkeypatch, na
     model.close()
 
 
-@pytest.mark.parametrize("name", [*SPECS, *QK_NORM])
+@pytest.mark.parametrize("name", [*SPECS, *QK_NORM, *RAGGED])
 def test_column_tiles_over_two_ctas(api, tmp_path, monkeypatch, name):
     """MLB_COLS_PAIR pins the tiles of 256 columns x 256 features of a CTA pair (0: never, 1: wherever they can run): 257 to 1100 columns, the last tile
     of one column, of one CTA's part and nearly whole; every position's logits."""
-    spec = dataclasses.replace({**SPECS, **QK_NORM}[name], max_context=1200)
+    spec = dataclasses.replace({**SPECS, **QK_NORM, **RAGGED}[name], max_context=1200)
     model = api.Model(write_model(tmp_path, spec, seed=111))
     text = random_prompts(spec.vocab, [1100], seed=113)[0]
     lens = (257, 384, 500, 512, 513, 1100)
