@@ -227,7 +227,8 @@ void mlb_kv_alloc_free(mlb_kv_alloc* a);
  * num_pages is the number of pages the pools hold. The page table is the caller's, so the kernel
  * checks it: a sequence whose position needs more than pt_stride pages is skipped, a page id
  * outside [0, num_pages) is replaced by page 0, and the call returns MLB_E_INVALID (nothing
- * outside the caller's buffers is read).
+ * outside the caller's buffers is read). A sequence with a negative position attends to nothing: neither
+ * its row of the page table nor the pools are read for it, and its row of out is NaN.
  * Allocates its split-combine scratch with cudaMalloc for the call and returns after the
  * stream has finished. */
 int mlb_op_attn_decode(const void* kpool, const void* vpool, int kv_dtype, const int32_t* page_table,

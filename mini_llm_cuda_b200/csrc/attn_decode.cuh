@@ -103,8 +103,10 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
     }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w = warp / HG, hgrp = warp % HG;
     const int lr = lane % LPR, grp = lane / LPR;
+    // An operator's caller may mark an idle sequence with a negative position: it has no pages, and nothing of its row of the table is read
+    // (the producer copies nothing, the sums stay empty, the row becomes 0 / 0).
     const int ctx = c.pos[b] + 1;
-    const int npages = (ctx + kKvBlock - 1) / kKvBlock;
+    const int npages = c.pos[b] < 0 ? 0 : c.pos[b] / kKvBlock + 1;
     // The splits are sized for the longest context; a split needs at least one page, and the CTAs
     // beyond the page count leave at once (fewer partials for the combine to read). Every CTA of a
     // (sequence, kv head) computes the same S.
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
         if (lane < NW) {
             const int* pt = p.page_table + kv_seq(c, b) * p.pt_stride;
             auto pool_index = [&](int pg) {
-                int page = pt[min(pg, npages - 1)];
+                int page = pt[pg];
                 if (p.num_pages > 0 && (unsigned)page >= (unsigned)p.num_pages) {
                     atomicExch(p.err, 5);
                     page = 0;
@@ -155,9 +157,9 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
             bool good = true;
             for (int s = s_first; s < s_end && good; ++s) {
                 const int end = min(npages, (s + 1) * pps);
-                int pg = s * pps + lane, page = pool_index(pg);
+                int pg = s * pps + lane, page = pg < end ? pool_index(pg) : 0;
                 for (; pg < end; pg += NW) {
-                    const int next = pool_index(pg + NW);      // on its way while this page waits for its stage
+                    const int next = pg + NW < end ? pool_index(pg + NW) : 0;      // on its way while this page waits for its stage
                     if (!waited && pg == npages - 1) {
                         pdl_wait();
                         waited = true;

@@ -167,6 +167,36 @@ def test_attention_op_skips_what_the_page_table_does_not_cover(api):
     assert (out.cpu().double() - case["want"]).abs().max().item() < 2e-5
 
 
+@pytest.mark.parametrize("heads,kv_heads,hd,dtype_name", [(4, 4, 64, "float32"), (8, 2, 128, "bfloat16")])
+@pytest.mark.parametrize("batch,splits", [(3, 1), (3, 3), (57, 1), (57, 3)])
+def test_attention_op_reads_no_table_entry_of_an_empty_sequence(api, heads, kv_heads, hd, dtype_name, batch, splits):
+    """Idle sequences are marked with negative positions. The word in front of the table and the last entry of every row are no page ids:
+    a read of either would set an error code. 57 sequences: one CTA per sequence and kv head takes its splits in turn."""
+    import torch
+    dtype = getattr(torch, dtype_name)
+    idle = [b % 3 != 1 for b in range(batch)]
+    case = make_attention_case(torch, batch, heads, kv_heads, hd, [1 if i else 6 + b % 90 for b, i in enumerate(idle)], dtype, 9, True)
+    n_entries, guard = batch * case["pt_stride"], -559038737
+    words = torch.full((1 + n_entries,), guard, dtype=torch.int32, device="cuda:0")
+    table = case["table"].clone()
+    table[:, -1] = guard
+    for b in range(batch):
+        if idle[b]:
+            table[b] = guard
+            case["pos"][b] = (-1, -2, -17, -40000)[b % 4]
+    words[1:] = table.flatten()
+    case["table"] = words[1:]
+    for fn in ("mlb_op_attn_decode", "mlb_op_attn_decode_static"):
+        rc, out = call_attention(api, torch, fn, case, batch, heads, kv_heads, hd, splits, dtype)
+        assert rc == 0, api.lib().mlb_last_error()
+        assert fn == "mlb_op_attn_decode" or api.lib().mlb_op_attn_decode_static_status(None) == 0
+        for b in range(batch):
+            if idle[b]:
+                assert out[b].isnan().all(), b
+            else:
+                assert (out[b].cpu().double() - case["want"][b]).abs().max().item() < 2e-5, b
+
+
 @pytest.mark.parametrize("N,K,batch", [(128, 64, 16), (256, 512, 32), (1408, 512, 256), (512, 1408, 100), (1552, 512, 20),
                                        (8192, 512, 300)])
 def test_tcgen05_gemm_matches_fp32_matmul(api, N, K, batch):
