@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "session.h"
+#include "step_shapes.h"
 #include "grid_host.h"
 #include "lean_host.h"
 #include "sgemv.cuh"
@@ -90,8 +91,8 @@ struct Chain {
         }
         auto up4 = [](int v) { return (v + 3) / 4 * 4; };
         g.xs_stride = up4(p.K); g.xs2_stride = up4(std::max(p.Kp, 4)); g.outs_stride = up4(std::max(p.hd, 64)); g.pacc_stride = up4(g.rows_per_cta + 4);
-        // as many sequences per CTA (three at most) as leave three stages; without room for one the other GEMV serves
-        int bt = std::min(s->B, 3);
+        // no more sequences per CTA than leave three stages; without room for one the other GEMV serves
+        int bt = sg_sequences(s->B, grid_x, s->sm_count);
         size_t fixed = 0;
         for (;; --bt) {
             if (bt == 0) return MLB_OK;

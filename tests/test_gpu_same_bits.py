@@ -149,14 +149,18 @@ def test_recurrence_over_columns_against_steps(api, tmp_path, monkeypatch, dk, d
     model.close()
 
 
-@pytest.mark.parametrize("name", ["fp8", "bf16", "fp32_qknorm_gated"])
+@pytest.mark.parametrize("name", ["fp8", "bf16", "fp32_qknorm_gated", "fp8_many_heads", "fp32_qknorm_many_heads"])
 def test_streamed_gemv_of_several_sequences(api, tmp_path, monkeypatch, name):
     """A CTA of the streamed GEMV takes up to three sequences: each gets the ids and logits that it gets alone. Two to seven
-    sequences: whole and ragged groups of three; down projections whose input leaves room for fewer (ffn_dim 9216: 108 KB for three)."""
+    sequences: whole and ragged groups of one to three; down projections whose input leaves room for fewer (ffn_dim 9216: 108 KB for
+    three); QKV cut into so few slabs that a CTA takes one sequence, and into 96 and 128."""
     for key, value in (("MLB_PREFILL", "step"), ("MLB_DECODE_PATH", "chain"), ("MLB_GEMV", "stream"), ("MLB_GEMM", "simt")):
         monkeypatch.setenv(key, value)
     spec = {**SPECS, "fp32_qknorm_gated": ModelSpec(dim=256, layers=2, heads=4, kv_heads=2, head_dim=64, ffn_dim=9216, vocab=500, qk_norm=True, query_gating=True,
-                                                    rms_eps=1e-5, max_context=64)}[name]
+                                                    rms_eps=1e-5, max_context=64),
+            "fp8_many_heads": dataclasses.replace(SPECS["fp8"], heads=16, kv_heads=4, layers=2, layer_types=["attention"] * 2),
+            "fp32_qknorm_many_heads": ModelSpec(dim=128, layers=1, heads=32, head_dim=64, ffn_dim=256, vocab=500, qk_norm=True, query_gating=True,
+                                                rms_eps=1e-5, max_context=64)}[name]
     model = api.Model(write_model(tmp_path, spec, seed=113))
     prompts = random_prompts(spec.vocab, [3 + b % 4 for b in range(7)], seed=115)
     sess = api.Session(model, 1)

@@ -278,3 +278,31 @@ def test_fp8_tensors_in_the_model_file(api, tmp_path):
     open(short, "wb").write(raw[:len(raw) - 64])
     with pytest.raises(api.MlbError):
         api.inspect_file(short)
+
+
+def run_host_program(tmp_path, includes, body):
+    """What a C++ program with `body` as its main prints, built against the library's host headers."""
+    import subprocess
+    src, exe = os.path.join(str(tmp_path), "p.cc"), os.path.join(str(tmp_path), "p")
+    with open(src, "w") as f:
+        f.write("".join(f"#include {i}\n" for i in includes) + "int main() {\n" + body + "\nreturn 0; }\n")
+    csrc = os.path.join(ROOT, "mini_llm_cuda_b200", "csrc")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I", csrc, src, "-o", exe], check=True)
+    return subprocess.run([exe], check=True, capture_output=True, text=True).stdout
+
+
+def test_sequences_of_a_streamed_gemv_cta(tmp_path):
+    """Every sequence has a CTA, no more waves than groups of three need, no group larger than its wave asks for, none at all where
+    the CTAs fit side by side."""
+    out = run_host_program(tmp_path, ["<cstdio>", '"step_shapes.h"'], """
+        for (int b = 1; b <= 64; ++b)
+            for (int slabs = 1; slabs <= 148; ++slabs) std::printf("%d %d %d\\n", b, slabs, mlb::sg_sequences(b, slabs, 148));""")
+    for batch, slabs, n in (map(int, line.split()) for line in out.splitlines()):
+        rows = -(-batch // n)
+        assert 1 <= n <= 3 and rows * n >= batch
+        assert rows * slabs <= 148 or rows <= -(-batch // 3), (batch, slabs, n)      # more rows than groups of three make only in one wave
+        assert n == 1 or rows < -(-batch // (n - 1)), (batch, slabs, n)              # with one sequence less to a CTA there would be more rows
+        if batch * slabs <= 148:
+            assert n == 1, (batch, slabs, n)
+        if slabs > 74 and batch in (2, 3, 4):
+            assert n == {2: 2, 3: 3, 4: 2}[batch], (batch, slabs, n)
