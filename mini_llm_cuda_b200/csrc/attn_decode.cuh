@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "ring.cuh"
+#include "step_shapes.h"
 
 namespace mlb {
 
@@ -52,7 +53,6 @@ struct AttnParams {
 };
 
 constexpr int kAttnStreams = 4;
-constexpr int kAttnLoopSplits = 4;                 // most splits that one CTA takes in turn
 template <typename KVT, int HD> constexpr int attn_page_bytes() { return kKvBlock * HD * (int)sizeof(KVT); }      // of K, or of V
 template <int G> constexpr int attn_heads_per_warp() { return G < 2 ? 1 : 2; }
 template <int G> constexpr int attn_threads() { return 32 * (kAttnStreams * (G / attn_heads_per_warp<G>()) + 1); }      // and the producer warp
@@ -63,9 +63,9 @@ template <typename KVT, int HD, int G> constexpr size_t attn_decode_smem() {
 
 // Launch grid. One CTA for all splits of a sequence where there are CTAs enough without them: no partial results in global memory, no
 // CTA that waits for others' tickets (64 sequences of 528 positions, 16 heads over 4 of 128, three splits: 26.7 us, 32 with a CTA each).
-inline dim3 attn_grid(const AttnParams& p, int B) {
+inline dim3 attn_grid(const AttnParams& p, int B, int sm_count) {
     const int groups = p.kv_heads * p.hg;
-    return dim3(p.splits <= kAttnLoopSplits && groups * B >= 148 ? 1 : p.splits, groups, B);
+    return dim3(attn_splits_in_turn(p.splits, (long)groups * B, sm_count) ? 1 : p.splits, groups, B);
 }
 
 template <typename KVT, int HD, int G>

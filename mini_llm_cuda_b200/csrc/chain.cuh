@@ -197,7 +197,7 @@ struct Chain {
         // per step); with the GPU already full the extra CTAs only re-read K/V (62 -> 69 us at 64 sequences)
         if (G >= 4 && G % 2 == 0 && s->splits * p.kv_heads * s->B < 2 * s->sm_count) { p.hg = G / 2; G = 2; }
         p.splits = s->splits;
-        const dim3 grid = attn_grid(p, s->B);
+        const dim3 grid = attn_grid(p, s->B, s->sm_count);
         auto launch = [&](auto kernel, size_t smem, int threads) {
             const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             return e == cudaSuccess ? launch_chain(s->use_pdl, kernel, grid, dim3(threads), smem, s->stream, c, p) : e;

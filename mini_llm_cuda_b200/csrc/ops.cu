@@ -61,7 +61,11 @@ int check_attn_args(const void* kpool, const void* vpool, int kv_dtype, const in
 
 template <typename KVT, int HD>
 cudaError_t launch_attn(const StepCtl& c, AttnParams p, int G, int B, cudaStream_t st) {
-    const dim3 grid = attn_grid(p, B);
+    int dev = 0, sm_count = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const dim3 grid = attn_grid(p, B, sm_count);
     auto launch = [&](auto kernel, size_t smem, int threads) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

@@ -14,4 +14,9 @@ inline int sg_sequences(int batch, int slabs, int sm_count) {
     return (batch + rows - 1) / rows;
 }
 
+// Decode attention: one CTA takes all splits of a sequence and group of query heads, in turn, where the sequences and groups alone fill the
+// SMs; else every split has a CTA. (Figures at attn_grid.)
+constexpr int kAttnLoopSplits = 4;                 // most splits that one CTA takes in turn
+inline bool attn_splits_in_turn(int splits, long sequence_groups, int sm_count) { return splits <= kAttnLoopSplits && sequence_groups >= sm_count; }
+
 }  // namespace mlb

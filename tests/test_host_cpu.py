@@ -306,3 +306,15 @@ def test_sequences_of_a_streamed_gemv_cta(tmp_path):
             assert n == 1, (batch, slabs, n)
         if slabs > 74 and batch in (2, 3, 4):
             assert n == {2: 2, 3: 3, 4: 2}[batch], (batch, slabs, n)
+
+
+def test_splits_in_turn_follow_the_devices_sms(tmp_path):
+    """One CTA takes a sequence's splits in turn where sequences and groups of heads give every SM of the device a CTA, whatever its number."""
+    out = run_host_program(tmp_path, ["<cstdio>", '"step_shapes.h"'], """
+        for (int sms : {20, 132, 148, 160})
+            for (int splits : {1, 4, 5})
+                for (long n : {sms - 1L, (long)sms}) std::printf("%d %ld %d %d\\n", splits, n, sms, (int)mlb::attn_splits_in_turn(splits, n, sms));""")
+    lines = [tuple(map(int, line.split())) for line in out.splitlines()]
+    assert len(lines) == 24
+    for splits, n, sms, turn in lines:
+        assert turn == (splits <= 4 and n >= sms)
