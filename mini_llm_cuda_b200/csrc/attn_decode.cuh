@@ -8,8 +8,8 @@
 // grid = (splits or 1, kv_heads, B), block = 4 streams x the head groups of a kv head.
 //
 // A stream takes the pages w, w + 4, .. of a split (w = 0 .. 3). The 16 rows of a head in a page are one contiguous block, so
-// one lane copies a page's K and V rows with two bulk copies into the stream's own ring of shared-memory stages: no registers hold
-// loads in flight. With four query heads or more per kv head a stream has a warp per two of them, which share its ring.
+// one lane copies a page's K and V rows (or a half or a quarter of them: attn_few_rows) with two bulk copies into the stream's own ring of
+// shared-memory stages: no registers hold loads in flight. With four query heads or more per kv head a stream has a warp per two of them, which share its ring.
 // In a decode session the K/V rows of earlier tokens were written by earlier steps, which are complete when a step's first
 // kernel starts (it is launched without overlap): only the page of the current position and the queries wait for the predecessor.
 // The scores of four positions per lane group and GW heads are summed over the lanes by a butterfly that leaves every lane
@@ -52,14 +52,8 @@ struct AttnParams {
     int splits;             // most splits of a sequence: grid.x CTAs of one each, or (grid.x = 1) one CTA that takes them in turn
 };
 
-constexpr int kAttnStreams = 4;
-template <typename KVT, int HD> constexpr int attn_page_bytes() { return kKvBlock * HD * (int)sizeof(KVT); }      // of K, or of V
 template <int G> constexpr int attn_heads_per_warp() { return G < 2 ? 1 : 2; }
 template <int G> constexpr int attn_threads() { return 32 * (kAttnStreams * (G / attn_heads_per_warp<G>()) + 1); }      // and the producer warp
-template <typename KVT, int HD> constexpr int attn_stages() { return 2; }
-template <typename KVT, int HD, int G> constexpr size_t attn_decode_smem() {
-    return (size_t)kAttnStreams * attn_stages<KVT, HD>() * 2 * attn_page_bytes<KVT, HD>() + (size_t)(kAttnStreams + kAttnLoopSplits) * G * (HD + 2) * 4;
-}
 
 // Launch grid. One CTA for all splits of a sequence where there are CTAs enough without them: no partial results in global memory, no
 // CTA that waits for others' tickets (64 sequences of 528 positions, 16 heads over 4 of 128, three splits: 26.7 us, 32 with a CTA each).
@@ -68,8 +62,10 @@ inline dim3 attn_grid(const AttnParams& p, int B, int sm_count) {
     return dim3(attn_splits_in_turn(p.splits, (long)groups * B, sm_count) ? 1 : p.splits, groups, B);
 }
 
-template <typename KVT, int HD, int G>
-__global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : (G == 4 ? 2 : 1)))
+static_assert(kAttnPageRows == kKvBlock, "rows of a page");
+// SR: rows of a page per stage (attn_few_rows)
+template <typename KVT, int HD, int G, int SR>
+__global__ void __launch_bounds__(attn_threads<G>(), attn_resident(G))
     attn_decode_kernel(const __grid_constant__ StepCtl c, const __grid_constant__ AttnParams p) {
     constexpr int EPL = 16 / sizeof(KVT);          // elements per lane per row
     constexpr int LPR = HD / EPL;                  // lanes per row
@@ -78,16 +74,17 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
     constexpr int GW = attn_heads_per_warp<G>();   // heads of a warp
     constexpr int HG = G / GW;                     // warps of a stream
     constexpr int CH = 4;                          // positions per lane group handled together
-    constexpr int CPP = kKvBlock / PPI / CH;       // chunks per page
+    constexpr int RB = HD * (int)sizeof(KVT);      // bytes per row
     constexpr int N = GW * CH;                     // scores of a lane group,
     constexpr int D = LPR / N;                     // each kept by D lanes
     constexpr int GL = D * CH;                     // lanes that hold a head's scores
-    constexpr int NST = attn_stages<KVT, HD>();
-    constexpr int PB = attn_page_bytes<KVT, HD>();
+    constexpr int NST = kAttnStages;
+    constexpr int SB = SR * RB;                    // bytes of K, and of V, per stage (SR rows of a page)
+    constexpr int CPS = SR / PPI / CH;             // chunks per stage
     constexpr int W = HD + 2;
-    static_assert(LPR <= 32 && PPI >= 1 && CPP >= 1 && D >= 1, "head_dim does not fit one warp row");
+    static_assert(LPR <= 32 && PPI >= 1 && CPS >= 1 && kKvBlock % SR == 0 && D >= 1, "head_dim does not fit one warp row");
     extern __shared__ __align__(128) unsigned char attn_sm[];
-    float* sred = reinterpret_cast<float*>(attn_sm + (size_t)NW * NST * 2 * PB);      // [stream][G][HD + 2] of a split
+    float* sred = reinterpret_cast<float*>(attn_sm + (size_t)NW * NST * 2 * SB);      // [stream][G][HD + 2] of a split
     float* spart = sred + NW * G * W;              // [split][G][HD + 2] where one CTA takes all splits
     __shared__ __align__(8) uint64_t bars[2 * NW * NST];
     __shared__ float wsm[G][64];
@@ -150,7 +147,7 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
                 }
                 return page;
             };
-            const uint32_t ring0 = smem_u32(attn_sm) + (uint32_t)(lane * NST * 2 * PB), f0 = full0 + 8u * lane * NST, e0 = empty0 + 8u * lane * NST;
+            const uint32_t ring0 = smem_u32(attn_sm) + (uint32_t)(lane * NST * 2 * SB), f0 = full0 + 8u * lane * NST, e0 = empty0 + 8u * lane * NST;
             bool waited = !early;
             int st = 0;
             uint32_t ph = 1;
@@ -158,21 +155,24 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
             for (int s = s_first; s < s_end && good; ++s) {
                 const int end = min(npages, (s + 1) * pps);
                 int pg = s * pps + lane, page = pg < end ? pool_index(pg) : 0;
-                for (; pg < end; pg += NW) {
+                for (; pg < end && good; pg += NW) {
                     const int next = pg + NW < end ? pool_index(pg + NW) : 0;      // on its way while this page waits for its stage
                     if (!waited && pg == npages - 1) {
                         pdl_wait();
                         waited = true;
                     }
-                    good = mbar_wait_bounded(e0 + 8u * st, ph, kRingSpinLimit, 0);
-                    if (!good) break;              // (the consumers' waits run out and report it)
-                    const uint32_t bytes = (uint32_t)min(kKvBlock, ctx - pg * kKvBlock) * (uint32_t)(PB / kKvBlock), bar = f0 + 8u * st;
-                    const size_t at = ((size_t)page * p.kv_heads + kvh) * PB;
-                    mbar_expect_tx(bar, 2 * bytes);
-                    bulk_g2s(ring0 + (uint32_t)(st * 2 * PB), static_cast<const unsigned char*>(p.kpool) + at, bytes, bar);
-                    bulk_g2s(ring0 + (uint32_t)(st * 2 * PB + PB), static_cast<const unsigned char*>(p.vpool) + at, bytes, bar);
+                    const int rows = min(kKvBlock, ctx - pg * kKvBlock);
+                    for (int r0 = 0; r0 < rows && good; r0 += SR) {
+                        good = mbar_wait_bounded(e0 + 8u * st, ph, kRingSpinLimit, 0);
+                        if (!good) break;          // (the consumers' waits run out and report it)
+                        const uint32_t bytes = (uint32_t)(min(SR, rows - r0) * RB), bar = f0 + 8u * st;
+                        const size_t at = (((size_t)page * p.kv_heads + kvh) * kKvBlock + r0) * RB;
+                        mbar_expect_tx(bar, 2 * bytes);
+                        bulk_g2s(ring0 + (uint32_t)(st * 2 * SB), static_cast<const unsigned char*>(p.kpool) + at, bytes, bar);
+                        bulk_g2s(ring0 + (uint32_t)(st * 2 * SB + SB), static_cast<const unsigned char*>(p.vpool) + at, bytes, bar);
+                        if (++st == NST) { st = 0; ph ^= 1u; }
+                    }
                     page = next;
-                    if (++st == NST) { st = 0; ph ^= 1u; }
                 }
             }
             if (!waited) pdl_wait();
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
     // the other warps; the producer takes no part in their barriers: it is pages ahead of them, or behind a full ring
     auto sync = []() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW * HG) : "memory"); };
     if (early) pdl_wait();
-    unsigned char* ring = attn_sm + (size_t)w * NST * 2 * PB;
+    unsigned char* ring = attn_sm + (size_t)w * NST * 2 * SB;
     const uint32_t my_full = full0 + 8u * w * NST, my_empty = empty0 + 8u * w * NST;
     bool ok = true;
 
@@ -207,15 +207,15 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
     float m, l[GW];                                // m: of the head whose score this lane keeps
     f32x2 acc[GW][EPL / 2];
     const int src0 = lane - lr, own_u = (lr / D) % CH;
-    // CH positions of every lane group; cnt: rows of the page that hold a position (what lies behind them may be no number)
+    // CH positions of every lane group; cnt: rows of the stage that hold a position (what lies behind them may be no number)
     auto use_chunk = [&](const unsigned char* kt, int cnt, int c0) {
         float s[N];
 #pragma unroll
         for (int u = 0; u < CH; u += 2) {
-            const unsigned char* row = kt + ((c0 + u) * PPI + grp) * (PB / kKvBlock) + lr * 16;
+            const unsigned char* row = kt + ((c0 + u) * PPI + grp) * RB + lr * 16;
             float k0[EPL], k1[EPL];
             Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(row), k0);
-            Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(row + PPI * (PB / kKvBlock)), k1);
+            Elem<KVT>::unpack(*reinterpret_cast<const uint4*>(row + PPI * RB), k1);
 #pragma unroll
             for (int g = 0; g < GW; ++g) {
                 f32x2 d = 0ull;
@@ -257,8 +257,8 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
         }
 #pragma unroll
         for (int u = 0; u < CH; ++u) {
-            uint4 raw = *reinterpret_cast<const uint4*>(kt + PB + ((c0 + u) * PPI + grp) * (PB / kKvBlock) + lr * 16);
-            if (cnt < kKvBlock && (c0 + u) * PPI + grp >= cnt) raw = make_uint4(0, 0, 0, 0);
+            uint4 raw = *reinterpret_cast<const uint4*>(kt + SB + ((c0 + u) * PPI + grp) * RB + lr * 16);
+            if (cnt < SR && (c0 + u) * PPI + grp >= cnt) raw = make_uint4(0, 0, 0, 0);
             float vv[EPL];
             Elem<KVT>::unpack(raw, vv);
 #pragma unroll
@@ -285,19 +285,23 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
         const int n = pages_of(s);
 #pragma unroll 1
         for (int i = 0; i < n; ++i) {
-            // a copy that never came: no further ones, nothing is handed back, the host reports the code
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(my_full + 8u * st, ph, kRingSpinLimit, 0));
+            const int left = ctx - (s * pps + w + NW * i) * kKvBlock;      // rows from the page's first on that hold a position
+#pragma unroll 1
+            for (int r0 = 0; r0 < kKvBlock && (r0 == 0 || r0 < left); r0 += SR) {
+                // a copy that never came: no further ones, nothing is handed back, the host reports the code
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(my_full + 8u * st, ph, kRingSpinLimit, 0));
+                if (!ok) break;
+                const unsigned char* kt = ring + st * 2 * SB;
+#pragma unroll 1
+                for (int cc = 0; cc < CPS; ++cc) use_chunk(kt, left - r0, cc * CH);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(my_empty + 8u * st);
+                if (++st == NST) { st = 0; ph ^= 1u; }
+            }
             if (!ok) {
                 if (lane == 0 && p.err != nullptr) atomicExch(p.err, 6);
                 break;
             }
-            const unsigned char* kt = ring + st * 2 * PB;
-            const int cnt = ctx - (s * pps + w + NW * i) * kKvBlock;
-#pragma unroll 1
-            for (int cc = 0; cc < CPP; ++cc) use_chunk(kt, cnt, cc * CH);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(my_empty + 8u * st);
-            if (++st == NST) { st = 0; ph ^= 1u; }
         }
         // merge the PPI lane groups of the warp
 #pragma unroll
@@ -390,6 +394,19 @@ __global__ void __launch_bounds__(attn_threads<G>(), G == 1 ? 5 : (G == 2 ? 3 : 
         p.abuf[((size_t)b * p.heads + h) * HD + e] = o;
         if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
     }
+}
+
+// The kernel for G query heads per CTA: launch(kernel, threads, shared memory), its shared-memory limit raised before.
+template <typename KVT, int HD, int G, typename Launch>
+inline cudaError_t attn_with_kernel(const dim3& grid, int sm_count, Launch launch) {
+    auto run = [&](auto kernel, int rows) {
+        const size_t smem = attn_smem(sizeof(KVT), HD, G, rows);
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e == cudaSuccess ? launch(kernel, attn_threads<G>(), smem) : e;
+    };
+    constexpr int FEW = attn_few_rows(sizeof(KVT), HD, G);
+    if (attn_whole_pages(sizeof(KVT), HD, G, (long)grid.x * grid.y * grid.z, sm_count)) return run(attn_decode_kernel<KVT, HD, G, kKvBlock>, kKvBlock);
+    return run(attn_decode_kernel<KVT, HD, G, FEW>, FEW);
 }
 
 }  // namespace mlb

@@ -198,16 +198,13 @@ struct Chain {
         if (G >= 4 && G % 2 == 0 && s->splits * p.kv_heads * s->B < 2 * s->sm_count) { p.hg = G / 2; G = 2; }
         p.splits = s->splits;
         const dim3 grid = attn_grid(p, s->B, s->sm_count);
-        auto launch = [&](auto kernel, size_t smem, int threads) {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            return e == cudaSuccess ? launch_chain(s->use_pdl, kernel, grid, dim3(threads), smem, s->stream, c, p) : e;
-        };
+        auto launch = [&](auto kernel, int threads, size_t smem) { return launch_chain(s->use_pdl, kernel, grid, dim3(threads), smem, s->stream, c, p); };
         cudaError_t e;
         switch (G) {
-            case 1: e = launch(attn_decode_kernel<KVT, HD, 1>, attn_decode_smem<KVT, HD, 1>(), attn_threads<1>()); break;
-            case 2: e = launch(attn_decode_kernel<KVT, HD, 2>, attn_decode_smem<KVT, HD, 2>(), attn_threads<2>()); break;
-            case 4: e = launch(attn_decode_kernel<KVT, HD, 4>, attn_decode_smem<KVT, HD, 4>(), attn_threads<4>()); break;
-            default: e = launch(attn_decode_kernel<KVT, HD, 8>, attn_decode_smem<KVT, HD, 8>(), attn_threads<8>()); break;
+            case 1: e = attn_with_kernel<KVT, HD, 1>(grid, s->sm_count, launch); break;
+            case 2: e = attn_with_kernel<KVT, HD, 2>(grid, s->sm_count, launch); break;
+            case 4: e = attn_with_kernel<KVT, HD, 4>(grid, s->sm_count, launch); break;
+            default: e = attn_with_kernel<KVT, HD, 8>(grid, s->sm_count, launch); break;
         }
         if (e != cudaSuccess) return fail(MLB_E_CUDA, "attention launch failed: %s", cudaGetErrorString(e));
         return MLB_OK;

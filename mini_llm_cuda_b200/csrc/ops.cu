@@ -66,17 +66,15 @@ cudaError_t launch_attn(const StepCtl& c, AttnParams p, int G, int B, cudaStream
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const dim3 grid = attn_grid(p, B, sm_count);
-    auto launch = [&](auto kernel, size_t smem, int threads) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
+    auto launch = [&](auto kernel, int threads, size_t smem) {
         kernel<<<grid, threads, smem, st>>>(c, p);
         return cudaGetLastError();
     };
     switch (G) {
-        case 1: return launch(attn_decode_kernel<KVT, HD, 1>, attn_decode_smem<KVT, HD, 1>(), attn_threads<1>());
-        case 2: return launch(attn_decode_kernel<KVT, HD, 2>, attn_decode_smem<KVT, HD, 2>(), attn_threads<2>());
-        case 4: return launch(attn_decode_kernel<KVT, HD, 4>, attn_decode_smem<KVT, HD, 4>(), attn_threads<4>());
-        default: return launch(attn_decode_kernel<KVT, HD, 8>, attn_decode_smem<KVT, HD, 8>(), attn_threads<8>());
+        case 1: return attn_with_kernel<KVT, HD, 1>(grid, sm_count, launch);
+        case 2: return attn_with_kernel<KVT, HD, 2>(grid, sm_count, launch);
+        case 4: return attn_with_kernel<KVT, HD, 4>(grid, sm_count, launch);
+        default: return attn_with_kernel<KVT, HD, 8>(grid, sm_count, launch);
     }
 }
 

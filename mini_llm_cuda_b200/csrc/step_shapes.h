@@ -19,4 +19,24 @@ inline int sg_sequences(int batch, int slabs, int sm_count) {
 constexpr int kAttnLoopSplits = 4;                 // most splits that one CTA takes in turn
 inline bool attn_splits_in_turn(int splits, long sequence_groups, int sm_count) { return splits <= kAttnLoopSplits && sequence_groups >= sm_count; }
 
+// Shared memory of decode attention: a ring of two stages of K and V rows for each of four streams of pages, the streams' and the splits' results.
+// A stage is a page of 16 rows, or fewer rows where that lets the CTAs which registers leave room for stand side by side on an SM: with pages
+// alone fp32 rows of 128 took 132 KB, one CTA per SM (64 sequences of 300 positions, 8 heads: 48.4 us in one split, 143 in eight; 35.0 and
+// 49.6 with stages of 4 rows), of 64 with one head per CTA 68 KB, three for five (24.2, 50.0 -> 19.8, 37.4 with 8). Where the launch has too few
+// CTAs for that, pages stay: a stage costs a wait and a hand-back (one sequence of 1000 positions, rows of 128: 28.1 us with pages, 33.5 with 4 rows).
+constexpr int kAttnStreams = 4, kAttnStages = 2, kAttnPageRows = 16;
+constexpr int attn_resident(int heads) { return heads == 1 ? 5 : (heads == 2 ? 3 : (heads == 4 ? 2 : 1)); }      // CTAs per SM, by registers
+constexpr long attn_smem(int kv_bytes, int head_dim, int heads, int rows) {
+    return (long)kAttnStreams * kAttnStages * 2 * rows * head_dim * kv_bytes + (long)(kAttnStreams + kAttnLoopSplits) * heads * (head_dim + 2) * 4;
+}
+// rows per stage where pages leave too little room; bf16 pages leave it, or gain nothing from less (rows of 128, one head: 139 us with pages, 149 with 8)
+constexpr int attn_few_rows(int kv_bytes, int head_dim, int heads) {
+    return kv_bytes == 2 || heads == 8 || (head_dim == 64 && heads > 1) ? kAttnPageRows : (head_dim == 128 && heads == 1 ? 4 : 8);
+}
+inline bool attn_whole_pages(int kv_bytes, int head_dim, int heads, long ctas, int sm_count) {
+    const long per_sm = std::min<long>(attn_resident(heads), (ctas + sm_count - 1) / sm_count);
+    return attn_few_rows(kv_bytes, head_dim, heads) == kAttnPageRows ||
+           attn_smem(kv_bytes, head_dim, heads, kAttnPageRows) <= 227 * 1024 / per_sm - 2048;      // (static shared memory, the system's share)
+}
+
 }  // namespace mlb

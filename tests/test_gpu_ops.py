@@ -106,6 +106,25 @@ def test_attention_op_many_sequences(api, group, hd, dtype_name, splits):
     assert err < 2e-5, err
 
 
+@pytest.mark.parametrize("heads,kv_heads,hd,batch", [(3, 3, 64, 170), (2, 2, 128, 76), (2, 2, 128, 230), (4, 2, 128, 76), (8, 2, 128, 76), (8, 2, 128, 150)])
+@pytest.mark.parametrize("splits", [1, 3, 5])
+def test_attention_op_stages_of_less_than_a_page(api, heads, kv_heads, hd, batch, splits):
+    """fp32 K/V and CTAs enough that stages hold 4 or 8 rows: contexts that end inside the first, on the edges of and inside the last stage of
+    a page; rows behind them hold no numbers."""
+    import torch
+    edges = [1, 3, 4, 5, 7, 8, 9, 12, 13, 15, 16, 17, 20, 24, 25, 63, 68, 72, 73, 129, 200]
+    ctx_list = [edges[b % len(edges)] for b in range(batch)]
+    case = make_attention_case(torch, batch, heads, kv_heads, hd, ctx_list, torch.float32, 7, False)
+    for b, ctx in enumerate(ctx_list):
+        if ctx % 16:
+            page = int(case["table"][b, ctx // 16])
+            case["kpool"][page, :, ctx % 16:] = float("nan")
+            case["vpool"][page, :, ctx % 16:] = float("inf")
+    rc, out = call_attention(api, torch, "mlb_op_attn_decode", case, batch, heads, kv_heads, hd, splits, torch.float32)
+    assert rc == 0, api.lib().mlb_last_error()
+    assert (out.cpu().double() - case["want"]).abs().max().item() < 2e-5
+
+
 def test_attention_op_rejects_bad_arguments(api):
     import torch
     case = make_attention_case(torch, 1, 4, 4, 64, [5], torch.float32, 1, False)

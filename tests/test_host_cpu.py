@@ -318,3 +318,27 @@ def test_splits_in_turn_follow_the_devices_sms(tmp_path):
     assert len(lines) == 24
     for splits, n, sms, turn in lines:
         assert turn == (splits <= 4 and n >= sms)
+
+
+def test_attention_ctas_stand_side_by_side(tmp_path):
+    """Rings of decode attention over fp32 K/V leave as many CTAs room on an SM as registers do, or as the launch has; whole pages where
+    they fit."""
+    out = run_host_program(tmp_path, ["<cstdio>", '"step_shapes.h"'], """
+        for (int kv : {2, 4})
+            for (int hd : {64, 128})
+                for (int heads : {1, 2, 4, 8})
+                    for (long ctas = 1; ctas <= 1000; ++ctas) {
+                        const bool pages = mlb::attn_whole_pages(kv, hd, heads, ctas, 148);
+                        std::printf("%d %d %d %ld %d %d %ld %ld\\n", kv, hd, heads, ctas, (int)pages, mlb::attn_resident(heads),
+                                    mlb::attn_smem(kv, hd, heads, pages ? 16 : mlb::attn_few_rows(kv, hd, heads)), mlb::attn_smem(kv, hd, heads, 16));
+                    }""")
+    seen = set()
+    for kv, hd, heads, ctas, pages, resident, smem, smem_pages in (map(int, line.split()) for line in out.splitlines()):
+        per_sm = min(resident, -(-ctas // 148))
+        if kv == 4:
+            assert per_sm * (smem + 2048) <= 227 * 1024, (hd, heads, ctas)
+            assert pages or per_sm * (smem_pages + 2048) > 227 * 1024, (hd, heads, ctas)
+        else:
+            assert pages
+        seen.add((kv, hd, heads, pages))
+    assert len([x for x in seen if not x[3]]) == 4      # fp32: 64 x 1 head, 128 x 1, 2 and 4
