@@ -87,7 +87,6 @@ __global__ void __launch_bounds__(attn_threads<G>(), attn_resident(G))
     float* sred = reinterpret_cast<float*>(attn_sm + (size_t)NW * NST * 2 * SB);      // [stream][G][HD + 2] of a split
     float* spart = sred + NW * G * W;              // [split][G][HD + 2] where one CTA takes all splits
     __shared__ __align__(8) uint64_t bars[2 * NW * NST];
-    __shared__ float wsm[G][64];
     __shared__ int is_last;
     const int b = blockIdx.z;
     pdl_launch_dependents();
@@ -367,33 +366,45 @@ __global__ void __launch_bounds__(attn_threads<G>(), attn_resident(G))
         __threadfence();
         if (tid == 0) p.ticket[tslot] = 0;
     }
-    // Combine: one warp per head turns the splits' (max, sum) pairs into normalised weights once;
-    // then every thread accumulates its output elements with independent loads.
-    auto get = [&](int g, int s, int e) {
-        return loop ? spart[(s * G + g) * W + e] : __ldcg(p.part + (((size_t)b * p.heads + h0 + g) * SG + s) * W + e);
-    };
-    for (int g = warp; g < G; g += NW * HG) {
-        float m0 = kNegBig, l0 = 0.f, m1 = kNegBig, l1 = 0.f;
-        if (lane < S) { m0 = get(g, lane, HD); l0 = get(g, lane, HD + 1); }
-        if (lane + 32 < S) { m1 = get(g, lane + 32, HD); l1 = get(g, lane + 32, HD + 1); }
-        float mx = fmaxf(m0, m1);
+    // Combine: a warp takes 32 output elements of a head. Its lanes turn the splits' (max, sum) pairs into normalised weights, which it hands
+    // round; the first eight splits' values are asked for with the pairs. (One warp of the CTA doing the weights for all, alone
+    // between two barriers, took 2.1 us of the 4.8 behind the last split at one head per CTA.)
+    auto combine = [&](auto shared) {
+        auto get = [&](int g, int s, int e) {
+            if constexpr (decltype(shared)::value) return spart[(s * G + g) * W + e];
+            else return __ldcg(p.part + (((size_t)b * p.heads + h0 + g) * SG + s) * W + e);
+        };
+        constexpr int AHEAD = 8;
+        for (int i = tid; i < G * HD; i += 32 * NW * HG) {
+            const int g = i / HD, e = i % HD;      // g: the warp's
+            const size_t at = ((size_t)b * p.heads + h0 + g) * HD;
+            float m0 = kNegBig, l0 = 0.f, m1 = kNegBig, l1 = 0.f, v[AHEAD];
+            if (lane < S) { m0 = get(g, lane, HD); l0 = get(g, lane, HD + 1); }
+            if (lane + 32 < S) { m1 = get(g, lane + 32, HD); l1 = get(g, lane + 32, HD + 1); }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float w0 = expf(m0 - mx), w1 = expf(m1 - mx);
-        const float lt = warp_sum(l0 * w0 + l1 * w1);
-        wsm[g][lane] = w0 / lt;
-        wsm[g][lane + 32] = w1 / lt;
-    }
-    sync();
-    for (int i = tid; i < G * HD; i += 32 * NW * HG) {
-        const int g = i / HD, e = i % HD, h = h0 + g;
-        float o = 0.f;
+            for (int s = 0; s < AHEAD; ++s) v[s] = s < S ? get(g, s, e) : 0.f;
+            float mx = fmaxf(m0, m1);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            float w0 = expf(m0 - mx), w1 = expf(m1 - mx);
+            const float lt = warp_sum(l0 * w0 + l1 * w1);
+            w0 /= lt;
+            w1 /= lt;
+            float o = 0.f;
+#pragma unroll
+            for (int s = 0; s < AHEAD; ++s) {
+                const float y = __shfl_sync(0xffffffffu, w0, s);
+                if (s < S) o = fmaf(y, v[s], o);
+            }
 #pragma unroll 4
-        for (int s = 0; s < S; ++s) o = fmaf(wsm[g][s], get(g, s, e), o);
-        if (p.gbuf) o *= p.gbuf[((size_t)b * p.heads + h) * HD + e];
-        p.abuf[((size_t)b * p.heads + h) * HD + e] = o;
-        if (p.abuf16) p.abuf16[((size_t)b * p.heads + h) * HD + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
-    }
+            for (int s = AHEAD; s < S; ++s) o = fmaf(__shfl_sync(0xffffffffu, s < 32 ? w0 : w1, s & 31), get(g, s, e), o);
+            if (p.gbuf) o *= p.gbuf[at + e];
+            p.abuf[at + e] = o;
+            if (p.abuf16) p.abuf16[at + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
+        }
+    };
+    if (loop) combine(std::true_type{});
+    else combine(std::false_type{});
 }
 
 // The kernel for G query heads per CTA: launch(kernel, threads, shared memory), its shared-memory limit raised before.

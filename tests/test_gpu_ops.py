@@ -125,6 +125,19 @@ def test_attention_op_stages_of_less_than_a_page(api, heads, kv_heads, hd, batch
     assert (out.cpu().double() - case["want"]).abs().max().item() < 2e-5
 
 
+@pytest.mark.parametrize("heads,kv_heads,hd,dtype_name", [(2, 2, 64, "bfloat16"), (1, 1, 128, "float32"), (4, 2, 64, "float32"), (8, 1, 128, "bfloat16")])
+@pytest.mark.parametrize("splits", [2, 7, 8, 9, 31, 32, 33, 64])
+def test_attention_op_combines_splits(api, heads, kv_heads, hd, dtype_name, splits):
+    """As many splits as the combine asks for ahead, one more or less, more than a warp has lanes; contexts with fewer pages than splits."""
+    import torch
+    dtype = getattr(torch, dtype_name)
+    ctx_list = [1100, 16 * splits, 16 * splits - 15, 33, 5]
+    case = make_attention_case(torch, 5, heads, kv_heads, hd, ctx_list, dtype, 11, True)
+    rc, out = call_attention(api, torch, "mlb_op_attn_decode", case, 5, heads, kv_heads, hd, splits, dtype)
+    assert rc == 0, api.lib().mlb_last_error()
+    assert (out.cpu().double() - case["want"]).abs().max().item() < 2e-5
+
+
 def test_attention_op_rejects_bad_arguments(api):
     import torch
     case = make_attention_case(torch, 1, 4, 4, 64, [5], torch.float32, 1, False)
