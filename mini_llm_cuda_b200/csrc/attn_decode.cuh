@@ -409,14 +409,15 @@ __global__ void __launch_bounds__(attn_threads<G>(), attn_resident(G))
 
 // The kernel for G query heads per CTA: launch(kernel, threads, shared memory), its shared-memory limit raised before.
 template <typename KVT, int HD, int G, typename Launch>
-inline cudaError_t attn_with_kernel(const dim3& grid, int sm_count, Launch launch) {
+inline cudaError_t attn_with_kernel(const AttnParams& p, const dim3& grid, int sm_count, Launch launch) {
     auto run = [&](auto kernel, int rows) {
         const size_t smem = attn_smem(sizeof(KVT), HD, G, rows);
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         return e == cudaSuccess ? launch(kernel, attn_threads<G>(), smem) : e;
     };
     constexpr int FEW = attn_few_rows(sizeof(KVT), HD, G);
-    if (attn_whole_pages(sizeof(KVT), HD, G, (long)grid.x * grid.y * grid.z, sm_count)) return run(attn_decode_kernel<KVT, HD, G, kKvBlock>, kKvBlock);
+    const long ctas = attn_ctas_with_work((long)grid.y * grid.z, (int)grid.x, p.pt_stride, p.min_pages_per_split);
+    if (attn_whole_pages(sizeof(KVT), HD, G, ctas, sm_count)) return run(attn_decode_kernel<KVT, HD, G, kKvBlock>, kKvBlock);
     return run(attn_decode_kernel<KVT, HD, G, FEW>, FEW);
 }
 

@@ -201,10 +201,10 @@ struct Chain {
         auto launch = [&](auto kernel, int threads, size_t smem) { return launch_chain(s->use_pdl, kernel, grid, dim3(threads), smem, s->stream, c, p); };
         cudaError_t e;
         switch (G) {
-            case 1: e = attn_with_kernel<KVT, HD, 1>(grid, s->sm_count, launch); break;
-            case 2: e = attn_with_kernel<KVT, HD, 2>(grid, s->sm_count, launch); break;
-            case 4: e = attn_with_kernel<KVT, HD, 4>(grid, s->sm_count, launch); break;
-            default: e = attn_with_kernel<KVT, HD, 8>(grid, s->sm_count, launch); break;
+            case 1: e = attn_with_kernel<KVT, HD, 1>(p, grid, s->sm_count, launch); break;
+            case 2: e = attn_with_kernel<KVT, HD, 2>(p, grid, s->sm_count, launch); break;
+            case 4: e = attn_with_kernel<KVT, HD, 4>(p, grid, s->sm_count, launch); break;
+            default: e = attn_with_kernel<KVT, HD, 8>(p, grid, s->sm_count, launch); break;
         }
         if (e != cudaSuccess) return fail(MLB_E_CUDA, "attention launch failed: %s", cudaGetErrorString(e));
         return MLB_OK;

@@ -71,10 +71,10 @@ cudaError_t launch_attn(const StepCtl& c, AttnParams p, int G, int B, cudaStream
         return cudaGetLastError();
     };
     switch (G) {
-        case 1: return attn_with_kernel<KVT, HD, 1>(grid, sm_count, launch);
-        case 2: return attn_with_kernel<KVT, HD, 2>(grid, sm_count, launch);
-        case 4: return attn_with_kernel<KVT, HD, 4>(grid, sm_count, launch);
-        default: return attn_with_kernel<KVT, HD, 8>(grid, sm_count, launch);
+        case 1: return attn_with_kernel<KVT, HD, 1>(p, grid, sm_count, launch);
+        case 2: return attn_with_kernel<KVT, HD, 2>(p, grid, sm_count, launch);
+        case 4: return attn_with_kernel<KVT, HD, 4>(p, grid, sm_count, launch);
+        default: return attn_with_kernel<KVT, HD, 8>(p, grid, sm_count, launch);
     }
 }
 

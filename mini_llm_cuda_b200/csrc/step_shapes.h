@@ -33,6 +33,11 @@ constexpr long attn_smem(int kv_bytes, int head_dim, int heads, int rows) {
 constexpr int attn_few_rows(int kv_bytes, int head_dim, int heads) {
     return kv_bytes == 2 || heads == 8 || (head_dim == 64 && heads > 1) ? kAttnPageRows : (head_dim == 128 && heads == 1 ? 4 : 8);
 }
+// CTAs with work where contexts fill half of the page table: a split with fewer than min_pages has none (8 sequences of 200 of 1024 positions, 8 heads:
+// 64 of 640 CTAs, which pages serve better: 601 us a step, 613 with 8 rows).
+inline long attn_ctas_with_work(long sequence_groups, int grid_splits, int table_pages, int min_pages) {
+    return sequence_groups * std::min(grid_splits, std::max(1, table_pages / 2 / std::max(1, min_pages)));
+}
 inline bool attn_whole_pages(int kv_bytes, int head_dim, int heads, long ctas, int sm_count) {
     const long per_sm = std::min<long>(attn_resident(heads), (ctas + sm_count - 1) / sm_count);
     return attn_few_rows(kv_bytes, head_dim, heads) == kAttnPageRows ||

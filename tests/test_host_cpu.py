@@ -342,3 +342,7 @@ def test_attention_ctas_stand_side_by_side(tmp_path):
             assert pages
         seen.add((kv, hd, heads, pages))
     assert len([x for x in seen if not x[3]]) == 4      # fp32: 64 x 1 head, 128 x 1, 2 and 4
+    out = run_host_program(tmp_path, ["<cstdio>", '"step_shapes.h"'], """
+        std::printf("%ld %ld %ld %ld\\n", mlb::attn_ctas_with_work(64, 10, 64, 11), mlb::attn_ctas_with_work(400, 1, 64, 11),
+                    mlb::attn_ctas_with_work(6, 8, 1, 1), mlb::attn_ctas_with_work(6, 8, 100, 0));""")
+    assert out.split() == ["128", "400", "6", "48"]
