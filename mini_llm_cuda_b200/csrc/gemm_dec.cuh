@@ -28,7 +28,7 @@ namespace mlb {
 constexpr int kGdF = 32;               // output features per CTA
 constexpr int kGdMaxStages = 16;
 constexpr int kGdMaxSplit = 4;         // k-ranges of a tile, a warp per range and 16 rows
-constexpr size_t kGdRing = 108 * 1024; // two CTAs per SM: the next launch's weights arrive under this one
+constexpr size_t kGdRing = 108 * 1024; // two CTAs per SM: the next launch's weights arrive under this one (part of it: gd_ring)
 
 struct GemmDecParams {
     int N, K, B;

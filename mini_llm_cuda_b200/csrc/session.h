@@ -10,6 +10,7 @@
 
 #include "../../include/mlb.h"
 #include "errors.h"
+#include "step_shapes.h"
 #include "attn_decode.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_dec.cuh"
@@ -290,17 +291,14 @@ static GdShape gd_pick(const mlb_session* s, int N, int nkb, int mode, bool w8, 
     while (g.np > 1 && (16 * (g.np / 2) >= s->B || (long)((N + kGdF - 1) / kGdF) * ((s->B + 16 * g.np - 1) / (16 * g.np)) < 96)) g.np >>= 1;
     g.w_bytes = kGdF * (w8 && !ext ? 64 : 128);
     const int ct = 16 * g.np;
-    // Two CTAs per SM share its shared memory, so that the next launch's weights arrive under this one; eight where there are more CTAs
-    // than two per SM: a CTA's own chain of barriers, operands and epilogue bounds those, and more of them side by side hide it (LM head of 8192
-    // features, 256 sequences, 1024 CTAs of 512: 35.5 us with two per SM, 20.8 with four, 15.3 with eight; of 32000 x 2048, e4m3, 64 sequences:
-    // 106 with two, 82 with eight).
     const long ctas = (long)((N + kGdF - 1) / kGdF) * ((s->B + 16 * g.np - 1) / (16 * g.np));
-    const size_t ring = ctas > 2L * s->sm_count ? kGdRing / 4 : kGdRing;
+    const size_t block = (size_t)g.split * (na * g.w_bytes + ct * 128);      // a stage of one k-block per copy
+    const size_t ring = gd_ring(kGdRing, ctas, s->sm_count, mode == TC_SWIGLU, block * std::min(2, (nkb + g.split - 1) / g.split + (ext ? 1 : 0)));
     // k-blocks per copy: as many as leave two stages
     size_t stage = 0;
     int n_iter = 1;
     for (g.g = 4;; g.g >>= 1) {
-        stage = (size_t)g.split * g.g * (na * g.w_bytes + ct * 128);
+        stage = block * g.g;
         n_iter = ((nkb + g.split - 1) / g.split + g.g - 1) / g.g + (ext ? 1 : 0);
         if (g.g == 1 || stage * std::min(2, n_iter) <= ring) break;
     }

@@ -1,6 +1,7 @@
 // Launch shapes of a decode step that follow from sizes alone: plain C++, so that their rules can be held to on the CPU.
 #pragma once
 #include <algorithm>
+#include <cstddef>
 
 namespace mlb {
 
@@ -42,6 +43,18 @@ inline bool attn_whole_pages(int kv_bytes, int head_dim, int heads, long ctas, i
     const long per_sm = std::min<long>(attn_resident(heads), (ctas + sm_count - 1) / sm_count);
     return attn_few_rows(kv_bytes, head_dim, heads) == kAttnPageRows ||
            attn_smem(kv_bytes, head_dim, heads, kAttnPageRows) <= 227 * 1024 / per_sm - 2048;      // (static shared memory, the system's share)
+}
+
+// Ring of a decode GEMM CTA. Two CTAs per SM share its shared memory, so that the next launch's weights arrive under this one. Where there are
+// more CTAs than two per SM, a CTA's own chain of barriers, operands and epilogue bounds the launch, and more of them side by side hide
+// it: a quarter or half of the ring, the least that holds two stages. LM heads of 256 sequences: 8192 x 512, stages of 12 KB, 35.5 us with
+// whole rings, 15.3 with quarters; step of four layers with 384 or 304 CTAs in one projection, whole / half / quarter (two, two, one
+// stage of 24 KB): QKV of 3072 x 1024 357 / 332 / 344 us, residual of 2432 x 896 616 / 584 / 606; QKV of 3072 x 2432 (48 KB: 2, 1, 1)
+// 560 / 605 / 605. Gate/up keeps the whole ring: its CTAs have twice the warps and operands (3584 x 512, 448 CTAs: 241 / 249 / 249 us, e4m3
+// 277 / 293 / 307).
+inline size_t gd_ring(size_t whole, long ctas, int sm_count, bool gate_up, size_t two_stages) {
+    if (ctas <= 2L * sm_count || gate_up) return whole;
+    return two_stages <= whole / 4 ? whole / 4 : (two_stages <= whole / 2 ? whole / 2 : whole);
 }
 
 }  // namespace mlb

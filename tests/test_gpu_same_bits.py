@@ -82,6 +82,28 @@ def test_step_projections_of_more_ctas_than_two_per_sm(api, tmp_path, monkeypatc
     model.close()
 
 
+@pytest.mark.parametrize("weight_dtype", ["bfloat16", "float8_e4m3"])
+def test_wide_step_projections_of_more_ctas_than_two_per_sm(api, tmp_path, monkeypatch, weight_dtype):
+    """QKV, delta-net projections, gate/up and residual launches (with and without the next layer's embedding) of 304 to 388 CTAs at 250 and 256
+    sequences, stages of one k-block per range, against the tcgen05 tiles."""
+    monkeypatch.setenv("MLB_PREFILL", "step")
+    spec = ModelSpec(dim=2432, layers=3, heads=16, head_dim=64, ffn_dim=2432, ple_dim=64, vocab=500, max_context=32, rms_eps=1e-5, kv_dtype="bfloat16",
+                     layer_types=["attention", "delta_net", "attention"], weight_dtype=weight_dtype)
+    model = api.Model(write_model(tmp_path, spec, seed=123))
+    for batch in (250, 256):
+        prompts = random_prompts(spec.vocab, [1 + b % 2 for b in range(batch)], seed=125)
+        got = {}
+        for tiles in ("mma", "tcgen05"):
+            monkeypatch.setenv("MLB_GEMM", tiles)
+            sess = api.Session(model, batch)
+            assert sess.path() == tiles
+            sess.prefill(prompts)
+            got[tiles] = sess.decode(2), sess.logits()
+            sess.close()
+        assert np.array_equal(got["mma"][0], got["tcgen05"][0]) and np.array_equal(got["mma"][1], got["tcgen05"][1]), batch
+    model.close()
+
+
 @pytest.mark.parametrize("name", [*SPECS, *QK_NORM, *RAGGED])
 def test_columns_against_the_decode_steps_kernels(api, tmp_path, monkeypatch, name):
     """129 to 256 columns (one set, whose k-ranges are those that every width takes): every position's logits."""

@@ -346,3 +346,20 @@ def test_attention_ctas_stand_side_by_side(tmp_path):
         std::printf("%ld %ld %ld %ld\\n", mlb::attn_ctas_with_work(64, 10, 64, 11), mlb::attn_ctas_with_work(400, 1, 64, 11),
                     mlb::attn_ctas_with_work(6, 8, 1, 1), mlb::attn_ctas_with_work(6, 8, 100, 0));""")
     assert out.split() == ["128", "400", "6", "48"]
+
+
+def test_rings_of_decode_gemms_hold_two_stages(tmp_path):
+    """A launch of more CTAs than two per SM takes the least of a quarter, half and whole ring in which a copy can run under the products;
+    gate/up launches and those of fewer CTAs the whole ring."""
+    out = run_host_program(tmp_path, ["<cstdio>", '"step_shapes.h"'], """
+        const size_t whole = 108 * 1024;
+        for (long ctas : {1, 296, 297, 1024})
+            for (int gate_up = 0; gate_up < 2; ++gate_up)
+                for (size_t kb = 4; kb <= 160; kb += 2)
+                    std::printf("%ld %d %zu %zu\\n", ctas, gate_up, kb, mlb::gd_ring(whole, ctas, 148, gate_up, kb * 1024) / 1024);""")
+    for ctas, gate_up, two_stages, ring in (map(int, line.split()) for line in out.splitlines()):
+        if ctas <= 296 or gate_up:
+            assert ring == 108
+        else:
+            assert ring in (27, 54, 108) and (ring >= two_stages or ring == 108)
+            assert ring == 27 or two_stages > ring // 2
