@@ -804,11 +804,6 @@ static cudaError_t gemm_cols_one(bool pdl, int ctas, cudaStream_t st, const CUte
                                  const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c, const QkvPostParams& q) {
     cudaError_t e = cudaFuncSetAttribute(gemm_cols_kernel<MODE, KVT, SUMS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGcSmem);
     if (e != cudaSuccess) return e;
-    if (SUMS) {
-        cudaFuncAttributes a;
-        if ((e = cudaFuncGetAttributes(&a, gemm_cols_kernel<MODE, KVT, SUMS, PAIR>)) != cudaSuccess) return e;
-        if (a.numRegs != kGcRegsLaunch) return cudaErrorInvalidConfiguration;      // its register shares would not add up
-    }
     const size_t smem = 1024 + (size_t)p.stages * (kGcM + (PAIR ? p.BN / 2 : p.BN)) * 128 + gc_staging(MODE);
     return launch_pdl_cluster(pdl, PAIR ? 2 : 1, gemm_cols_kernel<MODE, KVT, SUMS, PAIR>, dim3(ctas), dim3(kGcThreads), smem, st, x, w, w2, xx, wx, p, c, q);
 }
@@ -825,6 +820,30 @@ static cudaError_t gemm_cols_mode(int mode, int kv_dtype, bool pdl, int ctas, cu
             if (kv_dtype == MLB_DT_F32) return gemm_cols_one<TC_QKV, float, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
             return gemm_cols_one<TC_QKV, bf16_t, SUMS, PAIR>(pdl, ctas, st, x, w, w2, xx, wx, p, c, q);
     }
+}
+
+// The register shares of the kernels with sums add up only at kGcRegsLaunch registers a thread, which a compiler chooses: with another count their
+// warps would wait for registers without end.
+template <int MODE, typename KVT, bool PAIR>
+static cudaError_t gemm_cols_shares(bool* ok) {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, gemm_cols_kernel<MODE, KVT, true, PAIR>);
+    *ok = *ok && e == cudaSuccess && a.numRegs == kGcRegsLaunch;
+    return e;
+}
+template <bool PAIR>
+static cudaError_t gemm_cols_shares_of(bool* ok) {
+    cudaError_t e = gemm_cols_shares<TC_RAW, float, PAIR>(ok);
+    if (e == cudaSuccess) e = gemm_cols_shares<TC_RESID, float, PAIR>(ok);
+    if (e == cudaSuccess) e = gemm_cols_shares<TC_SWIGLU, float, PAIR>(ok);
+    if (e == cudaSuccess) e = gemm_cols_shares<TC_QKV, float, PAIR>(ok);
+    if (e == cudaSuccess) e = gemm_cols_shares<TC_QKV, bf16_t, PAIR>(ok);
+    return e;
+}
+cudaError_t gemm_cols_can_sum(bool* ok) {
+    *ok = true;
+    const cudaError_t e = gemm_cols_shares_of<false>(ok);
+    return e == cudaSuccess ? gemm_cols_shares_of<true>(ok) : e;
 }
 
 cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pair, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,

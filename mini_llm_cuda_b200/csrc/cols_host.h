@@ -58,6 +58,8 @@ cudaError_t embed_cols_launch(bool w8, bool pdl, cudaStream_t st, const StepCtl&
 // ---- projections of a chunk ----------------------------------------------------------------------
 struct GemmColsParams;
 struct QkvPostParams;
+// Whether launches with `sums` may be made: as the library's compiler left the kernels. The others serve without.
+cudaError_t gemm_cols_can_sum(bool* ok);
 // `mode` a GemmTcMode; raises the kernel's shared-memory limit on first use.
 cudaError_t gemm_cols_launch(int mode, int kv_dtype, bool sums, bool pair, bool pdl, int ctas, cudaStream_t st, const CUtensorMap& x, const CUtensorMap& w,
                              const CUtensorMap& w2, const CUtensorMap& xx, const CUtensorMap& wx, const GemmColsParams& p, const StepCtl& c,

@@ -924,7 +924,8 @@ static int model_widen(mlb_model* m, cudaStream_t st, bool* have) {
 // at 256, hidden under the next tile's k-loop where there are two buffers; the cheapest in the sum over a CTA's tiles wins. More ranges than
 // one: sums in registers (64 a thread, 128 in a pair) over accumulators in turn, except under a QK norm, which looks a head's features up in
 // tensor memory. A pair's two accumulators leave room for one range of a second pair. MLB_COLS_PAIR=0|1: never | wherever it can run.
-static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode, bool exts_apart, int split, int min_bn, bool qk_norm) {
+// Without sums (gemm_cols_can_sum, MLB_COLS_SUMS=0) every range has its accumulators until the tile's epilogue.
+static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode, bool exts_apart, int split, int min_bn, bool qk_norm, bool can_sum) {
     ColsGemm best{};
     double best_cost = -1.0;
     static const int bns[3] = {256, 128, 64};
@@ -935,7 +936,7 @@ static ColsGemm gc_pick(int sm_count, int T, int N, int nkb, int nkb_x, int mode
         if (exts_apart ? lo < nkb - nkb_x : hi > lo) ++mains;
         if (exts_apart && hi > nkb - nkb_x) ++exts;
     }
-    const bool sums = mains + exts > 1 && !(mode == TC_QKV && qk_norm) && exts < kGcMaxBufs;
+    const bool sums = can_sum && mains + exts > 1 && !(mode == TC_QKV && qk_norm) && exts < kGcMaxBufs;
     auto consider = [&](int bn, bool pair, int nbuf, double t_kb) {
         const int bn_out = mode == TC_SWIGLU ? bn / 2 : bn, rows = pair ? 2 * kGcM : kGcM, teams = pair ? sm_count / 2 : sm_count;
         const long tiles = (long)((T + rows - 1) / rows) * ((N + bn_out - 1) / bn_out);
@@ -994,12 +995,14 @@ static int setup_cols_path(mlb_session* s) {
     // The ranges of k-blocks are those of gemm_tc_kernel's launches with kTcRefCols columns, whatever the width of this set, so
     // that a prompt's cache does not depend on how it is cut into chunks.
     if ((rc = tc_probe_clusters(s))) return rc;
-    bool fits = true;
+    bool fits = true, can_sum = true;
+    CU(gemm_cols_can_sum(&can_sum));
+    if (const char* v = std::getenv("MLB_COLS_SUMS")) can_sum = can_sum && v[0] != '0';
     auto pick = [&](int N, int nkb, int nkb_x, int mode, bool apart) {
         const bool resid8 = w8 && mode == TC_RESID;
         const TcShape ref = tc_pick_shape(s, kTcRefCols, N, nkb, mode == TC_SWIGLU ? 2 : 1, w8, mode == TC_SWIGLU || resid8 ? 2 : 1);
         const ColsGemm g = gc_pick(s->sm_count, T, N, nkb, nkb_x, mode, apart, std::max(1, ref.split),
-                                    mode == TC_QKV && c.qk_norm ? c.head_dim : 64, c.qk_norm != 0);       // a tile holds whole heads for their norm
+                                    mode == TC_QKV && c.qk_norm ? c.head_dim : 64, c.qk_norm != 0, can_sum);       // a tile holds whole heads for their norm
         fits = fits && g.bn > 0;
         return g;
     };
@@ -1011,7 +1014,7 @@ static int setup_cols_path(mlb_session* s) {
     s->cg_down = pick(c.dim, kb(c.ffn_dim) + kb(c.ple_dim), kb(c.ple_dim), TC_RESID, ext2);
     s->cg_last = pick(c.dim, kb(c.ffn_dim), 0, TC_RESID, false);
     s->cg_head = pick(c.vocab, kb(c.dim), 0, TC_RAW, false);
-    if (!fits) return MLB_OK;      // a forced split that tensor memory does not hold
+    if (!fits) return MLB_OK;      // ranges that tensor memory does not hold (a forced split, no sums)
     if ((rc = sess_alloc(s, (void**)&s->xn16, (size_t)T * c.dim * 2, true))) return rc;
     if ((rc = sess_alloc(s, (void**)&s->a16, (size_t)T * std::max(nq, a_dn) * 2, true))) return rc;
     if ((rc = sess_alloc(s, (void**)&s->h16, (size_t)T * c.ffn_dim * 2, true))) return rc;

@@ -144,6 +144,28 @@ def test_column_tiles_over_two_ctas(api, tmp_path, monkeypatch, name):
     model.close()
 
 
+@pytest.mark.parametrize("name", ["bf16", "bf16_gqa_gated", "fp8", "fp8_eight_ranges"])
+def test_column_gemms_without_sums(api, tmp_path, monkeypatch, name):
+    """Kernels with sums in registers may be unusable as a compiler left them: prompts and scores run without them, on column GEMMs that hold every
+    range in tensor memory, or where they do not fit on the decode step's (eight ranges of codes and the embedding's)."""
+    spec = {**SPECS, "fp8_eight_ranges": dataclasses.replace(SPECS["fp8"], ffn_dim=4096, layers=2, layer_types=["attention"] * 2)}[name]
+    model = api.Model(write_model(tmp_path, dataclasses.replace(spec, max_context=700), seed=127))
+    text = random_prompts(spec.vocab, [600], seed=129)[0]
+    lens = (200,) if name == "fp8_eight_ranges" else (70, 200, 600)
+    got = {}
+    for sums in (None, "0"):
+        if sums:
+            monkeypatch.setenv("MLB_COLS_SUMS", sums)
+        sess = api.Session(model, 1)
+        for n in lens:
+            got[sums, n] = sess.score(text[:n])
+            assert sess.path(n) == ("tcgen05" if sums and name == "fp8_eight_ranges" else "cols")
+        sess.close()
+    for n in lens:
+        assert np.array_equal(got[None, n], got["0", n]), n
+    model.close()
+
+
 @pytest.mark.parametrize("dk,dv,heads,batch,uneven", [(64, 72, 3, 1, 0), (128, 128, 4, 1, 0), (64, 64, 4, 48, 0), (128, 72, 3, 48, 0), (64, 64, 4, 48, 1),
                                                       (128, 72, 3, 48, 1)])
 def test_recurrence_over_columns_against_steps(api, tmp_path, monkeypatch, dk, dv, heads, batch, uneven):
