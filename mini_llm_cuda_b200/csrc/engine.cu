@@ -6,7 +6,6 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
-#include <numeric>
 
 #include "session.h"
 #include "cols_host.h"
@@ -1493,47 +1492,13 @@ static int prefill_columns(mlb_session* s, const int32_t* tokens, const int32_t*
     // A chunk takes the next tokens of as many sequences as it can, an equal share each: the
     // delta-net recurrence is serial along a sequence and parallel across sequences. Columns stay grouped by
     // sequence, positions ascending.
-    std::vector<int> cursor(B, 0), take(B), order(B);
+    std::vector<int> cursor(B, 0), rest(B), take(B);
     long left = total;
     for (int slot = 0; left > 0; slot = (slot + 1) % kPlanSlots) {
         if ((rc = get(left))) return rc;
         const int want = (int)std::min<long>(left, cs->B);
-        // the largest equal share that fits; what is left over goes to the first sequences
-        int lo = 0, hi = want;
-        auto filled = [&](int share) {
-            long n = 0;
-            for (int b = 0; b < B; ++b) n += std::min(share, lens[b] - keep - cursor[b]);
-            return n;
-        };
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) / 2;
-            if (filled(mid) <= want) lo = mid; else hi = mid - 1;
-        }
-        int extra = want - (int)filled(lo);
-        // A share that ends inside an attention tile leaves the tile's other rows idle (256 sequences: 16 of 32 rows of every tile). It
-        // is rounded up to whole tiles, for as many of the sequences furthest behind as then fit; the others come with the next chunk
-        // (request of 256 prompts of 256 tokens, 8 heads of 64: 104.7 -> 95.5 ms).
-        std::fill(take.begin(), take.end(), 0);
-        bool all = true;
-        for (int b = 0; b < B; ++b) all = all && lens[b] - keep - cursor[b] <= lo;
-        if (has_attn && !f32 && !all && lo > 0 && (lo % qt || extra > 0)) {
-            const int share = (lo + qt - 1) / qt * qt;
-            std::iota(order.begin(), order.end(), 0);
-            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cursor[x] < cursor[y]; });
-            int room = want;
-            for (const int b : order) {
-                const int most = std::min(lens[b] - keep - cursor[b], share);
-                const int t = most <= room ? most : room / qt * qt;
-                take[b] = t;
-                room -= t;
-            }
-        } else {
-            for (int b = 0; b < B; ++b) {
-                const int rest = lens[b] - keep - cursor[b];
-                take[b] = std::min(rest, lo);
-                if (extra > 0 && take[b] < rest) { ++take[b]; --extra; }
-            }
-        }
+        for (int b = 0; b < B; ++b) rest[b] = lens[b] - keep - cursor[b];
+        cols_shares(rest, cursor, want, has_attn && !f32 ? qt : 0, take);
         const ColsLayout lay = cols_layout(cfg, s->B, cs->B);
         int* pl = s->plan_host + slot * s->plan_host_ints;
         CU(cudaEventSynchronize(s->plan_free[slot]));      // the slot's last plan has left it, also one of a call that failed half-way

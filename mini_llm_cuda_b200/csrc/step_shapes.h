@@ -1,7 +1,9 @@
-// Launch shapes of a decode step that follow from sizes alone: plain C++, so that their rules can be held to on the CPU.
+// Launch shapes of decode steps and prompt chunks that follow from sizes alone: plain C++, so that their rules can be held to on the CPU.
 #pragma once
 #include <algorithm>
 #include <cstddef>
+#include <numeric>
+#include <vector>
 
 namespace mlb {
 
@@ -55,6 +57,44 @@ inline bool attn_whole_pages(int kv_bytes, int head_dim, int heads, long ctas, i
 inline size_t gd_ring(size_t whole, long ctas, int sm_count, bool gate_up, size_t two_stages) {
     if (ctas <= 2L * sm_count || gate_up) return whole;
     return two_stages <= whole / 4 ? whole / 4 : (two_stages <= whole / 2 ? whole / 2 : whole);
+}
+
+// What a prompt chunk of `want` columns takes of each sequence: rest[b] tokens wait, cursor[b] were taken before. The largest equal share that
+// fits; what is left over goes to the first sequences, one token each. With attention tiles of `tile` > 0 queries a share that ends inside one
+// leaves the tile's other rows idle (256 sequences: 16 of 32 rows of every tile). It is rounded up to whole tiles, for as many of the sequences
+// furthest behind as then fit, the last of them with what room there is: the chunk is full either way, so that a prompt takes no more
+// chunks (request of 256 prompts of 256 tokens, 8 heads of 64: 104.7 -> 95.5 ms).
+inline void cols_shares(const std::vector<int>& rest, const std::vector<int>& cursor, int want, int tile, std::vector<int>& take) {
+    const int B = (int)rest.size();
+    take.assign(B, 0);
+    auto filled = [&](int share) {
+        long n = 0;
+        for (int r : rest) n += std::min(share, r);
+        return n;
+    };
+    int lo = 0, hi = want;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (filled(mid) <= want) lo = mid; else hi = mid - 1;
+    }
+    int extra = want - (int)filled(lo);
+    const bool all = std::all_of(rest.begin(), rest.end(), [&](int r) { return r <= lo; });
+    if (tile > 0 && !all && lo > 0 && (lo % tile || extra > 0)) {
+        const int share = (lo / tile + 1) * tile;      // (more than fits for all)
+        std::vector<int> order(B);
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cursor[x] < cursor[y]; });
+        int room = want;
+        for (const int b : order) {
+            take[b] = std::min(std::min(rest[b], share), room);
+            room -= take[b];
+        }
+    } else {
+        for (int b = 0; b < B; ++b) {
+            take[b] = std::min(rest[b], lo);
+            if (extra > 0 && take[b] < rest[b]) { ++take[b]; --extra; }
+        }
+    }
 }
 
 }  // namespace mlb

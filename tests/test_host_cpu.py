@@ -363,3 +363,38 @@ def test_rings_of_decode_gemms_hold_two_stages(tmp_path):
         else:
             assert ring in (27, 54, 108) and (ring >= two_stages or ring == 108)
             assert ring == 27 or two_stages > ring // 2
+
+
+def test_prompt_chunks_are_full(tmp_path):
+    """Shares of a chunk, in whole attention tiles where they can be: every chunk but the last is full, so a prompt takes as many chunks as its tokens
+    need; equal prompts get whole tiles."""
+    out = run_host_program(tmp_path, ["<cstdio>", '"step_shapes.h"'], """
+        unsigned state = 1;
+        auto rnd = [&](int n) { state = state * 1664525u + 1013904223u; return (int)((state >> 8) % (unsigned)n); };
+        for (int round = 0; round < 4000; ++round) {
+            const int batches[] = {1, 2, 3, 8, 37, 64, 200, 256}, B = batches[rnd(8)], longest = 1 + rnd(16000 / B), tile = (round % 4) ? 32 >> rnd(4) : 0;
+            std::vector<int> rest(B), cursor(B, 0), take;
+            long left = 0;
+            for (int& r : rest) left += r = rnd(5) ? rnd(longest + 1) : longest;
+            while (left > 0) {
+                const int want = (int)std::min<long>(left, 4096);
+                mlb::cols_shares(rest, cursor, want, tile, take);
+                long n = 0;
+                int parts = 0, bad = 0;
+                for (int b = 0; b < B; ++b) {
+                    bad += take[b] < 0 || take[b] > rest[b];
+                    parts += tile > 0 && take[b] % tile != 0 && take[b] < rest[b];
+                    n += take[b];
+                    rest[b] -= take[b];
+                    cursor[b] += take[b];
+                }
+                std::printf("%d %ld %d %d %d\\n", want, n, bad, tile, parts);
+                if (n != want) return 0;
+                left -= n;
+            }
+        }""")
+    lines = [tuple(map(int, line.split())) for line in out.splitlines()]
+    assert len(lines) > 4000
+    for want, n, bad, tile, parts in lines:
+        assert n == want and bad == 0
+        assert tile == 0 or parts <= 1 or want < 32 * 8, (want, tile, parts)
