@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "cols_host.h"
+#include "cols_math.h"
 #include "../../include/mlb.h"
 #include "gemm_cols.cuh"
 
@@ -148,10 +149,7 @@ __global__ void __launch_bounds__(kAcThreads, 1) attn_cols_kernel(AttnColsParams
         q[r][0] = pack2(x0.x, y0.x); q[r][1] = pack2(x0.y, y0.y); q[r][2] = pack2(x0.z, y0.z); q[r][3] = pack2(x0.w, y0.w);
         q[r][4] = pack2(x1.x, y1.x); q[r][5] = pack2(x1.y, y1.y); q[r][6] = pack2(x1.z, y1.z); q[r][7] = pack2(x1.w, y1.w);
     }
-    // x / sqrtf(HD), correctly rounded, without a division's branches: by its reciprocal (HD 64: a power of two), for HD 128 by the two-word
-    // reciprocal zh + zl of sqrtf(128) (Brisebarre, Muller, Raina 2004: division by a divisor known in advance; all 2^23 significands
-    // compared with the division). Infinities stay, as zl > 0; below 2^-90 a last place may differ, which no exponential sees.
-    auto scaled = [](float x) { return HD == 64 ? x * 0.125f : fmaf(x, 0x1.6a09e6p-4f, __fmul_rn(x, 0x1.9fcef4p-29f)); };
+    auto scaled = [](float x) { return HD == 64 ? x * 0.125f : over_sqrt128(x); };      // x / sqrtf(HD)
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
         const int n_t = np > 2 * pass ? ((np - 2 * pass + 3) / 4 + 1) / 2 : 0;         // tiles: of the pass's first w, which has the most pages

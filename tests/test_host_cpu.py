@@ -398,3 +398,23 @@ def test_prompt_chunks_are_full(tmp_path):
     for want, n, bad, tile, parts in lines:
         assert n == want and bad == 0
         assert tile == 0 or parts <= 1 or want < 32 * 8, (want, tile, parts)
+
+
+def test_scores_over_sqrt128_are_the_division(tmp_path):
+    """Prompt attention at head size 128 multiplies by a two-word reciprocal: the quotient for every significand, in a middle binade and
+    at both ends of the range in which it is meant to be exact; infinities, zeros and what is no number stay."""
+    out = run_host_program(tmp_path, ["<cstdio>", "<cstdint>", "<cstring>", "<initializer_list>", '"cols_math.h"'], """
+        volatile float divisor = std::sqrt(128.0f);
+        const float d = divisor;
+        long wrong = 0;
+        for (uint32_t exponent : {127u, 127u - 90u, 254u})
+            for (uint32_t frac = 0; frac < (1u << 23); ++frac) {
+                const uint32_t bits = (exponent << 23) | frac;
+                float x;
+                std::memcpy(&x, &bits, 4);
+                wrong += mlb::over_sqrt128(x) != x / d;
+                wrong += mlb::over_sqrt128(-x) != -x / d;
+            }
+        std::printf("%ld %g %g %g %g %d\\n", wrong, mlb::over_sqrt128(INFINITY), mlb::over_sqrt128(-INFINITY), mlb::over_sqrt128(0.f), mlb::over_sqrt128(-0.f),
+                    (int)std::isnan(mlb::over_sqrt128(NAN)));""")
+    assert out.split() == ["0", "inf", "-inf", "0", "-0", "1"]
