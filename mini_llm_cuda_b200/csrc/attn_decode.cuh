@@ -9,13 +9,14 @@
 //
 // A stream takes the pages w, w + 4, .. of a split (w = 0 .. 3). The 16 rows of a head in a page are one contiguous block, so
 // one lane copies a page's K and V rows (or a half or a quarter of them: attn_few_rows) with two bulk copies into the stream's own ring of
-// shared-memory stages: no registers hold loads in flight. With four query heads or more per kv head a stream has a warp per two of them, which share its ring.
+// shared-memory stages: no registers hold loads in flight. With four query heads or more per kv head a stream has a warp per two of
+// them, which share its ring.
 // In a decode session the K/V rows of earlier tokens were written by earlier steps, which are complete when a step's first
 // kernel starts (it is launched without overlap): only the page of the current position and the queries wait for the predecessor.
 // The scores of four positions per lane group and GW heads are summed over the lanes by a butterfly that leaves every lane
 // its share of them, so that a score is divided and its exponential taken once and not by every lane of the group. Sums,
 // maxima and products are those of a butterfly over every score, in its order.
-// What bounds it: with one head per kv head HBM and the start of each CTA (256 sequences of 320 positions, 8 heads of 64: 32.9 us,
+// What bounds it: with one head per kv head HBM and the start and end of each CTA (256 sequences of 320 positions, 8 heads of 64: 32.9 us,
 // 5.1 TB/s; 36.8 with per-thread loads); with four the chain of a chunk (scores, butterfly, exponentials, products: 550 cycles) under
 // few warps (64 sequences of 528, 16 heads over 4 of 128, three splits: 57.5 -> 27.7 us, 2.5 TB/s).
 // ------------------------------------------------------------------------------------

@@ -918,8 +918,8 @@ static int model_widen(mlb_model* m, cudaStream_t st, bool* have) {
 
 // Launch shape of a column GEMM: `T` columns, `N` output features, `nkb` k-blocks of 64, the last `nkb_x` of a second
 // operand pair (`exts_apart`: with accumulators of its own), in `split` ranges. Tensor memory (512 columns) bounds BN x
-// accumulators x buffers. A 128 x BN x 64 k-block takes about 0.43 / 0.36 / 0.26 us at BN = 256 / 128 / 64 with every SM at it: its
-// operand bytes (48 / 32 / 24 KB) at what an SM gets from L2. A pair of CTAs has one of 256 x 256 in 0.42 (32 KB each). An epilogue takes 3 us
+// accumulators x buffers. A 128 x BN x 64 k-block takes about 0.43 / 0.36 / 0.26 us at BN = 256 / 128 / 64 with every SM at it: the tensor
+// pipe's rate at 256 (1.44 PFLOP/s), its operands below (32, 24 KB at about 90 GB/s an SM). A pair of CTAs has one of 256 x 256 in 0.42. An epilogue takes 3 us
 // at 256, hidden under the next tile's k-loop where there are two buffers; the cheapest in the sum over a CTA's tiles wins. More ranges than
 // one: sums in registers (64 a thread, 128 in a pair) over accumulators in turn, except under a QK norm, which looks a head's features up in
 // tensor memory. A pair's two accumulators leave room for one range of a second pair. MLB_COLS_PAIR=0|1: never | wherever it can run.

@@ -11,9 +11,11 @@
 //   warps 2, 3 nothing: they complete the warpgroup that gives its registers to the epilogue's
 //   warps 4-11 epilogue of the other accumulator: two warps per TMEM lane quarter, half of the columns each
 // PAIR: two CTAs (the SMs of a TPC) share a tile of 256 columns x 256 features (tcgen05 cta_group::2): each loads its own 128 columns and half of
-// the weight rows, so that a k-block costs an SM 32 KB for 128 x 256 products where a lone CTA loads 32 KB for 128 x 128 or 48 KB for 128 x 256;
-// what an SM gets from L2 (about 100 GB/s with all of them at it) bounds the k-loop. 4096 columns, 2048 features: O 94 -> 61 us, down (K 5632)
-// 177 -> 105, QKV (3072) 88 -> 77, delta-net projections (6176) 142 -> 94 with pairs, the register shares below and staged residuals.
+// the weight rows. What bounds the k-loop: the tensor pipe at 256 features (128 x 256 x 64 in 0.43 us on every SM, 1.44 PFLOP/s; a pair's 256 x 256
+// 0.42, 1.48), below that the operands (32 KB in 0.36 us at 128 features, 24 KB in 0.26 at 64: about 90 GB/s an SM). A lone CTA whose epilogue adds up
+// ranges has registers for 128 features, a pair for 256: that is what pairs give. 4096 columns, 2048 features: O 94 -> 61 us, down
+// (K 5632) 177 -> 105, QKV (3072) 88 -> 77, delta-net projections (6176) 142 -> 94 with pairs, the register shares below and staged residuals;
+// gate/up (11264), which has no ranges to add up, 144 -> 140.
 // One CTA per SM walks tiles of the output; the epilogue of a tile runs under the k-loop of the next one where tensor
 // memory holds the accumulators twice.
 // FP8 weights come as an exact bf16 copy of their codes; their row scales are applied to the accumulator, and the bf16
@@ -37,8 +39,8 @@ constexpr int kGcM = 128;
 constexpr int kGcEpiWarps = 8;
 constexpr int kGcThreads = 128 + 32 * kGcEpiWarps;
 // Registers of a thread of a kernel with sums (SUMS), at launch (what 384 threads leave each), then of warps 0 - 3 and of the epilogue's:
-// 128 sums and an epilogue's values do not fit 168. The shares add up to what the block was launched with (checked before the launch: a
-// share that the block does not own would be waited for without end).
+// 128 sums and an epilogue's values do not fit 168. The shares add up to what the block was launched with (checked where a column set is made,
+// gemm_cols_can_sum: a share that the block does not own would be waited for without end).
 constexpr int kGcRegsLaunch = 168, kGcRegsFew = 40, kGcRegsMany = 232;
 static_assert(128 * kGcRegsFew + 32 * kGcEpiWarps * kGcRegsMany <= kGcThreads * kGcRegsLaunch, "register shares");
 constexpr int kGcMaxStages = 8;

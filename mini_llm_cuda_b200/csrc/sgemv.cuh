@@ -6,7 +6,7 @@
 // at a tenth of the HBM bandwidth. Here the matrix is cut into one contiguous slab of rows per CTA
 // (about one CTA per SM). A producer warp streams the slab with cp.async.bulk into a ring of
 // shared-memory stages guarded by mbarriers - and it starts BEFORE griddepcontrol.wait, because
-// weights do not depend on the predecessor kernel - while 15 consumer warps stage and normalise
+// weights do not depend on the predecessor kernel - while 31 consumer warps stage and normalise
 // the activation vector once, then take dot products out of shared memory two rows at a time.
 // Epilogues are the ones of gemv_kernel (same reference citations): plain store, residual (+ the
 // next layer's per-layer embedding), SwiGLU of a gate/up slab pair, QKV with per-head norm / RoPE /
