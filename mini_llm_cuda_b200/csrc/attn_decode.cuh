@@ -367,45 +367,61 @@ __global__ void __launch_bounds__(attn_threads<G>(), attn_resident(G))
         __threadfence();
         if (tid == 0) p.ticket[tslot] = 0;
     }
-    // Combine: a warp takes 32 output elements of a head. Its lanes turn the splits' (max, sum) pairs into normalised weights, which it hands
-    // round; the first eight splits' values are asked for with the pairs. (One warp of the CTA doing the weights for all, alone
-    // between two barriers, took 2.1 us of the 4.8 behind the last split at one head per CTA.)
-    auto combine = [&](auto shared) {
-        auto get = [&](int g, int s, int e) {
-            if constexpr (decltype(shared)::value) return spart[(s * G + g) * W + e];
-            else return __ldcg(p.part + (((size_t)b * p.heads + h0 + g) * SG + s) * W + e);
-        };
-        constexpr int AHEAD = 8;
-        for (int i = tid; i < G * HD; i += 32 * NW * HG) {
-            const int g = i / HD, e = i % HD;      // g: the warp's
-            const size_t at = ((size_t)b * p.heads + h0 + g) * HD;
-            float m0 = kNegBig, l0 = 0.f, m1 = kNegBig, l1 = 0.f, v[AHEAD];
-            if (lane < S) { m0 = get(g, lane, HD); l0 = get(g, lane, HD + 1); }
-            if (lane + 32 < S) { m1 = get(g, lane + 32, HD); l1 = get(g, lane + 32, HD + 1); }
+    // Combine: a warp takes 32 or 64 output elements of a head. Its lanes turn the splits' (max, sum) pairs into normalised weights, which it
+    // hands round; the splits' values are asked for eight at a time, the first with the pairs. (One warp of the CTA doing the weights for
+    // all, alone between two barriers, took 2.1 us of the 4.8 behind the last split at one head per CTA.) One code for results in shared
+    // and in global memory: a copy for each cost launches with one split, which run neither, 0.2 us (step of 3 sequences 213.6 -> 214.8 us).
+    constexpr int AHEAD = 8;                       // (of 32: a group's weights are in one register)
+    constexpr int PER = G * HD > 32 * NW * HG ? G * HD / (32 * NW * HG) : 1;      // outputs per lane
+    static_assert(HD % (32 * PER) == 0, "a warp's outputs are of one head");
+    const int first = warp * PER * 32;
+    if (first >= G * HD) return;
+    auto ld = [](const float* a) {
+        float x;
+        asm volatile("ld.relaxed.gpu.f32 %0, [%1];" : "=f"(x) : "l"(a) : "memory");
+        return x;
+    };
+    const int g = first / HD, e = first % HD + lane, of_split = loop ? G * W : W;
+    const float* part = loop ? spart + g * W : p.part + ((size_t)b * p.heads + h0 + g) * SG * W;
+    float m0 = kNegBig, l0 = 0.f, m1 = kNegBig, l1 = 0.f, w0 = 0.f, w1 = 0.f, o[PER];
+    if (lane < S) { m0 = ld(part + lane * of_split + HD); l0 = ld(part + lane * of_split + HD + 1); }
+    if (lane + 32 < S) { m1 = ld(part + (lane + 32) * of_split + HD); l1 = ld(part + (lane + 32) * of_split + HD + 1); }
 #pragma unroll
-            for (int s = 0; s < AHEAD; ++s) v[s] = s < S ? get(g, s, e) : 0.f;
+    for (int j = 0; j < PER; ++j) o[j] = 0.f;
+#pragma unroll 1
+    for (int s0 = 0; s0 < S; s0 += AHEAD) {
+        float v[AHEAD][PER];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+            for (int j = 0; j < PER; ++j) v[u][j] = s0 + u < S ? ld(part + (s0 + u) * of_split + e + 32 * j) : 0.f;
+        if (s0 == 0) {
             float mx = fmaxf(m0, m1);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            float w0 = expf(m0 - mx), w1 = expf(m1 - mx);
+            for (int q = 16; q > 0; q >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, q));
+            w0 = expf(m0 - mx);
+            w1 = expf(m1 - mx);
             const float lt = warp_sum(l0 * w0 + l1 * w1);
             w0 /= lt;
             w1 /= lt;
-            float o = 0.f;
-#pragma unroll
-            for (int s = 0; s < AHEAD; ++s) {
-                const float y = __shfl_sync(0xffffffffu, w0, s);
-                if (s < S) o = fmaf(y, v[s], o);
-            }
-#pragma unroll 4
-            for (int s = AHEAD; s < S; ++s) o = fmaf(__shfl_sync(0xffffffffu, s < 32 ? w0 : w1, s & 31), get(g, s, e), o);
-            if (p.gbuf) o *= p.gbuf[at + e];
-            p.abuf[at + e] = o;
-            if (p.abuf16) p.abuf16[at + (p.perm ? perm16(e) : e)] = __float2bfloat16_rn(p.perm ? o * kOperandScale : o);
         }
-    };
-    if (loop) combine(std::true_type{});
-    else combine(std::false_type{});
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const float y = __shfl_sync(0xffffffffu, s0 < 32 ? w0 : w1, (s0 + u) & 31);
+            if (s0 + u < S) {
+#pragma unroll
+                for (int j = 0; j < PER; ++j) o[j] = fmaf(y, v[u][j], o[j]);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int ej = e + 32 * j;
+        const size_t at = ((size_t)b * p.heads + h0 + g) * HD;
+        if (p.gbuf) o[j] *= p.gbuf[at + ej];
+        p.abuf[at + ej] = o[j];
+        if (p.abuf16) p.abuf16[at + (p.perm ? perm16(ej) : ej)] = __float2bfloat16_rn(p.perm ? o[j] * kOperandScale : o[j]);
+    }
 }
 
 // The kernel for G query heads per CTA: launch(kernel, threads, shared memory), its shared-memory limit raised before.
